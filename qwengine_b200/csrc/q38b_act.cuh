@@ -418,23 +418,4 @@ __device__ __forceinline__ void dequant_sub(const uint8_t* b, int s, float (&y)[
     }
 }
 
-template <int FMT, int KIND>
-__global__ void __launch_bounds__(128) dequant_rows_kernel(const uint8_t* __restrict__ W, long long row_bytes, int K, int rows,
-                                                            void* __restrict__ out) {
-    const int nsub = K >> 5;
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= (long long)rows * nsub) return;
-    const int r = (int)(id / nsub), sub = (int)(id % nsub);
-    const uint8_t* blk = W + (size_t)r * row_bytes + (size_t)(sub >> 3) * Unit<FMT>::BLOCK_BYTES;
-    float y[32];
-    dequant_sub<FMT>(blk, sub & 7, y);
-    const size_t o = (size_t)r * K + (size_t)sub * 32;
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-        if (KIND == 0) ((float*)out)[o + j] = y[j];
-        else if (KIND == 1) ((__half*)out)[o + j] = __float2half_rn(y[j]);
-        else ((__nv_bfloat16*)out)[o + j] = __float2bfloat16_rn(y[j]);
-    }
-}
-
 }  // namespace q38b

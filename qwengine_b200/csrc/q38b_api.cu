@@ -16,6 +16,18 @@
 
 using namespace q38b;
 
+const uint32_t* q38b_grid_source(const q38b_ctx* ctx, uint32_t type) {
+    switch (type) {
+        case T_IQ3_XXS: return ctx->d_cb_iq3xxs;
+        case T_IQ3_S: return ctx->d_cb_iq3s;
+        case T_IQ2_XXS: return ctx->d_code16[0];
+        case T_IQ2_XS: return ctx->d_code16[1];
+        case T_IQ2_S: return ctx->d_code16[2];
+        case T_IQ1_S: case T_IQ1_M: return ctx->d_code16[3];
+        default: return nullptr;
+    }
+}
+
 namespace {
 
 constexpr int NGROUPS = 2;
@@ -330,19 +342,6 @@ int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     }
 }
 
-// device table a format's decoders stage into shared memory (32-bit codebook words or 16-bit grid codes), or nullptr
-const uint32_t* codebook_of(const q38b_ctx* ctx, uint32_t type) {
-    switch (type) {
-        case T_IQ3_XXS: return ctx->d_cb_iq3xxs;
-        case T_IQ3_S: return ctx->d_cb_iq3s;
-        case T_IQ2_XXS: return ctx->d_code16[0];
-        case T_IQ2_XS: return ctx->d_code16[1];
-        case T_IQ2_S: return ctx->d_code16[2];
-        case T_IQ1_S: case T_IQ1_M: return ctx->d_code16[3];
-        default: return nullptr;
-    }
-}
-
 int dispatch_gemv1(q38b_ctx* ctx, uint32_t type, const Plan1& p1, cudaStream_t st) {
     switch (type) {
         case T_Q8_0: return launch_gemv1<T_Q8_0>(ctx, p1, st);
@@ -360,30 +359,6 @@ int dispatch_gemv1(q38b_ctx* ctx, uint32_t type, const Plan1& p1, cudaStream_t s
         case T_IQ1_M: return launch_gemv1<T_IQ1_M>(ctx, p1, st);
         default: return Q38B_ERR_UNSUPPORTED;
     }
-}
-
-template <int KIND>
-int launch_dequant(q38b_ctx* ctx, uint32_t type, const uint8_t* W, long long rb, int K, int rows, void* out, cudaStream_t st) {
-    const long long n = (long long)rows * (K / 32);
-    const unsigned blocks = (unsigned)((n + 127) / 128);
-    switch (type) {
-        case T_Q8_0: dequant_rows_kernel<T_Q8_0, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_Q4_K: dequant_rows_kernel<T_Q4_K, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_Q5_K: dequant_rows_kernel<T_Q5_K, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_Q6_K: dequant_rows_kernel<T_Q6_K, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ3_XXS: dequant_rows_kernel<T_IQ3_XXS, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ3_S: dequant_rows_kernel<T_IQ3_S, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ4_XS: dequant_rows_kernel<T_IQ4_XS, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_Q2_K: dequant_rows_kernel<T_Q2_K, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ2_XXS: dequant_rows_kernel<T_IQ2_XXS, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ2_XS: dequant_rows_kernel<T_IQ2_XS, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ2_S: dequant_rows_kernel<T_IQ2_S, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ1_S: dequant_rows_kernel<T_IQ1_S, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        case T_IQ1_M: dequant_rows_kernel<T_IQ1_M, KIND><<<blocks, 128, 0, st>>>(W, rb, K, rows, out); break;
-        default: return Q38B_ERR_UNSUPPORTED;
-    }
-    Q38B_CUDA(ctx, cudaGetLastError());
-    return Q38B_OK;
 }
 
 }  // namespace
@@ -701,7 +676,7 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
             g.static_weights = ctx->static_weights;
             for (int i = 0; i < n_peers; i++) g.y_peer[i] = y_peers[i];
             g.status = ctx->d_status;
-            g.codebook = codebook_of(ctx, type);
+            g.codebook = q38b_grid_source(ctx, type);
             g.K = K;
             g.M = M;
             g.accumulate = accumulate ? 1 : 0;
@@ -739,7 +714,7 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
     a.static_weights = ctx->static_weights;
     for (int i = 0; i < n_peers; i++) a.y_peer[i] = y_peers[i];
     a.status = ctx->d_status;
-    a.codebook = codebook_of(ctx, type);
+    a.codebook = q38b_grid_source(ctx, type);
     a.K = K;
     a.M = M;
     a.nb = nb;
@@ -809,7 +784,7 @@ int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* con
         for (int i = 0; i < n_peers; i++) a.y_peer_more[m - 1][i] = y_peers[m * n_peers + i];
     a.static_weights = ctx->static_weights;
     a.status = ctx->d_status;
-    a.codebook = codebook_of(ctx, type);
+    a.codebook = q38b_grid_source(ctx, type);
     a.K = K;
     a.nb = nb;
     a.accumulate = 0;
@@ -885,7 +860,7 @@ int q38b_gemv_group_peers(q38b_ctx* ctx, uint32_t type, int n_mats, const void* 
         for (int pr = 0; pr < n_peers; pr++) (i == 0 ? g.y_peer[pr] : g.y_peer_more[i - 1][pr]) = y_peers[i * n_peers + pr];
     g.static_weights = ctx->static_weights;
     g.status = ctx->d_status;
-    g.codebook = codebook_of(ctx, type);
+    g.codebook = q38b_grid_source(ctx, type);
     g.K = K;
     g.accumulate = 0;
     cudaStream_t st = (cudaStream_t)stream;
@@ -929,7 +904,7 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
         g.n_peers = 0;
         g.static_weights = ctx->static_weights;
         g.status = ctx->d_status;
-        g.codebook = codebook_of(ctx, type);
+        g.codebook = q38b_grid_source(ctx, type);
         g.K = K;
         g.M = M;
         g.accumulate = accumulate ? 1 : 0;
@@ -948,21 +923,6 @@ int q38b_gemv_f32(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes,
     int rc = q38b_quantize_q8k(ctx, x, x_ld, K, nb, q8k_scratch, K / 256, stream);
     if (rc != Q38B_OK) return rc;
     return q38b_gemv_q8k(ctx, type, W, row_bytes, K, M, q8k_scratch, K / 256, nb, y, y_ld, accumulate, stream);
-}
-
-int q38b_dequant_rows(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int rows, void* out, int out_kind,
-                      void* stream) {
-    if (!ctx || !W || !out || K <= 0 || K % 256 || rows < 1) return Q38B_ERR_ARG;
-    if (!known_format(type)) return Q38B_ERR_UNSUPPORTED;
-    if (row_bytes < q38b_row_bytes(type, K)) return Q38B_ERR_ARG;
-    if (((uintptr_t)W & 1) || (row_bytes & 1) || ((uintptr_t)out & 3)) return Q38B_ERR_ALIGN;
-    cudaStream_t st = (cudaStream_t)stream;
-    switch (out_kind) {
-        case Q38B_OUT_F32: return launch_dequant<0>(ctx, type, (const uint8_t*)W, (long long)row_bytes, K, rows, out, st);
-        case Q38B_OUT_F16: return launch_dequant<1>(ctx, type, (const uint8_t*)W, (long long)row_bytes, K, rows, out, st);
-        case Q38B_OUT_BF16: return launch_dequant<2>(ctx, type, (const uint8_t*)W, (long long)row_bytes, K, rows, out, st);
-        default: return Q38B_ERR_ARG;
-    }
 }
 
 }  // extern "C"

@@ -38,6 +38,8 @@ struct q38b_ctx {
     int pending_sync_seq = -1;        // >= 0: the next merged matvec or SwiGLU launch starts with cross-GPU barrier number seq of the run
 };
 
+// device table a format's decoders stage into shared memory (32-bit codebook words or 16-bit grid codes), or nullptr
+const uint32_t* q38b_grid_source(const q38b_ctx* ctx, uint32_t type);
 // 1 when q38b_gemv_group would run these matrices (single column) on the one-column kernel
 extern "C" int q38b_gemv_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M);
 // q38b_gemv_group with peer stores: y_peers[i * n_peers + r] is where peer r keeps the output of matrix i
