@@ -262,160 +262,4 @@ static __global__ void __launch_bounds__(256) swiglu_rows_inplace_kernel(float* 
     for (int i = threadIdx.x; i < n / 8; i += 256) dst[i] = src[i];
 }
 
-// ---------------------------------------------------------------------------------------------
-// Exact dequantizer: one thread per 32-weight sub-block.  Float operations are the ones of
-// dequantize_row_ref (src/quant/quant_ref.cpp:57-103, 165-225, 284-308) in the same order, each
-// individually rounded (no fused multiply-add), so fp32 outputs are bit-identical to it.
-// ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t g_u16(const uint8_t* p) { return *(const uint16_t*)p; }
-__device__ __forceinline__ uint32_t g_u32a2(const uint8_t* p) { return g_u16(p) | (g_u16(p + 2) << 16); }
-__device__ __forceinline__ float g_f16(const uint8_t* p) { return __half2float(__ushort_as_half((unsigned short)g_u16(p))); }
-
-template <int FMT>
-__device__ __forceinline__ void dequant_sub(const uint8_t* b, int s, float (&y)[32]) {
-    if (FMT == T_Q8_0) {
-        const uint8_t* q = b + 34 * s;
-        const float d = g_f16(q);
-#pragma unroll
-        for (int j = 0; j < 32; j++) y[j] = __fmul_rn((float)(int8_t)q[2 + j], d);
-    } else if (FMT == T_Q4_K || FMT == T_Q5_K) {
-        const float d = g_f16(b), mn = g_f16(b + 2);
-        const uint8_t* sc = b + 4;
-        int scv, mv;
-        if (s < 4) { scv = sc[s] & 63; mv = sc[s + 4] & 63; }
-        else { scv = (sc[s + 4] & 0xF) | ((sc[s - 4] >> 6) << 4); mv = (sc[s + 4] >> 4) | ((sc[s] >> 6) << 4); }
-        const float d1 = __fmul_rn(d, (float)scv), m1 = __fmul_rn(mn, (float)mv);
-        const uint8_t* q = b + (FMT == T_Q5_K ? 48 : 16) + 32 * (s >> 1);
-#pragma unroll
-        for (int l = 0; l < 32; l++) {
-            int v = (s & 1) ? (q[l] >> 4) : (q[l] & 0xF);
-            if (FMT == T_Q5_K) v += ((b[16 + l] >> s) & 1) << 4;
-            y[l] = __fsub_rn(__fmul_rn(d1, (float)v), m1);
-        }
-    } else if (FMT == T_Q6_K) {
-        const float d = g_f16(b + 208);
-        const int h = s >> 2, j = s & 3;
-        const uint8_t* ql = b + 64 * h + 32 * (j & 1);
-        const uint8_t* qh = b + 128 + 32 * h;
-        const int8_t* sc = (const int8_t*)(b + 192 + 8 * h + 2 * j);
-#pragma unroll
-        for (int l = 0; l < 32; l++) {
-            const int q = (int)(((ql[l] >> (4 * (j >> 1))) & 0xF) | (((qh[l] >> (2 * j)) & 3) << 4)) - 32;
-            y[l] = __fmul_rn(__fmul_rn(d, (float)sc[l >> 4]), (float)q);
-        }
-    } else if (FMT == T_IQ3_XXS) {
-        const float d = g_f16(b);
-        const uint32_t aux = g_u32a2(b + 66 + 4 * s);
-        const float db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)(aux >> 28))), 0.5f);
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t s7 = (aux >> (7 * l)) & 127u;
-            const uint32_t sg = s7 | ((uint32_t)(__popc(s7) & 1) << 7);
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const uint32_t gw = q38b_iq3xxs_grid[b[2 + 8 * s + 2 * l + hh]];
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    y[8 * l + 4 * hh + j] = __fmul_rn(__fmul_rn(db, (float)((gw >> (8 * j)) & 0xFF)), ((sg >> (4 * hh + j)) & 1) ? -1.f : 1.f);
-            }
-        }
-    } else if (FMT == T_IQ3_S) {
-        const float d = g_f16(b);
-        const uint32_t ls = (b[106 + (s >> 1)] >> (4 * (s & 1))) & 0xF;
-        const float db = __fmul_rn(d, (float)(1 + 2 * (int)ls));
-        const uint32_t qh = b[66 + s];
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t sg = b[74 + 4 * s + l];
-#pragma unroll
-            for (int hh = 0; hh < 2; hh++) {
-                const uint32_t idx = b[2 + 8 * s + 2 * l + hh] | (((qh >> (2 * l + hh)) & 1u) << 8);
-                const uint32_t gw = q38b_iq3s_grid[idx];
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-                    y[8 * l + 4 * hh + j] = __fmul_rn(__fmul_rn(db, (float)((gw >> (8 * j)) & 0xFF)), ((sg >> (4 * hh + j)) & 1) ? -1.f : 1.f);
-            }
-        }
-    } else if (FMT == T_Q2_K) {            // src/quant/quant_ref.cpp:33-55
-        const float d = g_f16(b + 80), mn = g_f16(b + 82);
-        const int n = s >> 2, j = s & 3;
-#pragma unroll
-        for (int half = 0; half < 2; half++) {
-            const uint32_t sc = b[2 * s + half];
-            const float dl = __fmul_rn(d, (float)(sc & 0xF)), ml = __fmul_rn(mn, (float)(sc >> 4));
-#pragma unroll
-            for (int l = 0; l < 16; l++)
-                y[16 * half + l] = __fsub_rn(__fmul_rn(dl, (float)((b[16 + 32 * n + 16 * half + l] >> (2 * j)) & 3)), ml);
-        }
-    } else if (FMT == T_IQ2_XXS || FMT == T_IQ2_XS || FMT == T_IQ2_S) {   // src/quant/quant_ref.cpp:105-168
-        const float d = g_f16(b);
-        const uint32_t a1 = FMT == T_IQ2_XXS ? g_u32a2(b + 6 + 8 * s) : 0u;
-        const uint32_t scb = FMT == T_IQ2_XXS ? 0u : b[(FMT == T_IQ2_XS ? 66 : 74) + s];
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            uint32_t code, sg;
-            float db;
-            if (FMT == T_IQ2_XXS) {
-                code = q38b_iq2xxs_codes[b[2 + 8 * s + l]];
-                const uint32_t s7 = (a1 >> (7 * l)) & 127u;
-                sg = s7 | ((uint32_t)(__popc(s7) & 1) << 7);
-                db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)(a1 >> 28))), 0.25f);
-            } else if (FMT == T_IQ2_XS) {
-                const uint32_t qv = g_u16(b + 2 + 2 * (4 * s + l));
-                code = q38b_iq2xs_codes[qv & 511u];
-                const uint32_t s7 = qv >> 9;
-                sg = s7 | ((uint32_t)(__popc(s7) & 1) << 7);
-                db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)((l < 2 ? scb : scb >> 4) & 0xF))), 0.25f);
-            } else {
-                code = q38b_iq2s_codes[b[2 + 4 * s + l] | (((uint32_t)b[66 + s] << (8 - 2 * l)) & 0x300u)];
-                sg = b[34 + 4 * s + l];
-                db = __fmul_rn(__fmul_rn(d, __fadd_rn(0.5f, (float)((l < 2 ? scb : scb >> 4) & 0xF))), 0.25f);
-            }
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                const uint32_t lv = (code >> (2 * j)) & 3u;
-                const float g = lv == 0 ? 8.f : lv == 1 ? 25.f : 43.f;
-                y[8 * l + j] = __fmul_rn(__fmul_rn(db, g), ((sg >> j) & 1) ? -1.f : 1.f);
-            }
-        }
-    } else if (FMT == T_IQ1_S) {           // src/quant/quant_ref.cpp:227-245
-        const float d = g_f16(b);
-        const uint32_t qh = g_u16(b + 34 + 2 * s);
-        const float dl = __fmul_rn(d, (float)(2 * (int)((qh >> 12) & 7) + 1));
-        const float delta = (qh & 0x8000u) ? -0.125f : 0.125f;
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t code = q38b_iq1s_codes[b[2 + 4 * s + l] | (((qh >> (3 * l)) & 7u) << 8)];
-#pragma unroll
-            for (int j = 0; j < 8; j++) y[8 * l + j] = __fmul_rn(dl, __fadd_rn((float)((int)((code >> (2 * j)) & 3u) - 1), delta));
-        }
-    } else if (FMT == T_IQ1_M) {           // src/quant/quant_ref.cpp:247-283
-        const uint32_t s0 = g_u16(b + 48), s1 = g_u16(b + 50), s2 = g_u16(b + 52), s3 = g_u16(b + 54);
-        const uint32_t su = (s0 >> 12) | ((s1 >> 8) & 0x00F0u) | ((s2 >> 4) & 0x0F00u) | (s3 & 0xF000u);
-        const float d = __half2float(__ushort_as_half((unsigned short)su));
-        const uint32_t scw = (s >> 1) == 0 ? s0 : (s >> 1) == 1 ? s1 : (s >> 1) == 2 ? s2 : s3;
-        const uint32_t t = scw >> (6 * (s & 1));
-        const float dl[2] = {__fmul_rn(d, (float)(2 * (int)(t & 7) + 1)), __fmul_rn(d, (float)(2 * (int)((t >> 3) & 7) + 1))};
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t hn = (b[32 + 2 * s + (l >> 1)] >> (4 * (l & 1))) & 0xFu;
-            const uint32_t code = q38b_iq1s_codes[b[4 * s + l] | ((hn & 7u) << 8)];
-            const float delta = (hn & 8u) ? -0.125f : 0.125f;
-#pragma unroll
-            for (int j = 0; j < 8; j++) y[8 * l + j] = __fmul_rn(dl[l >> 1], __fadd_rn((float)((int)((code >> (2 * j)) & 3u) - 1), delta));
-        }
-    } else if (FMT == T_IQ4_XS) {
-        const float d = g_f16(b);
-        const uint32_t sh = g_u16(b + 2);
-        const int ls = (int)(((b[4 + (s >> 1)] >> (4 * (s & 1))) & 0xF) | (((sh >> (2 * s)) & 3) << 4));
-        const float dl = __fmul_rn(d, (float)(ls - 32));
-        const uint8_t* q = b + 8 + 16 * s;
-#pragma unroll
-        for (int j = 0; j < 16; j++) {
-            y[j] = __fmul_rn(dl, (float)q38b_iq4nl_levels[q[j] & 0xF]);
-            y[j + 16] = __fmul_rn(dl, (float)q38b_iq4nl_levels[q[j] >> 4]);
-        }
-    }
-}
-
 }  // namespace q38b

@@ -502,7 +502,7 @@ Q38B_HD constexpr bool one_column_only(int fmt) {
 }
 
 // bytes of one 256-weight super-block
-Q38B_HD int block_bytes(int fmt) {
+Q38B_HD constexpr int block_bytes(int fmt) {
     switch (fmt) {
         case T_Q8_0: return 272; case T_Q4_K: return 144; case T_Q5_K: return 176; case T_Q6_K: return 210;
         case T_IQ3_XXS: return 98; case T_IQ3_S: return 110; case T_IQ4_XS: return 136;

@@ -64,16 +64,17 @@ __device__ __forceinline__ void words_a2(const uint8_t* p, uint32_t (&w)[N]) {
         prev = next;
     }
 }
-// N words from an address that is a multiple of 16 (ALIGNED: the K-quants' blocks when the rows are) or of 2
-template <int N, bool ALIGNED>
+// N words from an address that is a multiple of ALIGN = 16, 4 or 2
+template <int N, int ALIGN>
 __device__ __forceinline__ void words_of(const uint8_t* p, uint32_t (&w)[N]) {
-    if constexpr (ALIGNED && N % 4 == 0) {
+    if constexpr (ALIGN == 16) {
+        static_assert(N % 4 == 0, "whole 16-byte loads");
 #pragma unroll
         for (int i = 0; i < N / 4; i++) {
             const uint4 v = *(const uint4*)(p + 16 * i);
             w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
         }
-    } else if constexpr (ALIGNED) {
+    } else if constexpr (ALIGN == 4) {
 #pragma unroll
         for (int i = 0; i < N; i++) w[i] = *(const uint32_t*)(p + 4 * i);
     } else {
@@ -104,6 +105,7 @@ __device__ __forceinline__ uint32_t sign8(uint32_t s7) { return s7 | ((uint32_t)
 template <int FMT, bool ALIGNED>
 __device__ __forceinline__ void load_sub32(const uint8_t* b, int s, const uint32_t* tab, Sub32& o) {
     constexpr GridTable G = grid_table(FMT);
+    constexpr int AL = ALIGNED ? expand_alignment(FMT) : 2;   // what `b` is a multiple of
     o.sign = 0u;
     if constexpr (FMT == T_Q8_0) {
         const uint8_t* p = b + 34 * s;
@@ -115,19 +117,19 @@ __device__ __forceinline__ void load_sub32(const uint8_t* b, int s, const uint32
         for (int i = 0; i < 4; i++) o.off[i] = -128.0f;
     } else if constexpr (FMT == T_Q4_K || FMT == T_Q5_K) {
         uint32_t h[4];
-        words_of<4, ALIGNED>(b, h);
+        words_of<4, AL>(b, h);
         const float d = __half2float(__ushort_as_half((unsigned short)h[0])), mn = __half2float(__ushort_as_half((unsigned short)(h[0] >> 16)));
         // 6-bit scales and minima (get_scale_min_k4, src/quant/quant_ref.cpp:24-32): four bytes of the half of the block
         const uint32_t sc4 = s >= 4 ? ((h[3] & 0x0F0F0F0Fu) | ((h[1] >> 2) & 0x30303030u)) : (h[1] & 0x3F3F3F3Fu);
         const uint32_t mn4 = s >= 4 ? (((h[3] >> 4) & 0x0F0F0F0Fu) | ((h[2] >> 2) & 0x30303030u)) : (h[2] & 0x3F3F3F3Fu);
         o.a[0] = o.a[1] = __fmul_rn(d, (float)((sc4 >> (8 * (s & 3))) & 0xFFu));
         o.c[0] = o.c[1] = __fmul_rn(mn, (float)((mn4 >> (8 * (s & 3))) & 0xFFu));
-        words_of<8, ALIGNED>(b + (FMT == T_Q5_K ? 48 : 16) + 32 * (s >> 1), o.u);
+        words_of<8, AL>(b + (FMT == T_Q5_K ? 48 : 16) + 32 * (s >> 1), o.u);
 #pragma unroll
         for (int i = 0; i < 8; i++) o.u[i] = (o.u[i] >> (4 * (s & 1))) & 0x0F0F0F0Fu;
         if constexpr (FMT == T_Q5_K) {
             uint32_t qh[8];
-            words_of<8, ALIGNED>(b + 16, qh);
+            words_of<8, AL>(b + 16, qh);
 #pragma unroll
             for (int i = 0; i < 8; i++) o.u[i] |= ((qh[i] >> s) << 4) & 0x10101010u;
         }
@@ -146,7 +148,7 @@ __device__ __forceinline__ void load_sub32(const uint8_t* b, int s, const uint32
         for (int i = 0; i < 4; i++) o.off[i] = -32.0f;
     } else if constexpr (FMT == T_Q2_K) {            // src/quant/quant_ref.cpp:33-55
         const int n = s >> 2, j = s & 3;
-        words_of<8, ALIGNED>(b + 16 + 32 * n, o.u);
+        words_of<8, AL>(b + 16 + 32 * n, o.u);
 #pragma unroll
         for (int i = 0; i < 8; i++) o.u[i] = (o.u[i] >> (2 * j)) & 0x03030303u;
         const float d = s_f16(b + 80), mn = s_f16(b + 82);

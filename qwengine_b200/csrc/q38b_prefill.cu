@@ -4,23 +4,30 @@
 //
 // Replaces dequant_rows_f16 + gemm_f16 (cuBLAS) of the reference (src/cuda/prefill.cu:30-85, 802-851) by one kernel:
 // the weights never exist dequantized in global memory.  One CTA owns a 128-row weight tile and up to 512 tokens:
-//   * warps 0-7 (256 threads) decode one 32-weight sub-block each per K-slab of 64 (the exact dequantize_row_ref value,
-//     rounded once to bf16) and store it K-major with the 128-byte swizzle the tensor core expects (operand A);
-//   * one thread streams the matching activation tiles (operand B, 2 x [256 tokens x 64]) with tiled TMA loads
+//   * warps 0-15 own eight rows each.  They fetch the rows' raw blocks one super-block ahead (whole 16-byte units into
+//     registers, then their own piece of shared memory), a lane expands one 32-weight sub-block with word operations
+//     (q38b_expand.cuh) and stores it K-major with the 128-byte swizzle the tensor core expects (operand A);
+//   * one thread streams the matching activation tiles (operand B, [tokens x 64] per K-slab) with tiled TMA loads
 //     (hardware swizzle, zero fill past the last token; no multicast);
-//   * one thread issues tcgen05.mma (cta_group::1, kind::f16, M = 128, N = 256, K = 16) into two fp32 accumulators
-//     in tensor memory (2 x 256 columns) and commits each slab to the stage's "empty" mbarrier;
-//   * warps 0-3 read the accumulators back (tcgen05.ld 32x32b) and store Y, 32 consecutive rows per warp and token.
+//   * one thread issues tcgen05.mma (cta_group::1, kind::f16, M = 128, N = 16..256, K = 16) into one or two fp32
+//     accumulators in tensor memory and commits each stage to its "empty" mbarrier;
+//   * all 16 decode warps read the accumulators back (tcgen05.ld 32x32b) and store Y, 32 consecutive rows per warp and token.
+// Where row tiles and token tiles alone leave SMs idle, the CTAs of a cluster share a tile's K: each multiplies a range
+// of super-blocks and the partial sums meet through distributed shared memory, added in rank order.
+// Measured on B200, 17408 x 5120 IQ3_XXS / 5120 x 17408 IQ4_XS with 1024 tokens: 211 / 286 us -> 161 / 194 us; 77 tokens of a
+// whole Q4_K / Q6_K layer 698 -> 190 us.  Up to about 250 tokens the expanders set the pace (issue slots 66 % busy, the
+// shared-memory pipe 63-70 %), from 500 the tensor core and its shared-memory traffic do (tensor pipe 69 % busy).
 // All mbarrier waits are bounded; tensor memory is released before the kernel returns, also after a timeout.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
 #include <type_traits>
 
 #include "../../include/q38b200.h"
-#include "q38b_act.cuh"
+#include "q38b_expand.cuh"
 #include "q38b_internal.h"
 #include "q38b_pipe.cuh"
 
@@ -29,19 +36,25 @@ using namespace q38b;
 namespace {
 
 constexpr int PF_ROWS = 128;       // weight rows per CTA (MMA M)
-constexpr int PF_NTILE = 256;      // tokens per accumulator (MMA N)
-constexpr int PF_KSLAB = 64;       // K elements per stage: one 128-byte swizzle row of bf16
-// The two operands have rings of their own: the dequantized weights (16 KB per slab) four deep, so that the decoders,
-// whose loads come straight from L2 / HBM, run well ahead of the tensor core; the activation tiles (64 KB per slab) two.
-constexpr int PF_A_STAGES = 4, PF_B_STAGES = 2;
-constexpr int PF_A_BYTES = PF_ROWS * PF_KSLAB * 2;        // 16 KB
-constexpr int PF_B_BYTES = PF_NTILE * PF_KSLAB * 2;       // 32 KB per accumulator
-constexpr int PF_B_STAGE_BYTES = 2 * PF_B_BYTES;
-// two groups of 8 decode warps (group g takes the slabs with slab % 2 == g: each thread has two slab times for the load
-// and the decode of its 32 weights) + TMA warp + MMA warp
-constexpr int PF_DECODE_GROUPS = 2, PF_DECODE_WARPS = 8 * PF_DECODE_GROUPS;
-constexpr int PF_THREADS = 32 * (PF_DECODE_WARPS + 2);
-constexpr int PF_SMEM = 1024 + PF_A_STAGES * PF_A_BYTES + PF_B_STAGES * PF_B_STAGE_BYTES + 256;
+constexpr int PF_MAX_N = 256;      // tokens per accumulator (MMA N), at most
+constexpr int PF_KSLAB = 64;       // K elements per activation stage: one 128-byte swizzle row of bf16
+// The two operands have rings of their own: dequantized weights two deep in stages of half a super-block (two K-slabs,
+// 32 KB), activation tiles of one slab and one accumulator as deep as fits (four of 256 tokens, up to eight of fewer).
+constexpr int PF_A_STAGES = 2, PF_B_MAX_STAGES = 8;
+constexpr int PF_A_SLAB_BYTES = PF_ROWS * PF_KSLAB * 2;   // 16 KB
+constexpr int PF_A_BYTES = 2 * PF_A_SLAB_BYTES;
+constexpr int PF_DECODE_WARPS = 16, PF_WARP_ROWS = PF_ROWS / PF_DECODE_WARPS;
+constexpr int PF_THREADS = 32 * (PF_DECODE_WARPS + 2);    // + TMA warp + MMA warp
+constexpr int PF_MAX_SPLITS = 8;   // CTAs that share a tile's K (portable cluster size)
+
+// Raw bytes a warp keeps of each of its rows: a super-block (Q8_0, whose halves are self-contained, half of one), at the
+// low four bits of its global address, read in whole 16-byte pieces.  The distance between rows is an odd number of
+// pieces, so that the eight rows a load instruction touches start on different banks.
+__host__ __device__ constexpr int pf_raw_bytes(int fmt) { return fmt == T_Q8_0 ? 136 : block_bytes(fmt); }
+__host__ __device__ constexpr int pf_pieces(int fmt) { return (pf_raw_bytes(fmt) + 14 + 15) / 16; }
+__host__ __device__ constexpr int pf_pitch(int fmt) { return 16 * (pf_pieces(fmt) | 1); }
+__host__ __device__ constexpr int pf_raw_smem(int fmt) { return PF_ROWS * pf_pitch(fmt) + 16; }   // + what the last row's word loads read past its end
+__host__ __device__ constexpr int pf_fixed_smem(int fmt) { return 1024 + PF_A_STAGES * PF_A_BYTES + pf_raw_smem(fmt) + grid_table_bytes(fmt) + 16; }
 
 struct PrefillArgs {
     const uint8_t* W;
@@ -50,7 +63,11 @@ struct PrefillArgs {
     long long ldy;
     int* status;
     int K, M, B, accumulate;
-    int n_acc;             // accumulators in use per CTA: 1 (<= 256 tokens in this CTA) or 2
+    int n_acc;             // accumulators in use per CTA: 1 or 2
+    int n_tile;            // tokens per accumulator: a multiple of 16, at most 256
+    int b_stages;
+    int splits;            // CTAs of a cluster that share a tile's K
+    const uint32_t* grid_src;
 };
 
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
@@ -59,9 +76,9 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
            ((uint64_t)2 << 61);
 }
 
-// D format f32, A and B both bf16 (format code 1) or both fp16 (code 0), K-major, N = 256, M = 128
-__host__ __device__ constexpr uint32_t pf_idesc(bool f16) {
-    return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((uint32_t)(PF_NTILE >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
+// D format f32, A and B both bf16 (format code 1) or both fp16 (code 0), K-major, N = n_tile, M = 128
+__device__ __forceinline__ uint32_t pf_idesc(bool f16, int n_tile) {
+    return (1u << 4) | ((f16 ? 0u : 1u) << 7) | ((f16 ? 0u : 1u) << 10) | ((uint32_t)(n_tile >> 3) << 17) | ((uint32_t)(PF_ROWS >> 4) << 24);
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -71,12 +88,11 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Fast dequantization to bf16 pairs for the A operand (K-quants).  An integer n < 128 becomes the bf16 number 128 + n by
+// Packed dequantization of the K-quants Q4_K, Q5_K, Q6_K to operand pairs.  An integer n < 128 becomes the bf16 number 128 + n by
 // OR-ing it under the bit pattern 0x4300, the bias is subtracted exactly (bf16 holds every integer below 256), and one
 // packed bf16 fused multiply-add applies scale and minimum to two weights.  Against the exact dequantizer the scale and
 // the minimum are rounded to bf16 before instead of after the multiplication: a relative error of 2^-9 per weight, the
 // same size as the rounding of the product to bf16 that the tensor core's operand format imposes anyway.
-// p[j] = weights 2j, 2j + 1 of the 32-weight sub-block.
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t bf2_u32(__nv_bfloat162 v) { return *(const uint32_t*)&v; }
 __device__ __forceinline__ __nv_bfloat162 u32_bf2(uint32_t v) { return *(const __nv_bfloat162*)&v; }
@@ -107,96 +123,102 @@ struct OpF16 {
     static __device__ __forceinline__ uint32_t pack(float a, float b) { const V2 v = __floats2half2_rn(a, b); return *(const uint32_t*)&v; }
 };
 
-template <int FMT, typename OP>
-__device__ __forceinline__ bool fast_sub(const uint8_t* b, int s, uint32_t (&p)[16]) {
+// p[j] = weights 2j, 2j + 1 of the sub-block
+template <int FMT, bool F16>
+__device__ __forceinline__ void operand_pairs(const Sub32& o, uint32_t (&p)[16]) {
+    using OP = typename std::conditional<F16, OpF16, OpBf16>::type;
     using V2 = typename OP::V2;
-    if (FMT == T_Q4_K || FMT == T_Q5_K) {
-        if (((uintptr_t)b & 3) != 0) return false;   // the 32-bit loads below need it (blocks are multiples of 16 bytes; GGUF tensors are 32-byte aligned)
-        const uint32_t dd = *(const uint32_t*)b;
-        const float d = __half2float(__ushort_as_half((unsigned short)(dd & 0xFFFFu))), mn = __half2float(__ushort_as_half((unsigned short)(dd >> 16)));
-        const uint8_t* sc = b + 4;
-        int scv, mv;
-        if (s < 4) { scv = sc[s] & 63; mv = sc[s + 4] & 63; }
-        else { scv = (sc[s + 4] & 0xF) | ((sc[s - 4] >> 6) << 4); mv = (sc[s + 4] >> 4) | ((sc[s] >> 6) << 4); }
-        const V2 a2 = OP::splat(d * (float)scv), c2 = OP::splat(-(mn * (float)mv));
-        const V2 bias = OP::bias(0);
-        const uint32_t* q = (const uint32_t*)(b + (FMT == T_Q5_K ? 48 : 16) + 32 * (s >> 1));
-        const uint32_t* qh = (const uint32_t*)(b + 16);
-        const int sh = (s & 1) ? 4 : 0;
+    if constexpr (FMT == T_Q4_K || FMT == T_Q5_K || FMT == T_Q6_K) {
+        const V2 bias = OP::bias(FMT == T_Q6_K ? 32 : 0);
+        const V2 a0 = OP::splat(o.a[0]), a1 = FMT == T_Q6_K ? OP::splat(o.a[1]) : a0;
+        const V2 c = OP::splat(FMT == T_Q6_K ? 0.0f : -o.c[0]);
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            uint32_t t = (q[i] >> sh) & 0x0F0F0F0Fu;
-            if (FMT == T_Q5_K) t |= ((qh[i] >> s) & 0x01010101u) << 4;
             V2 lo, hi;
-            OP::bytes(t, bias, lo, hi);
-            p[2 * i] = OP::bits(__hfma2(lo, a2, c2));
-            p[2 * i + 1] = OP::bits(__hfma2(hi, a2, c2));
+            OP::bytes(o.u[i], bias, lo, hi);
+            const V2 a = i < 4 ? a0 : a1;
+            p[2 * i] = FMT == T_Q6_K ? OP::bits(__hmul2(lo, a)) : OP::bits(__hfma2(lo, a, c));
+            p[2 * i + 1] = FMT == T_Q6_K ? OP::bits(__hmul2(hi, a)) : OP::bits(__hfma2(hi, a, c));
         }
-        return true;
-    }
-    if (FMT == T_Q6_K) {
-        // sub-block s = 4h + j of the super-block: weights 128h + 32j .. + 31; ql nibble (low for j < 2) and two bits of qh
-        const float d = __half2float(__ushort_as_half(*(const unsigned short*)(b + 208)));
-        const int h = s >> 2, j = s & 3;
-        const uint16_t* ql = (const uint16_t*)(b + 64 * h + 32 * (j & 1));   // Q6_K blocks are 210 bytes: 2-byte aligned only
-        const uint16_t* qh = (const uint16_t*)(b + 128 + 32 * h);
-        const int8_t* sc = (const int8_t*)(b + 192 + 8 * h + 2 * j);
-        const V2 bias = OP::bias(32);                                        // the base + 32
-        const V2 a0 = OP::splat(d * (float)sc[0]), a1 = OP::splat(d * (float)sc[1]);
+    } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t lw = (uint32_t)ql[2 * i] | ((uint32_t)ql[2 * i + 1] << 16);
-            const uint32_t hw = (uint32_t)qh[2 * i] | ((uint32_t)qh[2 * i + 1] << 16);
-            const uint32_t t = ((lw >> (4 * (j >> 1))) & 0x0F0F0F0Fu) | (((hw >> (2 * j)) & 0x03030303u) << 4);
-            V2 lo, hi;
-            OP::bytes(t, bias, lo, hi);
-            const V2 a2 = i < 4 ? a0 : a1;
-            p[2 * i] = OP::bits(__hmul2(lo, a2));
-            p[2 * i + 1] = OP::bits(__hmul2(hi, a2));
-        }
-        return true;
+        for (int j = 0; j < 16; j++) p[j] = sub32_pair<FMT, F16>(o, j);
     }
-    return false;
 }
 
-constexpr int PF_PREFETCH_BLOCKS = 3;   // super-blocks (256 weights) of look-ahead of the L2 prefetch
+// true in one lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_peer_f32(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+
+// 16 accumulator columns of this warp's 32 rows
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
 
 // F16: operands are fp16 (weights dequantized to fp16, activations fp16) instead of bf16.
-template <int FMT, bool F16>
+// ALIGNED: every row starts at a multiple of expand_alignment(FMT).
+template <int FMT, bool F16, bool ALIGNED>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArgs a, const __grid_constant__ CUtensorMap xmap) {
-    using OP = typename std::conditional<F16, OpF16, OpBf16>::type;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint64_t* full_a = (uint64_t*)smem;              // [A stages] the 8 decode warps of the slab's group arrive
+    uint64_t* full_a = (uint64_t*)smem;              // [A stages] the 16 decode warps arrive
     uint64_t* empty_a = full_a + PF_A_STAGES;        // [A stages] tcgen05.commit
     uint64_t* full_b = empty_a + PF_A_STAGES;        // [B stages] TMA bytes
-    uint64_t* empty_b = full_b + PF_B_STAGES;        // [B stages] tcgen05.commit
-    uint64_t* acc_done = empty_b + PF_B_STAGES;      // [1]
+    uint64_t* empty_b = full_b + PF_B_MAX_STAGES;    // [B stages] tcgen05.commit
+    uint64_t* acc_done = empty_b + PF_B_MAX_STAGES;  // [1]
     uint32_t* tmem_slot = (uint32_t*)(acc_done + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    const int b_stage_bytes = a.n_tile * (PF_KSLAB * 2);
     uint8_t* stages = smem + 1024;                                   // ring of weight tiles
     uint8_t* stages_b = stages + PF_A_STAGES * PF_A_BYTES;            // ring of activation tiles
+    uint8_t* raw_all = stages_b + a.b_stages * b_stage_bytes;         // the decode warps' raw blocks
+    uint32_t* tab_smem = (uint32_t*)(raw_all + pf_raw_smem(FMT));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row0 = blockIdx.x * PF_ROWS;
-    const int tok0 = blockIdx.y * a.n_acc * PF_NTILE;
-    const int n_slabs = a.K / PF_KSLAB;
+    const int rank = a.splits > 1 ? (int)cluster_rank() : 0;
+    const int row0 = (int)(blockIdx.x / (unsigned)a.splits) * PF_ROWS;
+    const int tile_tok = a.n_acc * a.n_tile;
+    const int tok0 = blockIdx.y * tile_tok;
+    const int nsb = a.K >> 8;
+    const int sb_begin = nsb * rank / a.splits, sb_end = nsb * (rank + 1) / a.splits;   // this CTA's super-blocks (splits <= nsb: never none)
+    const uint32_t tmem_cols = a.n_acc == 2 ? 512u : a.n_tile > 128 ? 256u : a.n_tile > 64 ? 128u : a.n_tile > 32 ? 64u : 32u;
 
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < PF_A_STAGES; s++) {
-            mbar_init(smem_u32(&full_a[s]), 8);             // one arrival per decode warp of the slab's group
+            mbar_init(smem_u32(&full_a[s]), PF_DECODE_WARPS);   // one arrival per warp
             mbar_init(smem_u32(&empty_a[s]), 1);
         }
-        for (int s = 0; s < PF_B_STAGES; s++) {
+        for (int s = 0; s < a.b_stages; s++) {
             mbar_init(smem_u32(&full_b[s]), 1);
             mbar_init(smem_u32(&empty_b[s]), 1);
         }
         mbar_init(smem_u32(acc_done), 1);
         mbar_fence_init();
     }
-    if (warp == PF_DECODE_WARPS + 1) {   // this warp owns the tensor memory allocation (512 columns = two 128 x 256 fp32 accumulators)
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+    if (warp == PF_DECODE_WARPS + 1) {   // this warp owns the tensor memory allocation
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    fill_grid_table<FMT>(tab_smem, a.grid_src, tid, PF_THREADS);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -204,126 +226,208 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
     if (tid == 0 && (smem_u32(stages) & 1023u)) atomicOr(a.status, ST_TMEM_TIMEOUT);   // swizzled tiles need 1024-byte alignment
 
     if (warp < PF_DECODE_WARPS) {
-        // ---------------- operand A: decode 128 rows x 64 weights per slab ----------------
-        const int grp = warp >> 3, t = tid & 255;
-        const int r = t >> 1, half = t & 1;                      // row of the tile, which 32-weight half of the slab
-        const int grow = min(row0 + r, a.M - 1);                 // rows past the end repeat the last row (never stored)
-        const uint8_t* wrow = a.W + (size_t)grow * a.row_bytes;
-        for (int slab = grp; slab < n_slabs; slab += PF_DECODE_GROUPS) {
-            const int st = slab % PF_A_STAGES;
-            const uint32_t use = (uint32_t)(slab / PF_A_STAGES);
-            mbar_wait_bounded(smem_u32(&empty_a[st]), (use & 1u) ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
-            const int sub = slab * 2 + half;                     // 32-weight sub-block index within the row
-            // the weights come straight from HBM: ask L2 for this row's super-blocks a few slabs ahead (one line each)
-            if ((slab & 3) == 0 && half == 0) {
-                const size_t ahead = (size_t)((slab >> 2) + PF_PREFETCH_BLOCKS) * Unit<FMT>::BLOCK_BYTES;   // BLOCK_BYTES: bytes per 256 weights for every format
-                if (ahead < (size_t)a.row_bytes) {
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(wrow + ahead));
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(wrow + min(ahead + 128, (size_t)a.row_bytes - 2)));
+        // ---------------- operand A: decode 128 rows x 128 weights per stage ----------------
+        constexpr int RAW = pf_raw_bytes(FMT), PITCH = pf_pitch(FMT), ROUNDS = (pf_pieces(FMT) + 3) / 4;
+        constexpr int UNIT_HALVES = FMT == T_Q8_0 ? 1 : 2;
+        const uintptr_t w_begin = (uintptr_t)a.W, w_end = w_begin + (uintptr_t)(a.M - 1) * a.row_bytes + (uintptr_t)nsb * (RAW * 2 / UNIT_HALVES);
+        // fetching: lane / 4 is the row, lane % 4 the first of its pieces; rows past the end repeat the last row (never stored)
+        const uintptr_t fetch_row = w_begin + (uintptr_t)min(row0 + PF_WARP_ROWS * warp + (lane >> 2), a.M - 1) * a.row_bytes;
+        uint8_t* raw = raw_all + warp * (PF_WARP_ROWS * PITCH);
+        uint8_t* raw_put = raw + (lane >> 2) * PITCH + 16 * (lane & 3);
+        // A piece that reaches past the matrix's first or last byte is not loaded ahead but copied by halfwords when it is due:
+        // without that branch the loads stay in flight behind the work on the unit before (with it the compiler waited for
+        // them on the spot).
+        uint4 ahead[ROUNDS];
+        auto piece_at = [&](int unit, int r) { return ((fetch_row + (uintptr_t)unit * RAW) & ~(uintptr_t)15) + 16 * (uintptr_t)((lane & 3) + 4 * r); };
+        auto inside = [&](uintptr_t at, int unit) { return at >= w_begin && at + 16 <= w_end && at < fetch_row + (uintptr_t)(unit + 1) * RAW; };
+        auto fetch = [&](int unit) {
+#pragma unroll
+            for (int r = 0; r < ROUNDS; r++) {
+                const uintptr_t at = piece_at(unit, r);
+                if (inside(at, unit)) ahead[r] = __ldg((const uint4*)at);
+            }
+        };
+        auto put_raw = [&](int unit) {
+#pragma unroll
+            for (int r = 0; r < ROUNDS; r++) {
+                const uintptr_t at = piece_at(unit, r);
+                if (inside(at, unit)) {
+                    *(uint4*)(raw_put + 64 * r) = ahead[r];
+                } else if (at < fetch_row + (uintptr_t)(unit + 1) * RAW) {
+                    for (int h = 0; h < 16; h += 2)
+                        if (at + h >= w_begin && at + h < w_end) *(uint16_t*)(raw_put + 64 * r + h) = *(const uint16_t*)(at + h);
                 }
             }
-            uint32_t p[16];
-            const uint8_t* blk = wrow + (size_t)(sub >> 3) * Unit<FMT>::BLOCK_BYTES;
-            if (!fast_sub<FMT, OP>(blk, sub & 7, p)) {
-                float y[32];
-                dequant_sub<FMT>(blk, sub & 7, y);
+        };
+        // expanding: lane % 8 is the row, lane / 8 the sub-block of the half super-block.  The eight rows of a quarter warp
+        // store the same piece of their swizzled rows, which is eight different bank groups.
+        const int r7 = lane & 7, q = lane >> 3;
+        const uint32_t dec_lo = (uint32_t)w_begin + (uint32_t)min(row0 + PF_WARP_ROWS * warp + r7, a.M - 1) * (uint32_t)a.row_bytes;
+        const uint8_t* raw_get = raw + r7 * PITCH;
+        const uint32_t* tab = grid_copy<FMT>(tab_smem, lane);
+        uint8_t* put = stages + (q >> 1) * PF_A_SLAB_BYTES + (PF_WARP_ROWS * warp + r7) * 128;
+        const int unit_end = sb_end * 2 / UNIT_HALVES;
+        int st = 0;
+        uint32_t use = 0;
+        fetch(sb_begin * 2 / UNIT_HALVES);
+        for (int unit = sb_begin * 2 / UNIT_HALVES; unit < unit_end; unit++) {
+            put_raw(unit);
+            __syncwarp();
+            if (unit + 1 < unit_end) fetch(unit + 1);
+            const uint8_t* blk = raw_get + ((dec_lo + (uint32_t)unit * RAW) & 15u);
 #pragma unroll
-                for (int j = 0; j < 16; j++) p[j] = OP::pack(y[2 * j], y[2 * j + 1]);
-            }
-            // row r of the tile: 128 bytes; 16-byte chunk c goes to chunk c ^ (r & 7) (128-byte swizzle)
-            uint8_t* arow = stages + (size_t)st * PF_A_BYTES + (size_t)r * 128;
+            for (int half = 0; half < UNIT_HALVES; half++) {
+                Sub32 o;
+                load_sub32<FMT, ALIGNED>(blk, 4 * half + q, tab, o);
+                uint32_t p[16];
+                operand_pairs<FMT, F16>(o, p);
+                mbar_wait_bounded(smem_u32(&empty_a[st]), use ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
+                // row of the tile: 128 bytes; 16-byte chunk c goes to chunk c ^ (row & 7) (128-byte swizzle)
+                uint8_t* arow = put + st * PF_A_BYTES;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const int chunk = (4 * half + c) ^ (r & 7);
-                *(uint4*)(arow + 16 * chunk) = make_uint4(p[4 * c], p[4 * c + 1], p[4 * c + 2], p[4 * c + 3]);
+                for (int c = 0; c < 4; c++) *(uint4*)(arow + 16 * ((4 * (q & 1) + c) ^ r7)) = make_uint4(p[4 * c], p[4 * c + 1], p[4 * c + 2], p[4 * c + 3]);
+                fence_proxy_async();                                 // generic-proxy stores -> visible to the tensor core
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&full_a[st]));
+                if (++st == PF_A_STAGES) { st = 0; use ^= 1u; }
             }
-            fence_proxy_async();                                 // generic-proxy stores -> visible to the tensor core
-            __syncwarp();                                        // one arrival per warp: 256 arrivals on one barrier word serialise
-            if (lane == 0) mbar_arrive(smem_u32(&full_a[st]));
         }
     } else if (warp == PF_DECODE_WARPS) {
         // ---------------- operand B: activation tiles by TMA ----------------
         if (lane == 0) {
-            for (int slab = 0; slab < n_slabs; slab++) {
-                const int st = slab % PF_B_STAGES;
-                const uint32_t use = (uint32_t)(slab / PF_B_STAGES);
-                mbar_wait_bounded(smem_u32(&empty_b[st]), (use & 1u) ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
-                const uint32_t fb = smem_u32(&full_b[st]);
-                mbar_arrive_expect_tx(fb, (uint32_t)(a.n_acc * PF_B_BYTES));
-                uint8_t* b0 = stages_b + (size_t)st * PF_B_STAGE_BYTES;
-                for (int n = 0; n < a.n_acc; n++)
-                    tma_load_2d(smem_u32(b0 + n * PF_B_BYTES), &xmap, slab * PF_KSLAB, tok0 + n * PF_NTILE, fb);
-            }
+            int st = 0;
+            uint32_t use = 0;
+            for (int slab = 4 * sb_begin; slab < 4 * sb_end; slab++)
+                for (int n = 0; n < a.n_acc; n++) {
+                    mbar_wait_bounded(smem_u32(&empty_b[st]), use ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
+                    const uint32_t fb = smem_u32(&full_b[st]);
+                    mbar_arrive_expect_tx(fb, (uint32_t)b_stage_bytes);
+                    tma_load_2d(smem_u32(stages_b + st * b_stage_bytes), &xmap, slab * PF_KSLAB, tok0 + n * a.n_tile, fb);
+                    if (++st == a.b_stages) { st = 0; use ^= 1u; }
+                }
         }
     } else {
         // ---------------- MMA issue ----------------
-        if (lane == 0) {
-            for (int slab = 0; slab < n_slabs; slab++) {
-                const int sa = slab % PF_A_STAGES, sb = slab % PF_B_STAGES;
-                mbar_wait_bounded(smem_u32(&full_a[sa]), (uint32_t)(slab / PF_A_STAGES) & 1u, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
-                mbar_wait_bounded(smem_u32(&full_b[sb]), (uint32_t)(slab / PF_B_STAGES) & 1u, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t abase = smem_u32(stages + (size_t)sa * PF_A_BYTES);
-                const uint32_t bbase = smem_u32(stages_b + (size_t)sb * PF_B_STAGE_BYTES);
+        // The whole warp walks the rings and one elected lane issues: descriptors, addresses and counts are then the same in
+        // every lane and stay in uniform registers.  (Under `if (lane == 0)` an MMA took about 250 clocks to issue, four
+        // times what the tensor core needs for 16 tokens: 16384 x 5120 Q4_K, 16 tokens 62 -> 40 us.)
+        const uint32_t idesc = pf_idesc(F16, a.n_tile);
+        const uint64_t desc0 = umma_desc_sw128(0);
+        const uint32_t a_lo = (smem_u32(stages) & 0x3FFFFu) >> 4, b_lo = (smem_u32(stages_b) & 0x3FFFFu) >> 4;
+        int sa = 0, sb = 0;
+        uint32_t use_a = 0, use_b = 0, accum = 0;
+        for (int pair = 2 * sb_begin; pair < 2 * sb_end; pair++) {
+            mbar_wait_bounded(smem_u32(&full_a[sa]), use_a, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
 #pragma unroll
-                for (int k = 0; k < PF_KSLAB / 16; k++) {
-                    const uint64_t adesc = umma_desc_sw128(abase + 32 * k);
-                    for (int n = 0; n < a.n_acc; n++) {
-                        const uint64_t bdesc = umma_desc_sw128(bbase + n * PF_B_BYTES + 32 * k);
-                        const uint32_t accum = (slab > 0 || k > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                            ::"r"(tmem_base + (uint32_t)(n * PF_NTILE)), "l"(adesc), "l"(bdesc), "r"(pf_idesc(F16)), "r"(accum)
-                            : "memory");
+            for (int slab = 0; slab < 2; slab++) {
+                const uint64_t adesc = desc0 + (a_lo + (uint32_t)((sa * PF_A_BYTES + slab * PF_A_SLAB_BYTES) >> 4));
+                for (int n = 0; n < a.n_acc; n++) {
+                    mbar_wait_bounded(smem_u32(&full_b[sb]), use_b, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t bdesc = desc0 + (b_lo + (uint32_t)((sb * b_stage_bytes) >> 4));
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < PF_KSLAB / 16; k++)
+                            asm volatile(
+                                "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                                ::"r"(tmem_base + (uint32_t)(n * PF_MAX_N)), "l"(adesc + (uint64_t)(2 * k)), "l"(bdesc + (uint64_t)(2 * k)), "r"(idesc),
+                                  "r"(k > 0 ? 1u : accum)
+                                : "memory");
+                        // frees the stages once the tensor core has read them
+                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_b[sb])) : "memory");
+                        if (slab == 1 && n == a.n_acc - 1)
+                            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_a[sa])) : "memory");
                     }
+                    __syncwarp();
+                    if (++sb == a.b_stages) { sb = 0; use_b ^= 1u; }
                 }
-                // frees the two stages once the tensor core has read them
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_a[sa])) : "memory");
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_b[sb])) : "memory");
+                accum = 1u;
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_done)) : "memory");
+            if (++sa == PF_A_STAGES) { sa = 0; use_a ^= 1u; }
         }
+        if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_done)) : "memory");
+        __syncwarp();
     }
 
-    // ---------------- epilogue: warps 0-3 read the accumulators (warp w <-> TMEM lanes 32w..32w+31) ----------------
-    if (warp < 4) {
-        mbar_wait_bounded(smem_u32(acc_done), 0u, abort_flag, a.status, ST_TMEM_TIMEOUT);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = row0 + 32 * warp + lane;
-        const int n_tok = min(a.n_acc * PF_NTILE, a.B - tok0);
-        for (int c0 = 0; c0 < n_tok; c0 += 32) {
-            uint32_t v[32];
-            const uint32_t taddr = tmem_base + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                  "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                  "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                  "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                : "r"(taddr)
-                : "memory");
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row < a.M) {
+    // ---------------- epilogue: warp w reads the accumulators' lanes 32 (w % 4) .. + 31, 16 tokens at a time ----------------
+    const int n_tok = min(tile_tok, a.B - tok0), n_chunks = (n_tok + 15) >> 4;
+    const int quad = warp & 3, row = row0 + 32 * quad + lane;
+    auto acc_addr = [&](int chunk) {   // chunk of 16 tokens of the tile; an accumulator holds n_tile of them
+        const int t = 16 * chunk, acc = t >= a.n_tile ? 1 : 0;
+        return tmem_base + ((uint32_t)(32 * quad) << 16) + (uint32_t)(acc * PF_MAX_N + t - acc * a.n_tile);
+    };
+    auto store = [&](int chunk, const float (&v)[16]) {
+        if (row >= a.M) return;
 #pragma unroll
-                for (int j = 0; j < 32; j++) {
-                    if (c0 + j < n_tok) {
-                        float* yo = a.Y + (size_t)(tok0 + c0 + j) * a.ldy + row;
-                        const float val = __uint_as_float(v[j]);
-                        *yo = a.accumulate ? *yo + val : val;
-                    }
-                }
+        for (int j = 0; j < 16; j++) {
+            const int t = 16 * chunk + j;
+            if (t < n_tok) {
+                float* yo = a.Y + (size_t)(tok0 + t) * a.ldy + row;
+                *yo = a.accumulate ? *yo + v[j] : v[j];
             }
         }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    };
+    if (warp < PF_DECODE_WARPS) {
+        mbar_wait_bounded(smem_u32(acc_done), 0u, abort_flag, a.status, ST_TMEM_TIMEOUT);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
+    if (a.splits == 1) {
+        if (warp < PF_DECODE_WARPS)
+            for (int chunk = warp >> 2; chunk < n_chunks; chunk += PF_DECODE_WARPS / 4) {
+                uint32_t v[16];
+                float f[16];
+                tmem_ld16(acc_addr(chunk), v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) f[j] = __uint_as_float(v[j]);
+                store(chunk, f);
+            }
+    } else {
+        // Chunk c of the tile is finished by rank c % splits: the others put their sums of it into that CTA's (now idle)
+        // rings, [source][c / splits][16 tokens][128 rows], sources in rank order without the owner.
+        const int own_chunks = (n_chunks + a.splits - 1) / a.splits;
+        const uint32_t ring = smem_u32(stages);
+        cluster_sync_all();                                  // every CTA's tensor core has read its rings
+        if (warp < PF_DECODE_WARPS)
+            for (int chunk = warp >> 2; chunk < n_chunks; chunk += PF_DECODE_WARPS / 4) {
+                const int owner = chunk % a.splits;
+                if (owner == rank) continue;
+                uint32_t v[16];
+                tmem_ld16(acc_addr(chunk), v);
+                const int src = rank - (rank > owner ? 1 : 0);
+                const uint32_t dst = peer_smem(ring + (uint32_t)((src * own_chunks + chunk / a.splits) * (16 * PF_ROWS) + 32 * quad + lane) * 4u, (uint32_t)owner);
+#pragma unroll
+                for (int j = 0; j < 16; j++) st_peer_f32(dst + (uint32_t)(j * PF_ROWS * 4), v[j]);
+            }
+        cluster_sync_all();                                  // all sums have arrived; nobody touches another CTA's memory after this
+        if (warp < PF_DECODE_WARPS)
+            for (int own = warp >> 2; own * a.splits + rank < n_chunks; own += PF_DECODE_WARPS / 4) {
+                uint32_t v[16];
+                float f[16];
+                tmem_ld16(acc_addr(own * a.splits + rank), v);
+#pragma unroll
+                for (int j = 0; j < 16; j++) f[j] = 0.0f;
+                for (int r = 0; r < a.splits; r++) {
+                    if (r == rank) {
+#pragma unroll
+                        for (int j = 0; j < 16; j++) f[j] += __uint_as_float(v[j]);
+                        continue;
+                    }
+                    const float* in = (const float*)stages + (size_t)((r - (r > rank ? 1 : 0)) * own_chunks + own) * (16 * PF_ROWS) + 32 * quad + lane;
+#pragma unroll
+                    for (int j = 0; j < 16; j++) f[j] += in[j * PF_ROWS];
+                }
+                store(own * a.splits + rank, f);
+            }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == PF_DECODE_WARPS + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
 }
+
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -340,43 +444,86 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-template <int FMT, bool F16>
-int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, dim3 grid, cudaStream_t st) {
-    auto kern = prefill_kernel<FMT, F16>;
+// How a GEMM is cut: token tiles of n_acc x n_tile tokens and K shared by `splits` CTAs.
+struct PrefillCut { int n_acc, n_tile, tok_tiles, splits, b_stages; };
+
+// Picks the cut by its time in SM clocks: rounds of CTAs over the SMs, a K-slab at a time.  A slab takes about 700 clocks
+// to decode plus 1.35 per token (measured, 16384 x 5120 Q4_K: 16 tokens 41 us, 200 52 us, 512 78 us on one round of 128
+// CTAs); 9000 clocks start a CTA and drain it, 8 per token store the tile; a cluster's exchange costs 3000 and another 8
+// per token.  Clusters of three and more leave some SMs of a GPC unused (at M = 5120, 120 CTAs in threes take 60 us where
+// 160 in fours, 132 of which fit at once, take 88).  Against every cut of up to twice as many token tiles and up to
+// eight CTAs, over 11 shapes and 9 token counts, the cut picked was within 3 % of the fastest in all but five cases (9 %).
+// M = 5120, K = 17408, IQ4_XS, 512 tokens: 277 us unsplit, 101 us with three CTAs a tile.
+bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* best) {
+    const long long row_tiles = (M + PF_ROWS - 1) / PF_ROWS;
+    const int nsb = K / 256;
+    const int room = ctx->smem_optin - pf_fixed_smem(fmt);
+    double best_cost = 0.0;
+    bool found = false;
+    const int min_tiles = (B + 2 * PF_MAX_N - 1) / (2 * PF_MAX_N);
+    for (int want = min_tiles; want <= 2 * min_tiles + 1; want++) {
+        const int per = (B + want - 1) / want;
+        PrefillCut c;
+        c.n_acc = per > PF_MAX_N ? 2 : 1;
+        c.n_tile = ((per + c.n_acc - 1) / c.n_acc + 15) / 16 * 16;
+        const int tile = c.n_acc * c.n_tile;
+        c.tok_tiles = (B + tile - 1) / tile;
+        if (ctx->prefill_tiles && want != ctx->prefill_tiles) continue;
+        const int stage = c.n_tile * PF_KSLAB * 2;
+        c.b_stages = std::min(PF_B_MAX_STAGES, room / stage);
+        if (c.b_stages < 2) continue;
+        for (c.splits = 1; c.splits <= std::min(PF_MAX_SPLITS, nsb); c.splits++) {
+            if (ctx->prefill_splits && c.splits != ctx->prefill_splits) continue;
+            const int own_chunks = (tile / 16 + c.splits - 1) / c.splits;
+            if ((c.splits - 1) * own_chunks * (16 * PF_ROWS * 4) > PF_A_STAGES * PF_A_BYTES + c.b_stages * stage) continue;
+            const long long ctas = row_tiles * c.tok_tiles * c.splits;
+            const int slots = c.splits <= 2 ? ctx->sm_count : ctx->sm_count * 9 / 10 / c.splits * c.splits;
+            const double rounds = (double)((ctas + slots - 1) / slots);
+            const double slab = 700.0 + 1.35 * tile;
+            const double cost = rounds * (4.0 * ((nsb + c.splits - 1) / c.splits) * slab + 9000.0 + 8.0 * tile + (c.splits > 1 ? 3000.0 + 8.0 * tile : 0.0));
+            if (!found || cost < best_cost) { found = true; best_cost = cost; *best = c; }
+        }
+    }
+    return found;
+}
+
+template <int FMT, bool F16, bool ALIGNED>
+int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st) {
+    auto kern = prefill_kernel<FMT, F16, ALIGNED>;
     bool known = false;   // opt-in shared-memory size: once per context (= device) and kernel
     for (int i = 0; i < ctx->n_configured; i++) known |= ctx->configured[i] == (const void*)kern;
     if (!known) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ctx->smem_optin);
         if (e != cudaSuccess) { ctx->last_cuda = (int)e; return Q38B_ERR_CUDA; }
         if (ctx->n_configured < (int)(sizeof(ctx->configured) / sizeof(ctx->configured[0]))) ctx->configured[ctx->n_configured++] = (const void*)kern;
     }
-    kern<<<grid, PF_THREADS, PF_SMEM, st>>>(a, map);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) { ctx->last_cuda = (int)e; return Q38B_ERR_CUDA; }
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)((a.M + PF_ROWS - 1) / PF_ROWS * cut.splits), (unsigned)cut.tok_tiles);
+    cfg.blockDim = dim3(PF_THREADS);
+    cfg.dynamicSmemBytes = (size_t)(pf_fixed_smem(FMT) + cut.b_stages * cut.n_tile * PF_KSLAB * 2);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)cut.splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cut.splits > 1 ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, map);
+    if (e != cudaSuccess) { (void)cudaGetLastError(); ctx->last_cuda = (int)e; return Q38B_ERR_CUDA; }
     return Q38B_OK;
 }
 
 template <int FMT>
-int launch_prefill(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, dim3 grid, cudaStream_t st, bool f16) {
-    return f16 ? launch_prefill_op<FMT, true>(ctx, a, map, grid, st) : launch_prefill_op<FMT, false>(ctx, a, map, grid, st);
+int launch_prefill(q38b_ctx* ctx, PrefillArgs a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st, bool f16) {
+    if constexpr (expand_alignment(FMT) > 2) {
+        constexpr int AL = expand_alignment(FMT) - 1;
+        if ((((uintptr_t)a.W | (uintptr_t)a.row_bytes) & AL) == 0)
+            return f16 ? launch_prefill_op<FMT, true, true>(ctx, a, map, cut, st) : launch_prefill_op<FMT, false, true>(ctx, a, map, cut, st);
+    }
+    return f16 ? launch_prefill_op<FMT, true, false>(ctx, a, map, cut, st) : launch_prefill_op<FMT, false, false>(ctx, a, map, cut, st);
 }
 
-int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* X, long long ldx, int B,
-                     float* Y, long long ldy, int accumulate, void* stream, bool f16);
-
-}  // namespace
-
-extern "C" int q38b_gemm_prefill(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* X,
-                                 long long ldx, int B, float* Y, long long ldy, int accumulate, void* stream) {
-    return gemm_prefill_any(ctx, type, W, row_bytes, K, M, X, ldx, B, Y, ldy, accumulate, stream, false);
-}
-
-extern "C" int q38b_gemm_prefill_f16(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* X,
-                                     long long ldx, int B, float* Y, long long ldy, int accumulate, void* stream) {
-    return gemm_prefill_any(ctx, type, W, row_bytes, K, M, X, ldx, B, Y, ldy, accumulate, stream, true);
-}
-
-namespace {
 int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* X, long long ldx, int B,
                      float* Y, long long ldy, int accumulate, void* stream, bool f16) {
     if (!ctx || !W || !X || !Y || K <= 0 || K % 256 || M < 1 || B < 1 || ldx < K || ldy < M) return Q38B_ERR_ARG;
@@ -385,10 +532,12 @@ int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     if (((uintptr_t)W & 1) || (row_bytes & 1) || ((uintptr_t)X & 15) || ((ldx * 2) & 15) || ((uintptr_t)Y & 3)) return Q38B_ERR_ALIGN;
     EncodeTiledFn enc = encode_fn();
     if (!enc) return Q38B_ERR_UNSUPPORTED;
+    PrefillCut cut;
+    if (!prefill_cut(ctx, (int)type, K, M, B, &cut)) return Q38B_ERR_NOMEM;
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)B};
     const cuuint64_t strides[1] = {(cuuint64_t)ldx * 2};
-    const cuuint32_t box[2] = {PF_KSLAB, PF_NTILE};
+    const cuuint32_t box[2] = {PF_KSLAB, (cuuint32_t)cut.n_tile};
     const cuuint32_t estr[2] = {1, 1};
     if (enc(&map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)X, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -403,26 +552,38 @@ int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     a.M = M;
     a.B = B;
     a.accumulate = accumulate ? 1 : 0;
-    const int row_tiles = (M + PF_ROWS - 1) / PF_ROWS;
-    a.n_acc = B > PF_NTILE ? 2 : 1;   // 512 tokens per CTA (two accumulators) halve the dequantization work per token
-    const int tok_per_cta = a.n_acc * PF_NTILE;
-    const dim3 grid((unsigned)row_tiles, (unsigned)((B + tok_per_cta - 1) / tok_per_cta));
+    a.n_acc = cut.n_acc;
+    a.n_tile = cut.n_tile;
+    a.b_stages = cut.b_stages;
+    a.splits = cut.splits;
+    a.grid_src = q38b_grid_source(ctx, type);
     cudaStream_t st = (cudaStream_t)stream;
     switch (type) {
-        case T_Q8_0: return launch_prefill<T_Q8_0>(ctx, a, map, grid, st, f16);
-        case T_Q4_K: return launch_prefill<T_Q4_K>(ctx, a, map, grid, st, f16);
-        case T_Q5_K: return launch_prefill<T_Q5_K>(ctx, a, map, grid, st, f16);
-        case T_Q6_K: return launch_prefill<T_Q6_K>(ctx, a, map, grid, st, f16);
-        case T_IQ3_XXS: return launch_prefill<T_IQ3_XXS>(ctx, a, map, grid, st, f16);
-        case T_IQ3_S: return launch_prefill<T_IQ3_S>(ctx, a, map, grid, st, f16);
-        case T_IQ4_XS: return launch_prefill<T_IQ4_XS>(ctx, a, map, grid, st, f16);
-        case T_Q2_K: return launch_prefill<T_Q2_K>(ctx, a, map, grid, st, f16);
-        case T_IQ2_XXS: return launch_prefill<T_IQ2_XXS>(ctx, a, map, grid, st, f16);
-        case T_IQ2_XS: return launch_prefill<T_IQ2_XS>(ctx, a, map, grid, st, f16);
-        case T_IQ2_S: return launch_prefill<T_IQ2_S>(ctx, a, map, grid, st, f16);
-        case T_IQ1_S: return launch_prefill<T_IQ1_S>(ctx, a, map, grid, st, f16);
-        case T_IQ1_M: return launch_prefill<T_IQ1_M>(ctx, a, map, grid, st, f16);
+#define Q38B_CASE(T) case T: return launch_prefill<T>(ctx, a, map, cut, st, f16)
+        Q38B_CASE(T_Q8_0); Q38B_CASE(T_Q4_K); Q38B_CASE(T_Q5_K); Q38B_CASE(T_Q6_K); Q38B_CASE(T_IQ3_XXS); Q38B_CASE(T_IQ3_S); Q38B_CASE(T_IQ4_XS);
+        Q38B_CASE(T_Q2_K); Q38B_CASE(T_IQ2_XXS); Q38B_CASE(T_IQ2_XS); Q38B_CASE(T_IQ2_S); Q38B_CASE(T_IQ1_S); Q38B_CASE(T_IQ1_M);
+#undef Q38B_CASE
         default: return Q38B_ERR_UNSUPPORTED;
     }
 }
+
 }  // namespace
+
+// Test hook (not in the public header): the prefill GEMM cuts the tokens into `tiles` tiles and shares a tile's K among
+// `splits` CTAs (0: its own rule), so that tests reach every cut with small matrices.
+extern "C" int q38b_debug_set_prefill_cut(q38b_ctx* ctx, int tiles, int splits) {
+    if (!ctx || tiles < 0 || splits < 0 || splits > PF_MAX_SPLITS) return Q38B_ERR_ARG;
+    ctx->prefill_tiles = tiles;
+    ctx->prefill_splits = splits;
+    return Q38B_OK;
+}
+
+extern "C" int q38b_gemm_prefill(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* X,
+                                 long long ldx, int B, float* Y, long long ldy, int accumulate, void* stream) {
+    return gemm_prefill_any(ctx, type, W, row_bytes, K, M, X, ldx, B, Y, ldy, accumulate, stream, false);
+}
+
+extern "C" int q38b_gemm_prefill_f16(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* X,
+                                     long long ldx, int B, float* Y, long long ldy, int accumulate, void* stream) {
+    return gemm_prefill_any(ctx, type, W, row_bytes, K, M, X, ldx, B, Y, ldy, accumulate, stream, true);
+}
