@@ -7,7 +7,7 @@
  *   - `type` is the ggml type id the reference's QuantFormat enum carries verbatim
  *     (include/q38rt/q38rt_types.h:36-67): Q8_0 = 8, Q2_K = 10, Q4_K = 12, Q5_K = 13, Q6_K = 14, IQ2_XXS = 16,
  *     IQ2_XS = 17, IQ3_XXS = 18, IQ1_S = 19, IQ3_S = 21, IQ2_S = 22, IQ4_XS = 23, IQ1_M = 29 (the last six of the
- *     list: one-column kernel, exact dequantizer and prefill GEMM; several columns run as one launch per column);
+ *     list: one-column kernel, exact dequantizer and prefill GEMM; several columns run in launches of up to four);
  *   - weights are row-major GGUF blocks exactly as in the file, `row_bytes` apart (src/cuda/gemv.cuh:26-29);
  *     M counts output rows, K the row length (a multiple of 256);
  *   - output column c of a multi-column call is y + c * y_ld (src/cuda/gemv.cuh:31-34);

@@ -30,7 +30,7 @@
 //    stream).  Define Q38RT_B200_EAGER_DEQUANT to make dequant_rows_f16 also write the fp16 rows (callers that read
 //    the scratch themselves, like the reference's kernel tests).  gemm_f16 on fp16 rows that no dequant_rows_f16 call
 //    recorded (the reference's BF16 projections, Engine::gemm_bf16) is not provided and ends the process with a message.
-//  * gemv_q8n runs one launch per column (each column is the gemv_q8 result bit for bit, as src/cuda/gemv.cuh:31-34
+//  * gemv_q8n runs launches of up to four columns (each column is the gemv_q8 result bit for bit, as src/cuda/gemv.cuh:31-34
 //    promises); the multi-column tensor-core kernel takes Q8_K activations (q38b_gemv_q8k).
 #pragma once
 #include <cuda_fp16.h>

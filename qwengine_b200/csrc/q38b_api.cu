@@ -177,6 +177,10 @@ constexpr int G1_WARPS = 8;                  // consumer warps of a CTA when two
 // ... when a CTA has the SM to itself (measured on B200: the row-group decoder wants its 80 registers, which 20 warps
 // leave it; the others gain from more warps in flight, 5120 x 17408 IQ4_XS 15.7 -> 12.5 us)
 constexpr int G1_WARPS_ONE = 24, G1_WARPS_ONE_RG = 20;
+// several columns: the columns' activations and sums take registers (Q4_K / Q5_K: 20 a column); with the producer 16 warps
+// (12) leave a thread 128 (168), where 17 leave it 96 and spill
+constexpr int G1_COLS = 4;
+constexpr int g1_warps_cols(int fmt) { return fmt == T_Q4_K || fmt == T_Q5_K ? 11 : 15; }
 constexpr int G1_SMEM_BUDGET = 113 * 1024;   // two CTAs per SM (228 KB of shared memory per SM, 1 KB reserved per CTA)
 
 
@@ -186,7 +190,8 @@ struct Plan1 {
     int smem;
     int rows;   // rows per tile: 8, 4 or 2
     int rg;     // 1: row-group mapping (tables in static shared memory, activations staged twice)
-    int occ;    // CTAs per SM: 2 (8 consumer warps) or 1 (16 consumer warps, the whole shared memory)
+    int occ;    // CTAs per SM: 2 (8 consumer warps) or 1 (24 consumer warps, the whole shared memory)
+    int nc;     // columns of the launch (more than one: the kernel for up to G1_COLS)
 };
 
 // The row-group decoders want every row to start 8 bytes aligned: W is 16-byte aligned, so the row stride decides.
@@ -194,12 +199,15 @@ bool rowgroup_eligible(uint32_t type, size_t row_bytes, int rows) { return type 
 
 // Shared-memory carve-up of the single-column kernel: barriers | activation scales | activations | codebook |
 // per-tile slice sums | ring of stages (8 row slots of one 1024-weight slice each).
-int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int G1_ROWS, int occ, Plan1* p) {
+int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int G1_ROWS, int occ, int nc, Plan1* p) {
     const int bb = block_bytes((int)type);
     p->occ = occ;
+    p->nc = nc;
+    p->a.nc = nc;
+    const int sum_cols = nc > 1 ? G1_COLS : 1;   // columns a tile's sums are kept for
     const int nsb = K / 256;
-    const int rg = ctx->rowgroup && rowgroup_eligible(type, row_bytes, G1_ROWS) ? 1 : 0;
-    const int warps = occ == 1 ? (rg ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
+    const int rg = nc == 1 && ctx->rowgroup && rowgroup_eligible(type, row_bytes, G1_ROWS) ? 1 : 0;
+    const int warps = nc > 1 ? g1_warps_cols((int)type) : occ == 1 ? (rg ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
     const int cb_entries = rg ? 0 : type == T_IQ3_XXS ? 256 : type == T_IQ3_S ? 512 : 0;   // row groups keep their tables in static shared memory
     const int budget = (occ == 1 ? ctx->smem_optin : std::min(ctx->smem_optin, G1_SMEM_BUDGET)) - 128 - (rg ? RG_STATIC_BYTES : 0);
     Gemv1Args& a = p->a;
@@ -214,8 +222,8 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     }
     for (int i = n_mats; i < G1_MAX_MATS; i++) a.tile_start[i] = a.n_tiles;
     a.off_actd = 1664;   // barriers (1536 bytes), flags
-    a.off_actq = a.off_actd + a.n_slices * 4 * 32;
-    a.off_cb = a.off_actq + a.n_slices * (rg ? 4 * ACTR_BLOCK_BYTES : 1024);
+    a.off_actq = a.off_actd + nc * a.n_slices * 4 * 32;
+    a.off_cb = a.off_actq + nc * a.n_slices * (rg ? 4 * ACTR_BLOCK_BYTES : 1024);
     const int packed = nsb * bb;
     // stage shape: 8 whole rows in one bulk copy when the rows are packed and small enough, else 8 per-row copies of a
     // K-chunk of `chunk_slices` slices (bulk copies are issue-rate limited: keep each above ~2 KB)
@@ -244,7 +252,7 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
             // tile buffers: a warp can run at most (stages + warps) units ahead of a tile that is still being finished
             const int tb = (warps + stages * a.chunk_slices + 2 * a.n_slices - 1) / a.n_slices + 1;
             if (tb > G1_MAX_TILEBUF) continue;
-            a.off_stage = align_up(a.off_red + tb * a.n_slices * G1_ROWS * 4, 128);
+            a.off_stage = align_up(a.off_red + tb * a.n_slices * G1_ROWS * sum_cols * 4, 128);
             if (a.off_stage + stages * a.stage_bytes + align_up(3 * bb, 128) > budget) continue;
             a.n_stages = stages;
             a.n_tilebuf = tb;
@@ -270,21 +278,27 @@ int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_m
         for (int rows : cands1) {
             if (rows == 16 && !(ctx->rowgroup && rowgroup_eligible(type, row_bytes, 16))) continue;
             memset(best, 0, sizeof(*best));
-            if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 1, best) == Q38B_OK) return Q38B_OK;
+            if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 1, 1, best) == Q38B_OK) return Q38B_OK;
         }
     }
     const int cands[3] = {8, 4, 2};
     for (int rows : cands) {
         memset(best, 0, sizeof(*best));
-        if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 2, best) == Q38B_OK) return Q38B_OK;
+        if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 2, 1, best) == Q38B_OK) return Q38B_OK;
     }
     return Q38B_ERR_NOMEM;
 }
 
-template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2>
+// Two to four columns in one launch: one CTA per SM, tiles of eight rows.
+int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nc, Plan1* p) {
+    memset(p, 0, sizeof(*p));
+    return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, p) : Q38B_ERR_NOMEM;
+}
+
+template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2, int NC = 1>
 int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
-    constexpr int WARPS = OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
-    auto kern = gemv1_kernel<FMT, WARPS, ROWS, RG, A32, OCC>;
+    constexpr int WARPS = NC > 1 ? g1_warps_cols(FMT) : OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
+    auto kern = gemv1_kernel<FMT, WARPS, ROWS, RG, A32, OCC, NC>;
     const int rc = ensure_kernel_smem(ctx, (const void*)kern, (OCC == 1 ? ctx->smem_optin : G1_SMEM_BUDGET) - (RG ? RG_STATIC_BYTES : 0), true);
     if (rc != Q38B_OK) return rc;
     if (ctx->check_occupancy) {   // test hook: count launches whose CTAs would not be resident as often as planned
@@ -310,8 +324,14 @@ int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
 
 template <int FMT>
 int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
+    if (p.nc > 1) {
+        if (p.a.xd32) return launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS>(ctx, p, st);
+        if constexpr (one_column_only(FMT)) return launch_gemv1_rows<FMT, 8, false, false, 1, G1_COLS>(ctx, p, st);
+        return Q38B_ERR_ARG;
+    }
     if (p.a.xd32) {   // per-32 activations: lane-per-granule mapping only
         if (p.rg) return Q38B_ERR_ARG;
+        if (p.occ == 1) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, true, 1>(ctx, p, st) : Q38B_ERR_ARG;
         switch (p.rows) {
             case 8: return launch_gemv1_rows<FMT, 8, false, true>(ctx, p, st);
             case 4: return launch_gemv1_rows<FMT, 4, false, true>(ctx, p, st);
@@ -650,13 +670,37 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
     if (((uintptr_t)W & 15) || (row_bytes % al) || ((uintptr_t)q8k & 3) || ((uintptr_t)y & 3)) return Q38B_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
     if (one_column_only((int)type) && nb > 1) {
-        // formats that only the one-column kernel decodes: one launch per column (every column is the nb = 1 result)
-        for (int c = 0; c < nb; c++) {
+        // formats without mma fragments: launches of up to four columns of the one-column kernel's arithmetic (every column is the nb = 1 result)
+        for (int c = 0; c < nb;) {
+            Plan1 p;
+            int n = std::min(G1_COLS, (nb - c + (nb - c > G1_COLS)) / (nb - c > G1_COLS ? 2 : 1));   // 5 columns: 3 + 2
+            if (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, &p) != Q38B_OK) n = 1;
+            const uint8_t* xq = (const uint8_t*)q8k + (size_t)c * q8k_stride * Q8K_BYTES;
             float* peers_c[7];
             for (int i = 0; i < n_peers; i++) peers_c[i] = y_peers[i] + (size_t)c * y_ld;
-            const int rc = q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, (const uint8_t*)q8k + (size_t)c * q8k_stride * Q8K_BYTES, q8k_stride, 1,
-                                                 y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers, stream);
+            int rc;
+            if (n == 1) {
+                rc = q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, xq, q8k_stride, 1, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers, stream);
+            } else {
+                Gemv1Args& g = p.a;
+                g.W = (const uint8_t*)W;
+                g.row_bytes = (long long)row_bytes;
+                g.xq = xq;
+                g.xq_ld = q8k_stride * Q8K_BYTES;
+                g.y = y + (size_t)c * y_ld;
+                g.y_ld = y_ld;
+                g.n_peers = n_peers;
+                for (int i = 0; i < n_peers; i++) g.y_peer[i] = peers_c[i];
+                g.static_weights = ctx->static_weights;
+                g.status = ctx->d_status;
+                g.codebook = q38b_grid_source(ctx, type);
+                g.K = K;
+                g.M = M;
+                g.accumulate = accumulate ? 1 : 0;
+                rc = dispatch_gemv1(ctx, type, p, st);
+            }
             if (rc != Q38B_OK) return rc;
+            c += n;
         }
         return Q38B_OK;
     }
@@ -734,6 +778,10 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
 int q38b_gemvn_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M, int nb) {
     if (!ctx || n_mats < 1 || n_mats > GEMV_MAX_MATS || !known_format(type) || K <= 0 || K % 256 || nb < 1 || nb > 8) return 0;
     if (row_bytes < q38b_row_bytes(type, K)) return 0;
+    if (one_column_only((int)type)) {
+        Plan1 p1;
+        return nb > 1 && nb <= G1_COLS && plan_gemv1_cols(ctx, type, K, M, n_mats, row_bytes, nb, &p1) == Q38B_OK;
+    }
     Plan p;
     memset(&p, 0, sizeof(p));
     return plan_gemv(ctx, type, K, M, n_mats, nb, &p) == Q38B_OK;
@@ -757,6 +805,30 @@ int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* con
     for (int i = 0; i < n_mats; i++) {
         if (!W[i] || !y[i] || M[i] < 1 || y_ld[i] < M[i]) return Q38B_ERR_ARG;
         if (((uintptr_t)W[i] & 15) || ((uintptr_t)y[i] & 3)) return Q38B_ERR_ALIGN;
+    }
+    if (one_column_only((int)type)) {   // up to four columns (plannable says so) of the one-column kernel's arithmetic
+        Plan1 p1;
+        const int rc1 = plan_gemv1_cols(ctx, type, K, M, n_mats, row_bytes, nb, &p1);
+        if (rc1 != Q38B_OK) return rc1;
+        Gemv1Args& g = p1.a;
+        for (int i = 0; i < n_mats; i++) {
+            (i == 0 ? g.W : g.W_more[i - 1]) = (const uint8_t*)W[i];
+            (i == 0 ? g.y : g.y_more[i - 1]) = y[i];
+            (i == 0 ? g.y_ld : g.y_ld_more[i - 1]) = y_ld[i];
+            (i == 0 ? g.M : g.M_more[i - 1]) = M[i];
+            for (int pr = 0; pr < n_peers; pr++) (i == 0 ? g.y_peer[pr] : g.y_peer_more[i - 1][pr]) = y_peers[i * n_peers + pr];
+        }
+        g.row_bytes = (long long)row_bytes;
+        g.xq = (const uint8_t*)q8k;
+        g.xq_ld = q8k_stride * Q8K_BYTES;
+        g.x_f32 = x_f32;
+        g.x_f32_ld = x_f32_ld;
+        g.n_peers = n_peers;
+        g.static_weights = ctx->static_weights;
+        g.status = ctx->d_status;
+        g.codebook = q38b_grid_source(ctx, type);
+        g.K = K;
+        return dispatch_gemv1(ctx, type, p1, (cudaStream_t)stream);
     }
     Plan p;
     memset(&p, 0, sizeof(p));
@@ -884,23 +956,35 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     if (row_bytes < q38b_row_bytes(type, K)) return Q38B_ERR_ARG;
     const int al = format_alignment(type);
     if (((uintptr_t)W & 15) || (row_bytes % al) || ((uintptr_t)q & 3) || (act_ld & 3) || ((uintptr_t)d & 3) || ((uintptr_t)y & 3)) return Q38B_ERR_ALIGN;
-    // One launch of the one-column kernel per column: every column is the single-column result by construction (the
-    // promise of src/cuda/gemv.cuh:31-34 of the reference), at nb times the cost of one column.
-    const int saved_rg = ctx->rowgroup, saved_one = ctx->one_cta;
+    // The one-column kernel on its lane-per-granule mapping, or launches of up to four columns of the same arithmetic: every
+    // column is the single-column result (the promise of src/cuda/gemv.cuh:31-34 of the reference).
+    const int saved_rg = ctx->rowgroup;
     ctx->rowgroup = 0;
-    ctx->one_cta = 0;
     int rc = Q38B_OK;
-    for (int c = 0; c < nb && rc == Q38B_OK; c++) {
-        Plan1 p1;
-        memset(&p1, 0, sizeof(p1));
-        if (plan_gemv1(ctx, type, K, &M, 1, row_bytes, &p1) != Q38B_OK) { rc = Q38B_ERR_NOMEM; break; }
-        Gemv1Args& g = p1.a;
+    for (int c = 0; c < nb && rc == Q38B_OK;) {
+        Plan1 p;
+        int n = std::min(G1_COLS, (nb - c + (nb - c > G1_COLS)) / (nb - c > G1_COLS ? 2 : 1));
+        if (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, &p) != Q38B_OK) n = 1;
+        if (n == 1) {
+            memset(&p, 0, sizeof(p));
+            if (!ctx->one_cta || plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, &p) != Q38B_OK) {   // one CTA per SM, or what fits two
+                const int saved_one = ctx->one_cta;
+                ctx->one_cta = 0;
+                rc = plan_gemv1(ctx, type, K, &M, 1, row_bytes, &p);
+                ctx->one_cta = saved_one;
+                if (rc != Q38B_OK) { rc = Q38B_ERR_NOMEM; break; }
+            }
+        }
+        Gemv1Args& g = p.a;
         g.W = (const uint8_t*)W;
         g.row_bytes = (long long)row_bytes;
         g.xq = (const uint8_t*)(q + (size_t)c * act_ld);
+        g.xq_ld = act_ld;
         g.xd32 = d + (size_t)c * (act_ld / 32);
+        g.xd32_ld = act_ld / 32;
         g.x_f32 = nullptr;
         g.y = y + (size_t)c * y_ld;
+        g.y_ld = y_ld;
         g.n_peers = 0;
         g.static_weights = ctx->static_weights;
         g.status = ctx->d_status;
@@ -908,11 +992,10 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
         g.K = K;
         g.M = M;
         g.accumulate = accumulate ? 1 : 0;
-        cudaStream_t st = (cudaStream_t)stream;
-        rc = dispatch_gemv1(ctx, type, p1, st);
+        rc = dispatch_gemv1(ctx, type, p, (cudaStream_t)stream);
+        c += n;
     }
     ctx->rowgroup = saved_rg;
-    ctx->one_cta = saved_one;
     return rc;
 }
 

@@ -35,7 +35,7 @@ namespace q38b {
 
 // ggml type ids (the reference keeps them verbatim: include/q38rt/q38rt_types.h:36-67)
 enum : int { T_Q8_0 = 8, T_Q4_K = 12, T_Q5_K = 13, T_Q6_K = 14, T_IQ3_XXS = 18, T_IQ3_S = 21, T_IQ4_XS = 23,
-              // one-column kernel, dequantizer and prefill GEMM only (several columns run one after the other):
+              // one-column kernel (up to four columns a launch), dequantizer and prefill GEMM only:
               T_Q2_K = 10, T_IQ2_XXS = 16, T_IQ2_XS = 17, T_IQ1_S = 19, T_IQ2_S = 22, T_IQ1_M = 29 };
 
 #if !defined(__CUDA_ARCH__)

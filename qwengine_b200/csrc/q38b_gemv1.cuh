@@ -8,9 +8,15 @@
 // except through the per-tile reduction: each (tile, slice) writes its row sums to its own slot and arrives on the
 // tile's mbarrier; the warp that took the tile's last slice waits for the others, adds the slices in order
 // (deterministic) and stores y.
+//
+// With NC = 4 the same kernel takes two to four columns: a granule is decoded once (q38b_decode1n.cuh) and multiplied with
+// each column, whose result is the single-column launch's, bit for bit.  It serves the formats without mma fragments and
+// the per-32 activations; before, they ran one launch per column (bound by issue: the decoding is most of the work).
+// Measured: four columns of 17408 x 5120 IQ3_XXS, per-32 activations, 83 -> 31 us.
 #pragma once
 #include "q38b_act.cuh"
 #include "q38b_decode1.cuh"
+#include "q38b_decode1n.cuh"
 #include "q38b_pipe.cuh"
 
 namespace q38b {
@@ -40,6 +46,10 @@ struct Gemv1Args {
     int static_weights;     // 1: W was written long before this launch, the producer need not wait for earlier kernels
     int* status;
     const uint32_t* codebook;
+    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes), x_f32 and xd32 (floats), and of each
+    // matrix's output (floats; the peers' as well)
+    int nc;
+    long long xq_ld, x_f32_ld, xd32_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
     int K, M, accumulate;
     int nsb;                // super-blocks per row
     int n_slices;           // ceil(nsb / 4)
@@ -86,12 +96,14 @@ constexpr int RG_STATIC_BYTES = 4 * (RG_CB_WORDS + RG_SGN_WORDS);
 // OCC: CTAs per SM the kernel is built for: 1 (NWARPS = 24 consumer warps, 20 for row groups, all of the SM's shared
 // memory: one set of tables and one quantized column per SM, deeper rings, larger tiles; the default plan) or 2 (eight
 // consumer warps and half the shared memory each, for shapes whose one-CTA plan does not fit).
-template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC>
+// NC: columns at most (1 or 4).
+template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC, int NC = 1>
 __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gemv1Args a) {
     constexpr int G1_ROWS = ROWS;
     static_assert(!RG || (FMT == T_IQ3_XXS && ROWS % 4 == 0), "row-group mapping: IQ3_XXS, tiles of 4, 8 or 16 rows");
     static_assert(RG || ROWS <= 8, "the lane-per-granule mapping reduces at most eight rows per unit");
-    static_assert(!(RG && A32), "per-32 activations run on the lane-per-granule mapping");
+    static_assert(!(RG && (A32 || NC > 1)), "per-32 activations and several columns run on the lane-per-granule mapping");
+    const int nc = NC == 1 ? 1 : a.nc;
     // tables of the row-group decoders: static shared memory (their addresses become immediates of the loads); kernels
     // without them have no static shared memory at all, so that two CTAs of 113 KB still fit an SM
     uint32_t* rg_cb = nullptr;
@@ -231,7 +243,66 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         peer_sync_poll(a.sync, ctid, a.status);
         named_bar_sync(14, NWARPS * 32);
     }
-    if (a.x_f32) {
+    const int act_ld = a.n_slices * 1024, actd_ld = a.n_slices * 32;   // between the columns' staged values (bytes) and scales (floats)
+    if constexpr (NC > 1) {
+        // the same two ways for several columns: the blocks (words, scales) of all of them are dealt to the threads
+        const int nsb4 = a.n_slices * 4;
+        if (a.x_f32) {
+            constexpr int QB = 3;
+            for (int b0 = cw; b0 < nc * nsb4; b0 += QB * NWARPS) {
+                float4 lo4[QB], hi4[QB];
+#pragma unroll
+                for (int j = 0; j < QB; j++) {
+                    const int b = b0 + j * NWARPS, c = b / nsb4, sb = b - c * nsb4;
+                    lo4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    hi4[j] = lo4[j];
+                    if (c < nc && sb < a.nsb) {
+                        const float* src = a.x_f32 + (size_t)c * a.x_f32_ld + (size_t)sb * 256 + 8 * lane;
+                        lo4[j] = *(const float4*)src;
+                        hi4[j] = *(const float4*)(src + 4);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < QB; j++) {
+                    const int b = b0 + j * NWARPS, c = b / nsb4, sb = b - c * nsb4;
+                    if (c >= nc) continue;
+                    uint32_t w0 = 0, w1 = 0;
+                    float d = 0.0f;
+                    if (sb < a.nsb) {
+                        const float v[8] = {lo4[j].x, lo4[j].y, lo4[j].z, lo4[j].w, hi4[j].x, hi4[j].y, hi4[j].z, hi4[j].w};
+                        int s8;
+                        q8k_block_core(v, w0, w1, s8, d);
+                    }
+                    if (lane == 0) actd[c * actd_ld + sb * 8] = d;
+                    uint8_t* dst = actq + c * act_ld + (sb >> 2) * 1024;
+                    const int k0 = (sb & 3) * 256 + 8 * lane;
+                    static_assert(A32 || FMT != T_IQ4_XS, "its columns of floats run on the multi-column kernel");
+                    *(uint2*)(dst + act_slice_pos(FMT, k0)) = make_uint2(w0, w1);
+                }
+            }
+        } else {
+            const int n_d = A32 ? actd_ld : nsb4, n_w = a.n_slices * 256;
+            for (int i = ctid; i < nc * n_d; i += NWARPS * 32) {
+                const int c = i / n_d, k = i - c * n_d;
+                if (A32) actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xd32_ld + k] : 0.0f;
+                else actd[c * actd_ld + k * 8] = k < a.nsb ? *(const float*)(a.xq + (size_t)c * a.xq_ld + (size_t)k * Q8K_BYTES) : 0.0f;
+            }
+#pragma unroll 4
+            for (int i = ctid; i < nc * n_w; i += NWARPS * 32) {
+                const int c = i / n_w, w = i - c * n_w, sb = w >> 6, wi = w & 63;
+                const uint8_t* src = a.xq + (size_t)c * a.xq_ld;
+                const uint32_t v = sb >= a.nsb ? 0u : A32 ? *(const uint32_t*)(src + 4 * (size_t)w) : *(const uint32_t*)(src + (size_t)sb * Q8K_BYTES + 4 + 4 * wi);
+                uint8_t* dst = actq + c * act_ld + (sb >> 2) * 1024;
+                const int k0 = (sb & 3) * 256 + 4 * wi;
+                if (FMT == T_IQ4_XS) {
+#pragma unroll
+                    for (int b = 0; b < 4; b++) dst[act_slice_pos(FMT, ((k0 + b) & ~31) + act_stage_pos(FMT, (k0 + b) & 31))] = (uint8_t)(v >> (8 * b));
+                } else {
+                    *(uint32_t*)(dst + act_slice_pos(FMT, k0)) = v;
+                }
+            }
+        }
+    } else if (a.x_f32) {
         // quantize the column here (every CTA, the same arithmetic as quantize_q8k_kernel): one warp per 256 values.  The
         // loads of three blocks go out together, so the warp pays the round trip to L2 once per three blocks.
         constexpr int QB = 3;
@@ -347,7 +418,7 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         const SP st = stage0_sp + (stage * a.stage_bytes + cslice * SLICE_BYTES);
         // low address bits of row 0 of the tile at this stage's first byte (the copy kept its low 4 address bits)
         const uint32_t src_lo = w_lo + (uint32_t)tr.row0 * rb32 + (a.contiguous ? 0u : (uint32_t)(chunk * a.chunk_slices * SLICE_BYTES));
-        float* rslot = red + ((size_t)tslot * a.n_slices + slice) * G1_ROWS;
+        float* rslot = red + ((size_t)tslot * a.n_slices + slice) * (G1_ROWS * NC);
         // a short last chunk holds fewer slices than the barrier expects: its last slice makes up the difference
         const int in_chunk = min(a.chunk_slices, a.n_slices - chunk * a.chunk_slices);
         const int n_arr = (cslice == in_chunk - 1) ? a.chunk_slices - in_chunk + 1 : 1;
@@ -382,29 +453,46 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
                 if (s == 0) rslot[G1_ROWS == 16 ? ps + row_of_sub : 4 * ps + sub] = v;
             }
         } else {
-        typename Gran<FMT>::Acts acts;
-        Gran<FMT>::template load_acts<A32>(acts, actq_sp + slice * 1024, actd_sp + slice * 128, lane);
+        typename Gran<FMT>::Acts acts[NC];
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+            Gran<FMT>::template load_acts<A32>(acts[c], actq_sp + (min(c, nc - 1) * act_ld + slice * 1024), actd_sp + (min(c, nc - 1) * actd_ld * 4 + slice * 128), lane);
         // granules past the end of the row (K not a multiple of 1024) contribute nothing
         const int gran_sb = slice * 4 + (LPR == 32 ? (lane >> 3) : ((lane & 15) >> 2));
         const bool live = gran_sb < a.nsb;
-        float acc[PASSES];
+        float acc[NC][PASSES];
 #pragma unroll
         for (int ps = 0; ps < PASSES; ps++) {
             const int r = LPR == 32 ? ps : 2 * ps + sub;
             const SP rowp = st + (r * a.slot_stride + (int)((src_lo + (uint32_t)r * rb_step) & 15u));
-            const float v = Gran<FMT>::template dot<A32>(rowp, acts, cb, lane);
-            acc[ps] = live ? v : 0.0f;
+            if constexpr (NC == 1) {
+                const float v = Gran<FMT>::template dot<A32>(rowp, acts[0], cb, lane);
+                acc[0][ps] = live ? v : 0.0f;
+            } else {
+                const typename GranN<FMT>::W g = GranN<FMT>::decode(rowp, cb, lane);
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    acc[c][ps] = 0.0f;
+                    if (c < nc) {
+                        const float v = GranN<FMT>::template apply<A32>(g, acts[c]);
+                        acc[c][ps] = live ? v : 0.0f;
+                    }
+                }
+            }
         }
         __syncwarp();
         if (lane == 0) mbar_arrive_n(smem_u32(&empty[stage]), n_arr);
 
         // sum over the lanes of each row: halving butterflies (each step halves the values a lane holds), then plain ones
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+        if (c >= nc) break;
         float rowsum;
         int myrow = 0;      // the row whose sum this lane ends up with
         {
             float v[PASSES];
 #pragma unroll
-            for (int i = 0; i < PASSES; i++) v[i] = acc[i];
+            for (int i = 0; i < PASSES; i++) v[i] = acc[c][i];
             constexpr int TOP = LPR == 32 ? 16 : 8;    // highest lane bit inside one row's lane set
             int n = PASSES, bit = TOP;
 #pragma unroll
@@ -430,7 +518,8 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         }
         // one lane per row writes: the lanes whose low bits (those folded by the plain butterflies) are zero
         constexpr int LOW_MASK = (LPR == 32 ? 32 : 16) / PASSES - 1;
-        if ((lane & LOW_MASK) == 0) rslot[myrow] = rowsum;
+        if ((lane & LOW_MASK) == 0) rslot[c * G1_ROWS + myrow] = rowsum;
+        }
         }
         __syncwarp();
         const uint32_t tb = smem_u32(&tbar[tslot]);
@@ -438,16 +527,18 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         if (slice == a.n_slices - 1) {
             // this warp finishes the tile: wait for the other slices, add them in slice order
             mbar_wait_bounded(tb, tile_par, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
-            const int row = tr.row0 + lane;
+            const int row = tr.row0 + lane % G1_ROWS, col = NC == 1 ? 0 : lane / G1_ROWS;   // NC > 1: eight rows and four columns are the 32 lanes
             float* ym = mi == 0 ? a.y : a.y_more[mi - 1];
             const int Mm = mi == 0 ? a.M : a.M_more[mi - 1];
-            if (lane < G1_ROWS && row < Mm) {
-                const float* rs = red + (size_t)tslot * a.n_slices * G1_ROWS + lane;
+            static_assert(NC == 1 || G1_ROWS * NC == 32, "one lane per row and column");
+            if (lane < G1_ROWS * NC && row < Mm && col < nc) {
+                const float* rs = red + (size_t)tslot * a.n_slices * (G1_ROWS * NC) + lane;
                 float v = 0.0f;
-                for (int s = 0; s < a.n_slices; s++) v += rs[s * G1_ROWS];
-                const float out = a.accumulate ? ym[row] + v : v;
-                ym[row] = out;
-                for (int pr = 0; pr < a.n_peers; pr++) (mi == 0 ? a.y_peer[pr] : a.y_peer_more[mi - 1][pr])[row] = out;   // fused all-gather: push to every peer
+                for (int s = 0; s < a.n_slices; s++) v += rs[s * (G1_ROWS * NC)];
+                const size_t at = NC == 1 ? (size_t)row : (size_t)col * (mi == 0 ? a.y_ld : a.y_ld_more[mi - 1]) + row;
+                const float out = a.accumulate ? ym[at] + v : v;
+                ym[at] = out;
+                for (int pr = 0; pr < a.n_peers; pr++) (mi == 0 ? a.y_peer[pr] : a.y_peer_more[mi - 1][pr])[at] = out;   // fused all-gather: push to every peer
             }
         }
         slice += NWARPS;
