@@ -621,13 +621,11 @@ int q38b_topk(q38b_ctx* ctx, const float* logits, long long ld, int n, int n_row
     if (n_chunks > TOPK_MAX_CHUNKS) return Q38B_ERR_UNSUPPORTED;
     if (((uintptr_t)logits & 3) || ((uintptr_t)vals & 3) || ((uintptr_t)idx & 3)) return Q38B_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t smem = (size_t)n_chunks * k * sizeof(TopkPair);
-    const int rc = ensure_kernel_smem(ctx, (const void*)topk_merge_kernel, ctx->smem_optin, false);
-    if (rc != Q38B_OK) return rc;
     TopkPair* lists = (TopkPair*)ctx->d_topk;
     topk_lists_kernel<<<dim3((unsigned)((n_chunks + TOPK_STAGE1_WARPS - 1) / TOPK_STAGE1_WARPS), (unsigned)n_rows), TOPK_STAGE1_WARPS * 32, 0, st>>>(
         logits, ld, n, k, lists, n_chunks);
-    topk_merge_kernel<<<(unsigned)n_rows, 32 * TOPK_LISTS_PER_LANE, smem, st>>>(lists, n_chunks, k, logits, ld, index_offset, vals, idx, (long long)out_ld);
+    auto merge = n_chunks * k <= 8 * TOPK_MERGE_THREADS ? topk_merge_kernel<8> : topk_merge_kernel<TOPK_MAX_ROUNDS>;
+    merge<<<(unsigned)n_rows, TOPK_MERGE_THREADS, 0, st>>>(lists, n_chunks, k, logits, ld, index_offset, vals, idx, (long long)out_ld);
     Q38B_CUDA(ctx, cudaGetLastError());
     return Q38B_OK;
 }
