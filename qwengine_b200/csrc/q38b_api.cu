@@ -246,8 +246,9 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     const int min_stages = (warps + a.chunk_slices - 1) / a.chunk_slices + 1;
     for (int rep_log2 = cb_entries ? cb1_rep_log2((int)type) : 0; rep_log2 >= (cb_entries ? cb1_rep_log2((int)type) : 0); rep_log2--) {   // the replica count is part of the format's decoder
         a.cb_rep_log2 = rep_log2;
-        a.off_sgn = a.off_cb + align_up((cb_entries * 4 << rep_log2) + 2 * code16_entries((int)type), 128);
-        a.off_red = a.off_sgn + (type == T_IQ3_XXS && !rg ? KSIGN_TABLE_BYTES : 0);
+        const bool xt = occ == 1 && gridx_copies((int)type) > 0;   // expanded grids
+        a.off_sgn = a.off_cb + align_up((cb_entries * 4 << rep_log2) + (xt ? gridx_bytes((int)type) : 2 * code16_entries((int)type)), 128);
+        a.off_red = a.off_sgn + ((type == T_IQ3_XXS && !rg) || (xt && gridx_signs((int)type)) ? KSIGN_TABLE_BYTES : 0);
         for (int stages = G1_MAX_STAGES; stages >= min_stages; stages--) {
             // tile buffers: a warp can run at most (stages + warps) units ahead of a tile that is still being finished
             const int tb = (warps + stages * a.chunk_slices + 2 * a.n_slices - 1) / a.n_slices + 1;

@@ -21,15 +21,14 @@ Q38B_HD int words32_sum(const Words32& g, const uint32_t (&q)[8]) {
 
 template <int FMT> struct GranN;
 
-// the i-quants with one float factor: fp16 d * dx [* 0.125] * integer sum
+// the formats with one float factor: fp16 d * dx * integer sum
 template <int FMT> struct GranNWords {
     using W = Words32;
-    static constexpr bool EIGHTH = FMT == T_IQ2_XXS || FMT == T_IQ2_XS || FMT == T_IQ2_S || FMT == T_IQ1_S || FMT == T_IQ1_M;
+    using Acts = typename Gran<FMT>::Acts;
     template <bool A32>
-    static Q38B_HD float apply(const W& g, const typename Gran<FMT>::Acts& a) {
-        const float f = (float)words32_sum(g, a.q);
-        return EIGHTH ? g.d * a.dx * 0.125f * f : g.d * a.dx * f;
-    }
+    static Q38B_HD void load_acts(Acts& a, SP aq, SP ad, int lane) { Gran<FMT>::template load_acts<A32>(a, aq, ad, lane); }
+    template <bool A32>
+    static Q38B_HD float apply(const W& g, const Acts& a) { return g.d * a.dx * (float)words32_sum(g, a.q); }
 };
 
 template <> struct GranN<T_IQ3_XXS> : GranNWords<T_IQ3_XXS> {
@@ -114,110 +113,152 @@ template <> struct GranN<T_Q8_0> : GranNWords<T_Q8_0> {
     }
 };
 
-Q38B_HD void iq2_words(uint32_t code, uint32_t sign8, uint32_t& w0, uint32_t& w1) {
-    w0 = negate_bytes(iq2_bytes(code & 0xFFu), sign_mask4(sign8 & 0xFu));
-    w1 = negate_bytes(iq2_bytes(code >> 8), sign_mask4(sign8 >> 4));
+// ---------------------------------------------------------------------------------------------------------------
+// IQ2_XXS, IQ2_XS, IQ2_S, IQ1_S, IQ1_M with the whole shared memory of an SM: the grid as eight bytes an entry (the
+// magnitudes 8, 25, 43; for IQ1 eight times the level number 0, 1, 2), in as many copies as fit 64 KB, so that one 64-bit
+// load replaces a 16-bit code, its expansion to two PRMT selectors and two PRMT; lane l reads copy l % copies (16 copies:
+// a half warp meets no bank).  The seven-bit sign codes of IQ2_XXS / IQ2_XS come as byte masks from the table IQ3_XXS has.
+// The integer sums are Gran<FMT>'s, which serves the plans with two CTAs an SM.  Measured with one column, 19456 x 2816
+// IQ2_XXS: 17.8 -> 13.7 us; 2816 x 9728 IQ2_S 10.9 -> 8.5 us; four columns 20.7 and 15.0 us.
+// ---------------------------------------------------------------------------------------------------------------
+Q38B_HD constexpr int gridx_copies(int fmt) { return fmt == T_IQ2_XXS || fmt == T_IQ2_XS ? 16 : fmt == T_IQ2_S ? 8 : fmt == T_IQ1_S || fmt == T_IQ1_M ? 4 : 0; }
+Q38B_HD constexpr int gridx_bytes(int fmt) { return code16_entries(fmt) * gridx_copies(fmt) * 8; }
+Q38B_HD constexpr bool gridx_signs(int fmt) { return fmt == T_IQ2_XXS || fmt == T_IQ2_XS; }
+// bytes 0..3 and 4..7 of the entry with 16-bit code `code`
+template <int FMT>
+Q38B_HD void gridx_entry(uint32_t code, uint32_t& lo, uint32_t& hi) {
+    constexpr uint32_t LEVELS = FMT == T_IQ1_S || FMT == T_IQ1_M ? 0x00100800u : 0x002B1908u;
+    lo = prmt(LEVELS, 0u, sel_from_codes(code & 0xFFu));
+    hi = prmt(LEVELS, 0u, sel_from_codes(code >> 8));
 }
 
-template <> struct GranN<T_IQ2_XXS> : GranNWords<T_IQ2_XXS> {
-    static Q38B_HD W decode(SP row, const Codebook1& cb, int lane) {
-        W g;
-        const SP p = row + 66 * (lane >> 3);
-        uint32_t a0, a1;
-        sp_ld8b_a2(p + (2 + 8 * (lane & 7)), sp_low2(p) ^ 2u, a0, a1);
+// A granule as looked up: grid bytes g, sign masks m (IQ2), delta of each group of eight (IQ1: the weight is g + c)
+struct RawGran { uint32_t g[8], m[8]; int c[4]; int s[2]; float d; };
+template <int FMT> struct GranX {
+    static constexpr bool IQ1 = FMT == T_IQ1_S || FMT == T_IQ1_M;
+    static constexpr int STRIDE = 8 * gridx_copies(FMT), STRIDE_LOG2 = gridx_copies(FMT) == 16 ? 7 : gridx_copies(FMT) == 8 ? 6 : 5;
+    struct Acts : Gran<FMT>::Acts { int bs[IQ1 ? 4 : 1]; };   // bs: sums of eight activations
+    using W = Words32;
+    template <bool A32>
+    static Q38B_HD void load_acts(Acts& a, SP aq, SP ad, int lane) {
+        Gran<FMT>::template load_acts<A32>(a, aq, ad, lane);
+        if (IQ1) {
 #pragma unroll
-        for (int l = 0; l < 4; l++) iq2_words(code16(cb, (a0 >> (8 * l)) & 0xFFu), ksign_byte((a1 >> (7 * l)) & 127u), g.w[2 * l], g.w[2 * l + 1]);
-        g.s[0] = g.s[1] = (int)(2u * (a1 >> 28) + 1u);
-        g.d = fp16_bits_to_float(sp_ld16(p, 0));
-        return g;
-    }
-};
-
-template <> struct GranN<T_IQ2_XS> : GranNWords<T_IQ2_XS> {
-    static Q38B_HD W decode(SP row, const Codebook1& cb, int lane) {
-        W g;
-        const SP p = row + 74 * (lane >> 3);
-        const int ib = lane & 7;
-        uint32_t w[2];
-        sp_ld8b_a2(p + (2 + 8 * ib), sp_low2(p) ^ 2u, w[0], w[1]);
-        const uint32_t sc = sp_ld8(p, 66 + ib);
-#pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t qv = (w[l >> 1] >> (16 * (l & 1))) & 0xFFFFu;
-            iq2_words(code16(cb, qv & 511u), ksign_byte(qv >> 9), g.w[2 * l], g.w[2 * l + 1]);
+            for (int l = 0; l < 4; l++) a.bs[IQ1 ? l : 0] = dp4a_ss(0x01010101u, a.q[2 * l], dp4a_ss(0x01010101u, a.q[2 * l + 1], 0));
         }
-        g.s[0] = (int)(2u * (sc & 0xFu) + 1u);
-        g.s[1] = (int)(2u * (sc >> 4) + 1u);
-        g.d = fp16_bits_to_float(sp_ld16(p, 0));
-        return g;
     }
-};
-
-template <> struct GranN<T_IQ2_S> : GranNWords<T_IQ2_S> {
-    static Q38B_HD W decode(SP row, const Codebook1& cb, int lane) {
-        W g;
-        const SP p = row + 82 * (lane >> 3);
-        const int ib = lane & 7;
-        const uint32_t qs = sp_ld16(p, 2 + 4 * ib) | (sp_ld16(p, 4 + 4 * ib) << 16);
-        const uint32_t sg = sp_ld16(p, 34 + 4 * ib) | (sp_ld16(p, 36 + 4 * ib) << 16);
-        const uint32_t qh = sp_ld8(p, 66 + ib), sc = sp_ld8(p, 74 + ib);
-#pragma unroll
-        for (int l = 0; l < 4; l++)
-            iq2_words(code16(cb, ((qs >> (8 * l)) & 0xFFu) | ((qh << (8 - 2 * l)) & 0x300u)), (sg >> (8 * l)) & 0xFFu, g.w[2 * l], g.w[2 * l + 1]);
-        g.s[0] = (int)(2u * (sc & 0xFu) + 1u);
-        g.s[1] = (int)(2u * (sc >> 4) + 1u);
-        g.d = fp16_bits_to_float(sp_ld16(p, 0));
-        return g;
+    static Q38B_HD void entry(const Codebook1& cb, uint32_t e_times_stride, uint32_t& lo, uint32_t& hi) { sp_ld64(cb.lane_base + (int)e_times_stride, 0, lo, hi); }
+    // bits [at, at + n) of w, times the entry stride
+    static Q38B_HD uint32_t index(uint32_t w, int at, int n) {
+        const uint32_t mask = ((1u << n) - 1u) << STRIDE_LOG2;
+        return (at >= STRIDE_LOG2 ? (w >> (at - STRIDE_LOG2)) : (w << (STRIDE_LOG2 - at))) & mask;
     }
-};
-
-template <> struct GranN<T_IQ1_S> : GranNWords<T_IQ1_S> {
-    static Q38B_HD W decode(SP row, const Codebook1& cb, int lane) {
-        W g;
-        const SP p = row + 50 * (lane >> 3);
+    static Q38B_HD void look_up(SP row, const Codebook1& cb, int lane, RawGran& o) {
+        const SP p = row + Unit<FMT>::BLOCK_BYTES * (lane >> 3);
         const int ib = lane & 7;
-        const uint32_t qs = sp_ld16(p, 2 + 4 * ib) | (sp_ld16(p, 4 + 4 * ib) << 16);
-        const uint32_t qh = sp_ld16(p, 34 + 2 * ib);
-        const bool minus = (qh & 0x8000u) != 0;
+        if constexpr (FMT == T_IQ2_XXS) {
+            uint32_t a0, a1;
+            sp_ld8b_a2(p + (2 + 8 * ib), sp_low2(p) ^ 2u, a0, a1);
 #pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t code = code16(cb, ((qs >> (8 * l)) & 0xFFu) | (((qh >> (3 * l)) & 7u) << 8));
-            g.w[2 * l] = iq1_bytes(code & 0xFFu, minus);
-            g.w[2 * l + 1] = iq1_bytes(code >> 8, minus);
+            for (int l = 0; l < 4; l++) {
+                entry(cb, index(a0, 8 * l, 8), o.g[2 * l], o.g[2 * l + 1]);
+                sp_ld64(cb.sign_base + (int)((l == 0 ? (a1 << 7) : (a1 >> (7 * l - 7))) & 0x3F80u), 0, o.m[2 * l], o.m[2 * l + 1]);
+            }
+            o.s[0] = o.s[1] = (int)(2u * (a1 >> 28) + 1u);
+            o.d = fp16_bits_to_float(sp_ld16(p, 0));
+        } else if constexpr (FMT == T_IQ2_XS) {
+            uint32_t w[2];
+            sp_ld8b_a2(p + (2 + 8 * ib), sp_low2(p) ^ 2u, w[0], w[1]);
+            const uint32_t sc = sp_ld8(p, 66 + ib);
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                const int at = 16 * (l & 1);
+                entry(cb, index(w[l >> 1], at, 9), o.g[2 * l], o.g[2 * l + 1]);
+                sp_ld64(cb.sign_base + (int)((w[l >> 1] >> (at + 2)) & 0x3F80u), 0, o.m[2 * l], o.m[2 * l + 1]);
+            }
+            o.s[0] = (int)(2u * (sc & 0xFu) + 1u);
+            o.s[1] = (int)(2u * (sc >> 4) + 1u);
+            o.d = fp16_bits_to_float(sp_ld16(p, 0));
+        } else if constexpr (FMT == T_IQ2_S) {
+            const uint32_t qs = sp_ld16(p, 2 + 4 * ib) | (sp_ld16(p, 4 + 4 * ib) << 16);
+            const uint32_t sg = sp_ld16(p, 34 + 4 * ib) | (sp_ld16(p, 36 + 4 * ib) << 16);
+            const uint32_t qh = sp_ld8(p, 66 + ib), sc = sp_ld8(p, 74 + ib);
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                entry(cb, index(qs, 8 * l, 8) | ((qh << (8 - 2 * l + STRIDE_LOG2)) & (0x300u << STRIDE_LOG2)), o.g[2 * l], o.g[2 * l + 1]);
+                o.m[2 * l] = sign_mask4((sg >> (8 * l)) & 0xFu);
+                o.m[2 * l + 1] = sign_mask4((sg >> (8 * l + 4)) & 0xFu);
+            }
+            o.s[0] = (int)(2u * (sc & 0xFu) + 1u);
+            o.s[1] = (int)(2u * (sc >> 4) + 1u);
+            o.d = fp16_bits_to_float(sp_ld16(p, 0));
+        } else if constexpr (FMT == T_IQ1_S) {
+            const uint32_t qs = sp_ld16(p, 2 + 4 * ib) | (sp_ld16(p, 4 + 4 * ib) << 16);
+            const uint32_t qh = sp_ld16(p, 34 + 2 * ib);
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                entry(cb, index(qs, 8 * l, 8) | (((qh >> (3 * l)) & 7u) << (8 + STRIDE_LOG2)), o.g[2 * l], o.g[2 * l + 1]);
+                o.c[l] = (qh & 0x8000u) ? -9 : -7;   // 8 (level - 1) + 1, or - 1
+            }
+            o.s[0] = o.s[1] = (int)(2u * ((qh >> 12) & 7u) + 1u);
+            o.d = fp16_bits_to_float(sp_ld16(p, 0));
+        } else {
+            const uint32_t qs = sp_ld16(p, 4 * ib) | (sp_ld16(p, 4 * ib + 2) << 16);
+            const uint32_t qh = sp_ld16(p, 32 + 2 * ib);
+            const uint32_t s0 = sp_ld16(p, 48), s1 = sp_ld16(p, 50), s2 = sp_ld16(p, 52), s3 = sp_ld16(p, 54);
+            const uint32_t su = (s0 >> 12) | ((s1 >> 8) & 0x00F0u) | ((s2 >> 4) & 0x0F00u) | (s3 & 0xF000u);
+            const uint32_t t = ((ib >> 1) == 0 ? s0 : (ib >> 1) == 1 ? s1 : (ib >> 1) == 2 ? s2 : s3) >> (6 * (ib & 1));
+#pragma unroll
+            for (int l = 0; l < 4; l++) {
+                const uint32_t hn = qh >> (4 * l);
+                entry(cb, index(qs, 8 * l, 8) | ((hn & 7u) << (8 + STRIDE_LOG2)), o.g[2 * l], o.g[2 * l + 1]);
+                o.c[l] = (hn & 8u) ? -9 : -7;
+            }
+            o.s[0] = (int)(2u * (t & 7u) + 1u);
+            o.s[1] = (int)(2u * ((t >> 3) & 7u) + 1u);
+            o.d = fp16_bits_to_float(su);
         }
-        g.s[0] = g.s[1] = (int)(2u * ((qh >> 12) & 7u) + 1u);
-        g.d = fp16_bits_to_float(sp_ld16(p, 0));
-        return g;
     }
-};
-
-template <> struct GranN<T_IQ1_M> : GranNWords<T_IQ1_M> {
-    static Q38B_HD W decode(SP row, const Codebook1& cb, int lane) {
-        W g;
-        const SP p = row + 56 * (lane >> 3);
-        const int ib = lane & 7;
-        const uint32_t qs = sp_ld16(p, 4 * ib) | (sp_ld16(p, 4 * ib + 2) << 16);
-        const uint32_t qh = sp_ld16(p, 32 + 2 * ib);
-        const uint32_t s0 = sp_ld16(p, 48), s1 = sp_ld16(p, 50), s2 = sp_ld16(p, 52), s3 = sp_ld16(p, 54);
-        const uint32_t su = (s0 >> 12) | ((s1 >> 8) & 0x00F0u) | ((s2 >> 4) & 0x0F00u) | (s3 & 0xF000u);
-        const uint32_t scw = (ib >> 1) == 0 ? s0 : (ib >> 1) == 1 ? s1 : (ib >> 1) == 2 ? s2 : s3;
-        const uint32_t t = scw >> (6 * (ib & 1));
+    // one column: no signed words, P - 2 N (IQ2) or P + c * (sum of the group's activations) (IQ1)
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        RawGran o;
+        look_up(row, cb, lane, o);
+        int S[2];
 #pragma unroll
-        for (int l = 0; l < 4; l++) {
-            const uint32_t hn = (qh >> (4 * l)) & 0xFu;
-            const uint32_t code = code16(cb, ((qs >> (8 * l)) & 0xFFu) | ((hn & 7u) << 8));
-            const bool minus = (hn & 8u) != 0;
-            g.w[2 * l] = iq1_bytes(code & 0xFFu, minus);
-            g.w[2 * l + 1] = iq1_bytes(code >> 8, minus);
+        for (int h = 0; h < 2; h++) {
+            int P = 0, N = 0;
+#pragma unroll
+            for (int i = 4 * h; i < 4 * h + 4; i++) {
+                P = dp4a_us(o.g[i], a.q[i], P);
+                if (!IQ1) N = dp4a_us(o.g[i] & o.m[i], a.q[i], N);
+            }
+            S[h] = IQ1 ? P + o.c[2 * h] * a.bs[0 + (IQ1 ? 2 * h : 0)] + o.c[2 * h + 1] * a.bs[IQ1 ? 2 * h + 1 : 0] : P - 2 * N;
         }
-        g.s[0] = (int)(2u * (t & 7u) + 1u);
-        g.s[1] = (int)(2u * ((t >> 3) & 7u) + 1u);
-        g.d = fp16_bits_to_float(su);
-        return g;
+        return o.d * a.dx * 0.125f * (float)(o.s[0] * S[0] + o.s[1] * S[1]);
     }
+    // several columns
+    static Q38B_HD W decode(SP row, const Codebook1& cb, int lane) {
+        RawGran o;
+        look_up(row, cb, lane, o);
+        W w;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if (IQ1) w.w[i] = ((o.g[i] | 0x80808080u) - (o.c[i >> 1] == -9 ? 0x09090909u : 0x07070707u)) ^ 0x80808080u;
+            else w.w[i] = negate_bytes(o.g[i], o.m[i]);
+        }
+        w.s[0] = o.s[0];
+        w.s[1] = o.s[1];
+        w.d = o.d;
+        return w;
+    }
+    template <bool A32>
+    static Q38B_HD float apply(const W& g, const Acts& a) { return g.d * a.dx * 0.125f * (float)words32_sum(g, a.q); }
 };
 
 template <> struct GranN<T_Q2_K> {
+    using Acts = Gran<T_Q2_K>::Acts;
+    template <bool A32>
+    static Q38B_HD void load_acts(Acts& a, SP aq, SP ad, int lane) { Gran<T_Q2_K>::load_acts<A32>(a, aq, ad, lane); }
     struct W { uint32_t w[8]; uint32_t sc; float d, dmin; };
     static Q38B_HD W decode(SP row, const Codebook1&, int lane) {
         W g;
@@ -244,6 +285,9 @@ template <> struct GranN<T_Q2_K> {
 
 template <int NBITS> struct GranNQ45K {
     using One = GranQ45K<NBITS>;
+    using Acts = typename One::Acts;
+    template <bool A32>
+    static Q38B_HD void load_acts(Acts& a, SP aq, SP ad, int lane) { One::template load_acts<A32>(a, aq, ad, lane); }
     struct W { uint32_t lo[8], hi[8]; int sc0, sc1, mn0, mn1; float d, dmin; };
     static Q38B_HD W decode(SP row, const Codebook1&, int lane) {
         W g;
@@ -297,6 +341,9 @@ template <> struct GranN<T_Q4_K> : GranNQ45K<4> {};
 template <> struct GranN<T_Q5_K> : GranNQ45K<5> {};
 
 template <> struct GranN<T_Q6_K> {
+    using Acts = Gran<T_Q6_K>::Acts;
+    template <bool A32>
+    static Q38B_HD void load_acts(Acts& a, SP aq, SP ad, int lane) { Gran<T_Q6_K>::load_acts<A32>(a, aq, ad, lane); }
     struct W { uint32_t w[8]; int sc[4]; float d; };
     static Q38B_HD W decode(SP row, const Codebook1&, int lane) {
         W g;

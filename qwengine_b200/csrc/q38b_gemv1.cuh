@@ -14,6 +14,8 @@
 // the per-32 activations; before, they ran one launch per column (bound by issue: the decoding is most of the work).
 // Measured: four columns of 17408 x 5120 IQ3_XXS, per-32 activations, 83 -> 31 us.
 #pragma once
+#include <type_traits>
+
 #include "q38b_act.cuh"
 #include "q38b_decode1.cuh"
 #include "q38b_decode1n.cuh"
@@ -104,6 +106,8 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     static_assert(RG || ROWS <= 8, "the lane-per-granule mapping reduces at most eight rows per unit");
     static_assert(!(RG && (A32 || NC > 1)), "per-32 activations and several columns run on the lane-per-granule mapping");
     const int nc = NC == 1 ? 1 : a.nc;
+    constexpr bool XT = OCC == 1 && gridx_copies(FMT) > 0;   // expanded grid tables: an SM's whole shared memory is this CTA's
+    using G = typename std::conditional<XT, GranX<FMT>, typename std::conditional<NC == 1, Gran<FMT>, GranN<FMT>>::type>::type;
     // tables of the row-group decoders: static shared memory (their addresses become immediates of the loads); kernels
     // without them have no static shared memory at all, so that two CTAs of 113 KB still fit an SM
     uint32_t* rg_cb = nullptr;
@@ -226,10 +230,19 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     } else if (CBN > 0) {
         const int rep = 1 << a.cb_rep_log2;
         for (int i = ctid; i < CBN * rep; i += NWARPS * 32) cbw[i] = a.codebook[i >> a.cb_rep_log2];
+    } else if constexpr (XT) {
+        // two copies of an entry are 16 bytes: a warp's stores cover 512 consecutive bytes
+        constexpr int PAIRS = gridx_copies(FMT) / 2;
+#pragma unroll 4
+        for (int i = ctid; i < code16_entries(FMT) * PAIRS; i += NWARPS * 32) {
+            uint32_t lo, hi;
+            gridx_entry<FMT>(((const uint16_t*)a.codebook)[i / PAIRS], lo, hi);
+            ((uint4*)cbw)[i] = make_uint4(lo, hi, lo, hi);
+        }
     } else if (code16_entries(FMT) > 0) {   // the grid as 16-bit codes, one copy (two entries per word)
         for (int i = ctid; i < code16_entries(FMT) / 2; i += NWARPS * 32) cbw[i] = a.codebook[i];
     }
-    if (FMT == T_IQ3_XXS && !RG) {
+    if ((FMT == T_IQ3_XXS && !RG) || (XT && gridx_signs(FMT))) {
         uint32_t* sg = (uint32_t*)(smem + a.off_sgn);
         for (int i = ctid; i < 128 * 16; i += NWARPS * 32) {   // code i / 16, replica i % 16
             uint32_t lo, hi;
@@ -377,7 +390,7 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     named_bar_sync(15, NWARPS * 32);
 
     Codebook1 cb;                                    // 32 replicas: lane l reads bank l
-    cb.lane_base = sp_from(cbw) + 4 * (lane & ((1 << cb1_rep_log2(FMT)) - 1));
+    cb.lane_base = sp_from(cbw) + (XT ? 8 * (lane & (gridx_copies(FMT) - 1)) : 4 * (lane & ((1 << cb1_rep_log2(FMT)) - 1)));
     cb.sign_base = sp_from(smem + a.off_sgn) + 8 * (lane & 15);
     const TablesR tabs{sp_from(rg_cb), sp_from(rg_sgn), 4u * (uint32_t)lane};
     const SP actq_sp = sp_from(actq), actd_sp = sp_from(actd);
@@ -453,10 +466,10 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
                 if (s == 0) rslot[G1_ROWS == 16 ? ps + row_of_sub : 4 * ps + sub] = v;
             }
         } else {
-        typename Gran<FMT>::Acts acts[NC];
+        typename G::Acts acts[NC];
 #pragma unroll
         for (int c = 0; c < NC; c++)
-            Gran<FMT>::template load_acts<A32>(acts[c], actq_sp + (min(c, nc - 1) * act_ld + slice * 1024), actd_sp + (min(c, nc - 1) * actd_ld * 4 + slice * 128), lane);
+            G::template load_acts<A32>(acts[c], actq_sp + (min(c, nc - 1) * act_ld + slice * 1024), actd_sp + (min(c, nc - 1) * actd_ld * 4 + slice * 128), lane);
         // granules past the end of the row (K not a multiple of 1024) contribute nothing
         const int gran_sb = slice * 4 + (LPR == 32 ? (lane >> 3) : ((lane & 15) >> 2));
         const bool live = gran_sb < a.nsb;
@@ -466,15 +479,17 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
             const int r = LPR == 32 ? ps : 2 * ps + sub;
             const SP rowp = st + (r * a.slot_stride + (int)((src_lo + (uint32_t)r * rb_step) & 15u));
             if constexpr (NC == 1) {
-                const float v = Gran<FMT>::template dot<A32>(rowp, acts[0], cb, lane);
+                float v;
+                if constexpr (XT) v = G::dot(rowp, acts[0], cb, lane);
+                else v = G::template dot<A32>(rowp, acts[0], cb, lane);
                 acc[0][ps] = live ? v : 0.0f;
             } else {
-                const typename GranN<FMT>::W g = GranN<FMT>::decode(rowp, cb, lane);
+                const typename G::W g = G::decode(rowp, cb, lane);
 #pragma unroll
                 for (int c = 0; c < NC; c++) {
                     acc[c][ps] = 0.0f;
                     if (c < nc) {
-                        const float v = GranN<FMT>::template apply<A32>(g, acts[c]);
+                        const float v = G::template apply<A32>(g, acts[c]);
                         acc[c][ps] = live ? v : 0.0f;
                     }
                 }
