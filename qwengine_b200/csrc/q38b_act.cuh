@@ -244,22 +244,35 @@ static __global__ void __launch_bounds__(BF16_THREADS) gemv_bf16_kernel(const ui
 // overwrites the first 2 n bytes of G's row b as 16-bit floats (fp16 like the reference, or bf16 for the bf16 GEMM).
 // One CTA per row: the whole result row is formed in shared memory first (2 n bytes), then copied over the row's start,
 // so no read of G can see a half written earlier.  n, ld multiples of 8; 2 n bytes of shared memory.
+// Bound by memory (10 bytes a value): 512 threads with four 16-byte loads each in flight; with 256 threads and 8-byte loads
+// 1024 x 17408 took 56 us, now 36 us (5.0 TB/s).
+constexpr int SWIGLU_ROWS_THREADS = 512;
 template <bool BF16>
-static __global__ void __launch_bounds__(256) swiglu_rows_inplace_kernel(float* G, const float* __restrict__ U, int n, long long ld) {
+static __global__ void __launch_bounds__(SWIGLU_ROWS_THREADS, 3) swiglu_rows_inplace_kernel(float* G, const float* __restrict__ U, int n, long long ld) {
     extern __shared__ __align__(16) uint8_t row_smem[];
-    uint32_t* h2 = (uint32_t*)row_smem;
     float* g = G + (size_t)blockIdx.x * ld;
     const float* u = U + (size_t)blockIdx.x * ld;
-    for (int i = threadIdx.x; i < n / 2; i += 256) {
-        const float2 a = *(const float2*)(g + 2 * i), b = *(const float2*)(u + 2 * i);
-        const float h0 = a.x / (1.0f + __expf(-a.x)) * b.x, h1 = a.y / (1.0f + __expf(-a.y)) * b.y;
-        if (BF16) { const __nv_bfloat162 v = __floats2bfloat162_rn(h0, h1); h2[i] = *(const uint32_t*)&v; }
-        else { const __half2 v = __floats2half2_rn(h0, h1); h2[i] = *(const uint32_t*)&v; }
+    auto value = [](float x, float y) { return x / (1.0f + __expf(-x)) * y; };
+    auto pack = [](float x, float y) {
+        uint32_t w;
+        if (BF16) { const __nv_bfloat162 v = __floats2bfloat162_rn(x, y); w = *(const uint32_t*)&v; }
+        else { const __half2 v = __floats2half2_rn(x, y); w = *(const uint32_t*)&v; }
+        return w;
+    };
+    const int n4 = n / 4;
+    for (int i0 = threadIdx.x; i0 < n4; i0 += 2 * SWIGLU_ROWS_THREADS) {
+        const int i1 = i0 + SWIGLU_ROWS_THREADS;
+        const bool two = i1 < n4;
+        const float4 a0 = ((const float4*)g)[i0], b0 = ((const float4*)u)[i0];
+        float4 a1 = make_float4(0.f, 0.f, 0.f, 0.f), b1 = a1;
+        if (two) { a1 = ((const float4*)g)[i1]; b1 = ((const float4*)u)[i1]; }
+        ((uint2*)row_smem)[i0] = make_uint2(pack(value(a0.x, b0.x), value(a0.y, b0.y)), pack(value(a0.z, b0.z), value(a0.w, b0.w)));
+        if (two) ((uint2*)row_smem)[i1] = make_uint2(pack(value(a1.x, b1.x), value(a1.y, b1.y)), pack(value(a1.z, b1.z), value(a1.w, b1.w)));
     }
     __syncthreads();
     uint4* dst = (uint4*)g;
     const uint4* src = (const uint4*)row_smem;
-    for (int i = threadIdx.x; i < n / 8; i += 256) dst[i] = src[i];
+    for (int i = threadIdx.x; i < n / 8; i += SWIGLU_ROWS_THREADS) dst[i] = src[i];
 }
 
 }  // namespace q38b

@@ -641,11 +641,11 @@ int q38b_swiglu_rows_inplace(q38b_ctx* ctx, float* G, const float* U, int B, int
     if (out_kind == Q38B_OUT_BF16) {
         const int rc = ensure_kernel_smem(ctx, (const void*)swiglu_rows_inplace_kernel<true>, ctx->smem_optin, false);
         if (rc != Q38B_OK) return rc;
-        swiglu_rows_inplace_kernel<true><<<(unsigned)B, 256, smem, st>>>(G, U, n, ld);
+        swiglu_rows_inplace_kernel<true><<<(unsigned)B, SWIGLU_ROWS_THREADS, smem, st>>>(G, U, n, ld);
     } else {
         const int rc = ensure_kernel_smem(ctx, (const void*)swiglu_rows_inplace_kernel<false>, ctx->smem_optin, false);
         if (rc != Q38B_OK) return rc;
-        swiglu_rows_inplace_kernel<false><<<(unsigned)B, 256, smem, st>>>(G, U, n, ld);
+        swiglu_rows_inplace_kernel<false><<<(unsigned)B, SWIGLU_ROWS_THREADS, smem, st>>>(G, U, n, ld);
     }
     Q38B_CUDA(ctx, cudaGetLastError());
     return Q38B_OK;
