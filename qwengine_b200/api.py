@@ -116,7 +116,8 @@ def status_string(status):
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The current stream's handle.  Asked for raw: torch.cuda.current_stream() builds a Stream object on every call."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 class Context:
