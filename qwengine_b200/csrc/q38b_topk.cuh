@@ -9,8 +9,8 @@
 //            in the order of their positions;
 //   stage 2: one CTA does the same over all lists, then every survivor counts the survivors before it: its place.
 // Both are chains of about 32 dependent steps of some 100 clocks each, whatever k is.  (Picking the k best one after the
-// other took 0.9 us a pick in both stages.  Norm, head and top 32 of 248320 logits: 237 -> 221 us; the pass of a small
-// model with 32003: 561 -> 545 us.)
+// other took 0.9 us a pick in both stages.  Norm, head and top 32 of 248320 logits: 241 -> 231 us, 228 us with the
+// first bits taken from the lanes' and warps' largest keys; the pass of a small model with 32003: 561 -> 545 us.)
 #pragma once
 #include <cstdint>
 
@@ -33,6 +33,13 @@ __device__ __forceinline__ uint32_t topk_key(float f) {
 
 struct TopkPair { uint32_t key; int idx; };   // idx = 0x7fffffff: nothing (a list shorter than k)
 
+// The bits of the k-th key that are known from bounds lo <= k-th key <= hi: where the two differ first, and what is above.
+struct TopkStart { int bit; uint32_t t; };   // bit < 0: nothing is open, t is the key
+__device__ __forceinline__ TopkStart topk_start(uint32_t lo, uint32_t hi) {
+    const int bit = 31 - __clz((int)(lo ^ hi));
+    return TopkStart{bit, bit < 0 ? hi : hi & ~((2u << bit) - 1u)};
+}
+
 // grid (chunks, columns).  lists: [column][chunk][k] pairs by ascending position, then empty ones.
 static __global__ void __launch_bounds__(TOPK_STAGE1_WARPS * 32) topk_lists_kernel(const float* __restrict__ x, long long x_ld, int n, int k,
                                                                              TopkPair* __restrict__ lists, int n_chunks) {
@@ -48,13 +55,18 @@ static __global__ void __launch_bounds__(TOPK_STAGE1_WARPS * 32) topk_lists_kern
         key[j] = i < here ? topk_key(xc[base + i]) : 0u;
     }
     // the largest t that at least k keys reach (0 when fewer are above 0: NaN logits fill up); keys past the end are 0
-    uint32_t t = 0u;
-    for (int bit = 31; bit >= 0; bit--) {
-        const uint32_t cand = t | (1u << bit);
-        int c = 0;
+    // (the lanes' largest keys are 32 keys: at least k <= 32 reach the smallest of them)
+    uint32_t top = 0u;
 #pragma unroll
-        for (int j = 0; j < 32; j++) c += key[j] >= cand;
-        c = (int)__reduce_add_sync(0xffffffffu, (unsigned)c);
+    for (int j = 0; j < 32; j++) top = max(top, key[j]);
+    const TopkStart start = topk_start(k <= 32 ? __reduce_min_sync(0xffffffffu, top) : 0u, __reduce_max_sync(0xffffffffu, top));
+    uint32_t t = start.t;
+    for (int bit = start.bit; bit >= 0; bit--) {
+        const uint32_t cand = t | (1u << bit);
+        int c4[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int j = 0; j < 32; j++) c4[j & 3] += key[j] >= cand;
+        const int c = (int)__reduce_add_sync(0xffffffffu, (unsigned)((c4[0] + c4[1]) + (c4[2] + c4[3])));
         if (c >= k) t = cand;
         if (c == k) break;
     }
@@ -110,9 +122,18 @@ static __global__ void __launch_bounds__(TOPK_MERGE_THREADS) topk_merge_kernel(c
         pos[r] = p.idx;
     }
     if (threadIdx.x == 0) n_best = 0;
-    int phase = 0, c_t = -1;
-    uint32_t t = 0u;
-    for (int bit = 31; bit >= 0 && c_t != k; bit--) {
+    // the same bounds from the largest key of each of the 32 warps
+    uint32_t top = 0u;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) top = max(top, key[r]);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = (int)top;
+    __syncthreads();
+    top = (uint32_t)slots[threadIdx.x & 31];
+    const TopkStart start = topk_start(k <= 32 ? __reduce_min_sync(0xffffffffu, top) : 0u, __reduce_max_sync(0xffffffffu, top));
+    int phase = 1, c_t = -1;
+    uint32_t t = start.t;
+    for (int bit = start.bit; bit >= 0 && c_t != k; bit--) {
         const uint32_t cand = t | (1u << bit);
         int c = 0;
 #pragma unroll
