@@ -121,9 +121,9 @@ int q38b_quantize_act_q8(q38b_ctx* ctx, const float* x_dev, int K, int n_rows, i
 /* Replaces gemv_q8n / gemv_q8 on ActQ8 activations (src/cuda/gemv.cuh:23-34, src/cuda/gemv.cu:206-233):
  * y_dev[c * y_ld + r] (+)= W[r,:] . x_c for c < nb, where x_c is the per-32 quantized column at q_dev + c * act_ld with
  * its scales at d_dev + c * act_ld / 32 (act_ld a multiple of 32, >= K).  The integer sums per 32 weights are exact and
- * each is scaled by its own activation scale.  Every column is computed by the one-column kernel, so column c equals
- * the nb = 1 call on that column bit for bit (the promise of src/cuda/gemv.cuh:31-34) and the cost grows linearly
- * with nb; the Q8_K entry points above are the fast path for several columns. */
+ * each is scaled by its own activation scale.  Every column has the one-column kernel's arithmetic, so column c equals
+ * the nb = 1 call on that column bit for bit (the promise of src/cuda/gemv.cuh:31-34); up to four columns share a launch
+ * and the decoding of the weights. */
 int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W_dev, size_t row_bytes, int K, int M, const int8_t* q_dev,
                      const float* d_dev, int nb, int act_ld, float* y_dev, int y_ld, int accumulate, void* stream);
 

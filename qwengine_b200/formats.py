@@ -30,7 +30,7 @@ IQ4_XS = BlockFormat("IQ4_XS", 23, 256, 136)
 FORMATS = {f.name: f for f in (IQ3_XXS, IQ3_S, IQ4_XS, Q4_K, Q5_K, Q6_K, Q8_0)}
 
 # The reference's other six matvec formats (src/cuda/gemv.cu:206-213): decoded by the one-column kernel, the exact
-# dequantizer and the prefill GEMM; calls with several columns run one column after the other (no tensor-core fragment
+# dequantizer and the prefill GEMM; several columns run in launches of up to four of that kernel (no tensor-core fragment
 # builders for them).
 Q2_K = BlockFormat("Q2_K", 10, 256, 84)
 IQ2_XXS = BlockFormat("IQ2_XXS", 16, 256, 66)
