@@ -67,6 +67,7 @@ struct PrefillArgs {
     int n_tile;            // tokens per accumulator: a multiple of 16, at most 256
     int b_stages;
     int splits;            // CTAs of a cluster that share a tile's K
+    int exact;             // Q4_K, Q5_K whose rows are only 2-byte aligned: no packed conversion
     const uint32_t* grid_src;
 };
 
@@ -94,9 +95,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 // the minimum are rounded to bf16 before instead of after the multiplication: a relative error of 2^-9 per weight, the
 // same size as the rounding of the product to bf16 that the tensor core's operand format imposes anyway.
 // ---------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t bf2_u32(__nv_bfloat162 v) { return *(const uint32_t*)&v; }
 __device__ __forceinline__ __nv_bfloat162 u32_bf2(uint32_t v) { return *(const __nv_bfloat162*)&v; }
-__device__ __forceinline__ __nv_bfloat162 bf2_splat(float x) { return __float2bfloat162_rn(x); }
 // The same for fp16 operands (the reference's prefill path multiplies fp16 weights, src/cuda/prefill.cu:30-85): an integer
 // n < 1024 becomes the half 1024 + n under the bit pattern 0x6400.
 struct OpBf16 {
@@ -108,7 +107,6 @@ struct OpBf16 {
         hi = __hsub2(u32_bf2(__byte_perm(t, 0x43434343u, 0x5342)), bs);
     }
     static __device__ __forceinline__ uint32_t bits(V2 v) { return *(const uint32_t*)&v; }
-    static __device__ __forceinline__ uint32_t pack(float a, float b) { return bf2_u32(__floats2bfloat162_rn(a, b)); }
 };
 struct OpF16 {
     using V2 = __half2;
@@ -120,15 +118,15 @@ struct OpF16 {
         hi = __hsub2(*(const V2*)&h, bs);
     }
     static __device__ __forceinline__ uint32_t bits(V2 v) { return *(const uint32_t*)&v; }
-    static __device__ __forceinline__ uint32_t pack(float a, float b) { const V2 v = __floats2half2_rn(a, b); return *(const uint32_t*)&v; }
 };
 
-// p[j] = weights 2j, 2j + 1 of the sub-block
+// p[j] = weights 2j, 2j + 1 of the sub-block; exact: multiplied in fp32 and rounded once whatever the format
 template <int FMT, bool F16>
-__device__ __forceinline__ void operand_pairs(const Sub32& o, uint32_t (&p)[16]) {
+__device__ __forceinline__ void operand_pairs(const Sub32& o, bool exact, uint32_t (&p)[16]) {
     using OP = typename std::conditional<F16, OpF16, OpBf16>::type;
     using V2 = typename OP::V2;
-    if constexpr (FMT == T_Q4_K || FMT == T_Q5_K || FMT == T_Q6_K) {
+    constexpr bool PACKED = FMT == T_Q4_K || FMT == T_Q5_K || FMT == T_Q6_K;
+    if (PACKED && !exact) {
         const V2 bias = OP::bias(FMT == T_Q6_K ? 32 : 0);
         const V2 a0 = OP::splat(o.a[0]), a1 = FMT == T_Q6_K ? OP::splat(o.a[1]) : a0;
         const V2 c = OP::splat(FMT == T_Q6_K ? 0.0f : -o.c[0]);
@@ -280,7 +278,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                 Sub32 o;
                 load_sub32<FMT, ALIGNED>(blk, 4 * half + q, tab, o);
                 uint32_t p[16];
-                operand_pairs<FMT, F16>(o, p);
+                operand_pairs<FMT, F16>(o, !ALIGNED && (FMT == T_Q4_K || FMT == T_Q5_K) && a.exact, p);
                 mbar_wait_bounded(smem_u32(&empty_a[st]), use ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
                 // row of the tile: 128 bytes; 16-byte chunk c goes to chunk c ^ (row & 7) (128-byte swizzle)
                 uint8_t* arow = put + st * PF_A_BYTES;
@@ -557,6 +555,7 @@ int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     a.b_stages = cut.b_stages;
     a.splits = cut.splits;
     a.grid_src = q38b_grid_source(ctx, type);
+    a.exact = (((uintptr_t)W | row_bytes) & 3) != 0;   // such rows have always been multiplied exactly
     cudaStream_t st = (cudaStream_t)stream;
     switch (type) {
 #define Q38B_CASE(T) case T: return launch_prefill<T>(ctx, a, map, cut, st, f16)

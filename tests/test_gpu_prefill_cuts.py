@@ -36,7 +36,8 @@ def check(ctx, name, M, K, B, dt, tiles, splits, pad=0, shift=0, accumulate=Fals
     ref, mag = x.double() @ wq.double().t(), x.double().abs() @ wq.double().abs().t()
     got = y[:, :M].double() - (7.0 if accumulate else 0.0)
     err = ((got - ref).abs() - (7.0 * 2 ** -23 if accumulate else 0.0)) / mag
-    bound = (4e-3 if dt == torch.bfloat16 else 1e-3) if name in PACKED else 1e-5
+    packed = name == "Q6_K" or (name in PACKED and (w.data_ptr() | rb) % 4 == 0)   # rows of Q4_K, Q5_K that are 2-byte aligned only: exact
+    bound = (4e-3 if dt == torch.bfloat16 else 1e-3) if packed else 1e-5
     assert float(err.max()) < bound, (name, M, K, B, tiles, splits, float(err.max()))
     assert bool((y[:, M:] == 7.0).all())
 
