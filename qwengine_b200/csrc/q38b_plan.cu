@@ -191,7 +191,8 @@ void merge_plan(const q38b_pass* p, int nb, std::vector<Merged>& out, std::vecto
             std::vector<size_t> run;                              // the matvecs the quantize step would be folded into
             for (size_t k = j; on_column(k, col); k = next_in_run(k)) run.push_back(k);
             const size_t run_end = run.empty() ? j : next_real(run.back() + 1);
-            bool ok = !run.empty() && ops[i].off % 4 == 0;
+            // the kernels read the floats 16 bytes at a time; the buffer's length is the distance between its columns
+            bool ok = !run.empty() && ops[i].off % 4 == 0 && (nb == 1 || p->bufs[ops[i].a].n % 4 == 0);
             for (size_t k = run_end; ok && k < n; k++) {   // nobody else reads the Q8_K buffer before it is written again
                 const Op& o = ops[k];
                 if ((o.kind == OP_QUANT && o.b == col) || (o.kind == OP_SWIGLU && o.c == col)) break;
@@ -722,6 +723,28 @@ int q38b_debug_merge_plan(int n_ranks, int nb, int n_steps, const int* steps, in
         for (int t = 0; t < mg.n; t++) launch_of[mg.ops[t]] = mg.first_op;
     }
     return (int)merged.size();
+}
+
+// Test hook (not in the public header): whether a replay with nb columns folds a quantize step of K values at float
+// `src_off` of a buffer of `src_len` floats into the matvec behind it, an M-row matrix of format `type` that writes the
+// same buffer from `dst_off` (negative: another buffer).
+int q38b_debug_quantize_folds(uint32_t type, int nb, int K, int M, int src_len, int src_off, int dst_off) {
+    if (!q38b_format_supported(type) || nb < 1 || K <= 0 || K % 256 || M < 1) return Q38B_ERR_ARG;
+    q38b_ctx ctx;
+    ctx.sm_count = 148;
+    ctx.smem_optin = 232448;
+    q38b_pass p;
+    p.ctx = &ctx;
+    p.mats.push_back({type, nullptr, q38b_row_bytes(type, K), K, M, false});
+    p.bufs.push_back({nullptr, src_len, false, {}, 0, false});
+    p.bufs.push_back({nullptr, K, true, {}, 0, false});
+    p.bufs.push_back({nullptr, M, false, {}, 0, false});
+    p.ops.push_back({OP_QUANT, 0, 1, 0, 0, K, src_off});
+    p.ops.push_back({OP_GEMV, 0, 1, dst_off < 0 ? 2 : 0, 0, 0, std::max(dst_off, 0)});
+    std::vector<Merged> merged;
+    std::vector<char> skip;
+    merge_plan(&p, nb, merged, skip);
+    return merged.size() == 1 && merged[0].quant == 0;
 }
 
 int q38b_pass_kernel_count(const q38b_pass* p) {
