@@ -153,9 +153,16 @@ struct Merged { int first_op; int n; int ops[3]; int quant; };
 // number of ranks a matvec step's output is pushed to (0 for steps recorded with q38b_pass_op_gemv_local)
 int pushes(const q38b_pass* p, const Op& o) { return o.d ? 0 : p->bufs[o.c].n_peer_ranks; }
 
-// Which steps of a replay can share launches.  A quantize step is folded into the
-// matvecs that read its output when they follow it directly, nothing else reads that output before it is rewritten, and
-// all of them run on the one-column kernel.  Consecutive matvecs of one format, K and row stride on one column share a launch.
+// whether matvec step `o` writes any of the floats [lo, lo + n) of buffer `buf` (of a column; every column has the same)
+bool writes(const q38b_pass* p, const Op& o, int buf, long long lo, long long n) {
+    return o.c == buf && o.off < lo + n && lo < (long long)o.off + p->mats[o.a].M;
+}
+
+// Which steps of a replay can share launches.  A quantize step is folded into the matvecs that read its output when they
+// follow it directly, nothing else reads that output before it is rewritten, all of them run on a kernel that can quantize
+// its columns, and none of them writes over the floats (the CTAs of a launch read and store in no order, and a second
+// launch of the same run reads them again).  Consecutive matvecs of one format, K and row stride on one column share a
+// launch unless they write the same floats, where the later one's must stay.
 void merge_plan(const q38b_pass* p, int nb, std::vector<Merged>& out, std::vector<char>& skip) {
     const q38b_ctx* ctx = p->ctx;
     const std::vector<Op>& ops = p->ops;
@@ -201,7 +208,7 @@ void merge_plan(const q38b_pass* p, int nb, std::vector<Merged>& out, std::vecto
             for (size_t k : run) {
                 if (!ok) break;
                 const Mat& m = p->mats[ops[k].a];
-                if (m.K != ops[i].n) ok = false;
+                if (m.K != ops[i].n || writes(p, ops[k], ops[i].a, ops[i].off, ops[i].n)) ok = false;
                 else if (nb == 1 ? !q38b_gemv_group_plannable(ctx, m.type, 1, m.row_bytes, m.K, &m.M)
                                  : !q38b_gemvn_group_plannable(ctx, m.type, 1, m.row_bytes, m.K, &m.M, nb)) ok = false;
             }
@@ -224,6 +231,9 @@ void merge_plan(const q38b_pass* p, int nb, std::vector<Merged>& out, std::vecto
                 const Mat& m = p->mats[ops[k].a];
                 if (m.type != m0.type || m.K != m0.K || m.row_bytes != m0.row_bytes) break;
                 if (pushes(p, ops[k]) != pushes(p, ops[mg.first_op])) break;   // outputs pushed to the peers or not: one kind per launch
+                bool twice = false;
+                for (int t = 0; t < mg.n; t++) twice |= writes(p, ops[mg.ops[t]], ops[k].c, ops[k].off, m.M);
+                if (twice) break;
                 Ms[mg.n] = m.M;
                 if (nb == 1 ? !q38b_gemv_group_plannable(ctx, m0.type, mg.n + 1, m0.row_bytes, m0.K, Ms)
                             : !q38b_gemvn_group_plannable(ctx, m0.type, mg.n + 1, m0.row_bytes, m0.K, Ms, nb)) break;
