@@ -192,6 +192,7 @@ struct Plan1 {
     int rg;     // 1: row-group mapping (tables in static shared memory, activations staged twice)
     int occ;    // CTAs per SM: 2 (8 consumer warps) or 1 (24 consumer warps, the whole shared memory)
     int nc;     // columns of the launch (more than one: the kernel for up to G1_COLS)
+    int xt;     // 1: expanded grid tables (IQ2 / IQ1)
 };
 
 // The row-group decoders want every row to start 8 bytes aligned: W is 16-byte aligned, so the row stride decides.
@@ -199,9 +200,10 @@ bool rowgroup_eligible(uint32_t type, size_t row_bytes, int rows) { return type 
 
 // Shared-memory carve-up of the single-column kernel: barriers | activation scales | activations | codebook |
 // per-tile slice sums | ring of stages (8 row slots of one 1024-weight slice each).
-int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int G1_ROWS, int occ, int nc, Plan1* p) {
+int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int G1_ROWS, int occ, int nc, int xt, Plan1* p) {
     const int bb = block_bytes((int)type);
     p->occ = occ;
+    p->xt = xt;
     p->nc = nc;
     p->a.nc = nc;
     const int sum_cols = nc > 1 ? G1_COLS : 1;   // columns a tile's sums are kept for
@@ -246,7 +248,6 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     const int min_stages = (warps + a.chunk_slices - 1) / a.chunk_slices + 1;
     for (int rep_log2 = cb_entries ? cb1_rep_log2((int)type) : 0; rep_log2 >= (cb_entries ? cb1_rep_log2((int)type) : 0); rep_log2--) {   // the replica count is part of the format's decoder
         a.cb_rep_log2 = rep_log2;
-        const bool xt = occ == 1 && gridx_copies((int)type) > 0;   // expanded grids
         a.off_sgn = a.off_cb + align_up((cb_entries * 4 << rep_log2) + (xt ? gridx_bytes((int)type) : 2 * code16_entries((int)type)), 128);
         a.off_red = a.off_sgn + ((type == T_IQ3_XXS && !rg) || (xt && gridx_signs((int)type)) ? KSIGN_TABLE_BYTES : 0);
         for (int stages = G1_MAX_STAGES; stages >= min_stages; stages--) {
@@ -273,19 +274,23 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
 // one quantized column per SM, deeper rings, 16-row tiles for the row groups.  Measured on B200 it is faster than two
 // CTAs per SM for every shape of the benchmark pass (4.23 ms against 4.30 ms with only long rows and row groups on it,
 // 5.2 ms with none); the two-CTA plans remain for shapes whose one-CTA plan does not fit.
+// The expanded grids of IQ2 / IQ1 (64 KB, for two formats 16 KB of sign masks) are taken where eight rows fit beside them
+// (up to 30,720 weights a row for all five); longer rows keep the 16-bit codes and with them every length that has a plan.
 int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, Plan1* best) {
     if (ctx->one_cta) {
         const int cands1[4] = {16, 8, 4, 2};
         for (int rows : cands1) {
             if (rows == 16 && !(ctx->rowgroup && rowgroup_eligible(type, row_bytes, 16))) continue;
-            memset(best, 0, sizeof(*best));
-            if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 1, 1, best) == Q38B_OK) return Q38B_OK;
+            for (int xt = rows == 8 && gridx_copies((int)type) > 0; xt >= 0; xt--) {
+                memset(best, 0, sizeof(*best));
+                if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 1, 1, xt, best) == Q38B_OK) return Q38B_OK;
+            }
         }
     }
     const int cands[3] = {8, 4, 2};
     for (int rows : cands) {
         memset(best, 0, sizeof(*best));
-        if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 2, 1, best) == Q38B_OK) return Q38B_OK;
+        if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 2, 1, 0, best) == Q38B_OK) return Q38B_OK;
     }
     return Q38B_ERR_NOMEM;
 }
@@ -293,13 +298,13 @@ int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_m
 // Two to four columns in one launch: one CTA per SM, tiles of eight rows.
 int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nc, Plan1* p) {
     memset(p, 0, sizeof(*p));
-    return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, p) : Q38B_ERR_NOMEM;
+    return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p) : Q38B_ERR_NOMEM;
 }
 
-template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2, int NC = 1>
+template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2, int NC = 1, bool XT = false>
 int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     constexpr int WARPS = NC > 1 ? g1_warps_cols(FMT) : OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
-    auto kern = gemv1_kernel<FMT, WARPS, ROWS, RG, A32, OCC, NC>;
+    auto kern = gemv1_kernel<FMT, WARPS, ROWS, RG, A32, OCC, NC, XT>;
     const int rc = ensure_kernel_smem(ctx, (const void*)kern, (OCC == 1 ? ctx->smem_optin : G1_SMEM_BUDGET) - (RG ? RG_STATIC_BYTES : 0), true);
     if (rc != Q38B_OK) return rc;
     if (ctx->check_occupancy) {   // test hook: count launches whose CTAs would not be resident as often as planned
@@ -325,14 +330,15 @@ int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
 
 template <int FMT>
 int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
+    constexpr bool X = gridx_copies(FMT) > 0;
     if (p.nc > 1) {
-        if (p.a.xd32) return launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS>(ctx, p, st);
-        if constexpr (one_column_only(FMT)) return launch_gemv1_rows<FMT, 8, false, false, 1, G1_COLS>(ctx, p, st);
+        if (p.a.xd32) return launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS, X>(ctx, p, st);
+        if constexpr (one_column_only(FMT)) return launch_gemv1_rows<FMT, 8, false, false, 1, G1_COLS, X>(ctx, p, st);
         return Q38B_ERR_ARG;
     }
     if (p.a.xd32) {   // per-32 activations: lane-per-granule mapping only
         if (p.rg) return Q38B_ERR_ARG;
-        if (p.occ == 1) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, true, 1>(ctx, p, st) : Q38B_ERR_ARG;
+        if (p.occ == 1) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, true, 1, 1, X>(ctx, p, st) : Q38B_ERR_ARG;
         switch (p.rows) {
             case 8: return launch_gemv1_rows<FMT, 8, false, true>(ctx, p, st);
             case 4: return launch_gemv1_rows<FMT, 4, false, true>(ctx, p, st);
@@ -348,6 +354,9 @@ int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
         if (p.rg && p.rows == 4) return launch_gemv1_rows<FMT, 4, true>(ctx, p, st);
     }
     if (p.occ == 1) {
+        if constexpr (X) {
+            if (p.xt) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, false, 1, 1, true>(ctx, p, st) : Q38B_ERR_ARG;
+        }
         switch (p.rows) {
             case 8: return launch_gemv1_rows<FMT, 8, false, false, 1>(ctx, p, st);
             case 4: return launch_gemv1_rows<FMT, 4, false, false, 1>(ctx, p, st);
@@ -966,7 +975,7 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
         if (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, &p) != Q38B_OK) n = 1;
         if (n == 1) {
             memset(&p, 0, sizeof(p));
-            if (!ctx->one_cta || plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, &p) != Q38B_OK) {   // one CTA per SM, or what fits two
+            if (!ctx->one_cta || plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, gridx_copies((int)type) > 0, &p) != Q38B_OK) {   // one CTA per SM, or what fits two
                 const int saved_one = ctx->one_cta;
                 ctx->one_cta = 0;
                 rc = plan_gemv1(ctx, type, K, &M, 1, row_bytes, &p);

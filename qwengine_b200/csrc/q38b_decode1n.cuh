@@ -118,7 +118,7 @@ template <> struct GranN<T_Q8_0> : GranNWords<T_Q8_0> {
 // magnitudes 8, 25, 43; for IQ1 eight times the level number 0, 1, 2), in as many copies as fit 64 KB, so that one 64-bit
 // load replaces a 16-bit code, its expansion to two PRMT selectors and two PRMT; lane l reads copy l % copies (16 copies:
 // a half warp meets no bank).  The seven-bit sign codes of IQ2_XXS / IQ2_XS come as byte masks from the table IQ3_XXS has.
-// The integer sums are Gran<FMT>'s, which serves the plans with two CTAs an SM.  Measured with one column, 19456 x 2816
+// The integer sums are Gran<FMT>'s, which serves rows too long for these tables and the plans with two CTAs an SM.  Measured with one column, 19456 x 2816
 // IQ2_XXS: 17.8 -> 13.7 us; 2816 x 9728 IQ2_S 10.9 -> 8.5 us; four columns 20.7 and 15.0 us.
 // ---------------------------------------------------------------------------------------------------------------
 Q38B_HD constexpr int gridx_copies(int fmt) { return fmt == T_IQ2_XXS || fmt == T_IQ2_XS ? 16 : fmt == T_IQ2_S ? 8 : fmt == T_IQ1_S || fmt == T_IQ1_M ? 4 : 0; }

@@ -99,14 +99,16 @@ constexpr int RG_STATIC_BYTES = 4 * (RG_CB_WORDS + RG_SGN_WORDS);
 // memory: one set of tables and one quantized column per SM, deeper rings, larger tiles; the default plan) or 2 (eight
 // consumer warps and half the shared memory each, for shapes whose one-CTA plan does not fit).
 // NC: columns at most (1 or 4).
-template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC, int NC = 1>
+// XT: IQ2 / IQ1 with expanded grid tables (GranX), which want an SM's whole shared memory; without them the 16-bit codes.
+template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC, int NC = 1, bool XT = false>
 __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gemv1Args a) {
     constexpr int G1_ROWS = ROWS;
     static_assert(!RG || (FMT == T_IQ3_XXS && ROWS % 4 == 0), "row-group mapping: IQ3_XXS, tiles of 4, 8 or 16 rows");
     static_assert(RG || ROWS <= 8, "the lane-per-granule mapping reduces at most eight rows per unit");
     static_assert(!(RG && (A32 || NC > 1)), "per-32 activations and several columns run on the lane-per-granule mapping");
     const int nc = NC == 1 ? 1 : a.nc;
-    constexpr bool XT = OCC == 1 && gridx_copies(FMT) > 0;   // expanded grid tables: an SM's whole shared memory is this CTA's
+    static_assert(!XT || (OCC == 1 && gridx_copies(FMT) > 0), "expanded grids: IQ2 / IQ1 with one CTA per SM");
+    static_assert(XT || NC == 1 || gridx_copies(FMT) == 0, "several columns of IQ2 / IQ1 are decoded by GranX");
     using G = typename std::conditional<XT, GranX<FMT>, typename std::conditional<NC == 1, Gran<FMT>, GranN<FMT>>::type>::type;
     // tables of the row-group decoders: static shared memory (their addresses become immediates of the loads); kernels
     // without them have no static shared memory at all, so that two CTAs of 113 KB still fit an SM
