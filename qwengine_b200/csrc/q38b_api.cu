@@ -301,6 +301,17 @@ int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p) : Q38B_ERR_NOMEM;
 }
 
+// How many of `left` columns the next launch takes, with its plan in *p when that is more than one: as many as fit shared
+// memory (long rows of some formats: three or two), dealt evenly over the launches that are left.
+int next_cols(const q38b_ctx* ctx, uint32_t type, int K, int M, size_t row_bytes, int left, Plan1* p) {
+    int most = std::min(G1_COLS, left);
+    while (most > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, most, p) != Q38B_OK) most--;
+    const int launches = (left + most - 1) / most;
+    int n = (left + launches - 1) / launches;
+    while (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, p) != Q38B_OK) n--;
+    return n;
+}
+
 template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2, int NC = 1, bool XT = false>
 int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     constexpr int WARPS = NC > 1 ? g1_warps_cols(FMT) : OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
@@ -681,8 +692,7 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
         // formats without mma fragments: launches of up to four columns of the one-column kernel's arithmetic (every column is the nb = 1 result)
         for (int c = 0; c < nb;) {
             Plan1 p;
-            int n = std::min(G1_COLS, (nb - c + (nb - c > G1_COLS)) / (nb - c > G1_COLS ? 2 : 1));   // 5 columns: 3 + 2
-            if (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, &p) != Q38B_OK) n = 1;
+            const int n = next_cols(ctx, type, K, M, row_bytes, nb - c, &p);
             const uint8_t* xq = (const uint8_t*)q8k + (size_t)c * q8k_stride * Q8K_BYTES;
             float* peers_c[7];
             for (int i = 0; i < n_peers; i++) peers_c[i] = y_peers[i] + (size_t)c * y_ld;
@@ -900,6 +910,15 @@ int q38b_debug_gemv1_rows(uint32_t type, int K, int M, size_t row_bytes, int row
     return p1.occ * 100000 + p1.a.contiguous * 10000 + p1.rows * 100 + p1.a.n_stages;
 }
 
+// Test hook: how many of `left` columns the next launch of the one-column kernel takes on such a device.
+int q38b_debug_gemv1_cols(uint32_t type, int K, int M, size_t row_bytes, int left) {
+    q38b_ctx ctx;
+    ctx.sm_count = 148;
+    ctx.smem_optin = 232448;
+    Plan1 p1;
+    return known_format(type) && K > 0 && K % 256 == 0 && left >= 1 ? next_cols(&ctx, type, K, M, row_bytes, left, &p1) : 0;
+}
+
 int q38b_gemv_group(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const* W, size_t row_bytes, int K, const int* M,
                     const void* q8k, const float* x_f32, float* const* y, void* stream) {
     return q38b_gemv_group_peers(ctx, type, n_mats, W, row_bytes, K, M, q8k, x_f32, y, nullptr, 0, stream);
@@ -971,8 +990,7 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     int rc = Q38B_OK;
     for (int c = 0; c < nb && rc == Q38B_OK;) {
         Plan1 p;
-        int n = std::min(G1_COLS, (nb - c + (nb - c > G1_COLS)) / (nb - c > G1_COLS ? 2 : 1));
-        if (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, &p) != Q38B_OK) n = 1;
+        const int n = next_cols(ctx, type, K, M, row_bytes, nb - c, &p);
         if (n == 1) {
             memset(&p, 0, sizeof(p));
             if (!ctx->one_cta || plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, gridx_copies((int)type) > 0, &p) != Q38B_OK) {   // one CTA per SM, or what fits two

@@ -27,3 +27,23 @@ def test_long_rows_have_a_plan(lib, name, pad):
     for K in list(range(256, ALWAYS + 1, 256)) + [LONGEST[name]]:
         plan = lib.q38b_debug_gemv1_rows(f.type_id, K, 17408, f.row_bytes(K) + pad, 1, 1)
         assert plan // 100000 == 1, (name, K)
+
+
+@pytest.mark.parametrize("name", sorted(F.ALL_FORMATS))
+def test_columns_share_launches_at_every_length(lib, name):
+    """Columns of the one-column kernel's arithmetic: up to four a launch where they fit, else three or two, never one alone
+    beside others; the launches of a call take equal numbers or one less."""
+    fn = lib.q38b_debug_gemv1_cols
+    fn.argtypes = [C.c_uint32, C.c_int, C.c_int, C.c_size_t, C.c_int]
+    f = F.get(name)
+    for K in range(256, 17408 + 1, 256):
+        for pad in (0, 16):
+            for nb in range(1, 9):
+                took, left = [], nb
+                while left:
+                    took.append(fn(f.type_id, K, 5120, f.row_bytes(K) + pad, left))
+                    assert 1 <= took[-1] <= min(4, left)
+                    left -= took[-1]
+                assert max(took) - min(took) <= 1 and (nb == 1 or (nb == 3 and took == [2, 1]) or min(took) >= 2 or took == [2, 2, 1] or took == [2, 2, 2, 1]), (name, K, nb, took)
+            if K <= 8192:
+                assert fn(f.type_id, K, 5120, f.row_bytes(K), 4) == 4
