@@ -301,13 +301,12 @@ int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p) : Q38B_ERR_NOMEM;
 }
 
-// How many of `left` columns the next launch takes, with its plan in *p when that is more than one: as many as fit shared
-// memory (long rows of some formats: three or two), dealt evenly over the launches that are left.
+// How many of `left` columns the next launch takes, with its plan in *p when that is more than one: the most that fit shared
+// memory (four; three or two on long rows of some formats).  A column alone has a kernel of its own that decodes with more
+// warps, so that four columns of which three fit are faster as three and one (5120 x 12288 IQ2_XS: 37.1 us) than as two
+// and two (40.5 us).
 int next_cols(const q38b_ctx* ctx, uint32_t type, int K, int M, size_t row_bytes, int left, Plan1* p) {
-    int most = std::min(G1_COLS, left);
-    while (most > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, most, p) != Q38B_OK) most--;
-    const int launches = (left + most - 1) / most;
-    int n = (left + launches - 1) / launches;
+    int n = std::min(G1_COLS, left);
     while (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, p) != Q38B_OK) n--;
     return n;
 }

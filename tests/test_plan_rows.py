@@ -31,19 +31,15 @@ def test_long_rows_have_a_plan(lib, name, pad):
 
 @pytest.mark.parametrize("name", sorted(F.ALL_FORMATS))
 def test_columns_share_launches_at_every_length(lib, name):
-    """Columns of the one-column kernel's arithmetic: up to four a launch where they fit, else three or two, never one alone
-    beside others; the launches of a call take equal numbers or one less."""
+    """Columns of the one-column kernel's arithmetic: a launch takes the most that fit, four or at long rows of some formats
+    three or two, never one of several."""
     fn = lib.q38b_debug_gemv1_cols
     fn.argtypes = [C.c_uint32, C.c_int, C.c_int, C.c_size_t, C.c_int]
     f = F.get(name)
     for K in range(256, 17408 + 1, 256):
         for pad in (0, 16):
-            for nb in range(1, 9):
-                took, left = [], nb
-                while left:
-                    took.append(fn(f.type_id, K, 5120, f.row_bytes(K) + pad, left))
-                    assert 1 <= took[-1] <= min(4, left)
-                    left -= took[-1]
-                assert max(took) - min(took) <= 1 and (nb == 1 or (nb == 3 and took == [2, 1]) or min(took) >= 2 or took == [2, 2, 1] or took == [2, 2, 2, 1]), (name, K, nb, took)
+            took = [fn(f.type_id, K, 5120, f.row_bytes(K) + pad, left) for left in range(1, 9)]
+            assert took[0] == 1 and took[1] == 2 and took[3:] == took[3:4] * 5, (name, K, took)
+            assert 2 <= took[2] <= took[3] <= 4, (name, K, took)
             if K <= 8192:
-                assert fn(f.type_id, K, 5120, f.row_bytes(K), 4) == 4
+                assert took[2:4] == [3, 4]
