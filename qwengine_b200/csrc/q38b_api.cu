@@ -274,14 +274,15 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
 // one quantized column per SM, deeper rings, 16-row tiles for the row groups.  Measured on B200 it is faster than two
 // CTAs per SM for every shape of the benchmark pass (4.23 ms against 4.30 ms with only long rows and row groups on it,
 // 5.2 ms with none); the two-CTA plans remain for shapes whose one-CTA plan does not fit.
-// The expanded grids of IQ2 / IQ1 (64 KB, for two formats 16 KB of sign masks) are taken where eight rows fit beside them
-// (up to 30,720 weights a row for all five); longer rows keep the 16-bit codes and with them every length that has a plan.
+// The expanded grids of IQ2 / IQ1 (64 KB, for two formats 16 KB of sign masks) are taken where tiles of eight, four or two
+// rows fit beside them (5120 x 45056 IQ2_XS: 39.6 us in tiles of four, 61.3 us with the codes in tiles of eight); longer rows
+// (from 63,744 weights on) keep the 16-bit codes and with them every length that has a plan.
 int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, Plan1* best) {
     if (ctx->one_cta) {
         const int cands1[4] = {16, 8, 4, 2};
-        for (int rows : cands1) {
-            if (rows == 16 && !(ctx->rowgroup && rowgroup_eligible(type, row_bytes, 16))) continue;
-            for (int xt = rows == 8 && gridx_copies((int)type) > 0; xt >= 0; xt--) {
+        for (int xt = gridx_copies((int)type) > 0; xt >= 0; xt--) {
+            for (int rows : cands1) {
+                if (rows == 16 && !(ctx->rowgroup && rowgroup_eligible(type, row_bytes, 16))) continue;
                 memset(best, 0, sizeof(*best));
                 if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, rows, 1, 1, xt, best) == Q38B_OK) return Q38B_OK;
             }
@@ -365,7 +366,14 @@ int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     }
     if (p.occ == 1) {
         if constexpr (X) {
-            if (p.xt) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, false, 1, 1, true>(ctx, p, st) : Q38B_ERR_ARG;
+            if (p.xt) {
+                switch (p.rows) {
+                    case 8: return launch_gemv1_rows<FMT, 8, false, false, 1, 1, true>(ctx, p, st);
+                    case 4: return launch_gemv1_rows<FMT, 4, false, false, 1, 1, true>(ctx, p, st);
+                    case 2: return launch_gemv1_rows<FMT, 2, false, false, 1, 1, true>(ctx, p, st);
+                    default: return Q38B_ERR_ARG;
+                }
+            }
         }
         switch (p.rows) {
             case 8: return launch_gemv1_rows<FMT, 8, false, false, 1>(ctx, p, st);
