@@ -302,6 +302,32 @@ int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p) : Q38B_ERR_NOMEM;
 }
 
+// Whether one column with per-32 activations takes the plan `p` of one CTA per SM (else two).  These calls follow one another
+// without overlap, so a launch's start counts: where a row has few slices, or an SM one tile, two CTAs fill twice as many
+// small stages while the tables are set up (17408 x 1024 Q4_K: 7.6 us, one CTA 10.8 us; Q2_K 7.9 and 10.8 us; 1024 x 5120 Q4_K
+// 4.0 and 4.4 us); where there is more, the single set of tables and the longer ring win (5120 x 17408 IQ2_XS 29.1 and 18.6
+// us, IQ4_XS 21.1 and 16.9 us).  The lines are where the two met over 512 to 17408 rows of 512 to 17408 weights: the
+// expanded grids of IQ2 pay earliest; Q5_K and Q6_K lose with chunks of four slices (17408 x 8192 Q5_K: two CTAs 22.2 us, one
+// 28.0 us); Q4_K, which has the least to decode, gains on many rows at five and six slices only (17408 x 11008: 23.8 and
+// 28.2 us), IQ3_XXS from 14 on.
+bool act_q8_one_cta(const q38b_ctx* ctx, uint32_t type, const Plan1& p) {
+    const int n = p.a.n_slices, tiles = p.a.n_tiles, sms = ctx->sm_count;
+    switch (type) {
+        case T_Q8_0: return false;
+        case T_IQ2_XXS: case T_IQ2_XS: case T_IQ2_S: return n >= 3 || tiles <= 4 * sms;
+        case T_IQ1_M: return n >= 3;
+        case T_IQ4_XS: return n >= 4;
+        default: break;
+    }
+    if (tiles <= sms) return n >= 11;
+    switch (type) {
+        case T_Q5_K: case T_Q6_K: return n >= 3 && p.a.chunk_slices != 4;
+        case T_Q4_K: return n == 5 || n == 6 || (n >= 11 && tiles <= 3 * sms);
+        case T_IQ3_XXS: return n >= 14;
+        default: return n >= 5;   // IQ1_S, IQ3_S, Q2_K
+    }
+}
+
 // How many of `left` columns the next launch takes, with its plan in *p when that is more than one: the most that fit shared
 // memory (four; three or two on long rows of some formats).  A column alone has a kernel of its own that decodes with more
 // warps, so that four columns of which three fit are faster as three and one (5120 x 12288 IQ2_XS: 37.1 us) than as two
@@ -349,7 +375,10 @@ int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     }
     if (p.a.xd32) {   // per-32 activations: lane-per-granule mapping only
         if (p.rg) return Q38B_ERR_ARG;
-        if (p.occ == 1) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, true, 1, 1, X>(ctx, p, st) : Q38B_ERR_ARG;
+        if constexpr (FMT != T_Q8_0) {
+            if (p.occ == 1) return p.rows == 8 ? launch_gemv1_rows<FMT, 8, false, true, 1, 1, X>(ctx, p, st) : Q38B_ERR_ARG;
+        }
+        if (p.occ == 1) return Q38B_ERR_ARG;
         switch (p.rows) {
             case 8: return launch_gemv1_rows<FMT, 8, false, true>(ctx, p, st);
             case 4: return launch_gemv1_rows<FMT, 4, false, true>(ctx, p, st);
@@ -1000,12 +1029,15 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
         const int n = next_cols(ctx, type, K, M, row_bytes, nb - c, &p);
         if (n == 1) {
             memset(&p, 0, sizeof(p));
-            if (!ctx->one_cta || plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, gridx_copies((int)type) > 0, &p) != Q38B_OK) {   // one CTA per SM, or what fits two
+            const bool fits_one = ctx->one_cta && type != T_Q8_0 && plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, gridx_copies((int)type) > 0, &p) == Q38B_OK;
+            if (!fits_one || !act_q8_one_cta(ctx, type, p)) {
+                Plan1 two;
                 const int saved_one = ctx->one_cta;
                 ctx->one_cta = 0;
-                rc = plan_gemv1(ctx, type, K, &M, 1, row_bytes, &p);
+                const bool fits_two = plan_gemv1(ctx, type, K, &M, 1, row_bytes, &two) == Q38B_OK;
                 ctx->one_cta = saved_one;
-                if (rc != Q38B_OK) { rc = Q38B_ERR_NOMEM; break; }
+                if (fits_two) p = two;
+                else if (!fits_one) { rc = Q38B_ERR_NOMEM; break; }
             }
         }
         Gemv1Args& g = p.a;
