@@ -267,6 +267,17 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
     return Q38B_ERR_NOMEM;
 }
 
+// Whether the expanded grids pay: they are 64 KB a CTA to fill before its first row.  The IQ2 formats gain from the
+// smallest matrices on; IQ1 has less to gain: IQ1_M takes them from seven of a tile's slices per SM on (2048 x 1024 6.1 us with
+// the codes, 6.5 with the grids; 4096 x 2048 6.7 us either way; 6144 x 8192 14.7 and 13.0 us), IQ1_S from four tiles a CTA on
+// (2048 x 1024 5.9 and 6.2 us, 4096 x 4096 7.0 and 7.3 us, 6144 x 4096 8.8 and 8.4 us).
+bool gridx_pays(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats) {
+    if (type != T_IQ1_S && type != T_IQ1_M) return gridx_copies((int)type) > 0;
+    long long tiles = 0;
+    for (int i = 0; i < n_mats; i++) tiles += (Ms[i] + 7) / 8;
+    return type == T_IQ1_S ? tiles >= 4 * ctx->sm_count : tiles * ((K + 1023) / 1024) >= 7 * ctx->sm_count;
+}
+
 // Rows per tile: the largest of 8, 4, 2 that can be planned.  Measured on B200 for every shape of the benchmark pass,
 // eight rows win even where fewer rows would balance the CTAs better or let a tile be fetched by one copy: the cost per
 // (tile, slice) unit (activation loads, waits, lane reduction) outweighs both.
@@ -280,7 +291,7 @@ int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, in
 int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, Plan1* best) {
     if (ctx->one_cta) {
         const int cands1[4] = {16, 8, 4, 2};
-        for (int xt = gridx_copies((int)type) > 0; xt >= 0; xt--) {
+        for (int xt = gridx_pays(ctx, type, K, Ms, n_mats); xt >= 0; xt--) {
             for (int rows : cands1) {
                 if (rows == 16 && !(ctx->rowgroup && rowgroup_eligible(type, row_bytes, 16))) continue;
                 memset(best, 0, sizeof(*best));
