@@ -35,7 +35,8 @@ __host__ __device__ constexpr int grid_table_bytes(int fmt) { return grid_table(
 template <int FMT>
 __device__ __forceinline__ void fill_grid_table(uint32_t* tab, const uint32_t* src, int t, int n) {
     constexpr GridTable G = grid_table(FMT);
-    for (int e = t; e < G.entries; e += n) {
+#pragma unroll 8
+    for (int e = t; e < G.entries; e += n) {   // (a thread's loads go out together: one after the other they were most of a small call)
         if (G.words == 1) {
             const uint32_t w = src[e];
             for (int r = 0; r < G.copies; r++) tab[e * G.copies + r] = w;
