@@ -690,10 +690,16 @@ int q38b_topk(q38b_ctx* ctx, const float* logits, long long ld, int n, int n_row
     if (((uintptr_t)logits & 3) || ((uintptr_t)vals & 3) || ((uintptr_t)idx & 3)) return Q38B_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
     TopkPair* lists = (TopkPair*)ctx->d_topk;
-    topk_lists_kernel<<<dim3((unsigned)((n_chunks + TOPK_STAGE1_WARPS - 1) / TOPK_STAGE1_WARPS), (unsigned)n_rows), TOPK_STAGE1_WARPS * 32, 0, st>>>(
+    auto lists_kernel = k <= TOPK_FEW ? topk_lists_kernel<true> : topk_lists_kernel<false>;
+    lists_kernel<<<dim3((unsigned)((n_chunks + TOPK_STAGE1_WARPS - 1) / TOPK_STAGE1_WARPS), (unsigned)n_rows), TOPK_STAGE1_WARPS * 32, 0, st>>>(
         logits, ld, n, k, lists, n_chunks);
-    auto merge = n_chunks * k <= 8 * TOPK_MERGE_THREADS ? topk_merge_kernel<8> : topk_merge_kernel<TOPK_MAX_ROUNDS>;
-    merge<<<(unsigned)n_rows, TOPK_MERGE_THREADS, 0, st>>>(lists, n_chunks, k, logits, ld, index_offset, vals, idx, (long long)out_ld);
+    if (k <= TOPK_FEW) {
+        const int warps = (n_chunks * k + 32 * TOPK_FEW_ROUNDS - 1) / (32 * TOPK_FEW_ROUNDS);
+        topk_merge_few_kernel<<<(unsigned)n_rows, 32 * warps, 0, st>>>(lists, n_chunks, k, logits, ld, index_offset, vals, idx, (long long)out_ld);
+    } else {
+        auto merge = n_chunks * k <= 8 * TOPK_MERGE_THREADS ? topk_merge_kernel<8> : topk_merge_kernel<TOPK_MAX_ROUNDS>;
+        merge<<<(unsigned)n_rows, TOPK_MERGE_THREADS, 0, st>>>(lists, n_chunks, k, logits, ld, index_offset, vals, idx, (long long)out_ld);
+    }
     Q38B_CUDA(ctx, cudaGetLastError());
     return Q38B_OK;
 }

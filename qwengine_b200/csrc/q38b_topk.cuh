@@ -8,9 +8,12 @@
 //            keys at or above a candidate per bit -- and emits the keys above it and the first of the keys equal to it,
 //            in the order of their positions;
 //   stage 2: one CTA does the same over all lists, then every survivor counts the survivors before it: its place.
-// Both are chains of about 32 dependent steps of some 100 clocks each, whatever k is.  (Picking the k best one after the
-// other took 0.9 us a pick in both stages.  Norm, head and top 32 of 248320 logits: 241 -> 231 us, 228 us with the
-// first bits taken from the lanes' and warps' largest keys; the pass of a small model with 32003: 561 -> 545 us.)
+// Both are chains of about 25 dependent steps of some 100 clocks (where more than k keys reach the k-th, stage 2 searches
+// 31 steps more for the last position), whatever k is.  Up to TOPK_FEW elements are picked one after the other instead,
+// 0.45 us an element in both stages together: stage 1 keeps each lane's largest key and looks for its next one when the
+// warp has picked it, stage 2 lets every 256 candidates emit their best as a list and merges the heads of the lists.  Both
+// stages, 248320 logits, one column: k = 1 10.0 us (searched: 17.7), k = 8 13.3 (17.4), k = 16 17.9 (picked: 18.7; eight
+// columns 22.1 and 27.3), k = 32 20.1, k = 64 29.9.  (An earlier version that picked every k took 11.4 to 75.5 us.)
 #pragma once
 #include <cstdint>
 
@@ -21,6 +24,7 @@ constexpr int TOPK_CHUNK = 1024;
 constexpr int TOPK_MAX_CHUNKS = 384;
 constexpr int TOPK_STAGE1_WARPS = 2;          // 243 chunks of a 248320-word vocabulary over 148 SMs
 constexpr int TOPK_MERGE_THREADS = 1024;
+constexpr int TOPK_FEW = 8;                   // elements that are picked one by one, at most
 constexpr int TOPK_MAX_ROUNDS = TOPK_MAX_CHUNKS * TOPK_MAX_K / TOPK_MERGE_THREADS;   // candidates per thread of stage 2
 
 // unsigned order == float order (-0 and +0 are one key, as they compare equal); every NaN maps to 0, below -inf (0x007FFFFF)
@@ -40,7 +44,8 @@ __device__ __forceinline__ TopkStart topk_start(uint32_t lo, uint32_t hi) {
     return TopkStart{bit, bit < 0 ? hi : hi & ~((2u << bit) - 1u)};
 }
 
-// grid (chunks, columns).  lists: [column][chunk][k] pairs by ascending position, then empty ones.
+// grid (chunks, columns).  lists: [column][chunk][k] pairs by ascending position (up to TOPK_FEW: best first), then empty ones.
+template <bool FEW>
 static __global__ void __launch_bounds__(TOPK_STAGE1_WARPS * 32) topk_lists_kernel(const float* __restrict__ x, long long x_ld, int n, int k,
                                                                              TopkPair* __restrict__ lists, int n_chunks) {
     const int lane = threadIdx.x & 31;
@@ -53,6 +58,39 @@ static __global__ void __launch_bounds__(TOPK_STAGE1_WARPS * 32) topk_lists_kern
     for (int j = 0; j < 32; j++) {
         const int i = 32 * j + lane;
         key[j] = i < here ? topk_key(xc[base + i]) : 0u;
+    }
+    if constexpr (FEW) {
+        uint32_t live = 0u;                     // bit j: element j exists and has not been picked (its key is 0 afterwards)
+#pragma unroll
+        for (int j = 0; j < 32; j++) live |= (32 * j + lane < here ? 1u : 0u) << j;
+        uint32_t best = 0u;
+        int slot = -1;                          // this lane's largest key and its first place; -1: nothing left
+        auto scan = [&]() {
+            uint32_t m4[4] = {0u, 0u, 0u, 0u}, at = 0u;
+#pragma unroll
+            for (int j = 0; j < 32; j++) m4[j & 3] = max(m4[j & 3], key[j]);
+            best = max(max(m4[0], m4[1]), max(m4[2], m4[3]));
+#pragma unroll
+            for (int j = 0; j < 32; j++) at |= (key[j] == best ? 1u : 0u) << j;
+            slot = __ffs((int)(at & live)) - 1;
+        };
+        scan();
+        TopkPair mine{0u, 0x7fffffff};
+        for (int r = 0; r < k; r++) {
+            const uint32_t w = __reduce_max_sync(0xffffffffu, best);
+            const int p = slot >= 0 && best == w ? base + 32 * slot + lane : 0x7fffffff;
+            const int first = (int)__reduce_min_sync(0xffffffffu, (unsigned)p);
+            if (lane == r) mine = TopkPair{w, first};
+            if (p == first && p != 0x7fffffff) {
+                live &= ~(1u << slot);
+#pragma unroll
+                for (int j = 0; j < 32; j++)
+                    if (j == slot) key[j] = 0u;
+                scan();
+            }
+        }
+        if (lane < k) lists[((size_t)blockIdx.y * n_chunks + chunk) * k + lane] = mine;
+        return;
     }
     // the largest t that at least k keys reach (0 when fewer are above 0: NaN logits fill up); keys past the end are 0
     // (the lanes' largest keys are 32 keys: at least k <= 32 reach the smallest of them)
@@ -89,6 +127,58 @@ static __global__ void __launch_bounds__(TOPK_STAGE1_WARPS * 32) topk_lists_kern
         at += __popc(tk);
     }
     for (int r = at + lane; r < k; r += 32) out[r] = TopkPair{0u, 0x7fffffff};
+}
+
+// Stage 2 for k <= TOPK_FEW: grid (columns), a warp per 256 candidates.
+constexpr int TOPK_FEW_ROUNDS = 8;
+static_assert(TOPK_MAX_CHUNKS * TOPK_FEW <= 32 * 32 * TOPK_FEW_ROUNDS && TOPK_FEW <= 32, "a list per lane, a result per lane");
+static __global__ void __launch_bounds__(1024) topk_merge_few_kernel(const TopkPair* __restrict__ lists, int n_chunks, int k, const float* __restrict__ x,
+                                                                     long long x_ld, int index_offset, float* __restrict__ vals, int* __restrict__ idx,
+                                                                     long long out_ld) {
+    __shared__ TopkPair heads[32 * TOPK_FEW];
+    const TopkPair* src = lists + (size_t)blockIdx.x * n_chunks * k;
+    const int total = n_chunks * k, warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31, n_warps = (int)blockDim.x >> 5;
+    const TopkPair none{0u, 0x7fffffff};
+    uint32_t key[TOPK_FEW_ROUNDS];
+    int pos[TOPK_FEW_ROUNDS];
+#pragma unroll
+    for (int r = 0; r < TOPK_FEW_ROUNDS; r++) {
+        const int i = 32 * (TOPK_FEW_ROUNDS * warp + r) + lane;
+        const TopkPair p = i < total ? src[i] : none;
+        key[r] = p.key;
+        pos[r] = p.idx;
+    }
+    TopkPair mine = none;
+    for (int t = 0; t < k; t++) {
+        uint32_t best = 0u;
+        int at = 0x7fffffff;
+#pragma unroll
+        for (int r = 0; r < TOPK_FEW_ROUNDS; r++) best = max(best, key[r]);
+#pragma unroll
+        for (int r = 0; r < TOPK_FEW_ROUNDS; r++) at = min(at, key[r] == best ? pos[r] : 0x7fffffff);
+        const uint32_t w = __reduce_max_sync(0xffffffffu, best);
+        const int first = (int)__reduce_min_sync(0xffffffffu, (unsigned)(best == w ? at : 0x7fffffff));
+        if (lane == t) mine = TopkPair{w, first};
+#pragma unroll
+        for (int r = 0; r < TOPK_FEW_ROUNDS; r++)
+            if (pos[r] == first) { key[r] = 0u; pos[r] = 0x7fffffff; }
+    }
+    if (lane < k) heads[warp * k + lane] = mine;
+    __syncthreads();
+    if (warp > 0) return;
+    int taken = 0;
+    TopkPair head = lane < n_warps ? heads[lane * k] : none;
+    mine = none;
+    for (int t = 0; t < k; t++) {
+        const uint32_t w = __reduce_max_sync(0xffffffffu, head.key);
+        const int first = (int)__reduce_min_sync(0xffffffffu, (unsigned)(head.key == w ? head.idx : 0x7fffffff));
+        if (lane == t) mine = TopkPair{w, first};
+        if (head.idx == first && first != 0x7fffffff) head = ++taken < k ? heads[lane * k + taken] : none;
+    }
+    if (lane >= k) return;
+    const bool empty = mine.idx == 0x7fffffff;
+    vals[(size_t)blockIdx.x * out_ld + lane] = empty ? __uint_as_float(0x7FC00000u) : x[(size_t)blockIdx.x * x_ld + mine.idx];
+    idx[(size_t)blockIdx.x * out_ld + lane] = empty ? -1 : mine.idx + index_offset;
 }
 
 // Sum over the CTA of one count per thread; `slots`: [2][32] ints, used alternately so that one barrier per sum is enough.
