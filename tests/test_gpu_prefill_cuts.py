@@ -52,10 +52,34 @@ def test_cuts_all_formats(ctx, name, M, K, B, pad, shift, tiles, splits):
 @pytest.mark.parametrize("splits", [1, 2, 3, 4, 5, 7, 8])
 @pytest.mark.parametrize("B,tiles", [(16, 1), (77, 1), (250, 1), (250, 3), (258, 1), (530, 2)])
 def test_splits_and_tiles(ctx, splits, B, tiles):
-    if splits > 4 and B == 258:
-        pytest.skip("the partial sums of 512 tokens from more than three other CTAs do not fit")
     check(ctx, "IQ3_XXS", 200, 2304, B, torch.bfloat16, tiles, splits, accumulate=splits % 2 == 0)
     check(ctx, "Q5_K", 200, 2304, B, torch.float16, tiles, splits, accumulate=splits % 2 == 1)
+
+
+@pytest.mark.parametrize("name", ["IQ3_XXS", "Q5_K"])
+def test_full_tiles_fill_the_exchange(ctx, name):
+    """Two accumulators of 256 tokens: the partial sums of three other CTAs take the rings to the last byte, a fourth's have
+    no room (refused: the own rule never picks that cut)."""
+    for splits in (2, 3, 4):
+        check(ctx, name, 130, 2304, 512, torch.bfloat16, 1, splits)
+    f, K = F.get(name), 2304
+    w = torch.zeros((130, f.row_bytes(K)), dtype=torch.uint8, device="cuda")
+    x = torch.zeros((512, K), dtype=torch.bfloat16, device="cuda")
+    assert ctx.lib.q38b_debug_set_prefill_cut(ctx.h, 1, 5) == 0
+    try:
+        with pytest.raises(api.Q38BError) as e:
+            ctx.gemm_prefill(f, w, x, K)
+    finally:
+        ctx.lib.q38b_debug_set_prefill_cut(ctx.h, 0, 0)
+    assert e.value.status == -6      # Q38B_ERR_NOMEM
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q5_K"])
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("pad,shift", [(4, 4), (0, 8), (12, 0)])
+def test_packed_conversion_on_unaligned_rows(ctx, name, dt, pad, shift):
+    """Rows that are 4- but not 16-byte aligned: the packed conversion behind the word loads that assume two bytes only."""
+    check(ctx, name, 130, 1280, 33, dt, 1, 2, pad, shift)
 
 
 @pytest.mark.parametrize("M,K,B", [(5120, 5120, 9), (640, 17408, 77), (17000, 1024, 513), (1024, 512, 1030)])
