@@ -343,8 +343,9 @@ bool act_q8_one_cta(const q38b_ctx* ctx, uint32_t type, const Plan1& p) {
 // memory (four; three or two on long rows of some formats).  A column alone has a kernel of its own that decodes with more
 // warps, so that four columns of which three fit are faster as three and one (5120 x 12288 IQ2_XS: 37.1 us) than as two
 // and two (40.5 us).
+// Six are two threes (17408 x 5120 IQ2_XS: 50.6 us, as four and two 51.3 us).
 int next_cols(const q38b_ctx* ctx, uint32_t type, int K, int M, size_t row_bytes, int left, Plan1* p) {
-    int n = std::min(G1_COLS, left);
+    int n = left == 6 ? 3 : std::min(G1_COLS, left);
     while (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, p) != Q38B_OK) n--;
     return n;
 }

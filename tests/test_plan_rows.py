@@ -39,7 +39,7 @@ def test_columns_share_launches_at_every_length(lib, name):
     for K in range(256, 17408 + 1, 256):
         for pad in (0, 16):
             took = [fn(f.type_id, K, 5120, f.row_bytes(K) + pad, left) for left in range(1, 9)]
-            assert took[0] == 1 and took[1] == 2 and took[3:] == took[3:4] * 5, (name, K, took)
+            assert took[0] == 1 and took[1] == 2 and took[4:] == [took[3], took[2], took[3], took[3]], (name, K, took)
             assert 2 <= took[2] <= took[3] <= 4, (name, K, took)
             if K <= 8192:
                 assert took[2:4] == [3, 4]
