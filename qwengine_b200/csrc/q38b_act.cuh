@@ -245,10 +245,11 @@ static __global__ void __launch_bounds__(BF16_THREADS) gemv_bf16_kernel(const ui
 // One CTA per row: the whole result row is formed in shared memory first (2 n bytes), then copied over the row's start,
 // so no read of G can see a half written earlier.  n, ld multiples of 8; 2 n bytes of shared memory.
 // Bound by memory (10 bytes a value): 512 threads with four 16-byte loads each in flight; with 256 threads and 8-byte loads
-// 1024 x 17408 took 56 us, now 36 us (5.0 TB/s).
-constexpr int SWIGLU_ROWS_THREADS = 512;
-template <bool BF16>
-static __global__ void __launch_bounds__(SWIGLU_ROWS_THREADS, 3) swiglu_rows_inplace_kernel(float* G, const float* __restrict__ U, int n, long long ld) {
+// 1024 x 17408 took 56 us, now 35 us (5.1 TB/s).  Rows of less than 2048 values take fewer threads (512 threads leave warps
+// with nothing to load: 2500 x 512 8.6 us, with 128 threads 4.6 us; 2500 x 1024 10.5 and, with 256, 7.7 us).
+inline int swiglu_rows_threads(int n) { return n >= 2048 ? 512 : n >= 1024 ? 256 : 128; }
+template <bool BF16, int SWIGLU_ROWS_THREADS>
+static __global__ void __launch_bounds__(SWIGLU_ROWS_THREADS, 1536 / SWIGLU_ROWS_THREADS) swiglu_rows_inplace_kernel(float* G, const float* __restrict__ U, int n, long long ld) {
     extern __shared__ __align__(16) uint8_t row_smem[];
     float* g = G + (size_t)blockIdx.x * ld;
     const float* u = U + (size_t)blockIdx.x * ld;

@@ -712,15 +712,14 @@ int q38b_swiglu_rows_inplace(q38b_ctx* ctx, float* G, const float* U, int B, int
     const int smem = 2 * n;
     if (smem > ctx->smem_optin) return Q38B_ERR_NOMEM;
     cudaStream_t st = (cudaStream_t)stream;
-    if (out_kind == Q38B_OUT_BF16) {
-        const int rc = ensure_kernel_smem(ctx, (const void*)swiglu_rows_inplace_kernel<true>, ctx->smem_optin, false);
-        if (rc != Q38B_OK) return rc;
-        swiglu_rows_inplace_kernel<true><<<(unsigned)B, SWIGLU_ROWS_THREADS, smem, st>>>(G, U, n, ld);
-    } else {
-        const int rc = ensure_kernel_smem(ctx, (const void*)swiglu_rows_inplace_kernel<false>, ctx->smem_optin, false);
-        if (rc != Q38B_OK) return rc;
-        swiglu_rows_inplace_kernel<false><<<(unsigned)B, SWIGLU_ROWS_THREADS, smem, st>>>(G, U, n, ld);
-    }
+    const int threads = swiglu_rows_threads(n);
+    const bool bf = out_kind == Q38B_OUT_BF16;
+    auto kern = threads == 512 ? (bf ? swiglu_rows_inplace_kernel<true, 512> : swiglu_rows_inplace_kernel<false, 512>)
+              : threads == 256 ? (bf ? swiglu_rows_inplace_kernel<true, 256> : swiglu_rows_inplace_kernel<false, 256>)
+                               : (bf ? swiglu_rows_inplace_kernel<true, 128> : swiglu_rows_inplace_kernel<false, 128>);
+    const int rc = ensure_kernel_smem(ctx, (const void*)kern, ctx->smem_optin, false);
+    if (rc != Q38B_OK) return rc;
+    kern<<<(unsigned)B, (unsigned)threads, smem, st>>>(G, U, n, ld);
     Q38B_CUDA(ctx, cudaGetLastError());
     return Q38B_OK;
 }
