@@ -191,7 +191,10 @@ int q38b_dequant_rows(q38b_ctx* ctx, uint32_t type, const void* W_dev, size_t ro
  * What the tensor core multiplies, per format: Q8_0, IQ3_XXS, IQ3_S, IQ4_XS: the exact dequantize_row_ref value
  * (src/quant/quant_ref.cpp:323-351) rounded once to bf16; Q4_K, Q5_K, Q6_K: scale (d * sc) and minimum (dmin * m) are
  * rounded to bf16 first and applied to the exact integer by one bf16 fused multiply-add, so a weight may differ from
- * the rounded exact value by 2^-8 of its magnitude (outputs stay within 4e-3 of sum |w x|; the path's bound is 1e-2). */
+ * the rounded exact value by 2^-8 of its magnitude (outputs stay within 4e-3 of sum |w x|; the path's bound is 1e-2).
+ * The fp32 sum over K is one accumulation, or up to eight partial ones added in a fixed order: how many depends on B, M, K
+ * and the device's SM count.  The same call gives the same bits on the same device; the same token in a chunk of another
+ * length, or a row shard in place of the whole matrix, may differ in the last bits (about 1.5e-5 relative). */
 int q38b_gemm_prefill(q38b_ctx* ctx, uint32_t type, const void* W_dev, size_t row_bytes, int K, int M, const void* X_dev,
                       long long ldx, int B, float* Y_dev, long long ldy, int accumulate, void* stream);
 
@@ -268,9 +271,10 @@ int q38b_pass_run_host(q38b_pass* pass, int nb, int in_f32, const float* x_host,
 long long q38b_pass_weight_bytes(const q38b_pass* pass);
 /* Kernels one single-column run launches on this rank (after merging, see q38b_pass_set_merge). */
 int q38b_pass_kernel_count(const q38b_pass* pass);
-/* Single-column runs on one GPU merge steps by default: matvecs of one format and shape class that read the same
- * column share a launch (q38b_gemv_group), and a quantize step whose output only feeds the matvecs right after it is
- * folded into them.  Results are bit-identical either way; enabled = 0 replays one kernel per recorded step. */
+/* Runs merge steps by default: matvecs of one format and shape class that read the same columns share a launch, and a
+ * quantize step whose output only feeds the matvecs right after it is folded into them (not where one of them writes over
+ * its source, nor, with several columns, where the source buffer's length is no multiple of 4).  Results are bit-identical
+ * either way; enabled = 0 replays one kernel per recorded step. */
 int q38b_pass_set_merge(q38b_pass* pass, int enabled);
 /* ------------------------------------------------------------------------------------------------------------
  * GGUF files -> planner.  Replaces, for this path, the reference's GGUF v3 parser and split upload

@@ -1,4 +1,4 @@
-// q38b_act.cuh -- activation-side kernels (Q8_K quantizer, SwiGLU) and the exact row dequantizer.
+// q38b_act.cuh -- activation-side kernels: the quantizers, SwiGLU, residual add + RMSNorm, the bf16 matvec.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>

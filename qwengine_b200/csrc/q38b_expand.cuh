@@ -52,7 +52,7 @@ __device__ __forceinline__ void fill_grid_table(uint32_t* tab, const uint32_t* s
     }
 }
 
-// N words from a 2-byte aligned address (aligned loads and funnel shifts; up to two bytes past the last word are read)
+// N words from a 2-byte aligned address (aligned loads and funnel shifts; up to four bytes past the last word are read)
 template <int N>
 __device__ __forceinline__ void words_a2(const uint8_t* p, uint32_t (&w)[N]) {
     const uint32_t mis = (uint32_t)(uintptr_t)p & 2u;

@@ -64,7 +64,7 @@ struct Gemv1Args {
     int stage_bytes;
     int n_tilebuf;
     int cb_rep_log2;
-    int off_actd, off_actq, off_cb, off_sgn, off_red, off_stage;   // off_sgn: IQ3_XXS sign-mask table (KSIGN_TABLE_BYTES)
+    int off_actd, off_actq, off_cb, off_sgn, off_red, off_stage;   // off_sgn: sign-mask table of IQ3_XXS and the expanded IQ2_XXS / IQ2_XS (KSIGN_TABLE_BYTES)
 };
 
 // One block of the slice for every row pass of a row-group tile (B is a template argument: the alignment of the block's
@@ -95,9 +95,10 @@ constexpr int RG_STATIC_BYTES = 4 * (RG_CB_WORDS + RG_SGN_WORDS);
 // RG: the row-group mapping of q38b_decode1.cuh (IQ3_XXS, rows 8 bytes aligned): lane = (row of a group of four,
 // sub-block), tables in static shared memory, activations staged in the layout of actr_pos.
 // A32: the column is given in the reference GPU path's per-32 format (ActQ8: xq = int8 values, xd32 = one scale per 32).
-// OCC: CTAs per SM the kernel is built for: 1 (NWARPS = 24 consumer warps, 20 for row groups, all of the SM's shared
-// memory: one set of tables and one quantized column per SM, deeper rings, larger tiles; the default plan) or 2 (eight
-// consumer warps and half the shared memory each, for shapes whose one-CTA plan does not fit).
+// OCC: CTAs per SM the kernel is built for: 1 (NWARPS = 24 consumer warps, 20 for row groups, 15 or 11 for several columns,
+// all of the SM's shared memory: one set of tables and one quantized column per SM, deeper rings, larger tiles; the default
+// plan) or 2 (eight consumer warps and half the shared memory each, for shapes whose one-CTA plan does not fit and the
+// single per-32 columns that act_q8_one_cta names).
 // NC: columns at most (1 or 4).
 // XT: IQ2 / IQ1 with expanded grid tables (GranX), which want an SM's whole shared memory; without them the 16-bit codes.
 template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC, int NC = 1, bool XT = false>
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     const TablesR tabs{sp_from(rg_cb), sp_from(rg_sgn), 4u * (uint32_t)lane};
     const SP actq_sp = sp_from(actq), actd_sp = sp_from(actd);
     const SP stage0_sp = sp_from(smem + a.off_stage);
-    float* red = (float*)(smem + a.off_red);         // [n_tilebuf][n_slices][8]
+    float* red = (float*)(smem + a.off_red);         // [n_tilebuf][n_slices][NC][rows]
 
     constexpr int LPR = RG ? 8 : Gran<FMT>::LANES_PER_ROW;   // 32, or 16 when two rows share a warp pass; 8: row groups
     constexpr int PASSES = G1_ROWS * LPR / 32;       // row passes per stage

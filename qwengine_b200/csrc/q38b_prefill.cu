@@ -15,7 +15,7 @@
 // Where row tiles and token tiles alone leave SMs idle, the CTAs of a cluster share a tile's K: each multiplies a range
 // of super-blocks and the partial sums meet through distributed shared memory, added in rank order.
 // Measured on B200, 17408 x 5120 IQ3_XXS / 5120 x 17408 IQ4_XS with 1024 tokens: 211 / 286 us -> 161 / 194 us; 77 tokens of a
-// whole Q4_K / Q6_K layer 698 -> 190 us.  Up to about 250 tokens the expanders set the pace (issue slots 66 % busy, the
+// whole Q4_K / Q6_K layer 698 -> 199 us.  Up to about 250 tokens the expanders set the pace (issue slots 66 % busy, the
 // shared-memory pipe 63-70 %), from 500 the tensor core and its shared-memory traffic do (tensor pipe 69 % busy).
 // All mbarrier waits are bounded; tensor memory is released before the kernel returns, also after a timeout.
 #include <cuda.h>

@@ -1,5 +1,5 @@
 """The reference's other six matvec formats (IQ2_XXS, IQ2_XS, IQ2_S, IQ1_S, IQ1_M, Q2_K) on the GPU: exact dequantizer,
-one-column matvec (and several columns, run one after the other), per-32 activations, grouped launches and the prefill
+one-column matvec (and several columns, up to four a launch), per-32 activations, grouped launches and the prefill
 GEMM, against the CPU oracle, which is bit-identical to the compiled reference for these formats (tests/test_oracle.py)."""
 import numpy as np
 import pytest
