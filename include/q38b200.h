@@ -7,7 +7,7 @@
  *   - `type` is the ggml type id the reference's QuantFormat enum carries verbatim
  *     (include/q38rt/q38rt_types.h:36-67): Q8_0 = 8, Q2_K = 10, Q4_K = 12, Q5_K = 13, Q6_K = 14, IQ2_XXS = 16,
  *     IQ2_XS = 17, IQ3_XXS = 18, IQ1_S = 19, IQ3_S = 21, IQ2_S = 22, IQ4_XS = 23, IQ1_M = 29 (the last six of the
- *     list: one-column kernel, exact dequantizer and prefill GEMM; several columns run in launches of up to four);
+ *     list: one-column kernel, exact dequantizer and prefill GEMM; several columns share a launch);
  *   - weights are row-major GGUF blocks exactly as in the file, `row_bytes` apart (src/cuda/gemv.cuh:26-29);
  *     M counts output rows, K the row length (a multiple of 256);
  *   - output column c of a multi-column call is y + c * y_ld (src/cuda/gemv.cuh:31-34);
@@ -122,7 +122,7 @@ int q38b_quantize_act_q8(q38b_ctx* ctx, const float* x_dev, int K, int n_rows, i
  * y_dev[c * y_ld + r] (+)= W[r,:] . x_c for c < nb, where x_c is the per-32 quantized column at q_dev + c * act_ld with
  * its scales at d_dev + c * act_ld / 32 (act_ld a multiple of 32, >= K).  The integer sums per 32 weights are exact and
  * each is scaled by its own activation scale.  Every column has the one-column kernel's arithmetic, so column c equals
- * the nb = 1 call on that column bit for bit (the promise of src/cuda/gemv.cuh:31-34); up to four columns share a launch
+ * the nb = 1 call on that column bit for bit (the promise of src/cuda/gemv.cuh:31-34); the columns share a launch
  * and the decoding of the weights (three or two on rows so long that four do not fit shared memory, e.g. Q8_0 from
  * K = 10496, Q6_K and IQ2_XS at K = 17408). */
 int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W_dev, size_t row_bytes, int K, int M, const int8_t* q_dev,

@@ -57,6 +57,66 @@ __device__ __forceinline__ void q8k_block_core(const float (&v)[8], uint32_t& w0
     d = __fdiv_rn(1.0f, iscale);
 }
 
+// The same for NB blocks at a time (no sums), where every CTA of a several-column matvec forms all its columns' blocks and
+// instructions count: the two divisions of each block are made by one lane per block at the same time, and where the largest
+// magnitude is in [2^-100, 2^100] a product is rounded by adding 1.5 x 2^23, whose low byte then is the int8 value (|iscale * x|
+// <= 127 (1 + 2^-23) rounds to at most 127), instead of a conversion on the quarter-rate unit (a block's eight took it 64
+// clocks).  All other blocks (zeros, tiny, huge, infinite, NaN) are converted, out of line.  Seven columns of 5120 in the
+// prologue of the matvec: 10,300 -> 6,800 clocks from the columns' arrival to the first weight.  (One column has one block a warp:
+// there the longer code costs more than it saves, 27B-shaped pass 3810 -> 3850 us.)
+static __device__ __noinline__ uint2 q8k_convert(float4 a, float4 b, float iscale) {
+    const float x[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    int q[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) q[e] = __float2int_rn(__fmul_rn(iscale, x[e]));   // >= -127; the pack clamps at +127
+    return make_uint2(pack_s8x4(q[0], q[1], q[2], q[3]), pack_s8x4(q[4], q[5], q[6], q[7]));
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {   // NaN if any is
+    float r;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+template <int NB>
+__device__ __forceinline__ void q8k_blocks_core(const float (&v)[NB][8], uint32_t (&w0)[NB], uint32_t (&w1)[NB], float (&d)[NB]) {
+    const int lane = threadIdx.x & 31;
+    float mine = 1.0f;            // the leading element of block `lane`
+    uint32_t tops[NB];
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        const float (&x)[8] = v[b];
+        // Magnitudes compare like their bit patterns, so the block maximum is an integer maximum: one REDUX over the warp.
+        const float lane_top = max3_nan(max3_nan(fabsf(x[0]), fabsf(x[1]), fabsf(x[2])), max3_nan(fabsf(x[3]), fabsf(x[4]), fabsf(x[5])), max3_nan(fabsf(x[6]), fabsf(x[7]), 0.0f));
+        tops[b] = __reduce_max_sync(0xffffffffu, __float_as_uint(lane_top) & 0x7FFFFFFFu);
+        // First occurrence: the lowest lane that holds the maximum (ballot + find-first-set), there its first such element
+        const float top = __uint_as_float(tops[b]);
+        float lead = top;
+#pragma unroll
+        for (int e = 7; e >= 0; e--) lead = fabsf(x[e]) == top ? x[e] : lead;
+        const int owner = __ffs((int)__ballot_sync(0xffffffffu, lane_top == top)) - 1;
+        lead = __shfl_sync(0xffffffffu, lead, owner & 31);
+        if (lane == b) mine = lead;
+    }
+    const float my_iscale = __fdiv_rn(-127.0f, mine), my_d = __fdiv_rn(1.0f, my_iscale);
+#pragma unroll
+    for (int b = 0; b < NB; b++) {
+        const float iscale = __shfl_sync(0xffffffffu, my_iscale, b);
+        d[b] = __shfl_sync(0xffffffffu, my_d, b);
+        if (tops[b] - 0x0D800000u <= 0x71800000u - 0x0D800000u) {   // 2^-100 .. 2^100
+            uint32_t u[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) u[e] = __float_as_uint(__fadd_rn(__fmul_rn(iscale, v[b][e]), 12582912.0f));
+            w0[b] = prmt(prmt(u[0], u[1], 0x0040u), prmt(u[2], u[3], 0x0040u), 0x5410u);
+            w1[b] = prmt(prmt(u[4], u[5], 0x0040u), prmt(u[6], u[7], 0x0040u), 0x5410u);
+        } else if (tops[b] == 0u) {
+            w0[b] = w1[b] = 0u;
+            d[b] = 0.0f;
+        } else {
+            const uint2 w = q8k_convert(make_float4(v[b][0], v[b][1], v[b][2], v[b][3]), make_float4(v[b][4], v[b][5], v[b][6], v[b][7]), iscale);
+            w0[b] = w.x;
+            w1[b] = w.y;
+        }
+    }
+}
 // The block as ggml lays it out (float d | int8 qs[256] | int16 bsums[16], 292 bytes, 4-byte aligned) from the core's
 // outputs: lane l owns qs[8l .. 8l+7]; a bsum covers 16 values, i.e. a pair of lanes.
 __device__ __forceinline__ void q8k_block_from_regs(const float (&v)[8], uint8_t* blk) {
@@ -74,6 +134,7 @@ __device__ __forceinline__ void q8k_block_from_regs(const float (&v)[8], uint8_t
     if (lane == 0) words[0] = __float_as_uint(d);
 }
 
+constexpr int Q8K_BYTES = 292;   // float d | int8 qs[256] | int16 bsums[16]  (src/quant/quant_formats.h:95)
 constexpr int ACT_WARPS = 8;
 
 // One warp quantizes 256 floats at `src` (lane l holds elements 8l..8l+7) into the Q8_K block at `blk`.

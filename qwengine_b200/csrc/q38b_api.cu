@@ -10,7 +10,6 @@
 #include "../../include/q38b200.h"
 #include "q38b_act.cuh"
 #include "q38b_internal.h"
-#include "q38b_gemv.cuh"
 #include "q38b_topk.cuh"
 #include "q38b_gemv1.cuh"
 
@@ -28,13 +27,6 @@ const uint32_t* q38b_grid_source(const q38b_ctx* ctx, uint32_t type) {
     }
 }
 
-namespace {
-
-constexpr int NGROUPS = 2;
-constexpr int GEMV_WHOLE_ROW_K = 8192;          // longer rows run as K-parts (measured on B200: parts on K = 5120 / 6144 cost more per item than they even out)
-constexpr long long GEMV_PART_ITEMS = 131072;   // (tile, K-part) sums the scratch area of the multi-column kernel holds: 64 MB
-constexpr int GEMV_THREADS = 32 * (1 + NGROUPS * GROUP_WARPS);
-
 #define Q38B_CUDA(ctx, call)                                   \
     do {                                                       \
         cudaError_t e_ = (call);                               \
@@ -44,11 +36,9 @@ constexpr int GEMV_THREADS = 32 * (1 + NGROUPS * GROUP_WARPS);
         }                                                      \
     } while (0)
 
-int align_up(int v, int a) { return (v + a - 1) / a * a; }
-
 // Opt-in shared-memory size of a kernel, set once per context (= per device) and kernel; the record lives in the
 // context, so two contexts on two devices never disturb each other.
-int ensure_kernel_smem(q38b_ctx* ctx, const void* kern, int dyn_smem_bytes, bool max_carveout) {
+int q38b_ensure_kernel_smem(q38b_ctx* ctx, const void* kern, int dyn_smem_bytes, bool max_carveout) {
     for (int i = 0; i < ctx->n_configured; i++)
         if (ctx->configured[i] == kern) return Q38B_OK;
     Q38B_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_smem_bytes));
@@ -56,6 +46,12 @@ int ensure_kernel_smem(q38b_ctx* ctx, const void* kern, int dyn_smem_bytes, bool
     if (ctx->n_configured < (int)(sizeof(ctx->configured) / sizeof(ctx->configured[0]))) ctx->configured[ctx->n_configured++] = kern;
     return Q38B_OK;
 }
+
+namespace {
+
+constexpr long long GEMV_PART_ITEMS = 131072;   // (tile, K-part) sums the scratch area of the several-column kernel holds: 64 MB
+
+int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
 bool known_format(uint32_t t) {
     switch (t) {
@@ -73,104 +69,6 @@ int format_alignment(uint32_t t) {
         case T_Q2_K: return 4;
         default: return 2;
     }
-}
-
-// 4-super-block units per K-part: as long as two parts of activations for 8 columns and three stages of 16 rows fit
-static int gemv_units_per_part(uint32_t type) { return type == T_Q8_0 ? 2 : (type == T_Q6_K || type == T_Q5_K) ? 3 : 4; }
-
-struct Plan {
-    GemvArgs a;
-    int grid;
-    int smem;
-};
-
-// Carves the 227 KB of shared memory of one CTA: barriers | activation scales | activations | codebook |
-// reduction buffers | NGROUPS rings of n_stages stages of 16 row slots.
-int plan_gemv(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, int nb, Plan* p) {
-    if (one_column_only((int)type)) return Q38B_ERR_UNSUPPORTED;   // no fragment builders for these formats
-    const int bb = block_bytes((int)type);
-    const int nsb = K / 256;
-    int cb_entries = type == T_IQ3_XXS ? 256 : type == T_IQ3_S ? 512 : 0;
-    const int budget = ctx->smem_optin - 128;   // base is aligned up to 128 inside the kernel
-    GemvArgs& a = p->a;
-    a.nsb = nsb;
-    a.n_tiles = 0;
-    for (int i = 0; i < GEMV_MAX_MATS; i++) {
-        a.tile_start[i] = a.n_tiles;
-        if (i < n_mats) a.n_tiles += (Ms[i] + TILE_ROWS - 1) / TILE_ROWS;
-    }
-    for (int i = n_mats; i < GEMV_MAX_MATS; i++) a.tile_start[i] = a.n_tiles;
-    // K-parts for rows longer than 8192: up to 16 super-blocks each (12 for Q5_K / Q6_K, 8 for Q8_0: larger blocks),
-    // boundaries at multiples of 4 super-blocks.  A rule of K and the format alone, so that a sum is built from the same pieces whatever the
-    // column count, the row count or the GPU count.
-    const int n_units = (nsb + 3) / 4;
-    const int units_per_part = gemv_units_per_part(type);
-    a.n_parts = K <= GEMV_WHOLE_ROW_K ? 1 : (n_units + units_per_part - 1) / units_per_part;
-    if (a.n_parts > GEMV_MAX_PARTS) a.n_parts = GEMV_MAX_PARTS;   // longer parts; the plan fails below if they do not fit
-    int max_part = 0;
-    for (int q = 0; q <= a.n_parts; q++) a.part_sb0[q] = std::min(nsb, 4 * (int)((long long)n_units * q / a.n_parts));
-    for (int q = 0; q < a.n_parts; q++) max_part = std::max(max_part, a.part_sb0[q + 1] - a.part_sb0[q]);
-    if (a.n_parts > 1 && (long long)a.n_tiles * a.n_parts > ctx->part_items) return Q38B_ERR_NOMEM;   // the scratch area's size
-    // a CTA's range of (part, tile) items touches at most two neighbouring parts: it stages their activations only
-    a.act_sb = a.n_parts == 1 ? nsb : std::min(nsb, 2 * max_part);
-    a.off_actd = 256;
-    a.off_actq = a.off_actd + align_up(a.act_sb * 32, 16);
-    a.off_cb = a.off_actq + align_up(nb * a.act_sb * 256, 128);
-    // rows of a group land 16 bytes (32 for the formats read with 64-bit loads) further round the 32 banks
-    const int bank_skew = (type == T_Q4_K || type == T_Q5_K) ? 32 : 16;
-    for (int rep_log2 = cb_entries ? 5 : 0; rep_log2 >= 0; rep_log2 -= (rep_log2 == 5 ? 2 : 3)) {
-        a.cb_rep_log2 = rep_log2;
-        a.off_red = a.off_cb + align_up(cb_entries * 4 << rep_log2, 128);
-        a.off_stage = a.off_red + NGROUPS * 2 * GROUP_THREADS * 16;
-        const int avail = budget - a.off_stage;
-        // K-chunk sizes to try: the whole row (or part), then -- whole rows only -- fewer super-blocks, multiples of 4
-        // first (8 half super-blocks per 4 keep the 8 warps of a group evenly loaded)
-        for (int pass = 0; pass < 2; pass++)
-            for (int cs = max_part; cs >= (a.n_parts == 1 ? 1 : max_part); cs--) {
-                const bool even = cs == max_part || cs % 4 == 0;
-                if (even != (pass == 0)) continue;
-                int slot = align_up(cs * bb + 32, 16);
-                while (slot % 128 != bank_skew) slot += 16;
-                const int stage = TILE_ROWS * slot;
-                // one ring for both groups: each reads one stage while at least one more is being filled
-                const int stages = avail / stage;
-                if (stages < 3 && !(stages == 2 && cs == 1)) continue;
-                a.chunk_sb = cs;
-                a.n_chunks = (max_part + cs - 1) / cs;
-                a.n_stages = std::min(stages, MAX_STAGES);
-                a.slot_stride = slot;
-                a.stage_bytes = stage;
-                p->smem = a.off_stage + a.n_stages * stage + 128;
-                const long long items = (long long)a.n_tiles * a.n_parts;
-                p->grid = (int)std::max<long long>(1, std::min<long long>(ctx->sm_count, (items + NGROUPS - 1) / NGROUPS));
-                return Q38B_OK;
-            }
-        if (!cb_entries) break;
-    }
-    return Q38B_ERR_NOMEM;
-}
-
-template <int FMT>
-int launch_gemv(q38b_ctx* ctx, const Plan& p, cudaStream_t st) {
-    auto kern = p.a.n_parts > 1 ? gemv_kernel<FMT, NGROUPS, true> : gemv_kernel<FMT, NGROUPS, false>;
-    const int rc = ensure_kernel_smem(ctx, (const void*)kern, ctx->smem_optin, false);
-    if (rc != Q38B_OK) return rc;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)p.grid);
-    cfg.blockDim = dim3(GEMV_THREADS + (p.a.n_parts > 1 ? 32 : 0));   // K-parts: one more warp, which adds the parts up
-    cfg.dynamicSmemBytes = (size_t)p.smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = ctx->pdl ? 1 : 0;
-    GemvArgs a = p.a;
-    a.parts = ctx->d_parts;
-    a.part_count = ctx->d_part_count;
-    Q38B_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, a));
-    return Q38B_OK;
 }
 
 constexpr int G1_WARPS = 8;                  // consumer warps of a CTA when two CTAs share an SM
@@ -307,7 +205,7 @@ int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_m
     return Q38B_ERR_NOMEM;
 }
 
-// Two to four columns in one launch: one CTA per SM, tiles of eight rows.
+// Two to four columns of Q6_K in one launch: one CTA per SM, tiles of eight rows.
 int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nc, Plan1* p) {
     memset(p, 0, sizeof(*p));
     return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p) : Q38B_ERR_NOMEM;
@@ -339,11 +237,8 @@ bool act_q8_one_cta(const q38b_ctx* ctx, uint32_t type, const Plan1& p) {
     }
 }
 
-// How many of `left` columns the next launch takes, with its plan in *p when that is more than one: the most that fit shared
-// memory (four; three or two on long rows of some formats).  A column alone has a kernel of its own that decodes with more
-// warps, so that four columns of which three fit are faster as three and one (5120 x 12288 IQ2_XS: 37.1 us) than as two
-// and two (40.5 us).
-// Six are two threes (17408 x 5120 IQ2_XS: 50.6 us, as four and two 51.3 us).
+// How many of `left` columns the next launch of the one-column kernel takes (Q6_K with per-32 activations), with its plan in *p
+// when that is more than one: the most that fit shared memory, at most four; six are two threes.
 int next_cols(const q38b_ctx* ctx, uint32_t type, int K, int M, size_t row_bytes, int left, Plan1* p) {
     int n = left == 6 ? 3 : std::min(G1_COLS, left);
     while (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, p) != Q38B_OK) n--;
@@ -354,7 +249,7 @@ template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2, int NC = 1,
 int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     constexpr int WARPS = NC > 1 ? g1_warps_cols(FMT) : OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
     auto kern = gemv1_kernel<FMT, WARPS, ROWS, RG, A32, OCC, NC, XT>;
-    const int rc = ensure_kernel_smem(ctx, (const void*)kern, (OCC == 1 ? ctx->smem_optin : G1_SMEM_BUDGET) - (RG ? RG_STATIC_BYTES : 0), true);
+    const int rc = q38b_ensure_kernel_smem(ctx, (const void*)kern, (OCC == 1 ? ctx->smem_optin : G1_SMEM_BUDGET) - (RG ? RG_STATIC_BYTES : 0), true);
     if (rc != Q38B_OK) return rc;
     if (ctx->check_occupancy) {   // test hook: count launches whose CTAs would not be resident as often as planned
         int per_sm = 0;
@@ -381,8 +276,9 @@ template <int FMT>
 int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     constexpr bool X = gridx_copies(FMT) > 0;
     if (p.nc > 1) {
-        if (p.a.xd32) return launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS, X>(ctx, p, st);
-        if constexpr (one_column_only(FMT)) return launch_gemv1_rows<FMT, 8, false, false, 1, G1_COLS, X>(ctx, p, st);
+        if constexpr (FMT == T_Q6_K) {
+            if (p.a.xd32) return launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS>(ctx, p, st);
+        }
         return Q38B_ERR_ARG;
     }
     if (p.a.xd32) {   // per-32 activations: lane-per-granule mapping only
@@ -717,7 +613,7 @@ int q38b_swiglu_rows_inplace(q38b_ctx* ctx, float* G, const float* U, int B, int
     auto kern = threads == 512 ? (bf ? swiglu_rows_inplace_kernel<true, 512> : swiglu_rows_inplace_kernel<false, 512>)
               : threads == 256 ? (bf ? swiglu_rows_inplace_kernel<true, 256> : swiglu_rows_inplace_kernel<false, 256>)
                                : (bf ? swiglu_rows_inplace_kernel<true, 128> : swiglu_rows_inplace_kernel<false, 128>);
-    const int rc = ensure_kernel_smem(ctx, (const void*)kern, ctx->smem_optin, false);
+    const int rc = q38b_ensure_kernel_smem(ctx, (const void*)kern, ctx->smem_optin, false);
     if (rc != Q38B_OK) return rc;
     kern<<<(unsigned)B, (unsigned)threads, smem, st>>>(G, U, n, ld);
     Q38B_CUDA(ctx, cudaGetLastError());
@@ -727,6 +623,27 @@ int q38b_swiglu_rows_inplace(q38b_ctx* ctx, float* G, const float* U, int B, int
 int q38b_gemv_q8k(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* q8k,
                   long long q8k_stride, int nb, float* y, long long y_ld, int accumulate, void* stream) {
     return q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, q8k, q8k_stride, nb, y, y_ld, accumulate, nullptr, 0, stream);
+}
+
+// one matrix, columns of Q8_K blocks
+static ColsCall cols_call(uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* q8k, long long q8k_stride, int nb, float* y, long long y_ld,
+                          int accumulate, float* const* y_peers, int n_peers) {
+    ColsCall c;
+    c.type = type;
+    c.row_bytes = row_bytes;
+    c.K = K;
+    c.nb = nb;
+    c.n_mats = 1;
+    c.W[0] = W;
+    c.M[0] = M;
+    c.y[0] = y;
+    c.y_ld[0] = y_ld;
+    c.xq = q8k;
+    c.xq_ld = q8k_stride * Q8K_BYTES;
+    c.accumulate = accumulate ? 1 : 0;
+    c.y_peers = y_peers;
+    c.n_peers = n_peers;
+    return c;
 }
 
 int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* q8k,
@@ -742,34 +659,14 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
     if (((uintptr_t)W & 15) || (row_bytes % al) || ((uintptr_t)q8k & 3) || ((uintptr_t)y & 3)) return Q38B_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
     if (one_column_only((int)type) && nb > 1) {
-        // formats without mma fragments: launches of up to four columns of the one-column kernel's arithmetic (every column is the nb = 1 result)
+        // launches of as many columns as fit; every column is the nb = 1 result
         for (int c = 0; c < nb;) {
-            Plan1 p;
-            const int n = next_cols(ctx, type, K, M, row_bytes, nb - c, &p);
+            const int n = std::max(1, q38b_cols_fit(ctx, type, K, &M, 1, row_bytes, nb - c, false));
             const uint8_t* xq = (const uint8_t*)q8k + (size_t)c * q8k_stride * Q8K_BYTES;
             float* peers_c[7];
             for (int i = 0; i < n_peers; i++) peers_c[i] = y_peers[i] + (size_t)c * y_ld;
-            int rc;
-            if (n == 1) {
-                rc = q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, xq, q8k_stride, 1, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers, stream);
-            } else {
-                Gemv1Args& g = p.a;
-                g.W = (const uint8_t*)W;
-                g.row_bytes = (long long)row_bytes;
-                g.xq = xq;
-                g.xq_ld = q8k_stride * Q8K_BYTES;
-                g.y = y + (size_t)c * y_ld;
-                g.y_ld = y_ld;
-                g.n_peers = n_peers;
-                for (int i = 0; i < n_peers; i++) g.y_peer[i] = peers_c[i];
-                g.static_weights = ctx->static_weights;
-                g.status = ctx->d_status;
-                g.codebook = q38b_grid_source(ctx, type);
-                g.K = K;
-                g.M = M;
-                g.accumulate = accumulate ? 1 : 0;
-                rc = dispatch_gemv1(ctx, type, p, st);
-            }
+            const int rc = n == 1 ? q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, xq, q8k_stride, 1, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers, stream)
+                                  : q38b_cols_launch(ctx, cols_call(type, W, row_bytes, K, M, xq, q8k_stride, n, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers), stream);
             if (rc != Q38B_OK) return rc;
             c += n;
         }
@@ -798,64 +695,27 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
             return dispatch_gemv1(ctx, type, p1, st);
         }
     }
-    {   // more (tile, K-part) sums than the scratch area holds: one launch per block of rows
-        const int n_units = (K / 256 + 3) / 4, upp = gemv_units_per_part(type);
-        const int n_parts = K <= GEMV_WHOLE_ROW_K ? 1 : std::min(GEMV_MAX_PARTS, (n_units + upp - 1) / upp);
-        const long long rows_per_launch = ctx->part_items / n_parts * TILE_ROWS;
-        if (n_parts > 1 && M > rows_per_launch) {
-            for (long long m0 = 0; m0 < M; m0 += rows_per_launch) {
-                const int m = (int)std::min<long long>(rows_per_launch, M - m0);
-                float* peers_at[7];
-                for (int i = 0; i < n_peers; i++) peers_at[i] = y_peers[i] + m0;
-                const int rc = q38b_gemv_q8k_scatter(ctx, type, (const uint8_t*)W + (size_t)m0 * row_bytes, row_bytes, K, m, q8k, q8k_stride, nb, y + m0,
-                                                     y_ld, accumulate, n_peers ? peers_at : nullptr, n_peers, stream);
-                if (rc != Q38B_OK) return rc;
-            }
-            return Q38B_OK;
+    // more (tile, K-part) sums than the scratch area holds: one launch per block of rows
+    const long long rows_per_launch = q38b_cols_max_rows(ctx, type, K);
+    if (rows_per_launch > 0 && M > rows_per_launch) {
+        for (long long m0 = 0; m0 < M; m0 += rows_per_launch) {
+            const int m = (int)std::min<long long>(rows_per_launch, M - m0);
+            float* peers_at[7];
+            for (int i = 0; i < n_peers; i++) peers_at[i] = y_peers[i] + m0;
+            const int rc = q38b_gemv_q8k_scatter(ctx, type, (const uint8_t*)W + (size_t)m0 * row_bytes, row_bytes, K, m, q8k, q8k_stride, nb, y + m0,
+                                                 y_ld, accumulate, n_peers ? peers_at : nullptr, n_peers, stream);
+            if (rc != Q38B_OK) return rc;
         }
+        return Q38B_OK;
     }
-    Plan p;
-    memset(&p, 0, sizeof(p));
-    int rc = plan_gemv(ctx, type, K, &M, 1, nb, &p);
-    if (rc != Q38B_OK) return rc;
-    GemvArgs& a = p.a;
-    a.W = (const uint8_t*)W;
-    a.row_bytes = (long long)row_bytes;
-    a.xq = (const uint8_t*)q8k;
-    a.x_stride = q8k_stride;
-    a.y = y;
-    a.y_ld = y_ld;
-    a.n_peers = n_peers;
-    a.static_weights = ctx->static_weights;
-    for (int i = 0; i < n_peers; i++) a.y_peer[i] = y_peers[i];
-    a.status = ctx->d_status;
-    a.codebook = q38b_grid_source(ctx, type);
-    a.K = K;
-    a.M = M;
-    a.nb = nb;
-    a.accumulate = accumulate ? 1 : 0;
-    switch (type) {
-        case T_Q8_0: return launch_gemv<T_Q8_0>(ctx, p, st);
-        case T_Q4_K: return launch_gemv<T_Q4_K>(ctx, p, st);
-        case T_Q5_K: return launch_gemv<T_Q5_K>(ctx, p, st);
-        case T_Q6_K: return launch_gemv<T_Q6_K>(ctx, p, st);
-        case T_IQ3_XXS: return launch_gemv<T_IQ3_XXS>(ctx, p, st);
-        case T_IQ3_S: return launch_gemv<T_IQ3_S>(ctx, p, st);
-        case T_IQ4_XS: return launch_gemv<T_IQ4_XS>(ctx, p, st);
-        default: return Q38B_ERR_UNSUPPORTED;
-    }
+    return q38b_cols_launch(ctx, cols_call(type, W, row_bytes, K, M, q8k, q8k_stride, nb, y, y_ld, accumulate, y_peers, n_peers), stream);
 }
 
 int q38b_gemvn_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M, int nb) {
-    if (!ctx || n_mats < 1 || n_mats > GEMV_MAX_MATS || !known_format(type) || K <= 0 || K % 256 || nb < 1 || nb > 8) return 0;
+    if (!ctx || n_mats < 1 || n_mats > G1_MAX_MATS || !known_format(type) || K <= 0 || K % 256 || nb < 1 || nb > 8) return 0;
     if (row_bytes < q38b_row_bytes(type, K)) return 0;
-    if (one_column_only((int)type)) {
-        Plan1 p1;
-        return nb > 1 && nb <= G1_COLS && plan_gemv1_cols(ctx, type, K, M, n_mats, row_bytes, nb, &p1) == Q38B_OK;
-    }
-    Plan p;
-    memset(&p, 0, sizeof(p));
-    return plan_gemv(ctx, type, K, M, n_mats, nb, &p) == Q38B_OK;
+    if (one_column_only((int)type) && nb == 1) return 0;
+    return q38b_cols_fit(ctx, type, K, M, n_mats, row_bytes, nb, false) == nb;
 }
 
 int q38b_gemvn_group(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const* W, size_t row_bytes, int K, const int* M,
@@ -866,7 +726,7 @@ int q38b_gemvn_group(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const
 int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const* W, size_t row_bytes, int K, const int* M,
                        const void* q8k, long long q8k_stride, const float* x_f32, long long x_f32_ld, int nb, float* const* y,
                        const long long* y_ld, float* const* y_peers, int n_peers, void* stream) {
-    if (!ctx || !W || !M || !y || !y_ld || (!q8k == !x_f32) || n_mats < 1 || n_mats > GEMV_MAX_MATS) return Q38B_ERR_ARG;
+    if (!ctx || !W || !M || !y || !y_ld || (!q8k == !x_f32) || n_mats < 1 || n_mats > G1_MAX_MATS) return Q38B_ERR_ARG;
     if (n_peers < 0 || n_peers > 7 || (n_peers > 0 && !y_peers)) return Q38B_ERR_ARG;   // y_peers[i * n_peers + r]: peer r's copy of matrix i's output
     if (!q38b_gemvn_group_plannable(ctx, type, n_mats, row_bytes, K, M, nb)) return Q38B_ERR_UNSUPPORTED;
     const int al = format_alignment(type);
@@ -877,71 +737,25 @@ int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* con
         if (!W[i] || !y[i] || M[i] < 1 || y_ld[i] < M[i]) return Q38B_ERR_ARG;
         if (((uintptr_t)W[i] & 15) || ((uintptr_t)y[i] & 3)) return Q38B_ERR_ALIGN;
     }
-    if (one_column_only((int)type)) {   // up to four columns (plannable says so) of the one-column kernel's arithmetic
-        Plan1 p1;
-        const int rc1 = plan_gemv1_cols(ctx, type, K, M, n_mats, row_bytes, nb, &p1);
-        if (rc1 != Q38B_OK) return rc1;
-        Gemv1Args& g = p1.a;
-        for (int i = 0; i < n_mats; i++) {
-            (i == 0 ? g.W : g.W_more[i - 1]) = (const uint8_t*)W[i];
-            (i == 0 ? g.y : g.y_more[i - 1]) = y[i];
-            (i == 0 ? g.y_ld : g.y_ld_more[i - 1]) = y_ld[i];
-            (i == 0 ? g.M : g.M_more[i - 1]) = M[i];
-            for (int pr = 0; pr < n_peers; pr++) (i == 0 ? g.y_peer[pr] : g.y_peer_more[i - 1][pr]) = y_peers[i * n_peers + pr];
-        }
-        g.row_bytes = (long long)row_bytes;
-        g.xq = (const uint8_t*)q8k;
-        g.xq_ld = q8k_stride * Q8K_BYTES;
-        g.x_f32 = x_f32;
-        g.x_f32_ld = x_f32_ld;
-        g.n_peers = n_peers;
-        g.static_weights = ctx->static_weights;
-        g.status = ctx->d_status;
-        g.codebook = q38b_grid_source(ctx, type);
-        g.K = K;
-        return dispatch_gemv1(ctx, type, p1, (cudaStream_t)stream);
+    ColsCall c;
+    c.type = type;
+    c.row_bytes = row_bytes;
+    c.K = K;
+    c.nb = nb;
+    c.n_mats = n_mats;
+    for (int i = 0; i < n_mats; i++) {
+        c.W[i] = W[i];
+        c.M[i] = M[i];
+        c.y[i] = y[i];
+        c.y_ld[i] = y_ld[i];
     }
-    Plan p;
-    memset(&p, 0, sizeof(p));
-    const int rc = plan_gemv(ctx, type, K, M, n_mats, nb, &p);
-    if (rc != Q38B_OK) return rc;
-    GemvArgs& a = p.a;
-    a.W = (const uint8_t*)W[0];
-    a.y = y[0];
-    a.y_ld = y_ld[0];
-    a.M = M[0];
-    for (int i = 1; i < n_mats; i++) {
-        a.W_more[i - 1] = (const uint8_t*)W[i];
-        a.y_more[i - 1] = y[i];
-        a.y_ld_more[i - 1] = y_ld[i];
-        a.M_more[i - 1] = M[i];
-    }
-    a.row_bytes = (long long)row_bytes;
-    a.xq = (const uint8_t*)q8k;
-    a.x_stride = q8k_stride;
-    a.x_f32 = x_f32;
-    a.x_f32_ld = x_f32_ld;
-    a.n_peers = n_peers;
-    for (int i = 0; i < n_peers; i++) a.y_peer[i] = y_peers[i];
-    for (int m = 1; m < n_mats; m++)
-        for (int i = 0; i < n_peers; i++) a.y_peer_more[m - 1][i] = y_peers[m * n_peers + i];
-    a.static_weights = ctx->static_weights;
-    a.status = ctx->d_status;
-    a.codebook = q38b_grid_source(ctx, type);
-    a.K = K;
-    a.nb = nb;
-    a.accumulate = 0;
-    cudaStream_t st = (cudaStream_t)stream;
-    switch (type) {
-        case T_Q8_0: return launch_gemv<T_Q8_0>(ctx, p, st);
-        case T_Q4_K: return launch_gemv<T_Q4_K>(ctx, p, st);
-        case T_Q5_K: return launch_gemv<T_Q5_K>(ctx, p, st);
-        case T_Q6_K: return launch_gemv<T_Q6_K>(ctx, p, st);
-        case T_IQ3_XXS: return launch_gemv<T_IQ3_XXS>(ctx, p, st);
-        case T_IQ3_S: return launch_gemv<T_IQ3_S>(ctx, p, st);
-        case T_IQ4_XS: return launch_gemv<T_IQ4_XS>(ctx, p, st);
-        default: return Q38B_ERR_UNSUPPORTED;
-    }
+    c.xq = q8k;
+    c.xq_ld = q8k_stride * Q8K_BYTES;
+    c.x_f32 = x_f32;
+    c.x_f32_ld = x_f32_ld;
+    c.y_peers = y_peers;
+    c.n_peers = n_peers;
+    return q38b_cols_launch(ctx, c, stream);
 }
 
 int q38b_gemv_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M) {
@@ -1036,14 +850,24 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     if (row_bytes < q38b_row_bytes(type, K)) return Q38B_ERR_ARG;
     const int al = format_alignment(type);
     if (((uintptr_t)W & 15) || (row_bytes % al) || ((uintptr_t)q & 3) || (act_ld & 3) || ((uintptr_t)d & 3) || ((uintptr_t)y & 3)) return Q38B_ERR_ALIGN;
-    // The one-column kernel on its lane-per-granule mapping, or launches of up to four columns of the same arithmetic: every
+    // The one-column kernel on its lane-per-granule mapping, or several columns a launch with the same arithmetic: every
     // column is the single-column result (the promise of src/cuda/gemv.cuh:31-34 of the reference).
     const int saved_rg = ctx->rowgroup;
     ctx->rowgroup = 0;
     int rc = Q38B_OK;
     for (int c = 0; c < nb && rc == Q38B_OK;) {
         Plan1 p;
-        const int n = next_cols(ctx, type, K, M, row_bytes, nb - c, &p);
+        int n = nb - c > 1 ? q38b_cols_fit(ctx, type, K, &M, 1, row_bytes, nb - c, true) : 1;
+        if (n > 1) {
+            ColsCall call = cols_call(type, W, row_bytes, K, M, q + (size_t)c * act_ld, 0, n, y + (size_t)c * y_ld, y_ld, accumulate, nullptr, 0);
+            call.xq_ld = act_ld;
+            call.xd32 = d + (size_t)c * (act_ld / 32);
+            call.xd32_ld = act_ld / 32;
+            rc = q38b_cols_launch(ctx, call, stream);
+            c += n;
+            continue;
+        }
+        if (n == 0) n = type == T_Q6_K ? next_cols(ctx, type, K, M, row_bytes, nb - c, &p) : 1;
         if (n == 1) {
             memset(&p, 0, sizeof(p));
             const bool fits_one = ctx->one_cta && type != T_Q8_0 && plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, gridx_copies((int)type) > 0, &p) == Q38B_OK;

@@ -9,10 +9,6 @@
 // Compiles for the host too (the CPU unit test runs the 32 lanes one after the other).
 #pragma once
 #include "q38b_decode.cuh"
-#if !defined(__CUDA_ARCH__)
-#include <cstdio>
-#include <cstdlib>
-#endif
 
 namespace q38b {
 
@@ -34,59 +30,6 @@ Q38B_HD int dp4a_us(uint32_t a, uint32_t b, int c) {
     for (int i = 0; i < 4; i++) c += (int)(uint8_t)(a >> (8 * i)) * (int)(int8_t)(b >> (8 * i));
     return c;
 #endif
-}
-
-Q38B_HD uint32_t funnel_r(uint32_t lo, uint32_t hi, uint32_t sh) {   // (hi:lo) >> sh, sh in 0..31
-#if defined(__CUDA_ARCH__)
-    return __funnelshift_r(lo, hi, sh);
-#else
-    return sh ? (lo >> sh) | (hi << (32 - sh)) : lo;
-#endif
-}
-
-// ---------------------------------------------------------------------------------------------------------------
-// Staged bytes are addressed through SP: on the device a 32-bit shared-space address (loads are ld.shared with
-// immediate offsets, no 64-bit pointer arithmetic and no generic-to-shared conversion per load), on the host a pointer.
-// ---------------------------------------------------------------------------------------------------------------
-#if defined(__CUDA_ARCH__)
-struct SP { uint32_t a; };
-__device__ __forceinline__ SP sp_from(const void* p) { return SP{(uint32_t)__cvta_generic_to_shared(p)}; }
-__device__ __forceinline__ uint32_t sp_low2(SP p) { return p.a & 2u; }
-__device__ __forceinline__ uint32_t sp_ld8(SP p, int o = 0) { uint32_t v; asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(p.a + o)); return v; }
-__device__ __forceinline__ int sp_ld8s(SP p, int o = 0) { int v; asm volatile("ld.shared.s8 %0, [%1];" : "=r"(v) : "r"(p.a + o)); return v; }
-__device__ __forceinline__ uint32_t sp_ld16(SP p, int o = 0) { uint32_t v; asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(p.a + o)); return v; }
-__device__ __forceinline__ uint32_t sp_ld32(SP p, int o = 0) { uint32_t v; asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(p.a + o)); return v; }
-__device__ __forceinline__ float sp_ldf(SP p, int o = 0) { float v; asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(p.a + o)); return v; }
-__device__ __forceinline__ void sp_ld64(SP p, int o, uint32_t& x, uint32_t& y) {
-    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(x), "=r"(y) : "r"(p.a + o));
-}
-__device__ __forceinline__ void sp_ld128(SP p, int o, uint32_t (&v)[4]) {
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(p.a + o));
-}
-#else
-struct SP { const uint8_t* a; };
-inline SP sp_from(const void* p) { return SP{(const uint8_t*)p}; }
-inline uint32_t sp_low2(SP p) { return (uint32_t)((uintptr_t)p.a & 2); }
-inline uint32_t sp_ld8(SP p, int o = 0) { return p.a[o]; }
-inline int sp_ld8s(SP p, int o = 0) { return (int8_t)p.a[o]; }
-// the host versions refuse what the device would fault on: an address that is not a multiple of the access size
-inline void sp_check_aligned(const uint8_t* p, int n) { if ((uintptr_t)p % (uintptr_t)n) { fprintf(stderr, "misaligned %d-byte shared load\n", n); abort(); } }
-inline uint32_t sp_ld16(SP p, int o = 0) { uint16_t v; sp_check_aligned(p.a + o, 2); memcpy(&v, p.a + o, 2); return v; }
-inline uint32_t sp_ld32(SP p, int o = 0) { uint32_t v; sp_check_aligned(p.a + o, 4); memcpy(&v, p.a + o, 4); return v; }
-inline float sp_ldf(SP p, int o = 0) { float v; sp_check_aligned(p.a + o, 4); memcpy(&v, p.a + o, 4); return v; }
-inline void sp_ld64(SP p, int o, uint32_t& x, uint32_t& y) { sp_check_aligned(p.a + o, 8); memcpy(&x, p.a + o, 4); memcpy(&y, p.a + o + 4, 4); }
-inline void sp_ld128(SP p, int o, uint32_t (&v)[4]) { sp_check_aligned(p.a + o, 16); memcpy(v, p.a + o, 16); }
-#endif
-Q38B_HD SP operator+(SP p, int o) { return SP{p.a + o}; }
-Q38B_HD SP operator-(SP p, int o) { return SP{p.a - o}; }
-
-// 8 bytes from a 2-byte aligned address: three aligned words and two funnel shifts.  `mis` = address & 2.
-Q38B_HD void sp_ld8b_a2(SP p, uint32_t mis, uint32_t& lo, uint32_t& hi) {
-    const SP w = p - (int)mis;
-    const uint32_t sh = mis * 8;
-    const uint32_t w0 = sp_ld32(w, 0), w1 = sp_ld32(w, 4), w2 = sp_ld32(w, 8);
-    lo = funnel_r(w0, w1, sh);
-    hi = funnel_r(w1, w2, sh);
 }
 
 // Codebook replicated 32 x in shared memory: entry e for lane l is the word at base + e * 128 + l * 4.
@@ -135,13 +78,26 @@ template <int NWORDS> struct ActRegs {
 // keep one scale per super-block in slot 8 * sb; per-32 activations (the reference GPU path's ActQ8,
 // src/cuda/gemv.cuh:14-21) one scale per 32 weights in slot 8 * sb + j.  A32 selects the second.
 
+// Gran<FMT>: idot = a lane's exact integer sum over its granule (Q8_K activations: the sums of a super-block's lanes are added
+// as integers and scaled once, by the factors that block_scale reads; msum: the minima's part); dot<A32> = its value as a
+// float, for per-32 activations and for Q8_0, whose scales change inside a super-block.  FACTOR: as in Unit<FMT>.
 template <int FMT> struct Gran;
+
+template <class G, int FMT>
+Q38B_HD float gran_value(SP block, float dx, int sum, int msum) {
+    float d, m;
+    G::block_scale(block, d, m);
+    return Unit<FMT>::HAS_MIN ? block_value_min(d * dx, sum, m * dx, msum) : block_value(d * dx * Unit<FMT>::FACTOR, sum);
+}
+struct ScaleAt0 {   // fp16 d in front, no minima
+    static Q38B_HD void block_scale(SP block, float& d, float& m) { d = fp16_bits_to_float(sp_ld16(block, 0)); m = 0.0f; }
+};
 
 // ---------------------------------------------------------------------------------------------------------------
 // IQ3_XXS (layout and formula: see Unit<T_IQ3_XXS>).  sum = (2s+1) * (P - 2N): P = dot of the unsigned grid bytes,
 // N = dot of the grid bytes whose sign bit is set.
 // ---------------------------------------------------------------------------------------------------------------
-template <> struct Gran<T_IQ3_XXS> {
+template <> struct Gran<T_IQ3_XXS> : ScaleAt0 {
     static constexpr int WORDS = 8, LANES_PER_ROW = 32;
     using Acts = ActRegs<WORDS>;
     template <bool A32>
@@ -151,11 +107,16 @@ template <> struct Gran<T_IQ3_XXS> {
         a.q[0] = v[0]; a.q[1] = v[1]; a.q[2] = v[2]; a.q[3] = v[3];
         sp_ld128(aq, 512 + 16 * lane, v);
         a.q[4] = v[0]; a.q[5] = v[1]; a.q[6] = v[2]; a.q[7] = v[3];
-        a.dx = sp_ldf(ad, A32 ? 4 * lane : (lane >> 3) * 32) * 0.25f;
+        a.dx = sp_ldf(ad, A32 ? 4 * lane : (lane >> 3) * 32);
     }
     template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) { return dot(row, a, cb, lane); }
     static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ3_XXS>(row + 98 * (lane >> 3), a.dx, sum, ms);
+    }
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 98 * (lane >> 3);
         const int s = lane & 7;
         const SP ip = p + (2 + 8 * s);
@@ -174,15 +135,14 @@ template <> struct Gran<T_IQ3_XXS> {
             N = dp4a_us(g0 & m_lo, a.q[2 * l], N);
             N = dp4a_us(g1 & m_hi, a.q[2 * l + 1], N);
         }
-        const int sumi = (int)(2u * (aux >> 28) + 1u) * (P - 2 * N);
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * (float)sumi;
+        return (int)(2u * (aux >> 28) + 1u) * (P - 2 * N);
     }
 };
 
 // ---------------------------------------------------------------------------------------------------------------
 // IQ3_S: 512-entry codebook, 9th index bits in qh, explicit sign bytes
 // ---------------------------------------------------------------------------------------------------------------
-template <> struct Gran<T_IQ3_S> {
+template <> struct Gran<T_IQ3_S> : ScaleAt0 {
     static constexpr int WORDS = 8, LANES_PER_ROW = 32;
     using Acts = ActRegs<WORDS>;
     template <bool A32>
@@ -195,8 +155,13 @@ template <> struct Gran<T_IQ3_S> {
         a.dx = sp_ldf(ad, A32 ? 4 * lane : (lane >> 3) * 32);
     }
     template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) { return dot(row, a, cb, lane); }
     static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ3_S>(row + 110 * (lane >> 3), a.dx, sum, ms);
+    }
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 110 * (lane >> 3);
         const int s = lane & 7;
         uint32_t iw[2];
@@ -217,15 +182,14 @@ template <> struct Gran<T_IQ3_S> {
             N = dp4a_us(g0 & m_lo, a.q[2 * l], N);
             N = dp4a_us(g1 & m_hi, a.q[2 * l + 1], N);
         }
-        const int sumi = (int)(2u * ls + 1u) * (P - 2 * N);
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * (float)sumi;
+        return (int)(2u * ls + 1u) * (P - 2 * N);
     }
 };
 
 // ---------------------------------------------------------------------------------------------------------------
 // IQ4_XS: activations staged in the order the PRMT table lookup emits the weights (act_stage_pos)
 // ---------------------------------------------------------------------------------------------------------------
-template <> struct Gran<T_IQ4_XS> {
+template <> struct Gran<T_IQ4_XS> : ScaleAt0 {
     static constexpr int WORDS = 8, LANES_PER_ROW = 32;
     using Acts = ActRegs<WORDS>;
     template <bool A32>
@@ -238,8 +202,13 @@ template <> struct Gran<T_IQ4_XS> {
         a.dx = sp_ldf(ad, A32 ? 4 * lane : (lane >> 3) * 32);
     }
     template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) { return dot(row, a, cb, lane); }
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1&, int lane) {
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ4_XS>(row + 136 * (lane >> 3), a.dx, sum, ms);
+    }
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1&, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 136 * (lane >> 3);
         const int s = lane & 7;
         uint32_t w[4];
@@ -267,7 +236,7 @@ template <> struct Gran<T_IQ4_XS> {
         const uint32_t hdr = sp_ld32(p, 0);            // fp16 d | scales_h
         const uint32_t sl = sp_ld8(p, 4 + (s >> 1));
         const int ls = (int)(((sl >> (4 * (s & 1))) & 0xFu) | ((((hdr >> 16) >> (2 * s)) & 3u) << 4)) - 32;
-        return fp16_bits_to_float(hdr & 0xFFFFu) * a.dx * (float)(ls * dot);
+        return ls * dot;
     }
 };
 
@@ -295,8 +264,8 @@ template <int NBITS> struct GranQ45K {
 #pragma unroll
         for (int i = 0; i < 8; i++) { a.bs0 = dp4a_ss(0x01010101u, a.q[i], a.bs0); a.bs1 = dp4a_ss(0x01010101u, a.q[8 + i], a.bs1); }
     }
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1&, int lane) {
+    // sums of the two sub-blocks, scaled, and of their minima
+    static Q38B_HD void pair_sums(SP row, const Acts& a, int lane, int (&v)[2], int (&m)[2], uint32_t& dd) {
         const int pr = lane & 15, pp = pr & 3;
         const SP p = row + BB * (pr >> 2);
         uint32_t w[8], hd[4];
@@ -308,7 +277,8 @@ template <int NBITS> struct GranQ45K {
             w[4] = v[0]; w[5] = v[1]; w[6] = v[2]; w[7] = v[3];
         }
         sp_ld128(p, 0, hd);                        // d | dmin, scales[12]
-        const uint32_t dd = hd[0], u0 = hd[1], u1 = hd[2], u2 = hd[3];
+        dd = hd[0];
+        const uint32_t u0 = hd[1], u1 = hd[2], u2 = hd[3];
         // 6-bit scales / mins of sub-blocks 2pp, 2pp+1 (get_scale_min_k4, src/quant/quant_ref.cpp:24-32)
         const bool hi_half = pp >= 2;
         const uint32_t sc4 = hi_half ? ((u2 & 0x0F0F0F0Fu) | ((u0 >> 2) & 0x30303030u)) : (u0 & 0x3F3F3F3Fu);
@@ -341,12 +311,31 @@ template <int NBITS> struct GranQ45K {
                 hi = dp4a_ss(((w[i] >> 4) & 0x0F0F0F0Fu) | ((hb << 3) & 0x10101010u), a.q[8 + i], hi);
             }
         }
+        v[0] = sc0 * lo; v[1] = sc1 * hi;
+        m[0] = mn0 * a.bs0; m[1] = mn1 * a.bs1;
+    }
+    static Q38B_HD void block_scale(SP block, float& d, float& m) {
+        const uint32_t dd = sp_ld32(block, 0);
+        d = fp16_bits_to_float(dd & 0xFFFFu);
+        m = fp16_bits_to_float(dd >> 16);
+    }
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1&, int lane, int& msum) {
+        int v[2], m[2];
+        uint32_t dd;
+        pair_sums(row, a, lane, v, m, dd);
+        msum = m[0] + m[1];
+        return v[0] + v[1];
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1&, int lane) {
+        int v[2], m[2];
+        uint32_t dd;
+        pair_sums(row, a, lane, v, m, dd);
         const float d = fp16_bits_to_float(dd & 0xFFFFu), dmin = fp16_bits_to_float(dd >> 16);
-        if (A32)   // each sub-block of the pair has its own activation scale
-            return d * (a.dx * (float)(sc0 * lo) + a.dx1 * (float)(sc1 * hi)) - dmin * (a.dx * (float)(mn0 * a.bs0) + a.dx1 * (float)(mn1 * a.bs1));
-        const int sumi = sc0 * lo + sc1 * hi;
-        const int msum = mn0 * a.bs0 + mn1 * a.bs1;
-        return d * a.dx * (float)sumi - dmin * a.dx * (float)msum;
+        if (!A32) return block_value_min(d * a.dx, v[0] + v[1], dmin * a.dx, m[0] + m[1]);
+        // each sub-block of the pair has its own activation scale
+        const float kv = fmaf(a.dx1, (float)v[1], fmul_once(a.dx, (float)v[0])), km = fmaf(a.dx1, (float)m[1], fmul_once(a.dx, (float)m[0]));
+        return fmaf(-dmin, km, fmul_once(d, kv));
     }
 };
 template <> struct Gran<T_Q4_K> : GranQ45K<4> {};
@@ -361,15 +350,15 @@ template <> struct Gran<T_Q6_K> {
     struct Acts { uint32_t q[8]; float dx; float dxs[4]; };   // dxs: scales of the granule's four 32-weight groups (per-32 activations)
     template <bool A32>
     static Q38B_HD void load_acts(Acts& a, SP aq, SP ad, int lane) {
-        const int sb = lane >> 3, n = (lane >> 2) & 1, i = lane & 3;
+        const int sb = lane >> 3, n = (lane >> 2) & 1;
 #pragma unroll
         for (int j = 0; j < 4; j++) sp_ld64(aq, 256 * j + 8 * lane, a.q[2 * j], a.q[2 * j + 1]);
         a.dx = sp_ldf(ad, sb * 32);
 #pragma unroll
         for (int j = 0; j < 4; j++) a.dxs[j] = A32 ? sp_ldf(ad, sb * 32 + 16 * n + 4 * j) : a.dx;
     }
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1&, int lane) {
+    // sums of the granule's four groups of eight
+    static Q38B_HD void group_sums(SP row, const Acts& a, int lane, int (&d4)[4]) {
         const int n = (lane >> 2) & 1, i = lane & 3;
         const SP p = row + 210 * (lane >> 3);
         const uint32_t mis = sp_low2(p);
@@ -377,7 +366,7 @@ template <> struct Gran<T_Q6_K> {
         sp_ld8b_a2(p + (64 * n + 8 * i), mis, qa[0], qa[1]);
         sp_ld8b_a2(p + (64 * n + 32 + 8 * i), mis, qb[0], qb[1]);
         sp_ld8b_a2(p + (128 + 32 * n + 8 * i), mis, qh[0], qh[1]);
-        int d4[4] = {0, 0, 0, 0};
+        d4[0] = d4[1] = d4[2] = d4[3] = 0;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
             d4[0] = dp4a_ss(Unit<T_Q6_K>::q6(qa[k], qh[k] << 4), a.q[k], d4[0]);
@@ -385,17 +374,34 @@ template <> struct Gran<T_Q6_K> {
             d4[2] = dp4a_ss(Unit<T_Q6_K>::q6(qa[k] >> 4, qh[k]), a.q[4 + k], d4[2]);
             d4[3] = dp4a_ss(Unit<T_Q6_K>::q6(qb[k] >> 4, qh[k] >> 2), a.q[6 + k], d4[3]);
         }
-        const SP sc = p + (192 + 8 * n + (i >> 1));          // scale of group 8n + 2j + (i >> 1)
-        if (A32) {   // group j of the granule lies in 32-weight block 4n + j of the super-block
-            float acc = 0.0f;
-#pragma unroll
-            for (int j = 0; j < 4; j++) acc += a.dxs[j] * (float)(sp_ld8s(sc, 2 * j) * d4[j]);
-            return fp16_bits_to_float(sp_ld16(p, 208)) * acc;
-        }
-        int sumi = 0;
+    }
+    // int8 scale of group 8n + 2j + (i >> 1), j = 0..3: every second byte from here
+    static Q38B_HD SP scales(SP row, int lane) { return row + (210 * (lane >> 3) + 192 + 8 * ((lane >> 2) & 1) + ((lane & 3) >> 1)); }
+    static Q38B_HD void block_scale(SP block, float& d, float& m) { d = fp16_bits_to_float(sp_ld16(block, 208)); m = 0.0f; }
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1&, int lane, int& msum) {
+        int d4[4], sumi = 0;
+        group_sums(row, a, lane, d4);
+        const SP sc = scales(row, lane);
 #pragma unroll
         for (int j = 0; j < 4; j++) sumi += sp_ld8s(sc, 2 * j) * d4[j];
-        return fp16_bits_to_float(sp_ld16(p, 208)) * a.dx * (float)sumi;
+        msum = 0;
+        return sumi;
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        const SP p = row + 210 * (lane >> 3);
+        if (!A32) {
+            int ms;
+            const int sum = idot(row, a, cb, lane, ms);
+            return gran_value<Gran, T_Q6_K>(p, a.dx, sum, ms);
+        }
+        int d4[4];
+        group_sums(row, a, lane, d4);
+        const SP sc = scales(row, lane);
+        float acc = 0.0f;   // group j of the granule lies in 32-weight block 4n + j of the super-block
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc += a.dxs[j] * (float)(sp_ld8s(sc, 2 * j) * d4[j]);
+        return fp16_bits_to_float(sp_ld16(p, 208)) * acc;
     }
 };
 
@@ -430,7 +436,7 @@ template <> struct Gran<T_Q8_0> {
             dot = dp4a_ss(funnel_r(prev, next, sh), a.q[i], dot);
             prev = next;
         }
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * (float)dot;
+        return block_value(fp16_bits_to_float(sp_ld16(p, 0)) * a.dx, dot);
     }
 };
 
@@ -459,7 +465,7 @@ Q38B_HD void iq2_group(uint32_t code, uint32_t sign8, uint32_t q0, uint32_t q1, 
     N = dp4a_us(g1 & sign_mask4(sign8 >> 4), q1, N);
 }
 
-template <int FMT> struct GranPlain {   // the common activation side: one 32-weight sub-block per lane
+template <int FMT> struct GranPlain : ScaleAt0 {   // the common activation side: one 32-weight sub-block per lane
     static constexpr int WORDS = 8, LANES_PER_ROW = 32;
     using Acts = ActRegs<WORDS>;
     template <bool A32>
@@ -474,8 +480,8 @@ template <int FMT> struct GranPlain {   // the common activation side: one 32-we
 };
 
 template <> struct Gran<T_IQ2_XXS> : GranPlain<T_IQ2_XXS> {
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 66 * (lane >> 3);
         const int ib = lane & 7;
         uint32_t a0, a1;
@@ -484,14 +490,19 @@ template <> struct Gran<T_IQ2_XXS> : GranPlain<T_IQ2_XXS> {
 #pragma unroll
         for (int l = 0; l < 4; l++)
             iq2_group(code16(cb, (a0 >> (8 * l)) & 0xFFu), ksign_byte((a1 >> (7 * l)) & 127u), a.q[2 * l], a.q[2 * l + 1], P, N);
-        const int sumi = (int)(2u * (a1 >> 28) + 1u) * (P - 2 * N);
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * 0.125f * (float)sumi;
+        return (int)(2u * (a1 >> 28) + 1u) * (P - 2 * N);
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ2_XXS>(row + 66 * (lane >> 3), a.dx, sum, ms);
     }
 };
 
 template <> struct Gran<T_IQ2_XS> : GranPlain<T_IQ2_XS> {
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 74 * (lane >> 3);
         const int ib = lane & 7;
         uint32_t w[2];
@@ -503,14 +514,19 @@ template <> struct Gran<T_IQ2_XS> : GranPlain<T_IQ2_XS> {
             const uint32_t qv = (w[l >> 1] >> (16 * (l & 1))) & 0xFFFFu;
             iq2_group(code16(cb, qv & 511u), ksign_byte(qv >> 9), a.q[2 * l], a.q[2 * l + 1], P[l >> 1], N[l >> 1]);
         }
-        const int sumi = (int)(2u * (sc & 0xFu) + 1u) * (P[0] - 2 * N[0]) + (int)(2u * (sc >> 4) + 1u) * (P[1] - 2 * N[1]);
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * 0.125f * (float)sumi;
+        return (int)(2u * (sc & 0xFu) + 1u) * (P[0] - 2 * N[0]) + (int)(2u * (sc >> 4) + 1u) * (P[1] - 2 * N[1]);
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ2_XS>(row + 74 * (lane >> 3), a.dx, sum, ms);
     }
 };
 
 template <> struct Gran<T_IQ2_S> : GranPlain<T_IQ2_S> {
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 82 * (lane >> 3);
         const int ib = lane & 7;
         const uint32_t qs = sp_ld16(p, 2 + 4 * ib) | (sp_ld16(p, 4 + 4 * ib) << 16);
@@ -522,14 +538,19 @@ template <> struct Gran<T_IQ2_S> : GranPlain<T_IQ2_S> {
             const uint32_t idx = ((qs >> (8 * l)) & 0xFFu) | ((qh << (8 - 2 * l)) & 0x300u);
             iq2_group(code16(cb, idx), (sg >> (8 * l)) & 0xFFu, a.q[2 * l], a.q[2 * l + 1], P[l >> 1], N[l >> 1]);
         }
-        const int sumi = (int)(2u * (sc & 0xFu) + 1u) * (P[0] - 2 * N[0]) + (int)(2u * (sc >> 4) + 1u) * (P[1] - 2 * N[1]);
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * 0.125f * (float)sumi;
+        return (int)(2u * (sc & 0xFu) + 1u) * (P[0] - 2 * N[0]) + (int)(2u * (sc >> 4) + 1u) * (P[1] - 2 * N[1]);
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ2_S>(row + 82 * (lane >> 3), a.dx, sum, ms);
     }
 };
 
 template <> struct Gran<T_IQ1_S> : GranPlain<T_IQ1_S> {
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 50 * (lane >> 3);
         const int ib = lane & 7;
         const uint32_t qs = sp_ld16(p, 2 + 4 * ib) | (sp_ld16(p, 4 + 4 * ib) << 16);
@@ -542,20 +563,24 @@ template <> struct Gran<T_IQ1_S> : GranPlain<T_IQ1_S> {
             S = dp4a_ss(iq1_bytes(code & 0xFFu, minus), a.q[2 * l], S);
             S = dp4a_ss(iq1_bytes(code >> 8, minus), a.q[2 * l + 1], S);
         }
-        const int sumi = (int)(2u * ((qh >> 12) & 7u) + 1u) * S;
-        return fp16_bits_to_float(sp_ld16(p, 0)) * a.dx * 0.125f * (float)sumi;
+        return (int)(2u * ((qh >> 12) & 7u) + 1u) * S;
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ1_S>(row + 50 * (lane >> 3), a.dx, sum, ms);
     }
 };
 
 template <> struct Gran<T_IQ1_M> : GranPlain<T_IQ1_M> {
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1& cb, int lane, int& msum) {
+        msum = 0;
         const SP p = row + 56 * (lane >> 3);
         const int ib = lane & 7;
         const uint32_t qs = sp_ld16(p, 4 * ib) | (sp_ld16(p, 4 * ib + 2) << 16);
         const uint32_t qh = sp_ld16(p, 32 + 2 * ib);                 // nibble l: 3 index bits and the delta sign of group l
         const uint32_t s0 = sp_ld16(p, 48), s1 = sp_ld16(p, 50), s2 = sp_ld16(p, 52), s3 = sp_ld16(p, 54);
-        const uint32_t su = (s0 >> 12) | ((s1 >> 8) & 0x00F0u) | ((s2 >> 4) & 0x0F00u) | (s3 & 0xF000u);   // the scattered fp16 super-scale
         const uint32_t scw = (ib >> 1) == 0 ? s0 : (ib >> 1) == 1 ? s1 : (ib >> 1) == 2 ? s2 : s3;
         const uint32_t t = scw >> (6 * (ib & 1));
         int S[2] = {0, 0};
@@ -567,8 +592,18 @@ template <> struct Gran<T_IQ1_M> : GranPlain<T_IQ1_M> {
             S[l >> 1] = dp4a_ss(iq1_bytes(code & 0xFFu, minus), a.q[2 * l], S[l >> 1]);
             S[l >> 1] = dp4a_ss(iq1_bytes(code >> 8, minus), a.q[2 * l + 1], S[l >> 1]);
         }
-        const int sumi = (int)(2u * (t & 7u) + 1u) * S[0] + (int)(2u * ((t >> 3) & 7u) + 1u) * S[1];
-        return fp16_bits_to_float(su) * a.dx * 0.125f * (float)sumi;
+        return (int)(2u * (t & 7u) + 1u) * S[0] + (int)(2u * ((t >> 3) & 7u) + 1u) * S[1];
+    }
+    static Q38B_HD void block_scale(SP block, float& d, float& m) {
+        const uint32_t s0 = sp_ld16(block, 48), s1 = sp_ld16(block, 50), s2 = sp_ld16(block, 52), s3 = sp_ld16(block, 54);
+        d = fp16_bits_to_float((s0 >> 12) | ((s1 >> 8) & 0x00F0u) | ((s2 >> 4) & 0x0F00u) | (s3 & 0xF000u));   // the scattered fp16 super-scale
+        m = 0.0f;
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_IQ1_M>(row + 56 * (lane >> 3), a.dx, sum, ms);
     }
 };
 
@@ -590,8 +625,7 @@ template <> struct Gran<T_Q2_K> {
 #pragma unroll
         for (int i = 0; i < 4; i++) { a.bs0 = dp4a_ss(0x01010101u, a.q[i], a.bs0); a.bs1 = dp4a_ss(0x01010101u, a.q[4 + i], a.bs1); }
     }
-    template <bool A32>
-    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1&, int lane) {
+    static Q38B_HD int idot(SP row, const Acts& a, const Codebook1&, int lane, int& msum) {
         const SP p = row + 84 * (lane >> 3);
         const int ib = lane & 7, n = ib >> 2, j = ib & 3;
         int S0 = 0, S1 = 0;
@@ -601,10 +635,19 @@ template <> struct Gran<T_Q2_K> {
             S1 = dp4a_us((sp_ld32(p, 32 + 32 * n + 4 * i) >> (2 * j)) & 0x03030303u, a.q[4 + i], S1);
         }
         const uint32_t sc = sp_ld16(p, 2 * ib);                      // scale bytes of the two 16-weight groups
-        const int sumi = (int)(sc & 0xFu) * S0 + (int)((sc >> 8) & 0xFu) * S1;
-        const int msum = (int)((sc >> 4) & 0xFu) * a.bs0 + (int)(sc >> 12) * a.bs1;
-        const uint32_t dd = sp_ld32(p, 80);
-        return fp16_bits_to_float(dd & 0xFFFFu) * a.dx * (float)sumi - fp16_bits_to_float(dd >> 16) * a.dx * (float)msum;
+        msum = (int)((sc >> 4) & 0xFu) * a.bs0 + (int)(sc >> 12) * a.bs1;
+        return (int)(sc & 0xFu) * S0 + (int)((sc >> 8) & 0xFu) * S1;
+    }
+    static Q38B_HD void block_scale(SP block, float& d, float& m) {
+        const uint32_t dd = sp_ld32(block, 80);
+        d = fp16_bits_to_float(dd & 0xFFFFu);
+        m = fp16_bits_to_float(dd >> 16);
+    }
+    template <bool A32>
+    static Q38B_HD float dot(SP row, const Acts& a, const Codebook1& cb, int lane) {
+        int ms;
+        const int sum = idot(row, a, cb, lane, ms);
+        return gran_value<Gran, T_Q2_K>(row + 84 * (lane >> 3), a.dx, sum, ms);
     }
 };
 

@@ -9,10 +9,13 @@
 // tile's mbarrier; the warp that took the tile's last slice waits for the others, adds the slices in order
 // (deterministic) and stores y.
 //
-// With NC = 4 the same kernel takes two to four columns: a granule is decoded once (q38b_decode1n.cuh) and multiplied with
-// each column, whose result is the single-column launch's, bit for bit.  It serves the formats without mma fragments and
-// the per-32 activations; before, they ran one launch per column (bound by issue: the decoding is most of the work).
-// Measured: four columns of 17408 x 5120 IQ3_XXS, per-32 activations, 83 -> 31 us.
+// Q8_K columns of the lane-per-granule mapping: the eight (four) lanes of a super-block add exact integers and one lane per
+// row scales their sum, where every lane used to read the block's factors, convert and multiply: per granule and row some six
+// operations less (27B-shaped pass 3847 -> 3810 us, pass of a small model in 2-bit blocks 466 -> 458).  The sums are formed in
+// the order of the several-column kernel (q38b_gemv.cuh), so that a column's bits do not depend on how many share a launch.
+//
+// With NC = 4 the same kernel takes two to four columns of Q6_K with per-32 activations: a granule is decoded once
+// (q38b_decode1n.cuh) and multiplied with each column, whose result is the single-column launch's, bit for bit.
 #pragma once
 #include <type_traits>
 
@@ -48,10 +51,10 @@ struct Gemv1Args {
     int static_weights;     // 1: W was written long before this launch, the producer need not wait for earlier kernels
     int* status;
     const uint32_t* codebook;
-    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes), x_f32 and xd32 (floats), and of each
+    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes) and xd32 (floats), and of each
     // matrix's output (floats; the peers' as well)
     int nc;
-    long long xq_ld, x_f32_ld, xd32_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
+    long long xq_ld, xd32_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
     int K, M, accumulate;
     int nsb;                // super-blocks per row
     int n_slices;           // ceil(nsb / 4)
@@ -101,6 +104,9 @@ constexpr int RG_STATIC_BYTES = 4 * (RG_CB_WORDS + RG_SGN_WORDS);
 // single per-32 columns that act_q8_one_cta names).
 // NC: columns at most (1 or 4).
 // XT: IQ2 / IQ1 with expanded grid tables (GranX), which want an SM's whole shared memory; without them the 16-bit codes.
+template <int FMT, int NC, bool XT> struct GranOf { using type = typename std::conditional<XT, GranX<FMT>, Gran<FMT>>::type; };
+template <> struct GranOf<T_Q6_K, 4, false> { using type = GranN<T_Q6_K>; };
+
 template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC, int NC = 1, bool XT = false>
 __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gemv1Args a) {
     constexpr int G1_ROWS = ROWS;
@@ -109,8 +115,8 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     static_assert(!(RG && (A32 || NC > 1)), "per-32 activations and several columns run on the lane-per-granule mapping");
     const int nc = NC == 1 ? 1 : a.nc;
     static_assert(!XT || (OCC == 1 && gridx_copies(FMT) > 0), "expanded grids: IQ2 / IQ1 with one CTA per SM");
-    static_assert(XT || NC == 1 || gridx_copies(FMT) == 0, "several columns of IQ2 / IQ1 are decoded by GranX");
-    using G = typename std::conditional<XT, GranX<FMT>, typename std::conditional<NC == 1, Gran<FMT>, GranN<FMT>>::type>::type;
+    static_assert(NC == 1 || (FMT == T_Q6_K && A32 && !XT), "several columns: Q6_K with per-32 activations");
+    using G = typename GranOf<FMT, NC, XT>::type;
     // tables of the row-group decoders: static shared memory (their addresses become immediates of the loads); kernels
     // without them have no static shared memory at all, so that two CTAs of 113 KB still fit an SM
     uint32_t* rg_cb = nullptr;
@@ -261,62 +267,17 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     }
     const int act_ld = a.n_slices * 1024, actd_ld = a.n_slices * 32;   // between the columns' staged values (bytes) and scales (floats)
     if constexpr (NC > 1) {
-        // the same two ways for several columns: the blocks (words, scales) of all of them are dealt to the threads
-        const int nsb4 = a.n_slices * 4;
-        if (a.x_f32) {
-            constexpr int QB = 3;
-            for (int b0 = cw; b0 < nc * nsb4; b0 += QB * NWARPS) {
-                float4 lo4[QB], hi4[QB];
-#pragma unroll
-                for (int j = 0; j < QB; j++) {
-                    const int b = b0 + j * NWARPS, c = b / nsb4, sb = b - c * nsb4;
-                    lo4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    hi4[j] = lo4[j];
-                    if (c < nc && sb < a.nsb) {
-                        const float* src = a.x_f32 + (size_t)c * a.x_f32_ld + (size_t)sb * 256 + 8 * lane;
-                        lo4[j] = *(const float4*)src;
-                        hi4[j] = *(const float4*)(src + 4);
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < QB; j++) {
-                    const int b = b0 + j * NWARPS, c = b / nsb4, sb = b - c * nsb4;
-                    if (c >= nc) continue;
-                    uint32_t w0 = 0, w1 = 0;
-                    float d = 0.0f;
-                    if (sb < a.nsb) {
-                        const float v[8] = {lo4[j].x, lo4[j].y, lo4[j].z, lo4[j].w, hi4[j].x, hi4[j].y, hi4[j].z, hi4[j].w};
-                        int s8;
-                        q8k_block_core(v, w0, w1, s8, d);
-                    }
-                    if (lane == 0) actd[c * actd_ld + sb * 8] = d;
-                    uint8_t* dst = actq + c * act_ld + (sb >> 2) * 1024;
-                    const int k0 = (sb & 3) * 256 + 8 * lane;
-                    static_assert(A32 || FMT != T_IQ4_XS, "its columns of floats run on the multi-column kernel");
-                    *(uint2*)(dst + act_slice_pos(FMT, k0)) = make_uint2(w0, w1);
-                }
-            }
-        } else {
-            const int n_d = A32 ? actd_ld : nsb4, n_w = a.n_slices * 256;
-            for (int i = ctid; i < nc * n_d; i += NWARPS * 32) {
-                const int c = i / n_d, k = i - c * n_d;
-                if (A32) actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xd32_ld + k] : 0.0f;
-                else actd[c * actd_ld + k * 8] = k < a.nsb ? *(const float*)(a.xq + (size_t)c * a.xq_ld + (size_t)k * Q8K_BYTES) : 0.0f;
-            }
+        // several columns of per-32 activations: the words and scales of all of them are dealt to the threads
+        const int n_w = a.n_slices * 256;
+        for (int i = ctid; i < nc * actd_ld; i += NWARPS * 32) {
+            const int c = i / actd_ld, k = i - c * actd_ld;
+            actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xd32_ld + k] : 0.0f;
+        }
 #pragma unroll 4
-            for (int i = ctid; i < nc * n_w; i += NWARPS * 32) {
-                const int c = i / n_w, w = i - c * n_w, sb = w >> 6, wi = w & 63;
-                const uint8_t* src = a.xq + (size_t)c * a.xq_ld;
-                const uint32_t v = sb >= a.nsb ? 0u : A32 ? *(const uint32_t*)(src + 4 * (size_t)w) : *(const uint32_t*)(src + (size_t)sb * Q8K_BYTES + 4 + 4 * wi);
-                uint8_t* dst = actq + c * act_ld + (sb >> 2) * 1024;
-                const int k0 = (sb & 3) * 256 + 4 * wi;
-                if (FMT == T_IQ4_XS) {
-#pragma unroll
-                    for (int b = 0; b < 4; b++) dst[act_slice_pos(FMT, ((k0 + b) & ~31) + act_stage_pos(FMT, (k0 + b) & 31))] = (uint8_t)(v >> (8 * b));
-                } else {
-                    *(uint32_t*)(dst + act_slice_pos(FMT, k0)) = v;
-                }
-            }
+        for (int i = ctid; i < nc * n_w; i += NWARPS * 32) {
+            const int c = i / n_w, w = i - c * n_w, sb = w >> 6, wi = w & 63;
+            const uint32_t v = sb >= a.nsb ? 0u : *(const uint32_t*)(a.xq + (size_t)c * a.xq_ld + 4 * (size_t)w);
+            *(uint32_t*)(actq + c * act_ld + (sb >> 2) * 1024 + act_slice_pos(FMT, (sb & 3) * 256 + 4 * wi)) = v;
         }
     } else if (a.x_f32) {
         // quantize the column here (every CTA, the same arithmetic as quantize_q8k_kernel): one warp per 256 values.  The
@@ -476,15 +437,22 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         // granules past the end of the row (K not a multiple of 1024) contribute nothing
         const int gran_sb = slice * 4 + (LPR == 32 ? (lane >> 3) : ((lane & 15) >> 2));
         const bool live = gran_sb < a.nsb;
-        float acc[NC][PASSES];
+        // Q8_K columns: a super-block's lanes add exact integers, and one lane per row scales them (bits 1, 2, 4 of the lane
+        // number, 1, 2 with two rows a pass, are the place inside the super-block); per-32 columns and Q8_0: floats throughout.
+        constexpr bool INT_SUMS = NC == 1 && !A32 && FMT != T_Q8_0;
+        constexpr int SB_LANES = LPR / 4;
+        using Sum = typename std::conditional<INT_SUMS, int, float>::type;
+        Sum acc[NC][PASSES], mins[INT_SUMS && Unit<FMT>::HAS_MIN ? PASSES : 1];
+        auto row_at = [&](int r) { return st + (r * a.slot_stride + (int)((src_lo + (uint32_t)r * rb_step) & 15u)); };
 #pragma unroll
         for (int ps = 0; ps < PASSES; ps++) {
-            const int r = LPR == 32 ? ps : 2 * ps + sub;
-            const SP rowp = st + (r * a.slot_stride + (int)((src_lo + (uint32_t)r * rb_step) & 15u));
-            if constexpr (NC == 1) {
-                float v;
-                if constexpr (XT) v = G::dot(rowp, acts[0], cb, lane);
-                else v = G::template dot<A32>(rowp, acts[0], cb, lane);
+            const SP rowp = row_at(LPR == 32 ? ps : 2 * ps + sub);
+            if constexpr (INT_SUMS) {
+                int ms;
+                acc[0][ps] = G::idot(rowp, acts[0], cb, lane, ms);
+                if constexpr (Unit<FMT>::HAS_MIN) mins[ps] = ms;
+            } else if constexpr (NC == 1) {
+                const float v = G::template dot<A32>(rowp, acts[0], cb, lane);
                 acc[0][ps] = live ? v : 0.0f;
             } else {
                 const typename G::W g = G::decode(rowp, cb, lane);
@@ -498,45 +466,61 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
                 }
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive_n(smem_u32(&empty[stage]), n_arr);
+        if (!INT_SUMS) {   // (integer sums read the rows' factors below)
+            __syncwarp();
+            if (lane == 0) mbar_arrive_n(smem_u32(&empty[stage]), n_arr);
+        }
 
-        // sum over the lanes of each row: halving butterflies (each step halves the values a lane holds), then plain ones
+        // sum over the lanes of each row, neighbours first: halving butterflies (each step halves the values a lane holds)
+        // until one is left, then plain ones
 #pragma unroll
         for (int c = 0; c < NC; c++) {
         if (c >= nc) break;
-        float rowsum;
         int myrow = 0;      // the row whose sum this lane ends up with
-        {
-            float v[PASSES];
+        auto halve = [&](auto& v, int bit, int n) {   // n values a lane -> n / 2
+            const int h = n >> 1;
+            const bool up = (lane & bit) != 0;
 #pragma unroll
-            for (int i = 0; i < PASSES; i++) v[i] = acc[c][i];
-            constexpr int TOP = LPR == 32 ? 16 : 8;    // highest lane bit inside one row's lane set
-            int n = PASSES, bit = TOP;
-#pragma unroll
-            for (int step = 0; step < 3; step++) {
-                if (n > 1) {
-                    const int h = n >> 1;
-                    const bool up = (lane & bit) != 0;
-#pragma unroll
-                    for (int i = 0; i < (PASSES > 1 ? PASSES / 2 : 1); i++) {
-                        if (i < h && i + h < PASSES) {
-                            const float keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
-                            v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
-                        }
-                    }
-                    if (up) myrow += h;
-                    n = h;
-                    bit >>= 1;
+            for (int i = 0; i < (PASSES > 1 ? PASSES / 2 : 1); i++) {
+                if (i < h) {
+                    const auto keep = up ? v[i + h] : v[i], give = up ? v[i] : v[i + h];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
                 }
             }
-            rowsum = v[0];
-            for (; bit > 0; bit >>= 1) rowsum += __shfl_xor_sync(0xffffffffu, rowsum, bit);
-            if (LPR == 16) myrow = 2 * myrow + sub;
+        };
+        Sum v[PASSES > 1 ? PASSES : 2];
+#pragma unroll
+        for (int i = 0; i < PASSES; i++) v[i] = acc[c][i];
+        int n = PASSES;
+#pragma unroll
+        for (int bit = 1; bit < SB_LANES; bit <<= 1) {
+            if (n > 1) {
+                halve(v, bit, n);
+                if constexpr (INT_SUMS && Unit<FMT>::HAS_MIN) halve(mins, bit, n);
+                n >>= 1;
+                if (lane & bit) myrow += n;
+            } else {
+                v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
+                if constexpr (INT_SUMS && Unit<FMT>::HAS_MIN) mins[0] += __shfl_xor_sync(0xffffffffu, mins[0], bit);
+            }
         }
-        // one lane per row writes: the lanes whose low bits (those folded by the plain butterflies) are zero
-        constexpr int LOW_MASK = (LPR == 32 ? 32 : 16) / PASSES - 1;
-        if ((lane & LOW_MASK) == 0) rslot[c * G1_ROWS + myrow] = rowsum;
+        static_assert(PASSES <= SB_LANES, "one row a lane after the lanes of a super-block");
+        if (LPR == 16) myrow = 2 * myrow + sub;
+        float rowsum;
+        if constexpr (INT_SUMS) {
+            float d, m;
+            G::block_scale(row_at(myrow) + BB * (LPR == 32 ? (lane >> 3) : ((lane & 15) >> 2)), d, m);
+            __syncwarp();
+            if (lane == 0) mbar_arrive_n(smem_u32(&empty[stage]), n_arr);
+            const float dx = acts[0].dx;
+            rowsum = Unit<FMT>::HAS_MIN ? block_value_min(d * dx, v[0], m * dx, mins[0]) : block_value(d * dx * Unit<FMT>::FACTOR, v[0]);
+            rowsum = live ? rowsum : 0.0f;
+        } else {
+            rowsum = v[0];
+        }
+#pragma unroll
+        for (int bit = SB_LANES; bit < LPR; bit <<= 1) rowsum += __shfl_xor_sync(0xffffffffu, rowsum, bit);
+        if ((lane & (LPR - 1)) < PASSES) rslot[c * G1_ROWS + myrow] = rowsum;   // one lane per row writes
         }
         }
         __syncwarp();

@@ -41,6 +41,34 @@ struct q38b_ctx {
 
 // device table a format's decoders stage into shared memory (32-bit codebook words or 16-bit grid codes), or nullptr
 const uint32_t* q38b_grid_source(const q38b_ctx* ctx, uint32_t type);
+// Opt-in shared-memory size of a kernel, set once per context (= per device) and kernel
+int q38b_ensure_kernel_smem(q38b_ctx* ctx, const void* kern, int dyn_smem_bytes, bool max_carveout);
+
+// ---- several-column matvec (q38b_gemvn.cu) ----
+// One launch: up to three matrices of one format, K and row stride on nb columns, which come as Q8_K blocks (xq, xq_ld bytes
+// between the columns), as floats (x_f32) or in the per-32 format (xq = int8 values, xd32 = scales).
+struct ColsCall {
+    uint32_t type = 0;
+    size_t row_bytes = 0;
+    int K = 0, nb = 0, n_mats = 0, accumulate = 0, n_peers = 0;
+    const void* W[3] = {};
+    int M[3] = {};
+    float* y[3] = {};
+    long long y_ld[3] = {};
+    float* const* y_peers = nullptr;   // y_peers[i * n_peers + r]: peer r's copy of matrix i's output
+    const void* xq = nullptr;
+    long long xq_ld = 0;
+    const float* x_f32 = nullptr;
+    long long x_f32_ld = 0;
+    const float* xd32 = nullptr;
+    long long xd32_ld = 0;
+};
+int q38b_cols_launch(q38b_ctx* ctx, const ColsCall& c, void* stream);
+// the most of nb columns (at most eight) that one launch can take; 0: none (Q6_K with per-32 activations: the one-column kernel's)
+int q38b_cols_fit(const q38b_ctx* ctx, uint32_t type, int K, const int* M, int n_mats, size_t row_bytes, int nb, bool a32);
+// rows one launch can take (K-parts: the size of the scratch area); 0: any number
+long long q38b_cols_max_rows(const q38b_ctx* ctx, uint32_t type, int K);
+
 // 1 when q38b_gemv_group would run these matrices (single column) on the one-column kernel
 extern "C" int q38b_gemv_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M);
 // q38b_gemv_group with peer stores: y_peers[i * n_peers + r] is where peer r keeps the output of matrix i
