@@ -4,9 +4,9 @@
 //
 // Replaces dequant_rows_f16 + gemm_f16 (cuBLAS) of the reference (src/cuda/prefill.cu:30-85, 802-851) by one kernel:
 // the weights never exist dequantized in global memory.  One CTA owns a 128-row weight tile and up to 512 tokens:
-//   * warps 0-15 own eight rows each.  They fetch the rows' raw blocks one super-block ahead (whole 16-byte units into
-//     registers, then their own piece of shared memory), a lane expands one 32-weight sub-block with word operations
-//     (q38b_expand.cuh) and stores it K-major with the 128-byte swizzle the tensor core expects (operand A);
+//   * warps 0-15 fetch the rows' raw blocks one super-block ahead (whole 16-byte units into registers, then shared memory), a
+//     lane expands one 32-weight sub-block with word operations (q38b_expand.cuh) into operand A: from 257 tokens on K-major
+//     with the 128-byte swizzle in shared memory (a warp owns eight rows), up to 256 in tensor memory (a lane is a row);
 //   * one thread streams the matching activation tiles (operand B, [tokens x 64] per K-slab) with tiled TMA loads
 //     (hardware swizzle, zero fill past the last token; no multicast);
 //   * one thread issues tcgen05.mma (cta_group::1, kind::f16, M = 128, N = 16..256, K = 16) into one or two fp32
@@ -15,8 +15,8 @@
 // Where row tiles and token tiles alone leave SMs idle, the CTAs of a cluster share a tile's K: each multiplies a range
 // of super-blocks and the partial sums meet through distributed shared memory, added in rank order.
 // Measured on B200, 17408 x 5120 IQ3_XXS / 5120 x 17408 IQ4_XS with 1024 tokens: 211 / 286 us -> 161 / 194 us; 77 tokens of a
-// whole Q4_K / Q6_K layer 698 -> 199 us.  Up to about 250 tokens the expanders set the pace (issue slots 66 % busy, the
-// shared-memory pipe 63-70 %), from 500 the tensor core and its shared-memory traffic do (tensor pipe 69 % busy).
+// whole Q4_K / Q6_K layer 698 -> 199 us, 154 us with operand A in tensor memory.  Up to 256 tokens the expanders set the pace,
+// from 500 the activation tiles (64 bytes a clock and SM from L2) and the shared-memory traffic of 128-row tiles do.
 // All mbarrier waits are bounded; tensor memory is released before the kernel returns, also after a timeout.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -54,7 +54,18 @@ __host__ __device__ constexpr int pf_raw_bytes(int fmt) { return fmt == T_Q8_0 ?
 __host__ __device__ constexpr int pf_pieces(int fmt) { return (pf_raw_bytes(fmt) + 14 + 15) / 16; }
 __host__ __device__ constexpr int pf_pitch(int fmt) { return 16 * (pf_pieces(fmt) | 1); }
 __host__ __device__ constexpr int pf_raw_smem(int fmt) { return PF_ROWS * pf_pitch(fmt) + 16; }   // + what the last row's word loads read past its end
-__host__ __device__ constexpr int pf_fixed_smem(int fmt) { return 1024 + PF_A_STAGES * PF_A_BYTES + pf_raw_smem(fmt) + grid_table_bytes(fmt) + 16; }
+// Operand A in tensor memory (one accumulator, up to 256 tokens): a decode warp's lanes are 32 rows, an odd number of the
+// format's loads (16, 8 or 4 bytes) apart; two buffers, as four warps share a quarter of the rows.
+__host__ __device__ constexpr int pf_pitch_ta(int fmt, bool aligned) {
+    return aligned && (fmt == T_Q4_K || fmt == T_Q5_K) ? pf_pitch(fmt) : 16 * pf_pieces(fmt) + (aligned && fmt == T_IQ4_XS ? 8 : 4);
+}
+__host__ __device__ constexpr int pf_raw_ta(int fmt) { return (PF_ROWS * 16 * (pf_pieces(fmt) + 1) + 16 + 127) / 128 * 128; }   // one buffer, any pitch
+__host__ __device__ constexpr int pf_fixed_smem(int fmt, bool ta) {
+    return 1024 + (ta ? 2 * pf_raw_ta(fmt) : PF_A_STAGES * PF_A_BYTES + pf_raw_smem(fmt)) + grid_table_bytes(fmt) + 16;
+}
+constexpr int PF_TA_STAGE_COLS = 64;   // 128 rows x 128 K of 16-bit weights: 64 columns of tensor memory
+constexpr int PF_TA_MAX_STAGES = 6;
+__host__ __device__ constexpr int pf_ta_stages(int n_tile) { return (512 - (n_tile + 31) / 32 * 32) / PF_TA_STAGE_COLS < PF_TA_MAX_STAGES ? (512 - (n_tile + 31) / 32 * 32) / PF_TA_STAGE_COLS : PF_TA_MAX_STAGES; }
 
 struct PrefillArgs {
     const uint8_t* W;
@@ -162,6 +173,16 @@ __device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void st_peer_f32(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
+// 16 columns of this warp's 32 rows: 32 16-bit weights of a row
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]),
+        "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 // 16 accumulator columns of this warp's 32 rows
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
     asm volatile(
@@ -175,21 +196,28 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 
 // F16: operands are fp16 (weights dequantized to fp16, activations fp16) instead of bf16.
 // ALIGNED: every row starts at a multiple of expand_alignment(FMT).
-template <int FMT, bool F16, bool ALIGNED>
+// TA: operand A goes to tensor memory instead of shared memory (one accumulator, up to 256 tokens).  Up to there the kernel is
+// bound by shared-memory bandwidth: per 128 K the tensor core reads 32 KB of weights and 20 KB of activations (80 tokens), the
+// decode warps write the weights and move the raw blocks twice, 140 KB of traffic or 1100 clocks of some 1700 measured; from
+// tensor memory the weights cost none of it.  With one wait and one commit per 128 K and the unchecked fetch, 16384 x 5120 Q4_K,
+// 77 tokens 39.6 -> 27.9 us, 17408 x 5120 IQ3_XXS 51.4 -> 42.0, 5120 x 17408 Q6_K 55.1 -> 45.4, a Q4_K / Q6_K layer 199 -> 154 us.
+template <int FMT, bool F16, bool ALIGNED, bool TA>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArgs a, const __grid_constant__ CUtensorMap xmap) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* full_a = (uint64_t*)smem;              // [A stages] the 16 decode warps arrive
-    uint64_t* empty_a = full_a + PF_A_STAGES;        // [A stages] tcgen05.commit
-    uint64_t* full_b = empty_a + PF_A_STAGES;        // [B stages] TMA bytes
+    constexpr int MAX_A = TA ? PF_TA_MAX_STAGES : PF_A_STAGES;
+    const int a_stages = TA ? a.b_stages : PF_A_STAGES;
+    uint64_t* empty_a = full_a + MAX_A;              // [A stages] tcgen05.commit
+    uint64_t* full_b = empty_a + MAX_A;              // [B stages] TMA bytes
     uint64_t* empty_b = full_b + PF_B_MAX_STAGES;    // [B stages] tcgen05.commit
     uint64_t* acc_done = empty_b + PF_B_MAX_STAGES;  // [1]
     uint32_t* tmem_slot = (uint32_t*)(acc_done + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    const int b_stage_bytes = a.n_tile * (PF_KSLAB * 2);
-    uint8_t* stages = smem + 1024;                                   // ring of weight tiles
-    uint8_t* stages_b = stages + PF_A_STAGES * PF_A_BYTES;            // ring of activation tiles
+    const int b_stage_bytes = a.n_tile * (PF_KSLAB * 2) * (TA ? 2 : 1);   // TA: a stage is 128 K of both operands, one barrier each way
+    uint8_t* stages = smem + 1024;                                   // ring of weight tiles (TA: none)
+    uint8_t* stages_b = stages + (TA ? 0 : PF_A_STAGES * PF_A_BYTES); // ring of activation tiles
     uint8_t* raw_all = stages_b + a.b_stages * b_stage_bytes;         // the decode warps' raw blocks
-    uint32_t* tab_smem = (uint32_t*)(raw_all + pf_raw_smem(FMT));
+    uint32_t* tab_smem = (uint32_t*)(raw_all + (TA ? 2 * pf_raw_ta(FMT) : pf_raw_smem(FMT)));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = a.splits > 1 ? (int)cluster_rank() : 0;
     const int row0 = (int)(blockIdx.x / (unsigned)a.splits) * PF_ROWS;
@@ -197,12 +225,12 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
     const int tok0 = blockIdx.y * tile_tok;
     const int nsb = a.K >> 8;
     const int sb_begin = nsb * rank / a.splits, sb_end = nsb * (rank + 1) / a.splits;   // this CTA's super-blocks (splits <= nsb: never none)
-    const uint32_t tmem_cols = a.n_acc == 2 ? 512u : a.n_tile > 128 ? 256u : a.n_tile > 64 ? 128u : a.n_tile > 32 ? 64u : 32u;
+    const uint32_t tmem_cols = TA || a.n_acc == 2 ? 512u : a.n_tile > 128 ? 256u : a.n_tile > 64 ? 128u : a.n_tile > 32 ? 64u : 32u;
 
     if (tid == 0) {
         *abort_flag = 0;
-        for (int s = 0; s < PF_A_STAGES; s++) {
-            mbar_init(smem_u32(&full_a[s]), PF_DECODE_WARPS);   // one arrival per warp
+        for (int s = 0; s < a_stages; s++) {
+            mbar_init(smem_u32(&full_a[s]), PF_DECODE_WARPS + (TA ? 1 : 0));   // one arrival per warp (TA: and the activations')
             mbar_init(smem_u32(&empty_a[s]), 1);
         }
         for (int s = 0; s < a.b_stages; s++) {
@@ -225,20 +253,42 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
 
     if (warp < PF_DECODE_WARPS) {
         // ---------------- operand A: decode 128 rows x 128 weights per stage ----------------
-        constexpr int RAW = pf_raw_bytes(FMT), PITCH = pf_pitch(FMT), ROUNDS = (pf_pieces(FMT) + 3) / 4;
+        constexpr int RAW = pf_raw_bytes(FMT), PITCH = TA ? pf_pitch_ta(FMT, ALIGNED) : pf_pitch(FMT), ROUNDS = (pf_pieces(FMT) + 3) / 4;
         constexpr int UNIT_HALVES = FMT == T_Q8_0 ? 1 : 2;
         const uintptr_t w_begin = (uintptr_t)a.W, w_end = w_begin + (uintptr_t)(a.M - 1) * a.row_bytes + (uintptr_t)nsb * (RAW * 2 / UNIT_HALVES);
         // fetching: lane / 4 is the row, lane % 4 the first of its pieces; rows past the end repeat the last row (never stored)
-        const uintptr_t fetch_row = w_begin + (uintptr_t)min(row0 + PF_WARP_ROWS * warp + (lane >> 2), a.M - 1) * a.row_bytes;
-        uint8_t* raw = raw_all + warp * (PF_WARP_ROWS * PITCH);
+        // (TA: the four warps of a quarter of the rows, warp % 4, fetch eight of its 32 rows each)
+        const int first_row = TA ? 32 * (warp & 3) + PF_WARP_ROWS * (warp >> 2) : PF_WARP_ROWS * warp;
+        const uintptr_t fetch_row = w_begin + (uintptr_t)min(row0 + first_row + (lane >> 2), a.M - 1) * a.row_bytes;
+        uint8_t* raw = raw_all + first_row * PITCH;
         uint8_t* raw_put = raw + (lane >> 2) * PITCH + 16 * (lane & 3);
         // A piece that reaches past the matrix's first or last byte is not loaded ahead but copied by halfwords when it is due:
         // without that branch the loads stay in flight behind the work on the unit before (with it the compiler waited for
         // them on the spot).
-        uint4 ahead[ROUNDS];
+        uint4 ahead[ROUNDS] = {};
         auto piece_at = [&](int unit, int r) { return ((fetch_row + (uintptr_t)unit * RAW) & ~(uintptr_t)15) + 16 * (uintptr_t)((lane & 3) + 4 * r); };
         auto inside = [&](uintptr_t at, int unit) { return at >= w_begin && at + 16 <= w_end && at < fetch_row + (uintptr_t)(unit + 1) * RAW; };
+        // Every unit but the matrix's first and last: a piece is loaded where the unit can reach it at all, unchecked (it ends at
+        // most 29 bytes past the unit, where the next one lies).  The checks alone were a third of a unit's instructions.
+        const int row_first = min(row0 + first_row, a.M - 1), row_last = min(row0 + first_row + PF_WARP_ROWS - 1, a.M - 1), n_units = nsb * 2 / UNIT_HALVES;
+        auto interior = [&](int unit) { return (row_first > 0 || unit > 0) && (row_last < a.M - 1 || unit + 1 < n_units); };
+        auto reached = [&](int r) { return 4 * r + 3 < pf_pieces(FMT) || (lane & 3) + 4 * r < pf_pieces(FMT); };
+        auto put_piece = [&](int r) {
+            if constexpr (PITCH % 16 == 0) {
+                *(uint4*)(raw_put + 64 * r) = ahead[r];
+            } else {
+                uint32_t* to = (uint32_t*)(raw_put + 64 * r);
+                to[0] = ahead[r].x; to[1] = ahead[r].y; to[2] = ahead[r].z; to[3] = ahead[r].w;
+            }
+        };
         auto fetch = [&](int unit) {
+            if (interior(unit)) {
+                const uint8_t* at = (const uint8_t*)piece_at(unit, 0);
+#pragma unroll
+                for (int r = 0; r < ROUNDS; r++)
+                    if (reached(r)) ahead[r] = __ldg((const uint4*)(at + 64 * r));
+                return;
+            }
 #pragma unroll
             for (int r = 0; r < ROUNDS; r++) {
                 const uintptr_t at = piece_at(unit, r);
@@ -246,11 +296,17 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
             }
         };
         auto put_raw = [&](int unit) {
+            if (interior(unit)) {
+#pragma unroll
+                for (int r = 0; r < ROUNDS; r++)
+                    if (reached(r)) put_piece(r);
+                return;
+            }
 #pragma unroll
             for (int r = 0; r < ROUNDS; r++) {
                 const uintptr_t at = piece_at(unit, r);
                 if (inside(at, unit)) {
-                    *(uint4*)(raw_put + 64 * r) = ahead[r];
+                    put_piece(r);
                 } else if (at < fetch_row + (uintptr_t)(unit + 1) * RAW) {
                     for (int h = 0; h < 16; h += 2)
                         if (at + h >= w_begin && at + h < w_end) *(uint16_t*)(raw_put + 64 * r + h) = *(const uint16_t*)(at + h);
@@ -259,18 +315,21 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
         };
         // expanding: lane % 8 is the row, lane / 8 the sub-block of the half super-block.  The eight rows of a quarter warp
         // store the same piece of their swizzled rows, which is eight different bank groups.
-        const int r7 = lane & 7, q = lane >> 3;
-        const uint32_t dec_lo = (uint32_t)w_begin + (uint32_t)min(row0 + PF_WARP_ROWS * warp + r7, a.M - 1) * (uint32_t)a.row_bytes;
-        const uint8_t* raw_get = raw + r7 * PITCH;
+        // TA: a lane is a row of the warp's quarter, the warp's sub-block of the half is warp / 4.
+        const int r7 = TA ? lane : lane & 7, q = TA ? warp >> 2 : lane >> 3;
+        const uint32_t dec_lo = (uint32_t)w_begin + (uint32_t)min(row0 + (TA ? 32 * (warp & 3) : first_row) + r7, a.M - 1) * (uint32_t)a.row_bytes;
+        const uint8_t* raw_get = raw_all + ((TA ? 32 * (warp & 3) : first_row) + r7) * PITCH;
         const uint32_t* tab = grid_copy<FMT>(tab_smem, lane);
         uint8_t* put = stages + (q >> 1) * PF_A_SLAB_BYTES + (PF_WARP_ROWS * warp + r7) * 128;
         const int unit_end = sb_end * 2 / UNIT_HALVES;
-        int st = 0;
+        const uint32_t a_tmem = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)((a.n_tile + 31) / 32 * 32 + 16 * q);   // TA: this warp's columns of stage 0
+        int st = 0, buf = 0;
         uint32_t use = 0;
         fetch(sb_begin * 2 / UNIT_HALVES);
         for (int unit = sb_begin * 2 / UNIT_HALVES; unit < unit_end; unit++) {
             put_raw(unit);
-            __syncwarp();
+            if (TA) named_bar_sync(1 + (warp & 3), 128);   // (the buffer of two units before is free: its readers have come here since)
+            else __syncwarp();
             if (unit + 1 < unit_end) fetch(unit + 1);
             const uint8_t* blk = raw_get + ((dec_lo + (uint32_t)unit * RAW) & 15u);
 #pragma unroll
@@ -280,6 +339,15 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                 uint32_t p[16];
                 operand_pairs<FMT, F16>(o, !ALIGNED && (FMT == T_Q4_K || FMT == T_Q5_K) && a.exact, p);
                 mbar_wait_bounded(smem_u32(&empty_a[st]), use ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
+                if constexpr (TA) {
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    tmem_st16(a_tmem + (uint32_t)(st * PF_TA_STAGE_COLS), p);
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&full_a[st]));
+                    if (++st == a_stages) { st = 0; use ^= 1u; }
+                    continue;
+                }
                 // row of the tile: 128 bytes; 16-byte chunk c goes to chunk c ^ (row & 7) (128-byte swizzle)
                 uint8_t* arow = put + st * PF_A_BYTES;
 #pragma unroll
@@ -289,10 +357,28 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                 if (lane == 0) mbar_arrive(smem_u32(&full_a[st]));
                 if (++st == PF_A_STAGES) { st = 0; use ^= 1u; }
             }
+            if (TA) {   // the other buffer
+                buf ^= 1;
+                raw_put += buf ? pf_raw_ta(FMT) : -pf_raw_ta(FMT);
+                raw_get += buf ? pf_raw_ta(FMT) : -pf_raw_ta(FMT);
+            }
         }
     } else if (warp == PF_DECODE_WARPS) {
         // ---------------- operand B: activation tiles by TMA ----------------
-        if (lane == 0) {
+        if (TA) {
+            if (lane == 0) {
+                int st = 0;
+                uint32_t use = 0;
+                for (int pair = 2 * sb_begin; pair < 2 * sb_end; pair++) {
+                    mbar_wait_bounded(smem_u32(&empty_a[st]), use ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
+                    const uint32_t fb = smem_u32(&full_a[st]), to = smem_u32(stages_b + st * b_stage_bytes);
+                    mbar_arrive_expect_tx(fb, (uint32_t)b_stage_bytes);
+                    tma_load_2d(to, &xmap, 2 * pair * PF_KSLAB, tok0, fb);
+                    tma_load_2d(to + (uint32_t)(b_stage_bytes / 2), &xmap, (2 * pair + 1) * PF_KSLAB, tok0, fb);
+                    if (++st == a_stages) { st = 0; use ^= 1u; }
+                }
+            }
+        } else if (lane == 0) {
             int st = 0;
             uint32_t use = 0;
             for (int slab = 4 * sb_begin; slab < 4 * sb_end; slab++)
@@ -312,8 +398,33 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
         const uint32_t idesc = pf_idesc(F16, a.n_tile);
         const uint64_t desc0 = umma_desc_sw128(0);
         const uint32_t a_lo = (smem_u32(stages) & 0x3FFFFu) >> 4, b_lo = (smem_u32(stages_b) & 0x3FFFFu) >> 4;
+        const uint32_t a_tmem = tmem_base + (uint32_t)((a.n_tile + 31) / 32 * 32);   // TA: A stages behind the accumulator
         int sa = 0, sb = 0;
         uint32_t use_a = 0, use_b = 0, accum = 0;
+        if constexpr (TA) {
+            // One wait, eight MMA and one commit per 128 K: with a wait and a commit per 64 K and operand this warp set the pace
+            // (16384 x 5120 Q4_K, 16 or 77 tokens: 1300 clocks per 128 K, of which the tensor core needs 200 to 430).
+            for (int pair = 2 * sb_begin; pair < 2 * sb_end; pair++) {
+                mbar_wait_bounded(smem_u32(&full_a[sa]), use_a, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint64_t bdesc = desc0 + (b_lo + (uint32_t)((sa * b_stage_bytes) >> 4));
+                const uint32_t at = a_tmem + (uint32_t)(sa * PF_TA_STAGE_COLS), half_b = (uint32_t)(b_stage_bytes >> 5);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        asm volatile(
+                            "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                            "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+                            ::"r"(tmem_base), "r"(at + (uint32_t)(8 * k)), "l"(bdesc + (uint64_t)((k >> 2) * half_b + 2 * (k & 3))), "r"(idesc),
+                              "r"(k > 0 ? 1u : accum)
+                            : "memory");
+                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_a[sa])) : "memory");
+                }
+                __syncwarp();
+                accum = 1u;
+                if (++sa == a_stages) { sa = 0; use_a ^= 1u; }
+            }
+        } else
         for (int pair = 2 * sb_begin; pair < 2 * sb_end; pair++) {
             mbar_wait_bounded(smem_u32(&full_a[sa]), use_a, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
 #pragma unroll
@@ -342,7 +453,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                 }
                 accum = 1u;
             }
-            if (++sa == PF_A_STAGES) { sa = 0; use_a ^= 1u; }
+            if (++sa == a_stages) { sa = 0; use_a ^= 1u; }
         }
         if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_done)) : "memory");
         __syncwarp();
@@ -445,17 +556,20 @@ EncodeTiledFn encode_fn() {
 // How a GEMM is cut: token tiles of n_acc x n_tile tokens and K shared by `splits` CTAs.
 struct PrefillCut { int n_acc, n_tile, tok_tiles, splits, b_stages; };
 
-// Picks the cut by its time in SM clocks: rounds of CTAs over the SMs, a K-slab at a time.  A slab takes about 700 clocks
-// to decode plus 1.35 per token (measured, 16384 x 5120 Q4_K: 16 tokens 41 us, 200 52 us, 512 78 us on one round of 128
-// CTAs); 9000 clocks start a CTA and drain it, 8 per token store the tile; a cluster's exchange costs 3000 and another 8
-// per token.  Clusters of three and more leave some SMs of a GPC unused (at M = 5120, 120 CTAs in threes take 60 us where
-// 160 in fours, 132 of which fit at once, take 88).  Against every cut of up to twice as many token tiles and up to
-// eight CTAs, over 11 shapes and 9 token counts, the cut picked was within 3 % of the fastest in all but five cases (9 %).
-// M = 5120, K = 17408, IQ4_XS, 512 tokens: 277 us unsplit, 101 us with three CTAs a tile.
+// what a CTA receives from the others of its cluster (over the rings, idle by then; operand A in tensor memory: and what follows)
+int exchange_bytes(const PrefillCut& c) { return (c.splits - 1) * ((c.n_acc * c.n_tile / 16 + c.splits - 1) / c.splits) * (16 * PF_ROWS * 4); }
+
+// Picks the cut by its time in SM clocks: rounds of CTAs over the SMs, a K-slab at a time.  A slab takes about 800 clocks plus
+// 1.25 per token with operand A in shared memory (two accumulators), 480 plus the tokens squared over 140 with operand A in
+// tensor memory (measured, 16384 x 5120 Q4_K: 16 tokens 25 us, 77 27 us, 200 35 us, 256 43 us, 512 72 us on one round of 128 CTAs);
+// 9000 clocks start a CTA and drain it, 8 per token store the tile; a cluster's exchange costs 6000 and another 16 per token.
+// Clusters of three and more leave some SMs of a GPC unused (at M = 5120, 120 CTAs in threes take 60 us where 160 in fours, 132
+// of which fit at once, take 88), those of seven and eight more of them (2048 x 4096 IQ2_XS, 77 tokens: 128 CTAs in eights 21.8
+// us, 96 in sixes 14.4).  Against every cut of one to three token tiles and up to eight CTAs, over five shapes and 16 to 500
+// tokens, the cut picked is within 7 % of the fastest.  M = 5120, K = 17408, IQ4_XS, 512 tokens: 277 us unsplit, 101 us in threes.
 bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* best) {
     const long long row_tiles = (M + PF_ROWS - 1) / PF_ROWS;
     const int nsb = K / 256;
-    const int room = ctx->smem_optin - pf_fixed_smem(fmt);
     double best_cost = 0.0;
     bool found = false;
     const int min_tiles = (B + 2 * PF_MAX_N - 1) / (2 * PF_MAX_N);
@@ -467,27 +581,28 @@ bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* 
         const int tile = c.n_acc * c.n_tile;
         c.tok_tiles = (B + tile - 1) / tile;
         if (ctx->prefill_tiles && want != ctx->prefill_tiles) continue;
-        const int stage = c.n_tile * PF_KSLAB * 2;
-        c.b_stages = std::min(PF_B_MAX_STAGES, room / stage);
+        const bool ta = c.n_acc == 1;
+        const int room = ctx->smem_optin - pf_fixed_smem(fmt, ta);
+        const int stage = c.n_tile * PF_KSLAB * 2 * (ta ? 2 : 1);
+        c.b_stages = std::min(ta ? pf_ta_stages(c.n_tile) : PF_B_MAX_STAGES, room / stage);
         if (c.b_stages < 2) continue;
         for (c.splits = 1; c.splits <= std::min(PF_MAX_SPLITS, nsb); c.splits++) {
             if (ctx->prefill_splits && c.splits != ctx->prefill_splits) continue;
-            const int own_chunks = (tile / 16 + c.splits - 1) / c.splits;
-            if ((c.splits - 1) * own_chunks * (16 * PF_ROWS * 4) > PF_A_STAGES * PF_A_BYTES + c.b_stages * stage) continue;
+            if (ta ? 1024 + exchange_bytes(c) > ctx->smem_optin : exchange_bytes(c) > PF_A_STAGES * PF_A_BYTES + c.b_stages * stage) continue;
             const long long ctas = row_tiles * c.tok_tiles * c.splits;
-            const int slots = c.splits <= 2 ? ctx->sm_count : ctx->sm_count * 9 / 10 / c.splits * c.splits;
+            const int slots = c.splits <= 2 ? ctx->sm_count : (c.splits <= 6 ? ctx->sm_count * 9 / 10 : ctx->sm_count * 3 / 4) / c.splits * c.splits;
             const double rounds = (double)((ctas + slots - 1) / slots);
-            const double slab = 700.0 + 1.35 * tile;
-            const double cost = rounds * (4.0 * ((nsb + c.splits - 1) / c.splits) * slab + 9000.0 + 8.0 * tile + (c.splits > 1 ? 3000.0 + 8.0 * tile : 0.0));
+            const double slab = ta ? 480.0 + (double)tile * tile / 140.0 : 800.0 + 1.25 * tile;
+            const double cost = rounds * (4.0 * ((nsb + c.splits - 1) / c.splits) * slab + 9000.0 + 8.0 * tile + (c.splits > 1 ? 6000.0 + 16.0 * tile : 0.0));
             if (!found || cost < best_cost) { found = true; best_cost = cost; *best = c; }
         }
     }
     return found;
 }
 
-template <int FMT, bool F16, bool ALIGNED>
-int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st) {
-    auto kern = prefill_kernel<FMT, F16, ALIGNED>;
+template <int FMT, bool F16, bool ALIGNED, bool TA>
+int launch_prefill_as(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st) {
+    auto kern = prefill_kernel<FMT, F16, ALIGNED, TA>;
     bool known = false;   // opt-in shared-memory size: once per context (= device) and kernel
     for (int i = 0; i < ctx->n_configured; i++) known |= ctx->configured[i] == (const void*)kern;
     if (!known) {
@@ -499,7 +614,7 @@ int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& ma
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)((a.M + PF_ROWS - 1) / PF_ROWS * cut.splits), (unsigned)cut.tok_tiles);
     cfg.blockDim = dim3(PF_THREADS);
-    cfg.dynamicSmemBytes = (size_t)(pf_fixed_smem(FMT) + cut.b_stages * cut.n_tile * PF_KSLAB * 2);
+    cfg.dynamicSmemBytes = (size_t)std::max(pf_fixed_smem(FMT, TA) + cut.b_stages * cut.n_tile * PF_KSLAB * 2 * (TA ? 2 : 1), TA ? 1024 + exchange_bytes(cut) : 0);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -510,6 +625,11 @@ int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& ma
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, map);
     if (e != cudaSuccess) { (void)cudaGetLastError(); ctx->last_cuda = (int)e; return Q38B_ERR_CUDA; }
     return Q38B_OK;
+}
+
+template <int FMT, bool F16, bool ALIGNED>
+int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st) {
+    return cut.n_acc == 1 ? launch_prefill_as<FMT, F16, ALIGNED, true>(ctx, a, map, cut, st) : launch_prefill_as<FMT, F16, ALIGNED, false>(ctx, a, map, cut, st);
 }
 
 template <int FMT>
