@@ -123,8 +123,7 @@ int q38b_quantize_act_q8(q38b_ctx* ctx, const float* x_dev, int K, int n_rows, i
  * its scales at d_dev + c * act_ld / 32 (act_ld a multiple of 32, >= K).  The integer sums per 32 weights are exact and
  * each is scaled by its own activation scale.  Every column has the one-column kernel's arithmetic, so column c equals
  * the nb = 1 call on that column bit for bit (the promise of src/cuda/gemv.cuh:31-34); the columns share a launch
- * and the decoding of the weights (three or two on rows so long that four do not fit shared memory, e.g. Q8_0 from
- * K = 10496, Q6_K and IQ2_XS at K = 17408). */
+ * and the decoding of the weights, as many as fit shared memory. */
 int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W_dev, size_t row_bytes, int K, int M, const int8_t* q_dev,
                      const float* d_dev, int nb, int act_ld, float* y_dev, int y_ld, int accumulate, void* stream);
 

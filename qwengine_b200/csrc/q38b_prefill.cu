@@ -9,14 +9,14 @@
 //     with the 128-byte swizzle in shared memory (a warp owns eight rows), up to 256 in tensor memory (a lane is a row);
 //   * one thread streams the matching activation tiles (operand B, [tokens x 64] per K-slab) with tiled TMA loads
 //     (hardware swizzle, zero fill past the last token; no multicast);
-//   * one thread issues tcgen05.mma (cta_group::1, kind::f16, M = 128, N = 16..256, K = 16) into one or two fp32
+//   * one thread issues tcgen05.mma (kind::f16, M = 128, N = 16..256, K = 16; from 257 tokens on two CTAs as a pair, M = 256) into one or two fp32
 //     accumulators in tensor memory and commits each stage to its "empty" mbarrier;
 //   * all 16 decode warps read the accumulators back (tcgen05.ld 32x32b) and store Y, 32 consecutive rows per warp and token.
 // Where row tiles and token tiles alone leave SMs idle, the CTAs of a cluster share a tile's K: each multiplies a range
 // of super-blocks and the partial sums meet through distributed shared memory, added in rank order.
-// Measured on B200, 17408 x 5120 IQ3_XXS / 5120 x 17408 IQ4_XS with 1024 tokens: 211 / 286 us -> 161 / 194 us; 77 tokens of a
-// whole Q4_K / Q6_K layer 698 -> 199 us, 154 us with operand A in tensor memory.  Up to 256 tokens the expanders set the pace,
-// from 500 the activation tiles (64 bytes a clock and SM from L2) and the shared-memory traffic of 128-row tiles do.
+// Measured on B200, 17408 x 5120 IQ3_XXS / 5120 x 17408 IQ4_XS with 1024 tokens: 211 / 286 us -> 161 / 194 us; in pairs 143
+// for the former; 77 tokens of a whole Q4_K / Q6_K layer 698 -> 199 us, 154 us with operand A in tensor memory.  Up to 256 tokens the expanders set the pace,
+// from 500 the tensor core and the shared-memory traffic do.
 // All mbarrier waits are bounded; tensor memory is released before the kernel returns, also after a timeout.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -67,6 +67,8 @@ constexpr int PF_TA_STAGE_COLS = 64;   // 128 rows x 128 K of 16-bit weights: 64
 constexpr int PF_TA_MAX_STAGES = 6;
 __host__ __device__ constexpr int pf_ta_stages(int n_tile) { return (512 - (n_tile + 31) / 32 * 32) / PF_TA_STAGE_COLS < PF_TA_MAX_STAGES ? (512 - (n_tile + 31) / 32 * 32) / PF_TA_STAGE_COLS : PF_TA_MAX_STAGES; }
 
+enum : int { PF_SMEM = 0, PF_TMEM = 1, PF_PAIR = 2 };   // where operand A goes; PF_PAIR: shared memory of two CTAs
+
 struct PrefillArgs {
     const uint8_t* W;
     long long row_bytes;
@@ -95,6 +97,13 @@ __device__ __forceinline__ uint32_t pf_idesc(bool f16, int n_tile) {
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+                 "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+
+// the same, counted on a barrier of either CTA of a pair
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(map), "r"(x), "r"(y), "r"(bar)
                  : "memory");
 }
@@ -173,6 +182,19 @@ __device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void st_peer_f32(uint32_t addr, uint32_t v) { asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 
+// Arrives on a barrier of another CTA of the cluster.  (The weights it announces were made visible to the asynchronous proxy
+// before, in the shared memory of the SM that holds them, where the tensor core reads them; release and acquire at cluster scope
+// would add a memory fence of some 1800 clocks: 16384 x 5120 Q4_K, 1024 tokens 322 us against 138.)
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t addr) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory"); }
+// the barrier is arrived on when the tensor core has done all that was issued before (both CTAs of a pair: in each of them)
+template <bool PAIR>
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // 16 columns of this warp's 32 rows: 32 16-bit weights of a row
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile(
@@ -201,8 +223,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // decode warps write the weights and move the raw blocks twice, 140 KB of traffic or 1100 clocks of some 1700 measured; from
 // tensor memory the weights cost none of it.  With one wait and one commit per 128 K and the unchecked fetch, 16384 x 5120 Q4_K,
 // 77 tokens 39.6 -> 27.9 us, 17408 x 5120 IQ3_XXS 51.4 -> 42.0, 5120 x 17408 Q6_K 55.1 -> 45.4, a Q4_K / Q6_K layer 199 -> 154 us.
-template <int FMT, bool F16, bool ALIGNED, bool TA>
+// PAIR: two CTAs (a cluster of two, row tiles 2i and 2i + 1) multiply as one, M = 256 (cta_group::2): each expands its 128 rows and
+// loads half of every activation tile, CTA 0 issues, each CTA's tensor memory holds its own rows.  From 257 tokens on a slab of
+// 64 K moves 176 KB through an SM's shared memory otherwise (32 KB tiles written and read for each accumulator), 1375 clocks of
+// which the tensor core needs 1024; in pairs 112 KB, and half the activation bytes from L2 (16384 x 5120 Q4_K,
+// 1024 tokens 146 -> 132 us, 17408 x 5120 IQ3_XXS 161 -> 143; 512 tokens of the former 72 -> 66).
+template <int FMT, bool F16, bool ALIGNED, int MODE>
 __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArgs a, const __grid_constant__ CUtensorMap xmap) {
+    constexpr bool TA = MODE == PF_TMEM, PAIR = MODE == PF_PAIR;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t* full_a = (uint64_t*)smem;              // [A stages] the 16 decode warps arrive
     constexpr int MAX_A = TA ? PF_TA_MAX_STAGES : PF_A_STAGES;
@@ -213,13 +241,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
     uint64_t* acc_done = empty_b + PF_B_MAX_STAGES;  // [1]
     uint32_t* tmem_slot = (uint32_t*)(acc_done + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    const int b_stage_bytes = a.n_tile * (PF_KSLAB * 2) * (TA ? 2 : 1);   // TA: a stage is 128 K of both operands, one barrier each way
+    const int b_stage_bytes = a.n_tile * (PF_KSLAB * 2) * (TA ? 2 : 1) / (PAIR ? 2 : 1);   // TA: a stage is 128 K of both operands, one barrier each way
     uint8_t* stages = smem + 1024;                                   // ring of weight tiles (TA: none)
     uint8_t* stages_b = stages + (TA ? 0 : PF_A_STAGES * PF_A_BYTES); // ring of activation tiles
     uint8_t* raw_all = stages_b + a.b_stages * b_stage_bytes;         // the decode warps' raw blocks
     uint32_t* tab_smem = (uint32_t*)(raw_all + (TA ? 2 * pf_raw_ta(FMT) : pf_raw_smem(FMT)));
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rank = a.splits > 1 ? (int)cluster_rank() : 0;
+    const int half_id = PAIR ? (int)cluster_rank() : 0;   // which CTA of the pair this is
     const int row0 = (int)(blockIdx.x / (unsigned)a.splits) * PF_ROWS;
     const int tile_tok = a.n_acc * a.n_tile;
     const int tok0 = blockIdx.y * tile_tok;
@@ -230,7 +259,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
     if (tid == 0) {
         *abort_flag = 0;
         for (int s = 0; s < a_stages; s++) {
-            mbar_init(smem_u32(&full_a[s]), PF_DECODE_WARPS + (TA ? 1 : 0));   // one arrival per warp (TA: and the activations')
+            mbar_init(smem_u32(&full_a[s]), PF_DECODE_WARPS * (PAIR ? 2 : 1) + (TA ? 1 : 0));   // one arrival per warp (PAIR: of both CTAs, in CTA 0; TA: and the activations')
             mbar_init(smem_u32(&empty_a[s]), 1);
         }
         for (int s = 0; s < a.b_stages; s++) {
@@ -241,12 +270,18 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
         mbar_fence_init();
     }
     if (warp == PF_DECODE_WARPS + 1) {   // this warp owns the tensor memory allocation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        if constexpr (PAIR) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+        } else {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(tmem_cols) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
     }
     fill_grid_table<FMT>(tab_smem, a.grid_src, tid, PF_THREADS);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if (PAIR) cluster_sync_all();   // the other CTA's barriers are initialised
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     if (tid == 0 && (smem_u32(stages) & 1023u)) atomicOr(a.status, ST_TMEM_TIMEOUT);   // swizzled tiles need 1024-byte alignment
@@ -354,7 +389,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                 for (int c = 0; c < 4; c++) *(uint4*)(arow + 16 * ((4 * (q & 1) + c) ^ r7)) = make_uint4(p[4 * c], p[4 * c + 1], p[4 * c + 2], p[4 * c + 3]);
                 fence_proxy_async();                                 // generic-proxy stores -> visible to the tensor core
                 __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&full_a[st]));
+                if (lane == 0) {
+                    if (PAIR && half_id == 1) mbar_arrive_peer(peer_smem(smem_u32(&full_a[st]), 0u));
+                    else mbar_arrive(smem_u32(&full_a[st]));
+                }
                 if (++st == PF_A_STAGES) { st = 0; use ^= 1u; }
             }
             if (TA) {   // the other buffer
@@ -384,9 +422,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
             for (int slab = 4 * sb_begin; slab < 4 * sb_end; slab++)
                 for (int n = 0; n < a.n_acc; n++) {
                     mbar_wait_bounded(smem_u32(&empty_b[st]), use ^ 1u, abort_flag, a.status, ST_WAIT_EMPTY_TIMEOUT);
-                    const uint32_t fb = smem_u32(&full_b[st]);
-                    mbar_arrive_expect_tx(fb, (uint32_t)b_stage_bytes);
-                    tma_load_2d(smem_u32(stages_b + st * b_stage_bytes), &xmap, slab * PF_KSLAB, tok0 + n * a.n_tile, fb);
+                    const uint32_t fb = smem_u32(&full_b[st]), to = smem_u32(stages_b + st * b_stage_bytes);
+                    if constexpr (PAIR) {   // both halves count on CTA 0's barrier
+                        if (half_id == 0) mbar_arrive_expect_tx(fb, 2u * (uint32_t)b_stage_bytes);
+                        tma_load_2d_pair(to, &xmap, slab * PF_KSLAB, tok0 + n * a.n_tile + half_id * (a.n_tile / 2), peer_smem(fb, 0u));
+                    } else {
+                        mbar_arrive_expect_tx(fb, (uint32_t)b_stage_bytes);
+                        tma_load_2d(to, &xmap, slab * PF_KSLAB, tok0 + n * a.n_tile, fb);
+                    }
                     if (++st == a.b_stages) { st = 0; use ^= 1u; }
                 }
         }
@@ -395,7 +438,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
         // The whole warp walks the rings and one elected lane issues: descriptors, addresses and counts are then the same in
         // every lane and stay in uniform registers.  (Under `if (lane == 0)` an MMA took about 250 clocks to issue, four
         // times what the tensor core needs for 16 tokens: 16384 x 5120 Q4_K, 16 tokens 62 -> 40 us.)
-        const uint32_t idesc = pf_idesc(F16, a.n_tile);
+        const uint32_t idesc = pf_idesc(F16, a.n_tile) + (PAIR ? (uint32_t)(PF_ROWS >> 4) << 24 : 0u);   // PAIR: M = 256
         const uint64_t desc0 = umma_desc_sw128(0);
         const uint32_t a_lo = (smem_u32(stages) & 0x3FFFFu) >> 4, b_lo = (smem_u32(stages_b) & 0x3FFFFu) >> 4;
         const uint32_t a_tmem = tmem_base + (uint32_t)((a.n_tile + 31) / 32 * 32);   // TA: A stages behind the accumulator
@@ -418,13 +461,13 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                             ::"r"(tmem_base), "r"(at + (uint32_t)(8 * k)), "l"(bdesc + (uint64_t)((k >> 2) * half_b + 2 * (k & 3))), "r"(idesc),
                               "r"(k > 0 ? 1u : accum)
                             : "memory");
-                    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_a[sa])) : "memory");
+                    umma_commit<false>(smem_u32(&empty_a[sa]));
                 }
                 __syncwarp();
                 accum = 1u;
                 if (++sa == a_stages) { sa = 0; use_a ^= 1u; }
             }
-        } else
+        } else if (!(PAIR && half_id == 1))   // (CTA 0 of a pair issues for both)
         for (int pair = 2 * sb_begin; pair < 2 * sb_end; pair++) {
             mbar_wait_bounded(smem_u32(&full_a[sa]), use_a, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
 #pragma unroll
@@ -436,17 +479,24 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
                     const uint64_t bdesc = desc0 + (b_lo + (uint32_t)((sb * b_stage_bytes) >> 4));
                     if (elect_one()) {
 #pragma unroll
-                        for (int k = 0; k < PF_KSLAB / 16; k++)
-                            asm volatile(
-                                "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-                                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-                                ::"r"(tmem_base + (uint32_t)(n * PF_MAX_N)), "l"(adesc + (uint64_t)(2 * k)), "l"(bdesc + (uint64_t)(2 * k)), "r"(idesc),
-                                  "r"(k > 0 ? 1u : accum)
-                                : "memory");
-                        // frees the stages once the tensor core has read them
-                        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_b[sb])) : "memory");
-                        if (slab == 1 && n == a.n_acc - 1)
-                            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&empty_a[sa])) : "memory");
+                        for (int k = 0; k < PF_KSLAB / 16; k++) {
+                            const uint32_t to = tmem_base + (uint32_t)(n * PF_MAX_N), add = k > 0 ? 1u : accum;
+                            if constexpr (PAIR)
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(to), "l"(adesc + (uint64_t)(2 * k)),
+                                    "l"(bdesc + (uint64_t)(2 * k)), "r"(idesc), "r"(add)
+                                    : "memory");
+                            else
+                                asm volatile(
+                                    "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+                                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(to), "l"(adesc + (uint64_t)(2 * k)),
+                                    "l"(bdesc + (uint64_t)(2 * k)), "r"(idesc), "r"(add)
+                                    : "memory");
+                        }
+                        // frees the stages once the tensor core has read them (PAIR: in both CTAs)
+                        umma_commit<PAIR>(smem_u32(&empty_b[sb]));
+                        if (slab == 1 && n == a.n_acc - 1) umma_commit<PAIR>(smem_u32(&empty_a[sa]));
                     }
                     __syncwarp();
                     if (++sb == a.b_stages) { sb = 0; use_b ^= 1u; }
@@ -455,7 +505,7 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
             }
             if (++sa == a_stages) { sa = 0; use_a ^= 1u; }
         }
-        if (elect_one()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(acc_done)) : "memory");
+        if (!(PAIR && half_id == 1) && elect_one()) umma_commit<PAIR>(smem_u32(acc_done));
         __syncwarp();
     }
 
@@ -533,8 +583,10 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
     __syncthreads();
     if (warp == PF_DECODE_WARPS + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
+        else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
+    if (PAIR) cluster_sync_all();   // neither CTA leaves while the other may still signal it
 }
 
 
@@ -554,13 +606,13 @@ EncodeTiledFn encode_fn() {
 }
 
 // How a GEMM is cut: token tiles of n_acc x n_tile tokens and K shared by `splits` CTAs.
-struct PrefillCut { int n_acc, n_tile, tok_tiles, splits, b_stages; };
+struct PrefillCut { int n_acc, n_tile, tok_tiles, splits, b_stages, mode; };
 
 // what a CTA receives from the others of its cluster (over the rings, idle by then; operand A in tensor memory: and what follows)
 int exchange_bytes(const PrefillCut& c) { return (c.splits - 1) * ((c.n_acc * c.n_tile / 16 + c.splits - 1) / c.splits) * (16 * PF_ROWS * 4); }
 
 // Picks the cut by its time in SM clocks: rounds of CTAs over the SMs, a K-slab at a time.  A slab takes about 800 clocks plus
-// 1.25 per token with operand A in shared memory (two accumulators), 480 plus the tokens squared over 140 with operand A in
+// 1.25 per token with operand A in shared memory (two accumulators; in pairs 0.8), 480 plus the tokens squared over 140 with operand A in
 // tensor memory (measured, 16384 x 5120 Q4_K: 16 tokens 25 us, 77 27 us, 200 35 us, 256 43 us, 512 72 us on one round of 128 CTAs);
 // 9000 clocks start a CTA and drain it, 8 per token store the tile; a cluster's exchange costs 6000 and another 16 per token.
 // Clusters of three and more leave some SMs of a GPC unused (at M = 5120, 120 CTAs in threes take 60 us where 160 in fours, 132
@@ -577,22 +629,24 @@ bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* 
         const int per = (B + want - 1) / want;
         PrefillCut c;
         c.n_acc = per > PF_MAX_N ? 2 : 1;
-        c.n_tile = ((per + c.n_acc - 1) / c.n_acc + 15) / 16 * 16;
+        const int step = c.n_acc == 2 ? 32 : 16;   // (in pairs each CTA loads half of a tile)
+        c.n_tile = ((per + c.n_acc - 1) / c.n_acc + step - 1) / step * step;
         const int tile = c.n_acc * c.n_tile;
         c.tok_tiles = (B + tile - 1) / tile;
         if (ctx->prefill_tiles && want != ctx->prefill_tiles) continue;
         const bool ta = c.n_acc == 1;
         const int room = ctx->smem_optin - pf_fixed_smem(fmt, ta);
         const int stage = c.n_tile * PF_KSLAB * 2 * (ta ? 2 : 1);
-        c.b_stages = std::min(ta ? pf_ta_stages(c.n_tile) : PF_B_MAX_STAGES, room / stage);
-        if (c.b_stages < 2) continue;
+        if (room / stage < 2) continue;
         for (c.splits = 1; c.splits <= std::min(PF_MAX_SPLITS, nsb); c.splits++) {
             if (ctx->prefill_splits && c.splits != ctx->prefill_splits) continue;
+            c.mode = ta ? PF_TMEM : c.splits == 1 && row_tiles > 1 ? PF_PAIR : PF_SMEM;
+            c.b_stages = std::min(ta ? pf_ta_stages(c.n_tile) : PF_B_MAX_STAGES, room / (c.mode == PF_PAIR ? stage / 2 : stage));
             if (ta ? 1024 + exchange_bytes(c) > ctx->smem_optin : exchange_bytes(c) > PF_A_STAGES * PF_A_BYTES + c.b_stages * stage) continue;
-            const long long ctas = row_tiles * c.tok_tiles * c.splits;
+            const long long ctas = (c.mode == PF_PAIR ? (row_tiles + 1) / 2 * 2 : row_tiles) * c.tok_tiles * c.splits;
             const int slots = c.splits <= 2 ? ctx->sm_count : (c.splits <= 6 ? ctx->sm_count * 9 / 10 : ctx->sm_count * 3 / 4) / c.splits * c.splits;
             const double rounds = (double)((ctas + slots - 1) / slots);
-            const double slab = ta ? 480.0 + (double)tile * tile / 140.0 : 800.0 + 1.25 * tile;
+            const double slab = ta ? 480.0 + (double)tile * tile / 140.0 : c.mode == PF_PAIR ? 800.0 + 0.8 * tile : 800.0 + 1.25 * tile;
             const double cost = rounds * (4.0 * ((nsb + c.splits - 1) / c.splits) * slab + 9000.0 + 8.0 * tile + (c.splits > 1 ? 6000.0 + 16.0 * tile : 0.0));
             if (!found || cost < best_cost) { found = true; best_cost = cost; *best = c; }
         }
@@ -600,9 +654,10 @@ bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* 
     return found;
 }
 
-template <int FMT, bool F16, bool ALIGNED, bool TA>
+template <int FMT, bool F16, bool ALIGNED, int MODE>
 int launch_prefill_as(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st) {
-    auto kern = prefill_kernel<FMT, F16, ALIGNED, TA>;
+    constexpr bool TA = MODE == PF_TMEM, PAIR = MODE == PF_PAIR;
+    auto kern = prefill_kernel<FMT, F16, ALIGNED, MODE>;
     bool known = false;   // opt-in shared-memory size: once per context (= device) and kernel
     for (int i = 0; i < ctx->n_configured; i++) known |= ctx->configured[i] == (const void*)kern;
     if (!known) {
@@ -612,16 +667,17 @@ int launch_prefill_as(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& ma
     }
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3((unsigned)((a.M + PF_ROWS - 1) / PF_ROWS * cut.splits), (unsigned)cut.tok_tiles);
+    const int row_tiles = (a.M + PF_ROWS - 1) / PF_ROWS;
+    cfg.gridDim = dim3((unsigned)(PAIR ? (row_tiles + 1) / 2 * 2 : row_tiles * cut.splits), (unsigned)cut.tok_tiles);
     cfg.blockDim = dim3(PF_THREADS);
-    cfg.dynamicSmemBytes = (size_t)std::max(pf_fixed_smem(FMT, TA) + cut.b_stages * cut.n_tile * PF_KSLAB * 2 * (TA ? 2 : 1), TA ? 1024 + exchange_bytes(cut) : 0);
+    cfg.dynamicSmemBytes = (size_t)std::max(pf_fixed_smem(FMT, TA) + cut.b_stages * (cut.n_tile * PF_KSLAB * 2 * (TA ? 2 : 1) / (PAIR ? 2 : 1)), TA ? 1024 + exchange_bytes(cut) : 0);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)cut.splits;
+    attr[0].val.clusterDim.x = PAIR ? 2u : (unsigned)cut.splits;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = cut.splits > 1 ? 1 : 0;
+    cfg.numAttrs = PAIR || cut.splits > 1 ? 1 : 0;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a, map);
     if (e != cudaSuccess) { (void)cudaGetLastError(); ctx->last_cuda = (int)e; return Q38B_ERR_CUDA; }
     return Q38B_OK;
@@ -629,7 +685,11 @@ int launch_prefill_as(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& ma
 
 template <int FMT, bool F16, bool ALIGNED>
 int launch_prefill_op(q38b_ctx* ctx, const PrefillArgs& a, const CUtensorMap& map, const PrefillCut& cut, cudaStream_t st) {
-    return cut.n_acc == 1 ? launch_prefill_as<FMT, F16, ALIGNED, true>(ctx, a, map, cut, st) : launch_prefill_as<FMT, F16, ALIGNED, false>(ctx, a, map, cut, st);
+    switch (cut.mode) {
+        case PF_TMEM: return launch_prefill_as<FMT, F16, ALIGNED, PF_TMEM>(ctx, a, map, cut, st);
+        case PF_PAIR: return launch_prefill_as<FMT, F16, ALIGNED, PF_PAIR>(ctx, a, map, cut, st);
+        default: return launch_prefill_as<FMT, F16, ALIGNED, PF_SMEM>(ctx, a, map, cut, st);
+    }
 }
 
 template <int FMT>
@@ -655,7 +715,7 @@ int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     CUtensorMap map;
     const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)B};
     const cuuint64_t strides[1] = {(cuuint64_t)ldx * 2};
-    const cuuint32_t box[2] = {PF_KSLAB, (cuuint32_t)cut.n_tile};
+    const cuuint32_t box[2] = {PF_KSLAB, (cuuint32_t)(cut.mode == PF_PAIR ? cut.n_tile / 2 : cut.n_tile)};
     const cuuint32_t estr[2] = {1, 1};
     if (enc(&map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)X, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
