@@ -580,13 +580,14 @@ __global__ void __launch_bounds__(PF_THREADS, 1) prefill_kernel(const PrefillArg
             }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (PAIR) cluster_sync_all();   // the allocation is both CTAs': neither gives it back before the other's last read
+    else __syncthreads();
     if (warp == PF_DECODE_WARPS + 1) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
         else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(tmem_cols) : "memory");
     }
-    if (PAIR) cluster_sync_all();   // neither CTA leaves while the other may still signal it
+    if (PAIR) cluster_sync_all();   // neither CTA leaves before both have given it back
 }
 
 
