@@ -661,7 +661,7 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
     if (one_column_only((int)type) && nb > 1) {
         // launches of as many columns as fit; every column is the nb = 1 result
         for (int c = 0; c < nb;) {
-            const int n = std::max(1, q38b_cols_fit(ctx, type, K, &M, 1, row_bytes, nb - c, false));
+            const int n = std::max(1, q38b_cols_take(ctx, type, K, &M, 1, row_bytes, nb - c, false));
             const uint8_t* xq = (const uint8_t*)q8k + (size_t)c * q8k_stride * Q8K_BYTES;
             float* peers_c[7];
             for (int i = 0; i < n_peers; i++) peers_c[i] = y_peers[i] + (size_t)c * y_ld;
@@ -711,11 +711,13 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
     return q38b_cols_launch(ctx, cols_call(type, W, row_bytes, K, M, q8k, q8k_stride, nb, y, y_ld, accumulate, y_peers, n_peers), stream);
 }
 
+static bool gemvn_group_args(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, int nb) {
+    if (!ctx || n_mats < 1 || n_mats > G1_MAX_MATS || !known_format(type) || K <= 0 || K % 256 || nb < 1 || nb > 8) return false;
+    return row_bytes >= q38b_row_bytes(type, K) && !(one_column_only((int)type) && nb == 1);
+}
+
 int q38b_gemvn_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M, int nb) {
-    if (!ctx || n_mats < 1 || n_mats > G1_MAX_MATS || !known_format(type) || K <= 0 || K % 256 || nb < 1 || nb > 8) return 0;
-    if (row_bytes < q38b_row_bytes(type, K)) return 0;
-    if (one_column_only((int)type) && nb == 1) return 0;
-    return q38b_cols_fit(ctx, type, K, M, n_mats, row_bytes, nb, false) == nb;
+    return gemvn_group_args(ctx, type, n_mats, row_bytes, K, nb) && q38b_cols_take(ctx, type, K, M, n_mats, row_bytes, nb, false) == nb;
 }
 
 int q38b_gemvn_group(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const* W, size_t row_bytes, int K, const int* M,
@@ -728,7 +730,7 @@ int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* con
                        const long long* y_ld, float* const* y_peers, int n_peers, void* stream) {
     if (!ctx || !W || !M || !y || !y_ld || (!q8k == !x_f32) || n_mats < 1 || n_mats > G1_MAX_MATS) return Q38B_ERR_ARG;
     if (n_peers < 0 || n_peers > 7 || (n_peers > 0 && !y_peers)) return Q38B_ERR_ARG;   // y_peers[i * n_peers + r]: peer r's copy of matrix i's output
-    if (!q38b_gemvn_group_plannable(ctx, type, n_mats, row_bytes, K, M, nb)) return Q38B_ERR_UNSUPPORTED;
+    if (!gemvn_group_args(ctx, type, n_mats, row_bytes, K, nb)) return Q38B_ERR_UNSUPPORTED;
     const int al = format_alignment(type);
     if (row_bytes % al) return Q38B_ERR_ALIGN;
     if (q8k && (((uintptr_t)q8k & 3) || q8k_stride < K / 256)) return Q38B_ERR_ALIGN;
@@ -755,7 +757,8 @@ int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* con
     c.x_f32_ld = x_f32_ld;
     c.y_peers = y_peers;
     c.n_peers = n_peers;
-    return q38b_cols_launch(ctx, c, stream);
+    const int rc = q38b_cols_launch(ctx, c, stream);
+    return rc == Q38B_ERR_NOMEM ? Q38B_ERR_UNSUPPORTED : rc;
 }
 
 int q38b_gemv_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M) {
@@ -857,7 +860,7 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     int rc = Q38B_OK;
     for (int c = 0; c < nb && rc == Q38B_OK;) {
         Plan1 p;
-        int n = nb - c > 1 ? q38b_cols_fit(ctx, type, K, &M, 1, row_bytes, nb - c, true) : 1;
+        int n = nb - c > 1 ? q38b_cols_take(ctx, type, K, &M, 1, row_bytes, nb - c, true) : 1;
         if (n > 1) {
             ColsCall call = cols_call(type, W, row_bytes, K, M, q + (size_t)c * act_ld, 0, n, y + (size_t)c * y_ld, y_ld, accumulate, nullptr, 0);
             call.xq_ld = act_ld;

@@ -2,6 +2,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "../../include/q38b200.h"
@@ -26,39 +27,69 @@ int part_count(uint32_t type, int K, bool a32) {
     return cut_into_parts(type, K, a32) ? std::min(GEMV_MAX_PARTS, (nsb + most - 1) / most) : 1;
 }
 
-// Whether at most two of the rows g of a tile, `pitch` bytes apart, meet on a bank when their four lanes each read `bytes` side by
-// side (all eight rows with one load, four with a 64-bit load, which is served half a warp at a time).
-bool few_conflicts(int pitch, int bytes) {
-    int meet = 0;
-    for (int k = 1; k < (bytes == 8 ? 4 : 8); k++) {
-        const int d = k * pitch % 128;
-        meet += d < 4 * bytes || 128 - d < 4 * bytes;
-    }
-    return meet <= 1;
-}
-// bytes a lane takes from its row with the decoder's main load
-int lane_bytes(uint32_t type) {
+// How many different words the lanes of a decoder's main load want from the bank that most of them meet on, rows `pitch` bytes apart
+// (a 64-bit load is served half a warp, four rows, at a time).
+int bank_degree(uint32_t type, int pitch) {
+    int bytes, step;   // of a lane's load, and between the four lanes of a row
     switch (type) {
-        case T_Q4_K: case T_Q5_K: case T_Q8_0: return 8;
-        case T_IQ4_XS: case T_Q6_K: case T_Q2_K: return 4;
-        case T_IQ3_XXS: case T_IQ3_S: case T_IQ2_XS: return 2;
-        default: return 1;
+        case T_Q4_K: case T_Q5_K: bytes = step = 8; break;
+        case T_IQ4_XS: case T_Q2_K: bytes = step = 4; break;
+        case T_Q8_0: bytes = 2; step = 8; break;
+        case T_Q6_K: bytes = 2; step = 4; break;
+        case T_IQ3_XXS: case T_IQ3_S: case T_IQ2_XS: bytes = step = 2; break;
+        default: bytes = step = 1; break;
     }
+    int want[32] = {}, most = 1;
+    int seen[64], n = 0;
+    for (int g = 0; g < (bytes == 8 ? 4 : 8); g++)
+        for (int b = 0; b < 4 * step; b += std::max(4, step == 8 && bytes == 2 ? 8 : 4)) {
+            const int w = (g * pitch + b) / 4;
+            bool had = false;
+            for (int i = 0; i < n; i++) had |= seen[i] == w;
+            if (had) continue;
+            seen[n++] = w;
+            most = std::max(most, ++want[w % 32]);
+        }
+    return most;
+}
+// a 64-bit load wants the rows an odd multiple of 32 bytes apart, the others of 16
+int padded_pitch(uint32_t type, int bytes) {
+    const bool wide = type == T_Q4_K || type == T_Q5_K || type == T_Q8_0;
+    int pitch = align_up(bytes, 16);
+    while (wide ? pitch % 64 != 32 : pitch % 32 != 16) pitch += 16;
+    return pitch;
 }
 
 struct Plan {
     GemvArgs a;
     int grid;
     int smem;
+    double rating;   // of the division: the share of the launch left to the decoders
 };
 
 int table_bytes(uint32_t type) {
     return type == T_IQ3_XXS ? 1024 << cb1_rep_log2(T_IQ3_XXS) : type == T_IQ3_S ? 2048 << cb1_rep_log2(T_IQ3_S) : gridx_bytes((int)type);
 }
 
-// any: also a plan that leaves most warps without work.
 // Carves up the shared memory of one CTA: barriers | activation scales | activations | zeros | tables | unit sums | ring.
-int plan_gemv(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nb, bool a32, bool any, Plan* p) {
+//
+// How a tile's row is divided: into chunks of chunk_sb super-blocks (a stage each), a chunk into units of one, two or four
+// super-blocks, the units among kw warps; rows with few units leave warps for further groups, each with tiles of its own.  A
+// division is rated by the share of the launch that it leaves to the decoders:
+//   * units on the warps: work / (rounds of the warps), each unit with a fixed cost of 0.55 of a super-block;
+//   * nine warps and more keep the schedulers busy, as long as each scheduler has as many of them: 12 warps beat 18 (17408 x 2816
+//     IQ3_S, 3 x 4 warps 16.1 us, 6 x 3 17.5); of a last round of tiles that some groups sit out about half is lost, the others
+//     being faster meanwhile (6144 x 5120 IQ2_S, 2.6 tiles a CTA: two groups 13.4 us, one 14.3);
+//   * a copy costs the copy engine its bytes and 300 more;
+//   * one copy of 16 packed rows a stage loses 18 % to a copy per padded row (its rows meet on banks, and nothing of the stage can be
+//     read before all of it is there), and 4 % for every further row that meets on a bank: 17408 x 5120 Q8_0, seven columns, whose
+//     rows all meet in twos on two banks, 39.1 us in one copy, 27.0 in sixteen.  It is for rows of a few hundred bytes.
+// How far the ring runs ahead has no term: any two stages a group are enough.  Measured over all divisions of 593 shapes (thirteen
+// formats, 5120 and 17408 rows of 1024 to 17408 weights, two to eight columns, Q8_K and per-32) the division picked takes 1.2 % more
+// than the best on average and 18 % at most; rated by bytes under way, as before, it took 4.9 % more on average and 56 % at most.
+// With 356 shapes of 1024 to 12288 rows it is 1.6 % and 23 %.
+constexpr double UNIT_COST = 0.55, BUSY_WARPS = 9.0, COPY_BYTES = 300.0, ONE_COPY = 0.82, PER_ROW_MEETING = 0.04;
+int plan_gemv(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nb, bool a32, Plan* p) {
     const int bb = block_bytes((int)type), nsb = K / 256;
     const int budget = ctx->smem_optin;
     GemvArgs& a = p->a;
@@ -76,6 +107,8 @@ int plan_gemv(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_ma
     for (int q = 0; q <= a.n_parts; q++) a.part_sb0[q] = (int)((long long)nsb * q / a.n_parts);
     for (int q = 0; q < a.n_parts; q++) a.item_sb = std::max(a.item_sb, a.part_sb0[q + 1] - a.part_sb0[q]);
     if (a.n_parts > 1 && (long long)a.n_tiles * a.n_parts > ctx->part_items) return Q38B_ERR_NOMEM;   // the scratch area's size
+    const long long items = (long long)a.n_tiles * a.n_parts;
+    p->grid = (int)std::max<long long>(1, std::min<long long>(ctx->sm_count, items));
     // a CTA's range of (part, tile) items touches at most two neighbouring parts: it stages their activations only
     a.act_sb = a.n_parts == 1 ? nsb : std::min(nsb, 2 * a.item_sb);
     a.off_actd = GEMV_HEADER;
@@ -85,42 +118,38 @@ int plan_gemv(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_ma
     a.off_cb = a.off_zero + (wants_zeros((int)type) ? 384 : 0);
     a.off_sgn = a.off_cb + align_up(table_bytes(type), 128);
     a.off_red = a.off_sgn + (sign_table((int)type) ? 128 * 8 * SIGN_COPIES : 0);
-    // How a tile's row is divided: into chunks of chunk_sb super-blocks (a stage each), a chunk into units of one, two or four
-    // super-blocks, the units among kw warps; rows with few units leave warps for further groups, each with tiles of its own.
-    // Rated by the share of the warps' time that is work (a unit's fixed cost counts as UNIT_COST of a super-block) and by the
-    // bytes that the ring can have under way while a stage is being read.
-    constexpr double UNIT_COST = 0.4;
-    const int packed = nsb * bb, lb = lane_bytes(type);
-    const bool packed_rows = a.n_parts == 1 && (long long)row_bytes == packed && few_conflicts(packed, lb);
-    double best = 0.0;
+    const int packed = nsb * bb;
+    const bool packed_rows = a.n_parts == 1 && (long long)row_bytes == packed;
+    const double one_copy_worth = packed_rows ? ONE_COPY / (1.0 + PER_ROW_MEETING * (bank_degree(type, packed) - 1)) : 0.0;
+    const double cta_items = (double)items / p->grid;
+    p->rating = 0.0;
     for (int unit = 1; unit <= 4; unit *= 2)
-        for (int n_chunks = 1; n_chunks <= (best > 0.0 ? 4 : a.item_sb); n_chunks++) {
+        for (int n_chunks = 1; n_chunks <= (p->rating > 0.0 ? std::min(a.item_sb, 12) : a.item_sb); n_chunks++) {
             const int cs = std::min(a.item_sb, ((a.item_sb + n_chunks - 1) / n_chunks + unit - 1) / unit * unit);
             if ((a.item_sb + cs - 1) / cs != n_chunks) continue;
-            const bool one_copy = n_chunks == 1 && packed_rows;
-            // rows an odd multiple of 16 bytes apart (32 for 64-bit loads) meet no bank
-            int pitch = one_copy ? packed : align_up(cs * bb + 32, 16);
-            while (!one_copy && (lb == 8 ? pitch % 64 != 32 : pitch % 32 != 16)) pitch += 16;
-            const int stage = align_up(TILE_ROWS * pitch + 64, 128);
-            if (a.off_red + 2 * stage > budget) continue;
             const int slots = (a.item_sb + unit - 1) / unit, units = (cs + unit - 1) / unit;
-            const int copy = one_copy ? TILE_ROWS * packed : cs * bb;
-            if (best > 0.0 && copy < 512) break;
             const int least_rounds = (units + GEMV_MAX_WARPS - 1) / GEMV_MAX_WARPS;
-            for (int rounds = least_rounds; rounds <= std::min(units, least_rounds + 3); rounds++) {
-                const int kw = (units + rounds - 1) / rounds;
-                for (int groups = n_chunks == 1 ? GEMV_MAX_WARPS / kw : 1; groups >= 1; groups--) {
-                    const int off_stage = align_up(a.off_red + groups * GEMV_TILEBUF * slots * 64 * a.cols, 128);
-                    const int stages = std::min(GEMV_MAX_STAGES, (budget - off_stage) / stage) / groups * groups;
-                    if (stages < 2 * groups) continue;
-                    const double work = (double)a.item_sb / ((double)n_chunks * rounds * kw * (unit + UNIT_COST));
-                    const double warps = std::min(1.0, (kw * groups + 4) / 24.0);
-                    // bytes under way beside the stages being read, up to 48 KB; copies below 1.7 KB cost the copy engine's time
-                    const double ring = std::min(1.0, (double)(stages - groups) * stage / (48.0 * 1024)) * std::min(1.0, copy / 1700.0);
-                    const double score = work * warps * ring;
-                    if (score > best * 1.0001) {
-                        best = score;
-                        a.contiguous = one_copy ? 1 : 0;
+            for (int one_copy = n_chunks == 1 && packed_rows ? 1 : 0; one_copy >= 0; one_copy--) {
+                const int pitch = one_copy ? packed : padded_pitch(type, cs * bb + 32);
+                const int stage = align_up(TILE_ROWS * pitch + 64, 128);
+                if (a.off_red + 2 * stage > budget) continue;
+                const double copy = one_copy ? (double)TILE_ROWS * packed : (double)cs * bb;
+                const double copied = copy / (copy + COPY_BYTES) * (one_copy ? one_copy_worth : 1.0);
+                for (int rounds = least_rounds; rounds <= std::min(units, least_rounds + 5); rounds++) {
+                    const int kw = (units + rounds - 1) / rounds;
+                    const double rows = copied * a.item_sb / ((double)n_chunks * rounds * kw * (unit + UNIT_COST));
+                    if (rows <= p->rating) continue;
+                    for (int groups = n_chunks == 1 ? GEMV_MAX_WARPS / kw : 1; groups >= 1; groups--) {
+                        const int off_stage = align_up(a.off_red + groups * GEMV_TILEBUF * slots * 64 * a.cols, 128);
+                        const int stages = std::min(GEMV_MAX_STAGES, (budget - off_stage) / stage) / groups * groups;
+                        if (stages < 2 * groups) continue;
+                        const int warps = kw * groups;
+                        const double busy = std::min(1.0, warps / BUSY_WARPS) * warps / ((warps + 3) / 4 * 4);
+                        const double turns = cta_items / groups;
+                        const double rating = rows * busy * (a.n_parts == 1 ? std::sqrt(turns / std::ceil(turns)) : 1.0);
+                        if (rating <= p->rating) continue;
+                        p->rating = rating;
+                        a.contiguous = one_copy;
                         a.chunk_sb = cs;
                         a.unit_log2 = unit == 4 ? 2 : unit - 1;
                         a.kw = kw;
@@ -132,15 +161,10 @@ int plan_gemv(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_ma
                         a.off_stage = off_stage;
                         p->smem = off_stage + stages * stage;
                     }
-                    break;   // fewer groups are worth less
                 }
             }
         }
-    if (best == 0.0) return Q38B_ERR_NOMEM;
-    if (!any && a.kw * a.groups < std::min(8, (a.item_sb + 3) / 4)) return Q38B_ERR_NOMEM;   // fewer columns leave the ring room for chunks that feed the warps
-    const long long items = (long long)a.n_tiles * a.n_parts;
-    p->grid = (int)std::max<long long>(1, std::min<long long>(ctx->sm_count, items));
-    return Q38B_OK;
+    return p->rating > 0.0 ? Q38B_OK : Q38B_ERR_NOMEM;
 }
 
 template <int FMT, bool A32, bool PARTED>
@@ -178,22 +202,57 @@ int launch_format(q38b_ctx* ctx, const Plan& p, cudaStream_t st) {
 
 }  // namespace
 
+bool q38b_cols_in_parts(uint32_t type, int K) { return part_count(type, K, false) > 1; }
+
 long long q38b_cols_max_rows(const q38b_ctx* ctx, uint32_t type, int K) {
     const int parts = part_count(type, K, false);
     return parts == 1 ? 0 : ctx->part_items / parts * TILE_ROWS;
 }
 
-int q38b_cols_fit(const q38b_ctx* ctx, uint32_t type, int K, const int* M, int n_mats, size_t row_bytes, int nb, bool a32) {
+// A launch's time goes with about the 0.42nd power of its plan's rating down (5120 x 17408 IQ3_XXS, per-32: six columns at 0.213 47 us,
+// four at 0.473 34, seven at 0.048 92), so that all columns at once lose to two halves from a rating of a fifth of the halves' on:
+// there a long row's activations leave the ring two small stages that feed a few warps.
+int q38b_cols_take(const q38b_ctx* ctx, uint32_t type, int K, const int* M, int n_mats, size_t row_bytes, int left, bool a32) {
     if (a32 && type == T_Q6_K) return 0;
+    Plan all, half;
+    int n = std::min(8, left);
+    bool fits = plan_gemv(ctx, type, K, M, n_mats, row_bytes, n, a32, &all) == Q38B_OK;
+    while (n > 1 && (!fits || all.rating < 0.25)) {   // (no plan is rated above one and few above 0.8: others need no second look)
+        const int h = (n + 1) / 2;
+        const bool half_fits = plan_gemv(ctx, type, K, M, n_mats, row_bytes, h, a32, &half) == Q38B_OK;
+        if (fits && (!half_fits || all.rating >= 0.2 * half.rating)) break;
+        n = h;
+        fits = half_fits;
+        all = half;
+    }
+    return fits ? n : 0;
+}
+
+// Test hook (not in the public header): the division of a row for nb columns on a 148-SM device with 227 KB of shared memory a CTA, no
+// device needed: warps of a tile, groups, super-blocks a stage, stages, whether a stage is one copy, thousandths of the rating.
+extern "C" int q38b_debug_gemvn_plan(uint32_t type, int K, int M, size_t row_bytes, int nb, int a32, int* out) {
+    q38b_ctx ctx;
+    ctx.sm_count = 148;
+    ctx.smem_optin = 232448;
+    ctx.part_items = 131072;
     Plan p;
-    int n = std::min(8, nb);
-    while (n > 0 && plan_gemv(ctx, type, K, M, n_mats, row_bytes, n, a32, n == 1, &p) != Q38B_OK) n--;
-    return n;
+    const int rc = plan_gemv(&ctx, type, K, &M, 1, row_bytes, nb, a32 != 0, &p);
+    if (rc != Q38B_OK) return rc;
+    const int v[6] = {p.a.kw, p.a.groups, p.a.chunk_sb, p.a.n_stages, p.a.contiguous, (int)(1000.0 * p.rating)};
+    memcpy(out, v, sizeof(v));
+    return Q38B_OK;
+}
+extern "C" int q38b_debug_gemvn_take(uint32_t type, int K, int M, size_t row_bytes, int left, int a32) {
+    q38b_ctx ctx;
+    ctx.sm_count = 148;
+    ctx.smem_optin = 232448;
+    ctx.part_items = 131072;
+    return q38b_cols_take(&ctx, type, K, &M, 1, row_bytes, left, a32 != 0);
 }
 
 int q38b_cols_launch(q38b_ctx* ctx, const ColsCall& c, void* stream) {
     Plan p;
-    const int rc = plan_gemv(ctx, c.type, c.K, c.M, c.n_mats, c.row_bytes, c.nb, c.xd32 != nullptr, true, &p);
+    const int rc = plan_gemv(ctx, c.type, c.K, c.M, c.n_mats, c.row_bytes, c.nb, c.xd32 != nullptr, &p);
     if (rc != Q38B_OK) return rc;
     GemvArgs& a = p.a;
     for (int i = 0; i < c.n_mats; i++) {

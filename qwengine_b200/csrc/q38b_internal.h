@@ -64,8 +64,10 @@ struct ColsCall {
     long long xd32_ld = 0;
 };
 int q38b_cols_launch(q38b_ctx* ctx, const ColsCall& c, void* stream);
-// the most of nb columns (at most eight) that one launch can take; 0: none (Q6_K with per-32 activations: the one-column kernel's)
-int q38b_cols_fit(const q38b_ctx* ctx, uint32_t type, int K, const int* M, int n_mats, size_t row_bytes, int nb, bool a32);
+// how many of `left` columns the next of several launches takes (0: none has a plan; Q6_K with per-32 activations: the one-column kernel's)
+int q38b_cols_take(const q38b_ctx* ctx, uint32_t type, int K, const int* M, int n_mats, size_t row_bytes, int left, bool a32);
+// rows of Q8_K columns that are summed in K-parts (their sums are not the one-column kernel's)
+bool q38b_cols_in_parts(uint32_t type, int K);
 // rows one launch can take (K-parts: the size of the scratch area); 0: any number
 long long q38b_cols_max_rows(const q38b_ctx* ctx, uint32_t type, int K);
 
@@ -75,6 +77,7 @@ extern "C" int q38b_gemv_group_plannable(const q38b_ctx* ctx, uint32_t type, int
 extern "C" int q38b_gemv_group_peers(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const* W, size_t row_bytes, int K, const int* M,
                                      const void* q8k, const float* x_f32, float* const* y, float* const* y_peers, int n_peers, void* stream);
 // the same for the multi-column kernel (nb columns of Q8_K blocks, q8k_stride blocks apart; y[i][c * y_ld[i] + r]); no peers
+// (plannable: and better in one launch than in several)
 extern "C" int q38b_gemvn_group_plannable(const q38b_ctx* ctx, uint32_t type, int n_mats, size_t row_bytes, int K, const int* M, int nb);
 // the same with the columns given as floats (x_f32, x_f32_ld floats apart; quantized inside the kernel) instead of Q8_K
 // blocks, and with peer stores (y_peers[i * n_peers + r]: peer r's copy of matrix i's output)
