@@ -75,10 +75,10 @@ constexpr int G1_WARPS = 8;                  // consumer warps of a CTA when two
 // ... when a CTA has the SM to itself (measured on B200: the row-group decoder wants its 80 registers, which 20 warps
 // leave it; the others gain from more warps in flight, 5120 x 17408 IQ4_XS 15.7 -> 12.5 us)
 constexpr int G1_WARPS_ONE = 24, G1_WARPS_ONE_RG = 20;
-// several columns: the columns' activations and sums take registers (Q4_K / Q5_K: 20 a column); with the producer 16 warps
-// (12) leave a thread 128 (168), where 17 leave it 96 and spill
+// several columns: the columns' activations and sums take registers (Q4_K / Q5_K: 20 a column).  Two columns leave room for 19 warps
+// of 96 registers (17408 x 5120 Q5_K, per-32: 25.5 us with the 11 of the wide kernel, 19.3); three and four want 128 (168): 15 (11) warps
 constexpr int G1_COLS = 4;
-constexpr int g1_warps_cols(int fmt) { return fmt == T_Q4_K || fmt == T_Q5_K ? 11 : 15; }
+constexpr int g1_warps_cols(int fmt, int sum_cols) { return sum_cols == 2 ? 19 : fmt == T_Q4_K || fmt == T_Q5_K ? 11 : 15; }
 constexpr int G1_SMEM_BUDGET = 113 * 1024;   // two CTAs per SM (228 KB of shared memory per SM, 1 KB reserved per CTA)
 
 
@@ -89,7 +89,8 @@ struct Plan1 {
     int rows;   // rows per tile: 8, 4 or 2
     int rg;     // 1: row-group mapping (tables in static shared memory, activations staged twice)
     int occ;    // CTAs per SM: 2 (8 consumer warps) or 1 (24 consumer warps, the whole shared memory)
-    int nc;     // columns of the launch (more than one: the kernel for up to G1_COLS)
+    int nc;     // columns of the launch
+    int sum_cols;   // columns the kernel is built for: 1, 2 or G1_COLS
     int xt;     // 1: expanded grid tables (IQ2 / IQ1)
 };
 
@@ -98,16 +99,16 @@ bool rowgroup_eligible(uint32_t type, size_t row_bytes, int rows) { return type 
 
 // Shared-memory carve-up of the single-column kernel: barriers | activation scales | activations | codebook |
 // per-tile slice sums | ring of stages (8 row slots of one 1024-weight slice each).
-int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int G1_ROWS, int occ, int nc, int xt, Plan1* p) {
+int plan_gemv1_rows(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int G1_ROWS, int occ, int nc, int xt, Plan1* p, int sum_cols = 1) {
     const int bb = block_bytes((int)type);
     p->occ = occ;
     p->xt = xt;
     p->nc = nc;
     p->a.nc = nc;
-    const int sum_cols = nc > 1 ? G1_COLS : 1;   // columns a tile's sums are kept for
+    p->sum_cols = sum_cols;
     const int nsb = K / 256;
     const int rg = nc == 1 && ctx->rowgroup && rowgroup_eligible(type, row_bytes, G1_ROWS) ? 1 : 0;
-    const int warps = nc > 1 ? g1_warps_cols((int)type) : occ == 1 ? (rg ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
+    const int warps = nc > 1 ? g1_warps_cols((int)type, sum_cols) : occ == 1 ? (rg ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
     const int cb_entries = rg ? 0 : type == T_IQ3_XXS ? 256 : type == T_IQ3_S ? 512 : 0;   // row groups keep their tables in static shared memory
     const int budget = (occ == 1 ? ctx->smem_optin : std::min(ctx->smem_optin, G1_SMEM_BUDGET)) - 128 - (rg ? RG_STATIC_BYTES : 0);
     Gemv1Args& a = p->a;
@@ -205,10 +206,64 @@ int plan_gemv1(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_m
     return Q38B_ERR_NOMEM;
 }
 
-// Two to four columns of Q6_K in one launch: one CTA per SM, tiles of eight rows.
-int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nc, Plan1* p) {
-    memset(p, 0, sizeof(*p));
-    return ctx->one_cta ? plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p) : Q38B_ERR_NOMEM;
+// what cols_by_granule can ask for with Q8_K blocks; per-32 columns: every format
+constexpr bool granule_cols_q8k(int fmt, int sum_cols) {
+    return one_column_only(fmt) || fmt == T_Q8_0 || (sum_cols == 2 && (fmt == T_Q5_K || fmt == T_Q6_K));
+}
+// Two to four columns in one launch: one CTA per SM, tiles of eight rows.  Two columns that the kernel for two has no room for (its
+// 19 warps want a longer ring) take the one for four.
+int plan_gemv1_cols(const q38b_ctx* ctx, uint32_t type, int K, const int* Ms, int n_mats, size_t row_bytes, int nc, bool a32, Plan1* p) {
+    if (!ctx->one_cta) return Q38B_ERR_NOMEM;
+    for (int sum_cols = nc == 2 ? 2 : G1_COLS; sum_cols <= G1_COLS; sum_cols += 2) {
+        if (!a32 && !granule_cols_q8k((int)type, sum_cols)) continue;
+        memset(p, 0, sizeof(*p));
+        if (plan_gemv1_rows(ctx, type, K, Ms, n_mats, row_bytes, 8, 1, nc, gridx_copies((int)type) > 0, p, sum_cols) == Q38B_OK) return Q38B_OK;
+    }
+    return Q38B_ERR_NOMEM;
+}
+
+// Whether n = 2..4 columns on `rows` rows of nsb super-blocks take this kernel, which decodes a granule once for all of them and pays
+// a dp4a for each, instead of the several-column kernel, whose fragments cost the same for one column as for eight.  Same bits
+// either way; rows in K-parts never (other sums).  The lines are where the two met over 1024 to 65536 rows of 1024 to 17408 weights:
+// more warps and tables make this kernel's start longer (1024 x 1024: 5.0 to 6.5 us against 3.9 to 4.3), tiles of eight rows feed
+// more SMs where rows are few and long (1024 x 8192 IQ2_S: 1.26 times as fast).  Two columns of Q8_K blocks (several-column kernel
+// first, us): 17408 x 5120 IQ1_M 27.1 / 21.0, IQ2_S 24.8 / 22.0, Q5_K 20.2 / 18.6, Q6_K 26.3 / 21.1, but Q4_K 15.1 / 16.1 and 17408 x 2816
+// IQ2_XXS 14.6 / 15.0; Q2_K 5120 x 8192 12.4 / 13.2, x 17408 24.1 / 21.4.  Per-32 columns, which the other kernel scales every 32 weights
+// in floats: 17408 x 5120 Q2_K 24.9 / 17.8, Q4_K 20.2 / 16.4, IQ3_XXS 25.4 / 23.0, but IQ3_S 26.8 / 27.0 and 17408 x 1024 Q4_K 8.5 / 10.9.
+// Three and four columns gain less: Q8_0, whose fragments are scaled every 32 weights (5120 x 8192, three 18.2 / 15.8, four 18.5 / 17.2),
+// and long rows, whose activations leave the other kernel a short ring (5120 x 17408, per-32, three columns Q2_K 33.7 / 28.9, IQ1_M
+// 36.3 / 32.5; four IQ2_S 39.9 / 37.5).
+bool cols_by_granule(const q38b_ctx* ctx, uint32_t type, long long rows, int nsb, int n, bool a32) {
+    constexpr int NEVER = 1 << 30;
+    if ((!a32 && q38b_cols_in_parts(type, 256 * nsb)) || ctx->cols_route == 1) return false;
+    if (ctx->cols_route == 2) return true;
+    const bool few = rows <= 2048, many = rows >= 8192;
+    int from = NEVER;   // the shortest row
+    if (n == 2) {
+        switch (type) {
+            case T_Q8_0: from = many ? 4 : 8; break;
+            case T_Q6_K: from = few ? 11 : 8; break;
+            case T_IQ1_M: case T_IQ2_S: case T_IQ2_XS: from = few ? 20 : 8; break;
+            case T_IQ1_S: from = !few ? 16 : a32 ? 20 : 32; break;
+            case T_IQ2_XXS: from = a32 ? (few ? 20 : 16) : few ? 32 : 40; break;
+            case T_Q2_K: from = a32 ? (few ? 20 : 8) : few ? 32 : 49; break;
+            case T_Q4_K: from = a32 ? (few ? 11 : 8) : NEVER; break;
+            case T_Q5_K: from = a32 ? (few ? 11 : 8) : few ? 32 : many ? 20 : NEVER; break;
+            case T_IQ3_XXS: from = !a32 ? NEVER : few ? 32 : many ? 16 : 40; break;
+            case T_IQ4_XS: from = !a32 ? NEVER : few ? 20 : many ? 8 : 40; break;
+            default: from = !a32 ? NEVER : few ? 32 : 40; break;   // IQ3_S
+        }
+    } else {
+        switch (type) {
+            case T_Q8_0: from = n == 4 ? 24 : rows >= 16384 ? 4 : 20; break;
+            case T_Q2_K: from = a32 ? (n == 3 ? 20 : 64) : NEVER; break;
+            case T_IQ1_M: from = n == 3 ? 32 : 64; break;
+            case T_IQ2_S: from = n == 3 ? 48 : a32 ? 64 : NEVER; break;
+            case T_IQ2_XS: from = n == 3 ? 48 : NEVER; break;
+            default: break;
+        }
+    }
+    return nsb >= from;
 }
 
 // Whether one column with per-32 activations takes the plan `p` of one CTA per SM (else two).  These calls follow one another
@@ -237,17 +292,37 @@ bool act_q8_one_cta(const q38b_ctx* ctx, uint32_t type, const Plan1& p) {
     }
 }
 
-// How many of `left` columns the next launch of the one-column kernel takes (Q6_K with per-32 activations), with its plan in *p
-// when that is more than one: the most that fit shared memory, at most four; six are two threes.
+// How many of `left` columns the next launch of this kernel takes (Q6_K with per-32 activations, which has no other), with its plan
+// in *p when that is more than one: the most that fit shared memory, at most four; six are two threes.
 int next_cols(const q38b_ctx* ctx, uint32_t type, int K, int M, size_t row_bytes, int left, Plan1* p) {
     int n = left == 6 ? 3 : std::min(G1_COLS, left);
-    while (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, p) != Q38B_OK) n--;
+    while (n > 1 && plan_gemv1_cols(ctx, type, K, &M, 1, row_bytes, n, true, p) != Q38B_OK) n--;
+    return n;
+}
+
+// The next launch of `left` columns that keep the one-column kernel's bits: how many it takes (1: that kernel's single column) and
+// whether they go to the kernel that decodes a granule for all of them (its plan in *p).
+int next_launch(const q38b_ctx* ctx, uint32_t type, int K, const int* M, int n_mats, size_t row_bytes, int left, bool a32, bool* granule, Plan1* p) {
+    long long rows = 0;
+    for (int i = 0; i < n_mats; i++) rows += M[i];
+    auto by_granule = [&](int n) {
+        return n >= 2 && n <= G1_COLS && cols_by_granule(ctx, type, rows, K / 256, n, a32) && plan_gemv1_cols(ctx, type, K, M, n_mats, row_bytes, n, a32, p) == Q38B_OK;
+    };
+    *granule = by_granule(left);
+    if (*granule || left == 1) return left;
+    if (a32 && type == T_Q6_K) {
+        const int n = next_cols(ctx, type, K, M[0], row_bytes, left, p);
+        *granule = n > 1;
+        return n;
+    }
+    const int n = std::max(1, q38b_cols_take(ctx, type, K, M, n_mats, row_bytes, left, a32));
+    *granule = n < left && by_granule(n);
     return n;
 }
 
 template <int FMT, int ROWS, bool RG, bool A32 = false, int OCC = 2, int NC = 1, bool XT = false>
 int launch_gemv1_rows(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
-    constexpr int WARPS = NC > 1 ? g1_warps_cols(FMT) : OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
+    constexpr int WARPS = NC > 1 ? g1_warps_cols(FMT, NC) : OCC == 1 ? (RG ? G1_WARPS_ONE_RG : G1_WARPS_ONE) : G1_WARPS;
     auto kern = gemv1_kernel<FMT, WARPS, ROWS, RG, A32, OCC, NC, XT>;
     const int rc = q38b_ensure_kernel_smem(ctx, (const void*)kern, (OCC == 1 ? ctx->smem_optin : G1_SMEM_BUDGET) - (RG ? RG_STATIC_BYTES : 0), true);
     if (rc != Q38B_OK) return rc;
@@ -276,9 +351,11 @@ template <int FMT>
 int launch_gemv1(q38b_ctx* ctx, const Plan1& p, cudaStream_t st) {
     constexpr bool X = gridx_copies(FMT) > 0;
     if (p.nc > 1) {
-        if constexpr (FMT == T_Q6_K) {
-            if (p.a.xd32) return launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS>(ctx, p, st);
+        if (p.a.xd32) return p.sum_cols == 2 ? launch_gemv1_rows<FMT, 8, false, true, 1, 2, X>(ctx, p, st) : launch_gemv1_rows<FMT, 8, false, true, 1, G1_COLS, X>(ctx, p, st);
+        if constexpr (granule_cols_q8k(FMT, 2)) {
+            if (p.sum_cols == 2) return launch_gemv1_rows<FMT, 8, false, false, 1, 2, X>(ctx, p, st);
         }
+        if constexpr (granule_cols_q8k(FMT, G1_COLS)) return launch_gemv1_rows<FMT, 8, false, false, 1, G1_COLS, X>(ctx, p, st);
         return Q38B_ERR_ARG;
     }
     if (p.a.xd32) {   // per-32 activations: lane-per-granule mapping only
@@ -646,6 +723,32 @@ static ColsCall cols_call(uint32_t type, const void* W, size_t row_bytes, int K,
     return c;
 }
 
+// the columns of `c` on the one-column kernel's granules (p: their plan)
+static int granule_launch(q38b_ctx* ctx, Plan1& p, const ColsCall& c, cudaStream_t st) {
+    Gemv1Args& g = p.a;
+    for (int i = 0; i < c.n_mats; i++) {
+        (i == 0 ? g.W : g.W_more[i - 1]) = (const uint8_t*)c.W[i];
+        (i == 0 ? g.y : g.y_more[i - 1]) = c.y[i];
+        (i == 0 ? g.y_ld : g.y_ld_more[i - 1]) = c.y_ld[i];
+        (i == 0 ? g.M : g.M_more[i - 1]) = c.M[i];
+        for (int pr = 0; pr < c.n_peers; pr++) (i == 0 ? g.y_peer[pr] : g.y_peer_more[i - 1][pr]) = c.y_peers[i * c.n_peers + pr];
+    }
+    g.row_bytes = (long long)c.row_bytes;
+    g.xq = (const uint8_t*)c.xq;
+    g.xq_ld = c.xq_ld;
+    g.x_f32 = c.x_f32;
+    g.x_f32_ld = c.x_f32_ld;
+    g.xd32 = c.xd32;
+    g.xd32_ld = c.xd32_ld;
+    g.n_peers = c.n_peers;
+    g.static_weights = ctx->static_weights;
+    g.status = ctx->d_status;
+    g.codebook = q38b_grid_source(ctx, c.type);
+    g.K = c.K;
+    g.accumulate = c.accumulate;
+    return dispatch_gemv1(ctx, c.type, p, st);
+}
+
 int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_bytes, int K, int M, const void* q8k,
                           long long q8k_stride, int nb, float* y, long long y_ld, int accumulate, float* const* y_peers,
                           int n_peers, void* stream) {
@@ -658,15 +761,19 @@ int q38b_gemv_q8k_scatter(q38b_ctx* ctx, uint32_t type, const void* W, size_t ro
     const int al = format_alignment(type);
     if (((uintptr_t)W & 15) || (row_bytes % al) || ((uintptr_t)q8k & 3) || ((uintptr_t)y & 3)) return Q38B_ERR_ALIGN;
     cudaStream_t st = (cudaStream_t)stream;
-    if (one_column_only((int)type) && nb > 1) {
-        // launches of as many columns as fit; every column is the nb = 1 result
+    if (nb > 1 && !q38b_cols_in_parts(type, K)) {
+        // every column is what a launch of its own would give (but for the row groups of IQ3_XXS, a single column's)
         for (int c = 0; c < nb;) {
-            const int n = std::max(1, q38b_cols_take(ctx, type, K, &M, 1, row_bytes, nb - c, false));
+            Plan1 p1;
+            bool granule;
+            const int n = next_launch(ctx, type, K, &M, 1, row_bytes, nb - c, false, &granule, &p1);
             const uint8_t* xq = (const uint8_t*)q8k + (size_t)c * q8k_stride * Q8K_BYTES;
             float* peers_c[7];
             for (int i = 0; i < n_peers; i++) peers_c[i] = y_peers[i] + (size_t)c * y_ld;
-            const int rc = n == 1 ? q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, xq, q8k_stride, 1, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers, stream)
-                                  : q38b_cols_launch(ctx, cols_call(type, W, row_bytes, K, M, xq, q8k_stride, n, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers), stream);
+            const ColsCall call = cols_call(type, W, row_bytes, K, M, xq, q8k_stride, n, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers);
+            const int rc = granule ? granule_launch(ctx, p1, call, st)
+                         : n == 1 ? q38b_gemv_q8k_scatter(ctx, type, W, row_bytes, K, M, xq, q8k_stride, 1, y + (size_t)c * y_ld, y_ld, accumulate, peers_c, n_peers, stream)
+                                  : q38b_cols_launch(ctx, call, stream);
             if (rc != Q38B_OK) return rc;
             c += n;
         }
@@ -757,6 +864,11 @@ int q38b_gemvn_group_x(q38b_ctx* ctx, uint32_t type, int n_mats, const void* con
     c.x_f32_ld = x_f32_ld;
     c.y_peers = y_peers;
     c.n_peers = n_peers;
+    Plan1 p1;
+    long long rows = 0;
+    for (int i = 0; i < n_mats; i++) rows += M[i];
+    if (nb >= 2 && nb <= G1_COLS && cols_by_granule(ctx, type, rows, K / 256, nb, false) && plan_gemv1_cols(ctx, type, K, M, n_mats, row_bytes, nb, false, &p1) == Q38B_OK)
+        return granule_launch(ctx, p1, c, (cudaStream_t)stream);
     const int rc = q38b_cols_launch(ctx, c, stream);
     return rc == Q38B_ERR_NOMEM ? Q38B_ERR_UNSUPPORTED : rc;
 }
@@ -787,6 +899,13 @@ int q38b_debug_gemv1_cols(uint32_t type, int K, int M, size_t row_bytes, int lef
     ctx.smem_optin = 232448;
     Plan1 p1;
     return known_format(type) && K > 0 && K % 256 == 0 && left >= 1 ? next_cols(&ctx, type, K, M, row_bytes, left, &p1) : 0;
+}
+
+// Test hook: two to four columns by granules never (1), wherever there is a plan (2), by the rule (0)
+int q38b_debug_set_cols_route(q38b_ctx* ctx, int mode) {
+    if (!ctx || mode < 0 || mode > 2) return Q38B_ERR_ARG;
+    ctx->cols_route = mode;
+    return Q38B_OK;
 }
 
 int q38b_gemv_group(q38b_ctx* ctx, uint32_t type, int n_mats, const void* const* W, size_t row_bytes, int K, const int* M,
@@ -860,17 +979,17 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
     int rc = Q38B_OK;
     for (int c = 0; c < nb && rc == Q38B_OK;) {
         Plan1 p;
-        int n = nb - c > 1 ? q38b_cols_take(ctx, type, K, &M, 1, row_bytes, nb - c, true) : 1;
-        if (n > 1) {
-            ColsCall call = cols_call(type, W, row_bytes, K, M, q + (size_t)c * act_ld, 0, n, y + (size_t)c * y_ld, y_ld, accumulate, nullptr, 0);
-            call.xq_ld = act_ld;
-            call.xd32 = d + (size_t)c * (act_ld / 32);
-            call.xd32_ld = act_ld / 32;
+        bool granule;
+        const int n = next_launch(ctx, type, K, &M, 1, row_bytes, nb - c, true, &granule, &p);
+        ColsCall call = cols_call(type, W, row_bytes, K, M, q + (size_t)c * act_ld, 0, n, y + (size_t)c * y_ld, y_ld, accumulate, nullptr, 0);
+        call.xq_ld = act_ld;
+        call.xd32 = d + (size_t)c * (act_ld / 32);
+        call.xd32_ld = act_ld / 32;
+        if (n > 1 && !granule) {
             rc = q38b_cols_launch(ctx, call, stream);
             c += n;
             continue;
         }
-        if (n == 0) n = type == T_Q6_K ? next_cols(ctx, type, K, M, row_bytes, nb - c, &p) : 1;
         if (n == 1) {
             memset(&p, 0, sizeof(p));
             const bool fits_one = ctx->one_cta && type != T_Q8_0 && plan_gemv1_rows(ctx, type, K, &M, 1, row_bytes, 8, 1, 1, gridx_copies((int)type) > 0, &p) == Q38B_OK;
@@ -884,24 +1003,7 @@ int q38b_gemv_act_q8(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
                 else if (!fits_one) { rc = Q38B_ERR_NOMEM; break; }
             }
         }
-        Gemv1Args& g = p.a;
-        g.W = (const uint8_t*)W;
-        g.row_bytes = (long long)row_bytes;
-        g.xq = (const uint8_t*)(q + (size_t)c * act_ld);
-        g.xq_ld = act_ld;
-        g.xd32 = d + (size_t)c * (act_ld / 32);
-        g.xd32_ld = act_ld / 32;
-        g.x_f32 = nullptr;
-        g.y = y + (size_t)c * y_ld;
-        g.y_ld = y_ld;
-        g.n_peers = 0;
-        g.static_weights = ctx->static_weights;
-        g.status = ctx->d_status;
-        g.codebook = q38b_grid_source(ctx, type);
-        g.K = K;
-        g.M = M;
-        g.accumulate = accumulate ? 1 : 0;
-        rc = dispatch_gemv1(ctx, type, p, (cudaStream_t)stream);
+        rc = granule_launch(ctx, p, call, (cudaStream_t)stream);
         c += n;
     }
     ctx->rowgroup = saved_rg;

@@ -14,8 +14,9 @@
 // operations less (27B-shaped pass 3847 -> 3810 us, pass of a small model in 2-bit blocks 466 -> 458).  The sums are formed in
 // the order of the several-column kernel (q38b_gemv.cuh), so that a column's bits do not depend on how many share a launch.
 //
-// With NC = 4 the same kernel takes two to four columns of Q6_K with per-32 activations: a granule is decoded once
-// (q38b_decode1n.cuh) and multiplied with each column, whose result is the single-column launch's, bit for bit.
+// With NC = 2 or 4 the same kernel takes two to four columns: a granule is decoded once (q38b_decode1n.cuh) and multiplied with each
+// column, whose result is the single-column launch's, bit for bit.  cols_by_granule of q38b_api.cu says where that is faster than
+// the several-column kernel.
 #pragma once
 #include <type_traits>
 
@@ -51,10 +52,10 @@ struct Gemv1Args {
     int static_weights;     // 1: W was written long before this launch, the producer need not wait for earlier kernels
     int* status;
     const uint32_t* codebook;
-    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes) and xd32 (floats), and of each
+    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes), x_f32 and xd32 (floats), and of each
     // matrix's output (floats; the peers' as well)
     int nc;
-    long long xq_ld, xd32_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
+    long long xq_ld, x_f32_ld, xd32_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
     int K, M, accumulate;
     int nsb;                // super-blocks per row
     int n_slices;           // ceil(nsb / 4)
@@ -102,10 +103,10 @@ constexpr int RG_STATIC_BYTES = 4 * (RG_CB_WORDS + RG_SGN_WORDS);
 // all of the SM's shared memory: one set of tables and one quantized column per SM, deeper rings, larger tiles; the default
 // plan) or 2 (eight consumer warps and half the shared memory each, for shapes whose one-CTA plan does not fit and the
 // single per-32 columns that act_q8_one_cta names).
-// NC: columns at most (1 or 4).
+// NC: columns at most (1, 2 or 4).
 // XT: IQ2 / IQ1 with expanded grid tables (GranX), which want an SM's whole shared memory; without them the 16-bit codes.
-template <int FMT, int NC, bool XT> struct GranOf { using type = typename std::conditional<XT, GranX<FMT>, Gran<FMT>>::type; };
-template <> struct GranOf<T_Q6_K, 4, false> { using type = GranN<T_Q6_K>; };
+template <int FMT, int NC, bool XT> struct GranOf { using type = GranN<FMT>; };
+template <int FMT, bool XT> struct GranOf<FMT, 1, XT> { using type = typename std::conditional<XT, GranX<FMT>, Gran<FMT>>::type; };
 
 template <int FMT, int NWARPS, int ROWS, bool RG, bool A32, int OCC, int NC = 1, bool XT = false>
 __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gemv1Args a) {
@@ -115,7 +116,7 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     static_assert(!(RG && (A32 || NC > 1)), "per-32 activations and several columns run on the lane-per-granule mapping");
     const int nc = NC == 1 ? 1 : a.nc;
     static_assert(!XT || (OCC == 1 && gridx_copies(FMT) > 0), "expanded grids: IQ2 / IQ1 with one CTA per SM");
-    static_assert(NC == 1 || (FMT == T_Q6_K && A32 && !XT), "several columns: Q6_K with per-32 activations");
+    static_assert(NC == 1 || XT == (gridx_copies(FMT) > 0), "several columns of IQ2 / IQ1: expanded grids");
     using G = typename GranOf<FMT, NC, XT>::type;
     // tables of the row-group decoders: static shared memory (their addresses become immediates of the loads); kernels
     // without them have no static shared memory at all, so that two CTAs of 113 KB still fit an SM
@@ -267,17 +268,64 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
     }
     const int act_ld = a.n_slices * 1024, actd_ld = a.n_slices * 32;   // between the columns' staged values (bytes) and scales (floats)
     if constexpr (NC > 1) {
-        // several columns of per-32 activations: the words and scales of all of them are dealt to the threads
-        const int n_w = a.n_slices * 256;
-        for (int i = ctid; i < nc * actd_ld; i += NWARPS * 32) {
-            const int c = i / actd_ld, k = i - c * actd_ld;
-            actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xd32_ld + k] : 0.0f;
-        }
+        // the same two ways for several columns: the blocks (words, scales) of all of them are dealt to the warps (threads)
+        const int nsb4 = a.n_slices * 4;
+        auto put8 = [&](int c, int sb, int k0, uint32_t w0, uint32_t w1) {   // values k0 .. k0 + 7 of a slice, k0 a multiple of 8
+            uint8_t* dst = actq + c * act_ld + (sb >> 2) * 1024;
+            if (FMT == T_IQ4_XS) {
+#pragma unroll
+                for (int e = 0; e < 8; e++) {
+                    const int k = k0 + e;
+                    dst[act_slice_pos(FMT, (k & ~31) + act_stage_pos(FMT, k & 31))] = (uint8_t)((e < 4 ? w0 : w1) >> (8 * (e & 3)));
+                }
+            } else {
+                *(uint2*)(dst + act_slice_pos(FMT, k0)) = make_uint2(w0, w1);
+            }
+        };
+        if (!A32 && a.x_f32) {
+            constexpr int QB = 3;
+            for (int b0 = cw; b0 < nc * nsb4; b0 += QB * NWARPS) {
+                float4 lo4[QB], hi4[QB];
+#pragma unroll
+                for (int j = 0; j < QB; j++) {
+                    const int b = b0 + j * NWARPS, c = b / nsb4, sb = b - c * nsb4;
+                    lo4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    hi4[j] = lo4[j];
+                    if (c < nc && sb < a.nsb) {
+                        const float* src = a.x_f32 + (size_t)c * a.x_f32_ld + (size_t)sb * 256 + 8 * lane;
+                        lo4[j] = *(const float4*)src;
+                        hi4[j] = *(const float4*)(src + 4);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < QB; j++) {
+                    const int b = b0 + j * NWARPS, c = b / nsb4, sb = b - c * nsb4;
+                    if (c >= nc) continue;
+                    uint32_t w0 = 0, w1 = 0;
+                    float d = 0.0f;
+                    if (sb < a.nsb) {
+                        const float v[8] = {lo4[j].x, lo4[j].y, lo4[j].z, lo4[j].w, hi4[j].x, hi4[j].y, hi4[j].z, hi4[j].w};
+                        int s8;
+                        q8k_block_core(v, w0, w1, s8, d);
+                    }
+                    if (lane == 0) actd[c * actd_ld + sb * 8] = d;
+                    put8(c, sb, (sb & 3) * 256 + 8 * lane, w0, w1);
+                }
+            }
+        } else {
+            const int n_d = A32 ? actd_ld : nsb4, n_w = a.n_slices * 128;
+            for (int i = ctid; i < nc * n_d; i += NWARPS * 32) {
+                const int c = i / n_d, k = i - c * n_d;
+                if (A32) actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xd32_ld + k] : 0.0f;
+                else actd[c * actd_ld + k * 8] = k < a.nsb ? *(const float*)(a.xq + (size_t)c * a.xq_ld + (size_t)k * Q8K_BYTES) : 0.0f;
+            }
 #pragma unroll 4
-        for (int i = ctid; i < nc * n_w; i += NWARPS * 32) {
-            const int c = i / n_w, w = i - c * n_w, sb = w >> 6, wi = w & 63;
-            const uint32_t v = sb >= a.nsb ? 0u : *(const uint32_t*)(a.xq + (size_t)c * a.xq_ld + 4 * (size_t)w);
-            *(uint32_t*)(actq + c * act_ld + (sb >> 2) * 1024 + act_slice_pos(FMT, (sb & 3) * 256 + 4 * wi)) = v;
+            for (int i = ctid; i < nc * n_w; i += NWARPS * 32) {
+                const int c = i / n_w, w = i - c * n_w, sb = w >> 5, wi = w & 31;
+                const uint32_t* src = (const uint32_t*)(a.xq + (size_t)c * a.xq_ld + (A32 ? (size_t)sb * 256 : (size_t)sb * Q8K_BYTES + 4)) + 2 * wi;
+                const bool in = sb < a.nsb;
+                put8(c, sb, (sb & 3) * 256 + 8 * wi, in ? src[0] : 0u, in ? src[1] : 0u);
+            }
         }
     } else if (a.x_f32) {
         // quantize the column here (every CTA, the same arithmetic as quantize_q8k_kernel): one warp per 256 values.  The
@@ -439,31 +487,40 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         const bool live = gran_sb < a.nsb;
         // Q8_K columns: a super-block's lanes add exact integers, and one lane per row scales them (bits 1, 2, 4 of the lane
         // number, 1, 2 with two rows a pass, are the place inside the super-block); per-32 columns and Q8_0: floats throughout.
-        constexpr bool INT_SUMS = NC == 1 && !A32 && FMT != T_Q8_0;
+        constexpr bool INT_SUMS = !A32 && FMT != T_Q8_0, INT_MINS = INT_SUMS && Unit<FMT>::HAS_MIN;
         constexpr int SB_LANES = LPR / 4;
         using Sum = typename std::conditional<INT_SUMS, int, float>::type;
-        Sum acc[NC][PASSES], mins[INT_SUMS && Unit<FMT>::HAS_MIN ? PASSES : 1];
+        Sum acc[NC][PASSES], mins[NC][INT_MINS ? PASSES : 1];
         auto row_at = [&](int r) { return st + (r * a.slot_stride + (int)((src_lo + (uint32_t)r * rb_step) & 15u)); };
 #pragma unroll
         for (int ps = 0; ps < PASSES; ps++) {
             const SP rowp = row_at(LPR == 32 ? ps : 2 * ps + sub);
-            if constexpr (INT_SUMS) {
-                int ms;
-                acc[0][ps] = G::idot(rowp, acts[0], cb, lane, ms);
-                if constexpr (Unit<FMT>::HAS_MIN) mins[ps] = ms;
-            } else if constexpr (NC == 1) {
-                const float v = G::template dot<A32>(rowp, acts[0], cb, lane);
-                acc[0][ps] = live ? v : 0.0f;
-            } else {
+            if constexpr (NC > 1) {
                 const typename G::W g = G::decode(rowp, cb, lane);
+                float d = 0.0f, m = 0.0f;
+                if (!INT_SUMS) G::block_scale(rowp + (FMT == T_Q8_0 ? 34 * lane : BB * (LPR == 32 ? (lane >> 3) : ((lane & 15) >> 2))), d, m);
 #pragma unroll
                 for (int c = 0; c < NC; c++) {
-                    acc[c][ps] = 0.0f;
+                    acc[c][ps] = 0;
+                    if (INT_MINS) mins[c][ps] = 0;
                     if (c < nc) {
-                        const float v = G::template apply<A32>(g, acts[c]);
-                        acc[c][ps] = live ? v : 0.0f;
+                        if constexpr (INT_SUMS) {
+                            int ms;
+                            acc[c][ps] = G::isum(g, acts[c], ms);
+                            if constexpr (INT_MINS) mins[c][ps] = ms;
+                        } else {
+                            const float v = G::template apply<A32>(g, acts[c], d, m);
+                            acc[c][ps] = live ? v : 0.0f;
+                        }
                     }
                 }
+            } else if constexpr (INT_SUMS) {
+                int ms;
+                acc[0][ps] = G::idot(rowp, acts[0], cb, lane, ms);
+                if constexpr (INT_MINS) mins[0][ps] = ms;
+            } else {
+                const float v = G::template dot<A32>(rowp, acts[0], cb, lane);
+                acc[0][ps] = live ? v : 0.0f;
             }
         }
         if (!INT_SUMS) {   // (integer sums read the rows' factors below)
@@ -496,12 +553,12 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         for (int bit = 1; bit < SB_LANES; bit <<= 1) {
             if (n > 1) {
                 halve(v, bit, n);
-                if constexpr (INT_SUMS && Unit<FMT>::HAS_MIN) halve(mins, bit, n);
+                if constexpr (INT_MINS) halve(mins[c], bit, n);
                 n >>= 1;
                 if (lane & bit) myrow += n;
             } else {
                 v[0] += __shfl_xor_sync(0xffffffffu, v[0], bit);
-                if constexpr (INT_SUMS && Unit<FMT>::HAS_MIN) mins[0] += __shfl_xor_sync(0xffffffffu, mins[0], bit);
+                if constexpr (INT_MINS) mins[c][0] += __shfl_xor_sync(0xffffffffu, mins[c][0], bit);
             }
         }
         static_assert(PASSES <= SB_LANES, "one row a lane after the lanes of a super-block");
@@ -510,10 +567,12 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         if constexpr (INT_SUMS) {
             float d, m;
             G::block_scale(row_at(myrow) + BB * (LPR == 32 ? (lane >> 3) : ((lane & 15) >> 2)), d, m);
-            __syncwarp();
-            if (lane == 0) mbar_arrive_n(smem_u32(&empty[stage]), n_arr);
-            const float dx = acts[0].dx;
-            rowsum = Unit<FMT>::HAS_MIN ? block_value_min(d * dx, v[0], m * dx, mins[0]) : block_value(d * dx * Unit<FMT>::FACTOR, v[0]);
+            if (c == nc - 1) {
+                __syncwarp();
+                if (lane == 0) mbar_arrive_n(smem_u32(&empty[stage]), n_arr);
+            }
+            const float dx = acts[c].dx;
+            rowsum = INT_MINS ? block_value_min(d * dx, v[0], m * dx, mins[c][0]) : block_value(d * dx * Unit<FMT>::FACTOR, v[0]);
             rowsum = live ? rowsum : 0.0f;
         } else {
             rowsum = v[0];
@@ -529,10 +588,10 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
         if (slice == a.n_slices - 1) {
             // this warp finishes the tile: wait for the other slices, add them in slice order
             mbar_wait_bounded(tb, tile_par, abort_flag, a.status, ST_WAIT_FULL_TIMEOUT);
-            const int row = tr.row0 + lane % G1_ROWS, col = NC == 1 ? 0 : lane / G1_ROWS;   // NC > 1: eight rows and four columns are the 32 lanes
+            const int row = tr.row0 + lane % G1_ROWS, col = NC == 1 ? 0 : lane / G1_ROWS;   // NC > 1: one lane per row and column
             float* ym = mi == 0 ? a.y : a.y_more[mi - 1];
             const int Mm = mi == 0 ? a.M : a.M_more[mi - 1];
-            static_assert(NC == 1 || G1_ROWS * NC == 32, "one lane per row and column");
+            static_assert(NC == 1 || G1_ROWS * NC <= 32, "one lane per row and column");
             if (lane < G1_ROWS * NC && row < Mm && col < nc) {
                 const float* rs = red + (size_t)tslot * a.n_slices * (G1_ROWS * NC) + lane;
                 float v = 0.0f;

@@ -14,6 +14,7 @@ struct q38b_ctx {
     int rowgroup = 1;          // 0: the row-group mapping of the one-column kernel is not used (test hook q38b_debug_set_rowgroup)
     int one_cta = 1;           // one-column kernel with one CTA per SM where such a plan fits; 0: never (test hook q38b_debug_set_one_cta)
     int check_occupancy = 0, occupancy_shortfalls = 0;   // test hook q38b_debug_occupancy_shortfalls
+    int cols_route = 0;        // test hook q38b_debug_set_cols_route: 1 never, 2 always (where there is a plan) by granules
     int prefill_tiles = 0, prefill_splits = 0;   // test hook q38b_debug_set_prefill_cut
     int uniform_columns = 0;   // 1: single-column calls also run the tensor-core kernel (bit-identical to columns of wider calls)
     long long wait_budget_cycles = 4000000000LL;   // bounded waits on other GPUs (q38b_ctx_set_wait_budget_cycles)
