@@ -580,9 +580,7 @@ template <> struct Gran<T_IQ1_M> : GranPlain<T_IQ1_M> {
         const int ib = lane & 7;
         const uint32_t qs = sp_ld16(p, 4 * ib) | (sp_ld16(p, 4 * ib + 2) << 16);
         const uint32_t qh = sp_ld16(p, 32 + 2 * ib);                 // nibble l: 3 index bits and the delta sign of group l
-        const uint32_t s0 = sp_ld16(p, 48), s1 = sp_ld16(p, 50), s2 = sp_ld16(p, 52), s3 = sp_ld16(p, 54);
-        const uint32_t scw = (ib >> 1) == 0 ? s0 : (ib >> 1) == 1 ? s1 : (ib >> 1) == 2 ? s2 : s3;
-        const uint32_t t = scw >> (6 * (ib & 1));
+        const uint32_t t = sp_ld16(p, 48 + 2 * (ib >> 1)) >> (6 * (ib & 1));
         int S[2] = {0, 0};
 #pragma unroll
         for (int l = 0; l < 4; l++) {

@@ -92,8 +92,7 @@ template <int FMT> struct GranX {
         } else {
             const uint32_t qs = sp_ld16(p, 4 * ib) | (sp_ld16(p, 4 * ib + 2) << 16);
             const uint32_t qh = sp_ld16(p, 32 + 2 * ib);
-            const uint32_t s0 = sp_ld16(p, 48), s1 = sp_ld16(p, 50), s2 = sp_ld16(p, 52), s3 = sp_ld16(p, 54);
-            const uint32_t t = ((ib >> 1) == 0 ? s0 : (ib >> 1) == 1 ? s1 : (ib >> 1) == 2 ? s2 : s3) >> (6 * (ib & 1));
+            const uint32_t t = sp_ld16(p, 48 + 2 * (ib >> 1)) >> (6 * (ib & 1));
 #pragma unroll
             for (int l = 0; l < 4; l++) {
                 const uint32_t hn = qh >> (4 * l);
