@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <type_traits>
 
@@ -612,14 +613,32 @@ struct PrefillCut { int n_acc, n_tile, tok_tiles, splits, b_stages, mode; };
 // what a CTA receives from the others of its cluster (over the rings, idle by then; operand A in tensor memory: and what follows)
 int exchange_bytes(const PrefillCut& c) { return (c.splits - 1) * ((c.n_acc * c.n_tile / 16 + c.splits - 1) / c.splits) * (16 * PF_ROWS * 4); }
 
-// Picks the cut by its time in SM clocks: rounds of CTAs over the SMs, a K-slab at a time.  A slab takes about 800 clocks plus
-// 1.25 per token with operand A in shared memory (two accumulators; in pairs 0.8), 480 plus the tokens squared over 140 with operand A in
-// tensor memory (measured, 16384 x 5120 Q4_K: 16 tokens 25 us, 77 27 us, 200 35 us, 256 43 us, 512 72 us on one round of 128 CTAs);
-// 9000 clocks start a CTA and drain it, 8 per token store the tile; a cluster's exchange costs 6000 and another 16 per token.
-// Clusters of three and more leave some SMs of a GPC unused (at M = 5120, 120 CTAs in threes take 60 us where 160 in fours, 132
-// of which fit at once, take 88), those of seven and eight more of them (2048 x 4096 IQ2_XS, 77 tokens: 128 CTAs in eights 21.8
-// us, 96 in sixes 14.4).  Against every cut of one to three token tiles and up to eight CTAs, over five shapes and 16 to 500
-// tokens, the cut picked is within 7 % of the fastest.  M = 5120, K = 17408, IQ4_XS, 512 tokens: 277 us unsplit, 101 us in threes.
+// Clocks in which the expanders of a format bring 128 rows x 64 K into tensor memory
+double expand_clocks(int fmt) {
+    switch (fmt) {
+        case T_Q4_K: return 460.0;
+        case T_Q5_K: return 570.0;
+        case T_Q2_K: return 615.0;
+        case T_IQ1_S: return 645.0;
+        case T_IQ2_XXS: return 705.0;
+        case T_IQ2_XS: case T_IQ1_M: return 725.0;
+        case T_IQ2_S: return 745.0;
+        case T_IQ3_S: case T_IQ3_XXS: return 790.0;
+        case T_Q6_K: return 820.0;
+        case T_Q8_0: return 875.0;
+        default: return 940.0;   // IQ4_XS
+    }
+}
+// Picks the cut by its time in SM clocks: rounds of CTAs over the SMs, a K-slab at a time.  A slab takes the longer of what its
+// expanders and what its tokens take, added as fourth powers: the format's clocks against 2.5 a token with operand A in tensor memory,
+// 0.6 of them and 710 against 1.65 a token in pairs, 0.47 of them and 1000 against 2.3 with operand A in shared memory (their swizzled
+// stores and barriers are the same for every format).  10400 clocks start a CTA and drain it, 30 per token store the tile; a cluster's
+// exchange costs 500 and another 1.4 per token.  Clusters of three and more leave some SMs of a GPC unused (at M = 5120, 120 CTAs in threes
+// take 60 us where 160 in fours, 132 of which fit at once, take 88), those of seven and eight more of them (2048 x 4096 IQ2_XS, 77
+// tokens: 128 CTAs in eights 21.8 us, 96 in sixes 14.4).  The constants are fitted to every cut of as many to twice as many token tiles
+// and up to eight CTAs over 1547 calls (thirteen formats, twelve shapes, 16 to 2500 tokens): the cut picked takes 0.3 % more than the
+// fastest on average and over 5 % more in 42 of them; with one set of constants for all formats, measured on Q4_K, it was 3.7 % and 324
+// (5120 x 17408 on 1024 tokens, IQ4_XS 195 us in pairs, 184 in threes).  M = 5120, K = 17408, IQ4_XS, 512 tokens: 277 us unsplit, 101 us in threes.
 bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* best) {
     const long long row_tiles = (M + PF_ROWS - 1) / PF_ROWS;
     const int nsb = K / 256;
@@ -647,8 +666,10 @@ bool prefill_cut(const q38b_ctx* ctx, int fmt, int K, int M, int B, PrefillCut* 
             const long long ctas = (c.mode == PF_PAIR ? (row_tiles + 1) / 2 * 2 : row_tiles) * c.tok_tiles * c.splits;
             const int slots = c.splits <= 2 ? ctx->sm_count : (c.splits <= 6 ? ctx->sm_count * 9 / 10 : ctx->sm_count * 3 / 4) / c.splits * c.splits;
             const double rounds = (double)((ctas + slots - 1) / slots);
-            const double slab = ta ? 480.0 + (double)tile * tile / 140.0 : c.mode == PF_PAIR ? 800.0 + 0.8 * tile : 800.0 + 1.25 * tile;
-            const double cost = rounds * (4.0 * ((nsb + c.splits - 1) / c.splits) * slab + 9000.0 + 8.0 * tile + (c.splits > 1 ? 6000.0 + 16.0 * tile : 0.0));
+            const double expand = c.mode == PF_TMEM ? expand_clocks(fmt) : c.mode == PF_PAIR ? 710.0 + 0.6 * expand_clocks(fmt) : 1000.0 + 0.47 * expand_clocks(fmt);
+            const double multiply = (c.mode == PF_PAIR ? 1.65 : ta ? 2.5 : 2.3) * tile, e2 = expand * expand, m2 = multiply * multiply;
+            const double slab = std::sqrt(std::sqrt(e2 * e2 + m2 * m2));
+            const double cost = rounds * (4.0 * ((nsb + c.splits - 1) / c.splits) * slab + 10400.0 + 30.0 * tile + (c.splits > 1 ? 500.0 + 1.4 * tile : 0.0));
             if (!found || cost < best_cost) { found = true; best_cost = cost; *best = c; }
         }
     }
@@ -748,6 +769,19 @@ int gemm_prefill_any(q38b_ctx* ctx, uint32_t type, const void* W, size_t row_byt
 }
 
 }  // namespace
+
+// Test hook (not in the public header): the cut of a GEMM on a 148-SM device with 227 KB of shared memory a CTA, no device needed: token
+// tiles, tokens a tile, CTAs that share K, where operand A goes (0 shared memory, 1 tensor memory, 2 a pair's shared memory).
+extern "C" int q38b_debug_prefill_plan(uint32_t type, int K, int M, int B, int* out) {
+    q38b_ctx ctx;
+    ctx.sm_count = 148;
+    ctx.smem_optin = 232448;
+    PrefillCut c;
+    if (!prefill_cut(&ctx, (int)type, K, M, B, &c)) return Q38B_ERR_NOMEM;
+    const int v[4] = {c.tok_tiles, c.n_acc * c.n_tile, c.splits, c.mode};
+    memcpy(out, v, sizeof(v));
+    return Q38B_OK;
+}
 
 // Test hook (not in the public header): the prefill GEMM cuts the tokens into `tiles` tiles and shares a tile's K among
 // `splits` CTAs (0: its own rule), so that tests reach every cut with small matrices.
