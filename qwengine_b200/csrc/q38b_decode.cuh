@@ -228,7 +228,7 @@ Q38B_HD uint32_t negate_bytes(uint32_t g, uint32_t m) { return (g ^ m) + (m & 0x
 // Activation operand of one lane for one super-block (the CPU unit test's interface to the fragment builders).
 struct ActLane {
     const uint8_t* q;   // int8 activations of column g for this super-block (256 bytes, staged order); column 0's where !valid
-    bool valid;         // column g < nb
+    bool valid;         // column g < nb (for the test's own use: the fragments multiply column 0 there)
     float dx0, dx1;     // Q8_K block scales of columns 2t and 2t+1 (0 beyond nb)
 };
 
@@ -247,7 +247,7 @@ struct Codebook {
 //   cb       32-bit codebook: entry e at cb + (e << cb_shift); grid8: eight-byte grid entries likewise
 //   sgn      byte masks of the 128 seven-bit sign codes, SIGN_COPIES times: code c at sgn + 8 c SIGN_COPIES (TABLES; else they
 //            are computed, with seven operations where the look-up takes two)
-//   bsum     this lane's word of the staged sums of activations (see MINS_STAGED)
+//   bsum     this lane's word of the staged sums of activations (TABLES; see the minima below)
 constexpr int SIGN_COPIES = 8, SIGN_STRIDE_LOG2 = 6;   // (16 would meet no bank but cost the ring 8 KB)
 struct FragEnv {
     SP q, q_half[2];
@@ -255,7 +255,7 @@ struct FragEnv {
     int cb_shift;
     int t;
 };
-// The minima of the K-quants: sum over the sub-blocks of m * (sum of the sub-block's activations).  MINS_STAGED: the sums are
+// The minima of the K-quants: sum over the sub-blocks of m * (sum of the sub-block's activations).  TABLES: the sums are
 // staged as two digits, 64 hi + lo, and one k16 mma per digit and super-block forms the product (per column 8 lo | 8 hi bytes
 // a super-block, Q2_K 16 lo | 16 hi); else m is broadcast to every slot of a second mma per sub-block (per-32 activations,
 // whose scales differ by sub-block; the unit test).  Eight IMMA a super-block less: Q4_K's decoder 334 -> 275 clocks
@@ -343,7 +343,6 @@ template <int FMT> struct UnitRun {
     static constexpr int ACT_STEP = 8;           // bytes of a sub-block between the lanes t of a row
     static constexpr bool SCALE32 = false, HAS_MIN = false;
     static constexpr float FACTOR = 1.0f;
-    static constexpr int BSUM_BYTES = 0;
     static Q38B_HD float d32(SP, int) { return 0.0f; }
     static Q38B_HD void run(const uint8_t* pA, const uint8_t* pB, int h, const ActLane& act, const Codebook& cb, float (&acc)[4]) {
         unit_run<FMT>(pA, pB, h, act, cb, acc);
@@ -506,8 +505,8 @@ template <> struct Unit<T_IQ4_XS> : UnitRun<T_IQ4_XS> {
 // ------------------------------------------------------------------------------------------------
 // Q4_K (144 bytes: fp16 d, dmin | scales[12] | qs[128]) and Q5_K (176 bytes: ... | qh[32] | qs[128]).
 // w = d * sc * q - dmin * m (src/quant/quant_ref.cpp:57-76; src/cpu/cpu_kernels.cpp:386-433; Q5_K has no
-// reference code: q gets a fifth bit from qh).  The min term sum_s m_s * (sum of the sub-block's activations) is a
-// second mma whose A operand is m_s in every slot, so no activation block sums are needed.
+// reference code: q gets a fifth bit from qh).  The min term sum_s m_s * (sum of the sub-block's activations): mins()
+// from the sums that are staged beside Q8_K columns; with per-32 columns a second mma whose A operand is m_s in every slot.
 // ------------------------------------------------------------------------------------------------
 template <int FMT> struct UnitQ45K : UnitRun<FMT> {
     static constexpr int NBITS = FMT == T_Q5_K ? 5 : 4;
@@ -515,7 +514,6 @@ template <int FMT> struct UnitQ45K : UnitRun<FMT> {
     static constexpr int CODEBOOK_ENTRIES = 0;
     static constexpr int QS_OFF = NBITS == 5 ? 48 : 16;
     static constexpr bool HAS_MIN = true;
-    static constexpr int BSUM_BYTES = 16;        // staged sums per column and super-block (MINS_STAGED)
 
     struct Row { uint32_t dd, sc[2], mn[2], qh[NBITS == 5 ? 2 : 1]; };
 
@@ -876,7 +874,6 @@ template <> struct Unit<T_Q2_K> : UnitRun<T_Q2_K> {
     static constexpr int BLOCK_BYTES = 84, CODEBOOK_ENTRIES = 0, CODE16_ENTRIES = 0;
     static constexpr bool HAS_MIN = true;
     static constexpr int ACT_STEP = 4;
-    static constexpr int BSUM_BYTES = 32;
     struct Row { uint32_t sc[4], dd; };
     static Q38B_HD void mins(const Row& A, const Row& B, const FragEnv& e, int (&cm)[4]) {
         const uint32_t wA = e.t == 0 ? A.sc[0] : e.t == 1 ? A.sc[1] : e.t == 2 ? A.sc[2] : A.sc[3];

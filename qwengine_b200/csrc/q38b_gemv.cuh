@@ -13,7 +13,7 @@
 //     several groups of kw warps take tiles in turn;
 //   * activations (int8 values and scales of all columns) and the tables are staged in shared memory once per CTA, the columns
 //     32 (16) bytes off a multiple of 128, so that the four or eight columns of one load meet no bank;
-//   * rows longer than 8192 are cut into K-parts of 8 to 16 super-blocks (a rule of K and the format alone).  The work
+//   * rows longer than 8192 are cut into K-parts of at most 20 super-blocks, Q5_K / Q6_K 17, Q8_0 10 (a rule of K and the format alone).  The work
 //     items (part, tile), part-major, are dealt to the CTAs as equal contiguous ranges: a CTA then needs the
 //     activations of at most two neighbouring parts, which leaves the shared memory to the weight stages, and 320
 //     tiles of 68 super-blocks keep 148 SMs evenly busy instead of 24 of them working a second round.  A part's sums
@@ -56,7 +56,7 @@ constexpr uint32_t PART_EMPTY = 0xFFFFFFFFu;   // a slot of the K-part scratch a
 // Columns of staged activations lie this many bytes off a multiple of 128: the four (8-byte loads of a half warp) or eight
 // (4-byte loads of the k16 formats) columns that meet in one load then fall on different banks.
 __host__ __device__ constexpr int act_skew(int fmt) { return fmt == T_Q6_K || fmt == T_Q2_K ? 16 : 32; }
-// bytes of staged activation sums per column and super-block (MINS_STAGED of q38b_decode.cuh)
+// bytes of staged activation sums per column and super-block (mins() of q38b_decode.cuh)
 __host__ __device__ constexpr int bsum_bytes(int fmt, bool a32) { return a32 ? 0 : fmt == T_Q4_K || fmt == T_Q5_K ? 16 : fmt == T_Q2_K ? 32 : 0; }
 __host__ __device__ constexpr bool sign_table(int fmt) { return fmt == T_IQ3_XXS || fmt == T_IQ2_XXS || fmt == T_IQ2_XS; }
 // a run of zeros beside the activations (q_half of FragEnv)
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(32 * (2 + GEMV_MAX_WARPS), 1) gemv_kernel(cons
     };
     Block at = {0, 0};
     step(at, cw);
-    // Sums of a block's activations, as digits (MINS_STAGED).  Floats: a lane has eight values in a row (w0, w1); blocks: words
+    // Sums of a block's activations, as digits (mins() of q38b_decode.cuh).  Floats: a lane has eight values in a row (w0, w1); blocks: words
     // l % 4 and l % 4 + 4 of 32.  Either way four lanes have a sub-block; sixteen values are two of them or one word of each.
     constexpr int BS = bsum_bytes(FMT, A32);
     const bool floats = !A32 && a.x_f32;

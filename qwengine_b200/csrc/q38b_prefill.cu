@@ -5,18 +5,20 @@
 // Replaces dequant_rows_f16 + gemm_f16 (cuBLAS) of the reference (src/cuda/prefill.cu:30-85, 802-851) by one kernel:
 // the weights never exist dequantized in global memory.  One CTA owns a 128-row weight tile and up to 512 tokens:
 //   * warps 0-15 fetch the rows' raw blocks one super-block ahead (whole 16-byte units into registers, then shared memory), a
-//     lane expands one 32-weight sub-block with word operations (q38b_expand.cuh) into operand A: from 257 tokens on K-major
-//     with the 128-byte swizzle in shared memory (a warp owns eight rows), up to 256 in tensor memory (a lane is a row);
+//     lane expands one 32-weight sub-block with word operations (q38b_expand.cuh) into operand A: for token tiles over 256
+//     K-major with the 128-byte swizzle in shared memory (a warp owns eight rows), for tiles of at most 256 in tensor memory
+//     (a lane is a row);
 //   * one thread streams the matching activation tiles (operand B, [tokens x 64] per K-slab) with tiled TMA loads
 //     (hardware swizzle, zero fill past the last token; no multicast);
-//   * one thread issues tcgen05.mma (kind::f16, M = 128, N = 16..256, K = 16; from 257 tokens on two CTAs as a pair, M = 256) into one or two fp32
+//   * one thread issues tcgen05.mma (kind::f16, M = 128, N = 16..256, K = 16; tiles over 256 tokens whose K is not shared: two
+//     CTAs as a pair, M = 256) into one or two fp32
 //     accumulators in tensor memory and commits each stage to its "empty" mbarrier;
 //   * all 16 decode warps read the accumulators back (tcgen05.ld 32x32b) and store Y, 32 consecutive rows per warp and token.
 // Where row tiles and token tiles alone leave SMs idle, the CTAs of a cluster share a tile's K: each multiplies a range
 // of super-blocks and the partial sums meet through distributed shared memory, added in rank order.
 // Measured on B200, 17408 x 5120 IQ3_XXS / 5120 x 17408 IQ4_XS with 1024 tokens: 211 / 286 us -> 161 / 194 us; in pairs 143
-// for the former; 77 tokens of a whole Q4_K / Q6_K layer 698 -> 199 us, 154 us with operand A in tensor memory.  Up to 256 tokens the expanders set the pace,
-// from 500 the tensor core and the shared-memory traffic do.
+// for the former; 77 tokens of a whole Q4_K / Q6_K layer 698 -> 199 us, 154 us with operand A in tensor memory.  In tiles of at most 256 tokens
+// the expanders set the pace, in tiles of 500 the tensor core and the shared-memory traffic do.
 // All mbarrier waits are bounded; tensor memory is released before the kernel returns, also after a timeout.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -55,7 +57,7 @@ __host__ __device__ constexpr int pf_raw_bytes(int fmt) { return fmt == T_Q8_0 ?
 __host__ __device__ constexpr int pf_pieces(int fmt) { return (pf_raw_bytes(fmt) + 14 + 15) / 16; }
 __host__ __device__ constexpr int pf_pitch(int fmt) { return 16 * (pf_pieces(fmt) | 1); }
 __host__ __device__ constexpr int pf_raw_smem(int fmt) { return PF_ROWS * pf_pitch(fmt) + 16; }   // + what the last row's word loads read past its end
-// Operand A in tensor memory (one accumulator, up to 256 tokens): a decode warp's lanes are 32 rows, an odd number of the
+// Operand A in tensor memory (one accumulator, a tile of up to 256 tokens): a decode warp's lanes are 32 rows, an odd number of the
 // format's loads (16, 8 or 4 bytes) apart; two buffers, as four warps share a quarter of the rows.
 __host__ __device__ constexpr int pf_pitch_ta(int fmt, bool aligned) {
     return aligned && (fmt == T_Q4_K || fmt == T_Q5_K) ? pf_pitch(fmt) : 16 * pf_pieces(fmt) + (aligned && fmt == T_IQ4_XS ? 8 : 4);
@@ -219,14 +221,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 
 // F16: operands are fp16 (weights dequantized to fp16, activations fp16) instead of bf16.
 // ALIGNED: every row starts at a multiple of expand_alignment(FMT).
-// TA: operand A goes to tensor memory instead of shared memory (one accumulator, up to 256 tokens).  Up to there the kernel is
+// TA: operand A goes to tensor memory instead of shared memory (one accumulator: tiles of up to 256 tokens, also of longer
+// calls that are cut so).  Up to there the kernel is
 // bound by shared-memory bandwidth: per 128 K the tensor core reads 32 KB of weights and 20 KB of activations (80 tokens), the
 // decode warps write the weights and move the raw blocks twice, 140 KB of traffic or 1100 clocks of some 1700 measured; from
 // tensor memory the weights cost none of it.  With one wait and one commit per 128 K and the unchecked fetch, 16384 x 5120 Q4_K,
 // 77 tokens 39.6 -> 27.9 us, 17408 x 5120 IQ3_XXS 51.4 -> 42.0, 5120 x 17408 Q6_K 55.1 -> 45.4, a Q4_K / Q6_K layer 199 -> 154 us.
 // PAIR: two CTAs (a cluster of two, row tiles 2i and 2i + 1) multiply as one, M = 256 (cta_group::2): each expands its 128 rows and
-// loads half of every activation tile, CTA 0 issues, each CTA's tensor memory holds its own rows.  From 257 tokens on a slab of
-// 64 K moves 176 KB through an SM's shared memory otherwise (32 KB tiles written and read for each accumulator), 1375 clocks of
+// loads half of every activation tile, CTA 0 issues, each CTA's tensor memory holds its own rows.  For tiles over 256 tokens whose K is not
+// shared, where there are two row tiles; alone a slab of 64 K moves 176 KB through an SM's shared memory (32 KB tiles written and read for each accumulator), 1375 clocks of
 // which the tensor core needs 1024; in pairs 112 KB, and half the activation bytes from L2 (16384 x 5120 Q4_K,
 // 1024 tokens 146 -> 132 us, 17408 x 5120 IQ3_XXS 161 -> 143; 512 tokens of the former 72 -> 66).
 template <int FMT, bool F16, bool ALIGNED, int MODE>
