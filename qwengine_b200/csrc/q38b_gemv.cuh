@@ -28,7 +28,7 @@
 // per tile, fragments of half a super-block; one-column arithmetic in launches of four columns for IQ2 / IQ1 / Q2_K and per-32
 // columns): seven columns, 2 x 17408 x 5120 IQ3_XXS 41.8 -> 37.2 us, 65536 x 5120 Q6_K 78.5 -> 70.6; two columns, 2 x 17408 x
 // 5120 Q4_K 27.9 -> 22.0; four columns, 2 x 17408 x 5120 IQ2_XS 46.9 -> 37.0, IQ1_S 45.1 -> 30.3, 5120 x 17408 Q2_K 34.1 -> 26.4;
-// the 7-column pass 7.04 -> 6.38 ms, the four-column pass on 2- and 3-bit blocks 697 -> 588 us.
+// the 7-column pass 7.04 -> 6.38 ms (6.11 with the divisions as they are rated now), the four-column pass on 2- and 3-bit blocks 697 -> 588 us.
 // Every column is computed by the same instructions whatever nb is, so column c of an nb-column call is
 // bit-identical to a 1-column call on that column (the reference promises the same: src/cuda/gemv.cuh:31-34).
 //

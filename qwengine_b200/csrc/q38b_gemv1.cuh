@@ -11,7 +11,7 @@
 //
 // Q8_K columns of the lane-per-granule mapping: the eight (four) lanes of a super-block add exact integers and one lane per
 // row scales their sum, where every lane used to read the block's factors, convert and multiply: per granule and row some six
-// operations less (27B-shaped pass 3847 -> 3810 us, pass of a small model in 2-bit blocks 466 -> 458).  The sums are formed in
+// operations less (27B-shaped pass 3883 -> 3840 us, pass of a small model in 2-bit blocks 466 -> 458).  The sums are formed in
 // the order of the several-column kernel (q38b_gemv.cuh), so that a column's bits do not depend on how many share a launch.
 //
 // With NC = 2 or 4 the same kernel takes two to four columns: a granule is decoded once (q38b_decode1n.cuh) and multiplied with each
