@@ -737,9 +737,8 @@ static int granule_launch(q38b_ctx* ctx, Plan1& p, const ColsCall& c, cudaStream
     g.xq = (const uint8_t*)c.xq;
     g.xq_ld = c.xq_ld;
     g.x_f32 = c.x_f32;
-    g.x_f32_ld = c.x_f32_ld;
+    g.xf_ld = c.x_f32 ? c.x_f32_ld : c.xd32_ld;
     g.xd32 = c.xd32;
-    g.xd32_ld = c.xd32_ld;
     g.n_peers = c.n_peers;
     g.static_weights = ctx->static_weights;
     g.status = ctx->d_status;

@@ -52,10 +52,11 @@ struct Gemv1Args {
     int static_weights;     // 1: W was written long before this launch, the producer need not wait for earlier kernels
     int* status;
     const uint32_t* codebook;
-    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes), x_f32 and xd32 (floats), and of each
-    // matrix's output (floats; the peers' as well)
+    // NC > 1: columns in use (1 .. NC), the distances between columns of xq (bytes) and of x_f32 or xd32 (floats), and of each
+    // matrix's output (floats; the peers' as well).  One field for x_f32 and xd32, never both given: every launch pays for the arguments' bytes
+    // (decode pass of a small model, 63 launches, 458.9 us with eight bytes more, 457.2)
     int nc;
-    long long xq_ld, x_f32_ld, xd32_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
+    long long xq_ld, xf_ld, y_ld, y_ld_more[G1_MAX_MATS - 1];
     int K, M, accumulate;
     int nsb;                // super-blocks per row
     int n_slices;           // ceil(nsb / 4)
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
                     lo4[j] = make_float4(0.f, 0.f, 0.f, 0.f);
                     hi4[j] = lo4[j];
                     if (c < nc && sb < a.nsb) {
-                        const float* src = a.x_f32 + (size_t)c * a.x_f32_ld + (size_t)sb * 256 + 8 * lane;
+                        const float* src = a.x_f32 + (size_t)c * a.xf_ld + (size_t)sb * 256 + 8 * lane;
                         lo4[j] = *(const float4*)src;
                         hi4[j] = *(const float4*)(src + 4);
                     }
@@ -316,7 +317,7 @@ __global__ void __launch_bounds__(32 * (1 + NWARPS), OCC) gemv1_kernel(const Gem
             const int n_d = A32 ? actd_ld : nsb4, n_w = a.n_slices * 128;
             for (int i = ctid; i < nc * n_d; i += NWARPS * 32) {
                 const int c = i / n_d, k = i - c * n_d;
-                if (A32) actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xd32_ld + k] : 0.0f;
+                if (A32) actd[c * actd_ld + k] = k < a.nsb * 8 ? a.xd32[(size_t)c * a.xf_ld + k] : 0.0f;
                 else actd[c * actd_ld + k * 8] = k < a.nsb ? *(const float*)(a.xq + (size_t)c * a.xq_ld + (size_t)k * Q8K_BYTES) : 0.0f;
             }
 #pragma unroll 4
